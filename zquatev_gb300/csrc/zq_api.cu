@@ -20,6 +20,7 @@
 #include "zq_common.cuh"
 #include "zq_kernels.h"
 #include "zq_context.h"
+#include "zq_resident.h"
 #include "../../include/zquatev_gb300.h"
 
 #include <algorithm>
@@ -287,6 +288,7 @@ int solve_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, bool
 
   tm.mark("start", c->st);
   TridiagView<double> v = tridiag_bind<double>(tri_ws, dD, n, ldd, NBMAX, d, e, tau);
+  v.ctas = resident_ctas(n, c->coop);
   prof_begin(PC_TRIDIAG, c->st);
   if (int rc = tridiagonalize<double>(v, nb, c->st)) return rc;
   prof_end(PC_TRIDIAG, c->st);

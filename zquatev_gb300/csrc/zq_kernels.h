@@ -36,6 +36,8 @@ struct TridiagView {
   double* e;       // quaternion subdiagonal (4 doubles each, n)
   double* tau;     // 1 if reflector j exists else 0 (n)
   int* tc_err;     // FP32: tensor-core products allowed (their timeout flag); null: CUDA cores only
+  void* rws;       // exchange area of the resident reduction (zq_resident.cu)
+  int ctas;        // CTAs it may use (0: the per-column kernels only)
   int coop;        // 1: the FP32 panels may run as one cooperative launch each (no other solve runs beside it)
 };
 

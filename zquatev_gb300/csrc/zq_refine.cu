@@ -27,6 +27,7 @@
 //   tol_converged; the caller gets the number of iterations and that value.
 #include "zq_common.cuh"
 #include "zq_kernels.h"
+#include "zq_resident.h"
 
 #include <algorithm>
 #include <cstdio>
@@ -637,6 +638,7 @@ int refined_solve(RefineArgs& ra) {
   TridiagView<float> vf = tridiag_bind<float>(tri_ws, Mf, n, n2, NBMAX, d, e, tau);
   vf.tc_err = tc_err;  // tensor-core products where fp32_products_on_tensor_cores allows them
   vf.coop = ra.coop;
+  vf.ctas = resident_ctas(n, ra.coop != 0);
   if (int rc = tridiagonalize<float>(vf, ra.nb, st)) return rc;
   if (int rc = phase_reduce(e, n, offd, phi, st)) return rc;
   mark(1, st);

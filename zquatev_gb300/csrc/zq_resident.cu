@@ -1,0 +1,818 @@
+// Quaternion tridiagonalisation with the matrix resident in shared memory.
+//
+// Same reduction and outputs as zq_tridiag.cu (one quaternion reflector per
+// column; reference blocked.cc:45-546, unblocked.cc:44-131): d, the quaternion
+// subdiagonal e, tau, and w_j stored in column j below the diagonal. Here the
+// lower triangles of A and B are loaded once, as T x T tiles dealt round robin
+// over the shared memories of a group of G co-resident CTAs, and stay there:
+// per column every tile takes the previous column's rank-2 update and the
+// mat-vec with the current reflector in one sweep, and only vectors travel
+// between the CTAs (through L2), with three group barriers per column:
+//
+//   sweep j    tiles -= w_{j-1} y_{j-1}^H + y_{j-1} w_{j-1}^H (structured), then the
+//              tile's products with w_j; column j + 1 is published
+//      -- barrier --
+//   rows       g = H w_j: each CTA sums the tile partials of its share of the
+//              rows, and its part of c = w_j^H g
+//      -- barrier --
+//   column     y_j = g - (c/2) w_j and column j + 1 brought up to date on the
+//              CTA's rows, with its norm partials
+//      -- barrier --
+//              every CTA forms reflector j + 1 from the norm partials
+//
+// Why: the per-column kernels of zq_tridiag.cu cost ~22 us (FP32) to ~75 us
+// (FP64) per column in launches, memory round trips and FP64 work on few SMs,
+// at orders where the arithmetic takes a few; and GB300's FP64 pipe (2 FMA per
+// clock per SM) makes the split of the FP64 work over all SMs matter more than
+// operand reuse, hence small tiles. Reduction before and after: FP64 n = 384
+// 29 -> 6.3 ms, n = 750 60 -> 19.6 ms (7.2 ms of FP64 pipe time); FP32 n = 1023
+// 23.5 -> 9.8 ms. What remains per column (FP32, n = 600, cycles): reflector
+// scalars 3100, vectors 1100, sweep 2100, rows 3100, column 3400, barriers
+// 3 x 2500: chains of L2 round trips and dependent FP64 instructions.
+//
+// Tile work: one warp per tile, lane (tr, tc) = (lane & 7, lane >> 3) owns
+// rows tr + 8 i and columns tc + 4 q of the tile, stored so that a lane only
+// touches its own 16-byte-aligned slots (no bank conflicts, no barriers around
+// the tiles). The lanes' row and column products meet by a halving exchange
+// (each step every lane keeps half of its values), so the sums cost about one
+// add per value. A diagonal tile holds both triangles and forms row products
+// only.
+//
+// Tiles are dealt in the order of their columns from the last one back, so
+// that the live tiles of every stage are spread evenly.
+//
+// The group is one cooperative launch; every wait is bounded (the abort flag
+// and the caller's error flag are raised, NaN is left in d, and all CTAs return).
+#include "zq_common.cuh"
+#include "zq_kernels.h"
+#include "zq_resident.h"
+
+#include <atomic>
+
+namespace zq {
+namespace {
+
+constexpr int RT_THREADS = 256;
+constexpr int RT_WARPS = RT_THREADS / 32;
+constexpr int RT_SMEM_MAX = 227 * 1024 - 1024;  // dynamic shared memory per CTA (static part below 1 KB)
+
+template <typename R> __device__ __forceinline__ Q4<R> q_zero() { return Q4<R>{R(0), R(0), R(0), R(0)}; }
+__device__ __forceinline__ Q4<float> q_ldcg(const Q4<float>* p) {
+  const float4 v = __ldcg(reinterpret_cast<const float4*>(p));
+  return Q4<float>{v.x, v.y, v.z, v.w};
+}
+__device__ __forceinline__ Q4<double> q_ldcg(const Q4<double>* p) {
+  const double2 u = __ldcg(reinterpret_cast<const double2*>(p)), v = __ldcg(reinterpret_cast<const double2*>(p) + 1);
+  return Q4<double>{u.x, u.y, v.x, v.y};
+}
+__device__ __forceinline__ void q_store(Q4<float>* p, const Q4<float>& q) {
+  *reinterpret_cast<float4*>(p) = make_float4(q.ax, q.ay, q.bx, q.by);
+}
+__device__ __forceinline__ void q_store(Q4<double>* p, const Q4<double>& q) {
+  reinterpret_cast<double2*>(p)[0] = make_double2(q.ax, q.ay);
+  reinterpret_cast<double2*>(p)[1] = make_double2(q.bx, q.by);
+}
+// a lane's tile slot e: FP32 one 16-byte slot, FP64 two 16-byte planes
+template <int EL> __device__ __forceinline__ Q4<float> t_load(const float* t, int e, int lane) {
+  const float4 v = reinterpret_cast<const float4*>(t)[e * 32 + lane];
+  return Q4<float>{v.x, v.y, v.z, v.w};
+}
+template <int EL> __device__ __forceinline__ void t_store(float* t, int e, int lane, const Q4<float>& q) {
+  reinterpret_cast<float4*>(t)[e * 32 + lane] = make_float4(q.ax, q.ay, q.bx, q.by);
+}
+template <int EL> __device__ __forceinline__ Q4<double> t_load(const double* t, int e, int lane) {
+  const double2 u = reinterpret_cast<const double2*>(t)[e * 32 + lane];
+  const double2 v = reinterpret_cast<const double2*>(t)[(EL + e) * 32 + lane];
+  return Q4<double>{u.x, u.y, v.x, v.y};
+}
+template <int EL> __device__ __forceinline__ void t_store(double* t, int e, int lane, const Q4<double>& q) {
+  reinterpret_cast<double2*>(t)[e * 32 + lane] = make_double2(q.ax, q.ay);
+  reinterpret_cast<double2*>(t)[(EL + e) * 32 + lane] = make_double2(q.bx, q.by);
+}
+
+// the structured rank-2 term at (r, c): row vectors (w, y)_r, column vectors (w, y)_c
+//   A: wa_r conj(ya_c) + conj(wb_r) yb_c + ya_r conj(wa_c) + conj(yb_r) wb_c
+//   B: wb_r conj(ya_c) - conj(wa_r) yb_c + yb_r conj(wa_c) - conj(ya_r) wb_c
+template <typename R>
+__device__ __forceinline__ Q4<R> rank2(const Q4<R>& wr, const Q4<R>& yr, const Q4<R>& wc, const Q4<R>& yc) {
+  Q4<R> t;
+  t.ax = wr.ax * yc.ax; t.ax = fma(wr.ay, yc.ay, t.ax);
+  t.ay = wr.ay * yc.ax; t.ay = fma(-wr.ax, yc.ay, t.ay);
+  t.bx = wr.bx * yc.ax; t.bx = fma(wr.by, yc.ay, t.bx);
+  t.by = wr.by * yc.ax; t.by = fma(-wr.bx, yc.ay, t.by);
+  t.ax = fma(wr.bx, yc.bx, t.ax); t.ax = fma(wr.by, yc.by, t.ax);
+  t.ay = fma(wr.bx, yc.by, t.ay); t.ay = fma(-wr.by, yc.bx, t.ay);
+  t.bx = fma(-wr.ax, yc.bx, t.bx); t.bx = fma(-wr.ay, yc.by, t.bx);
+  t.by = fma(-wr.ax, yc.by, t.by); t.by = fma(wr.ay, yc.bx, t.by);
+  t.ax = fma(yr.ax, wc.ax, t.ax); t.ax = fma(yr.ay, wc.ay, t.ax);
+  t.ay = fma(yr.ay, wc.ax, t.ay); t.ay = fma(-yr.ax, wc.ay, t.ay);
+  t.bx = fma(yr.bx, wc.ax, t.bx); t.bx = fma(yr.by, wc.ay, t.bx);
+  t.by = fma(yr.by, wc.ax, t.by); t.by = fma(-yr.bx, wc.ay, t.by);
+  t.ax = fma(yr.bx, wc.bx, t.ax); t.ax = fma(yr.by, wc.by, t.ax);
+  t.ay = fma(yr.bx, wc.by, t.ay); t.ay = fma(-yr.by, wc.bx, t.ay);
+  t.bx = fma(-yr.ax, wc.bx, t.bx); t.bx = fma(-yr.ay, wc.by, t.bx);
+  t.by = fma(-yr.ax, wc.by, t.by); t.by = fma(yr.ay, wc.bx, t.by);
+  return t;
+}
+// g_r += M(r, c) w_c:  ga += a wa - conj(b) wb,  gb += b wa + conj(a) wb
+template <typename R>
+__device__ __forceinline__ void row_prod(R* g, const Q4<R>& m, const Q4<R>& w) {
+  g[0] = fma(m.ax, w.ax, g[0]); g[0] = fma(-m.ay, w.ay, g[0]); g[0] = fma(-m.bx, w.bx, g[0]); g[0] = fma(-m.by, w.by, g[0]);
+  g[1] = fma(m.ax, w.ay, g[1]); g[1] = fma(m.ay, w.ax, g[1]); g[1] = fma(-m.bx, w.by, g[1]); g[1] = fma(m.by, w.bx, g[1]);
+  g[2] = fma(m.bx, w.ax, g[2]); g[2] = fma(-m.by, w.ay, g[2]); g[2] = fma(m.ax, w.bx, g[2]); g[2] = fma(m.ay, w.by, g[2]);
+  g[3] = fma(m.bx, w.ay, g[3]); g[3] = fma(m.by, w.ax, g[3]); g[3] = fma(m.ax, w.by, g[3]); g[3] = fma(-m.ay, w.bx, g[3]);
+}
+// g_c += M(c, r) w_r from the stored (r, c):  ga += conj(a) wa + conj(b) wb,  gb += -b wa + a wb
+template <typename R>
+__device__ __forceinline__ void col_prod(R* g, const Q4<R>& m, const Q4<R>& w) {
+  g[0] = fma(m.ax, w.ax, g[0]); g[0] = fma(m.ay, w.ay, g[0]); g[0] = fma(m.bx, w.bx, g[0]); g[0] = fma(m.by, w.by, g[0]);
+  g[1] = fma(m.ax, w.ay, g[1]); g[1] = fma(-m.ay, w.ax, g[1]); g[1] = fma(m.bx, w.by, g[1]); g[1] = fma(-m.by, w.bx, g[1]);
+  g[2] = fma(-m.bx, w.ax, g[2]); g[2] = fma(m.by, w.ay, g[2]); g[2] = fma(m.ax, w.bx, g[2]); g[2] = fma(-m.ay, w.by, g[2]);
+  g[3] = fma(-m.bx, w.ay, g[3]); g[3] = fma(-m.by, w.ax, g[3]); g[3] = fma(m.ax, w.by, g[3]); g[3] = fma(m.ay, w.bx, g[3]);
+}
+// v[0..N) summed over the lanes that differ in the bits of MASK, MASK/2, ..., LOW:
+// each step halves the values a lane keeps; returns in v[0..N / lanes)
+template <int N, int MASK, int LOW, typename R>
+__device__ __forceinline__ void scatter_sum(R* v, int lane) {
+  if constexpr (MASK >= LOW) {
+    const bool up = lane & MASK;
+#pragma unroll
+    for (int k = 0; k < N / 2; ++k) {
+      const R keep = up ? v[N / 2 + k] : v[k], send = up ? v[k] : v[N / 2 + k];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, MASK);
+    }
+    scatter_sum<N / 2, MASK / 2, LOW, R>(v, lane);
+  }
+}
+
+// tile t in dealing order: column blocks from the last one back
+__device__ __forceinline__ void rt_tile(int t, int nt, int& I, int& J) {
+  int a, b;
+  tri_tile(t, a, b);
+  J = nt - 1 - a;
+  I = J + b;
+}
+
+// Barrier of one group (bounded). ctr only grows; `target` is this CTA's count.
+__device__ __forceinline__ bool group_barrier(unsigned* ctr, unsigned& target, int G, unsigned* abt, int* err,
+                                              long long limit, int* s_ok) {
+  __syncthreads();
+  if (G > 1) {
+    if (threadIdx.x == 0) {
+      target += (unsigned)G;
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
+      unsigned v;
+      int ok = 1, spins = 0;
+      const long long t0 = clock64();
+      for (;;) {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
+        if ((int)(v - target) >= 0) break;
+        if ((++spins & 63) == 0) {
+          if (*reinterpret_cast<volatile unsigned*>(abt)) { ok = 0; break; }
+          if (clock64() - t0 > limit) {
+            atomicExch(abt, 1u);
+            if (err) atomicExch(err, 1);
+            ok = 0;
+            break;
+          }
+        }
+      }
+      *s_ok = ok;
+    }
+    __syncthreads();
+    return *s_ok != 0;
+  }
+  return true;
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+  __syncthreads();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ double pow2_biased(int be) {
+  return be < 1 ? 0.0 : __longlong_as_double((long long)be << 52);
+}
+
+// Sum of `count` doubles (written by other CTAs) by one warp; every lane gets it.
+__device__ __forceinline__ double warp_gather(const double* p, int count, int lane) {
+  double s = 0.0;
+  for (int i = lane; i < count; i += 32) s += __ldcg(p + i);
+  return warp_sum(s);
+}
+__device__ __forceinline__ unsigned mag_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ unsigned long long mag_bits(double v) { return abs_bits(v); }
+__device__ __forceinline__ double mag_value(unsigned b) { return (double)__uint_as_float(b); }
+__device__ __forceinline__ double mag_value(unsigned long long b) { return bits_to_double(b); }
+
+// CTAs that own rows in the vector phases: enough to spread the sums, few
+// enough that one warp gathers their partials in one or two steps
+template <typename R> __host__ __device__ __forceinline__ int row_ctas(int G) {
+  const int most = sizeof(R) == 8 ? 96 : 32;
+  return G < most ? G : most;
+}
+
+// One matrix reduced by the group (CL: the group is one cluster). Returns
+// false when a wait ran out.
+//
+// An FP64 instruction holds its SM quadrant's pipe for 64 cycles whatever the
+// number of lanes, so the vector phases keep one real component per lane (the
+// four lanes of a row exchange theirs by shuffles) and the reflector's scalars
+// come from two reciprocal square roots: with ss = |x|^2 and q2 = |x_1|^2,
+// g = sqrt(ss q2) = |x||x_1|, s = |x|/|x_1| = ss / g and f = 1 / sqrt(ss + g).
+// The matrix is scaled by a power of two once (largest entry in [1, 2)), so no
+// sum of squares needs a scale of its own.
+template <typename R, int T, int LPR, bool CL>
+__device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int rank, int G, unsigned char* smem,
+                              unsigned& target, int* err, long long limit) {
+  constexpr int RR = T / 8, CC = T / 4, EL = RR * CC;  // rows, columns and entries per lane
+  constexpr int NRV = RR * 4 / 4;                      // row sums a lane ends with (4 column lanes)
+  constexpr int NCV = CC * 4 / 8;                      // column sums a lane ends with (8 row lanes)
+  constexpr int TILE = T * T * 4;                      // reals per tile
+  __shared__ R s_head[8];                              // f, f m (4)
+  __shared__ double s_red[RT_WARPS];
+  __shared__ double s_c;
+  __shared__ int s_ok;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tr = lane & 7, tc = lane >> 3;
+  const int n = tk.n, k0 = tk.k0, m = n - k0;
+  const int64_t ld = tk.ld;
+  cplx<R>* A = tk.M + k0 + (int64_t)k0 * ld;
+  cplx<R>* B = A + n;
+  const int nt = (m + T - 1) / T;
+  const int ntiles = nt * (nt + 1) / 2;
+  const int mine = ntiles > rank ? (ntiles - rank + G - 1) / G : 0;
+  const int NR = row_ctas<R>(G);
+  auto barrier = [&]() {
+    if constexpr (CL) {
+      cluster_barrier();
+      return true;
+    } else {
+      return group_barrier(gr.counter, target, G, gr.abort, err, limit, &s_ok);
+    }
+  };
+
+  // shared memory: tiles | w (previous, current) | y | own rows (w, g, x) | needed blocks
+  R* tiles = reinterpret_cast<R*>(smem);
+  const int cap = (ntiles + G - 1) / G;
+  Q4<R>* wbuf[2];
+  wbuf[0] = reinterpret_cast<Q4<R>*>(tiles + (size_t)cap * TILE);
+  wbuf[1] = wbuf[0] + m;
+  Q4<R>* ys = wbuf[1] + m;
+  const int rmax = (m + NR - 1) / NR;
+  R* own_w = reinterpret_cast<R*>(ys + m);
+  R* own_g = own_w + 4 * rmax;
+  R* own_x = own_g + 4 * rmax;
+  unsigned char* need = reinterpret_cast<unsigned char*>(own_x + 4 * rmax);
+
+  // load the tiles; clear the vectors; mark the row blocks this CTA's tiles touch
+  for (int b = tid; b < nt; b += RT_THREADS) need[b] = 0;
+  for (int r = tid; r < m; r += RT_THREADS) { wbuf[0][r] = q_zero<R>(); wbuf[1][r] = q_zero<R>(); ys[r] = q_zero<R>(); }
+  __syncthreads();
+  decltype(mag_bits(R(0))) mb = 0;
+  for (int q = warp; q < mine; q += RT_WARPS) {
+    int I, J;
+    rt_tile(rank + q * G, nt, I, J);
+    if (lane == 0) { need[I] = 1; need[J] = 1; }
+    R* tl = tiles + (size_t)q * TILE;
+#pragma unroll 4
+    for (int e = 0; e < EL; ++e) {
+      const int r = I * T + tr + 8 * (e % RR), c = J * T + tc + 4 * (e / RR);
+      Q4<R> v = q_zero<R>();
+      if (r < m && c < m) {
+        const bool low = r >= c;
+        const int64_t o = low ? r + (int64_t)c * ld : c + (int64_t)r * ld;
+        const cplx<R> a = A[o], b = B[o];
+        v = low ? Q4<R>{a.x, a.y, b.x, b.y} : Q4<R>{a.x, -a.y, -b.x, -b.y};
+        if (r == c) { v.ay = 0; v.bx = 0; v.by = 0; }
+        mb = max(mb, max(max(mag_bits(v.ax), mag_bits(v.ay)), max(mag_bits(v.bx), mag_bits(v.by))));
+      }
+      t_store<EL>(tl, e, lane, v);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, o));
+  if (lane == 0) s_red[warp] = mag_value(mb);
+  __syncthreads();
+  if (tid == 0) {
+    unsigned long long b = 0;
+    for (int q = 0; q < RT_WARPS; ++q) b = max(b, abs_bits(s_red[q]));
+    gr.npart[rank] = bits_to_double(b);
+  }
+  if (!barrier()) return false;
+  double scale = 1.0;
+  {
+    unsigned long long b = 0;
+    for (int i = lane; i < G; i += 32) b = max(b, abs_bits(__ldcg(gr.npart + i)));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
+    const int be = (int)(b >> 52);
+    // FP32 data: the scale and its inverse stay normal numbers of R
+    const int lim = sizeof(R) == 8 ? 1022 : 126;
+    if (b != 0) scale = pow2_biased(be < 1023 - lim ? 1023 - lim : (be > 1023 + lim ? 1023 + lim : be));
+  }
+  const R inv = (R)bits_to_double((2046ull << 52) - (unsigned long long)__double_as_longlong(scale));
+  for (int q = warp; q < mine; q += RT_WARPS) {
+    R* tl = tiles + (size_t)q * TILE;
+#pragma unroll 4
+    for (int e = 0; e < EL; ++e) {
+      Q4<R> v = t_load<EL>(tl, e, lane);
+      v.ax *= inv; v.ay *= inv; v.bx *= inv; v.by *= inv;
+      t_store<EL>(tl, e, lane, v);
+    }
+  }
+  // this CTA's rows: its share of [j, m) for the column j being formed
+  int rows0 = 0, nrows = 0;
+  auto partition = [&](int j) {
+    const int per = (m - j + NR - 1) / NR;
+    rows0 = j + rank * per;
+    nrows = (rank >= NR || rows0 >= m) ? 0 : (rows0 + per < m ? per : m - rows0);
+  };
+  // sum over the block of per-lane values, left in thread 0 (ss: one per thread)
+  auto cta_sum = [&](double v, int items) {
+    const int nw = items <= 32 ? 1 : RT_WARPS;
+    if (nw == 1) return warp == 0 ? warp_sum(v) : 0.0;
+    if (warp * 32 < items) v = warp_sum(v);
+    if (lane == 0) s_red[warp] = warp * 32 < items ? v : 0.0;
+    __syncthreads();
+    if (warp == 0) {
+      v = lane < RT_WARPS ? s_red[lane] : 0.0;
+#pragma unroll
+      for (int o = RT_WARPS / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    }
+    return v;
+  };
+  // |x|^2 of the own rows below the diagonal of column j, from the components'
+  // squares, and |x_1|^2 for everybody (row j + 1)
+  auto publish_norms = [&](int j, R x, int idx, double ss) {
+    const int items = 4 * nrows;
+    const double t = cta_sum(ss, items);
+    if (tid == 0 && rank < NR) gr.npart[rank] = t;
+    const int i1 = j + 1 - rows0;  // row j + 1 among the own rows
+    if (nrows > 0 && i1 >= 0 && i1 < nrows && (idx >> 5) == (4 * i1) >> 5 && idx < RT_THREADS) {
+      double q = (double)x * (double)x;   // only the four lanes of row j + 1 are used
+      q += __shfl_xor_sync(0xffffffffu, q, 1);
+      q += __shfl_xor_sync(0xffffffffu, q, 2);
+      if (idx == 4 * i1) *gr.q2 = q;
+    }
+  };
+  // column 0 as it is
+  partition(0);
+  {
+    double ss = 0.0;
+    R x0 = R(0);
+    for (int idx = tid; idx < ((4 * nrows + 31) & ~31); idx += RT_THREADS) {
+      R x = R(0);
+      if (idx < 4 * nrows) {
+        const int r = rows0 + (idx >> 2), k = idx & 3;
+        const R* src = reinterpret_cast<const R*>((k < 2 ? A : B) + r);
+        x = src[k & 1] * inv;
+        if (r == 0) { if (k) x = R(0); else tk.d[k0] = (double)x * scale; }
+        own_x[idx] = x;
+        reinterpret_cast<R*>(gr.x)[4 * r + k] = x;
+        if (r > 0) ss += (double)x * (double)x;
+      }
+      if (idx == tid) x0 = x;
+    }
+    publish_norms(0, x0, tid, ss);
+  }
+  if (!barrier()) return false;
+
+  for (int j = 0; j + 1 < m; ++j) {
+    Q4<R>* wp = wbuf[(j & 1) ^ 1];
+    Q4<R>* wn = wbuf[j & 1];
+    // ------------------------------------------------ reflector j
+    double ej = 0.0;  // component of e_j (lanes 0..3 of warp 0)
+    if (warp == 0) {
+      const R x1 = __ldcg(reinterpret_cast<const R*>(gr.x + j + 1) + (lane & 3));
+      const double q2 = __ldcg(gr.q2);
+      const double ss = warp_gather(gr.npart, NR, lane);
+      double f = 0.0, h = 0.0, s = 0.0;
+      bool unit = false;               // x_1 = 0: the head is 1
+      const bool last = m - 1 - j < 2;  // one row left: the entry itself is e
+      if (!last && ss > 0.0) {
+        const double t = ss * q2;
+        if (t > 0.0) {
+          const double rg = rsqrt(t);
+          s = ss * rg;
+          f = rsqrt(fma(t, rg, ss));
+          h = fma(f, s, f);
+        } else {
+          f = rsqrt(ss);
+          unit = true;
+        }
+      }
+      ej = last ? (double)x1 : (unit ? ((lane & 3) == 0 ? -ss * f : 0.0) : (ss == 0.0 ? 0.0 : -s * (double)x1));
+      if (!last && !(ss >= 0.0)) ej = ss;  // not a number: keep it visible
+      const double mk_ = unit ? ((lane & 3) == 0 ? 1.0 : 0.0) : (double)x1 * h;
+      if (lane < 4) {
+        s_head[1 + lane] = (R)mk_;
+        if (lane == 0) s_head[0] = (R)f;
+      }
+    }
+    // w (as x for now) and y_{j-1} of the blocks this CTA's tiles touch
+    for (int r = tid + (j >= 2 ? j - 2 : 0); r < m; r += RT_THREADS) {
+      if (!need[r / T]) continue;
+      Q4<R> x = q_zero<R>(), y = q_zero<R>();
+      if (r > j) x = q_ldcg(gr.x + r);
+      if (j > 0 && r >= j) y = q_ldcg(gr.y + r);
+      wn[r] = x;
+      ys[r] = y;
+    }
+    __syncthreads();
+    const R f = s_head[0];
+    const Q4<R> w1{s_head[1], s_head[2], s_head[3], s_head[4]};  // w at row j + 1
+    for (int r = tid + (j >= 2 ? j - 2 : 0); r < m; r += RT_THREADS) {
+      if (r <= j || !need[r / T]) continue;
+      const Q4<R> x = wn[r];
+      wn[r] = r == j + 1 ? w1 : Q4<R>{x.ax * f, x.ay * f, x.bx * f, x.by * f};
+    }
+    __syncthreads();
+    // ------------------------------------------------ sweep
+    const int Jlo = (j + 1) / T;                       // first live column block
+    const int live = (nt - Jlo) * (nt - Jlo + 1) / 2;  // tiles in dealing order
+    for (int q = warp; rank + q * G < live; q += RT_WARPS) {
+      int I, J;
+      rt_tile(rank + q * G, nt, I, J);
+      R* tl = tiles + (size_t)q * TILE;
+      const bool diag = I == J;
+      const bool publish = J == Jlo && tc == (((j + 1) - J * T) & 3);
+      const int pubq = ((j + 1) - J * T) >> 2;
+      Q4<R> v[EL];
+#pragma unroll
+      for (int e = 0; e < EL; ++e) v[e] = t_load<EL>(tl, e, lane);
+      R rs[RR * 4], cs[CC * 4];
+#pragma unroll
+      for (int k = 0; k < RR * 4; ++k) rs[k] = R(0);
+#pragma unroll
+      for (int k = 0; k < CC * 4; ++k) cs[k] = R(0);
+      Q4<R> wr[RR], yr[RR], nr[RR];
+#pragma unroll
+      for (int i = 0; i < RR; ++i) {
+        const int r0 = I * T + tr + 8 * i, r = min(r0, m - 1);
+        wr[i] = wp[r]; yr[i] = ys[r]; nr[i] = wn[r];
+        if (r0 >= m) { wr[i] = q_zero<R>(); yr[i] = q_zero<R>(); nr[i] = q_zero<R>(); }
+      }
+#pragma unroll
+      for (int c = 0; c < CC; ++c) {
+        const int cc = J * T + tc + 4 * c, cl = min(cc, m - 1);
+        Q4<R> wc = wp[cl], yc = ys[cl], nc = wn[cl];
+        if (cc >= m) { wc = q_zero<R>(); yc = q_zero<R>(); nc = q_zero<R>(); }
+#pragma unroll
+        for (int i = 0; i < RR; ++i) {
+          const int e = c * RR + i;
+          const Q4<R> u = rank2(wr[i], yr[i], wc, yc);
+          v[e].ax -= u.ax; v[e].ay -= u.ay; v[e].bx -= u.bx; v[e].by -= u.by;
+          if (diag && tr + 8 * i == tc + 4 * c) { v[e].ay = 0; v[e].bx = 0; v[e].by = 0; }
+          row_prod(rs + 4 * i, v[e], nc);
+          col_prod(cs + 4 * c, v[e], nr[i]);
+          t_store<EL>(tl, e, lane, v[e]);
+          if (publish && c == pubq) {
+            const int r = I * T + tr + 8 * i;
+            if (r > j && r < m) q_store(gr.col + r, v[e]);
+          }
+        }
+      }
+      // row sums over the four column lanes, column sums over the eight row lanes
+      scatter_sum<RR * 4, 16, 8, R>(rs, lane);
+      {
+        // column lane tc is left with values [tc NRV, (tc + 1) NRV) of (row, component)
+        const int k = tc * NRV;
+        const int r = I * T + tr + 8 * (k / 4);
+        if (r < m) {
+          R* o = reinterpret_cast<R*>(gr.part + (size_t)J * m + r) + (k & 3);
+#pragma unroll
+          for (int q2 = 0; q2 < NRV; ++q2) o[q2] = rs[q2];
+        }
+      }
+      if (!diag) {
+        scatter_sum<CC * 4, 4, 1, R>(cs, lane);
+        const int k = tr * NCV;
+        const int c = J * T + tc + 4 * (k / 4);
+        if (c < m) {
+          R* o = reinterpret_cast<R*>(gr.part + (size_t)I * m + c) + (k & 3);
+#pragma unroll
+          for (int q2 = 0; q2 < NCV; ++q2) o[q2] = cs[q2];
+        }
+      }
+    }
+    if (rank == G - 1 && warp == 0 && lane < 4) {
+      tk.e[4 * (size_t)(k0 + j) + lane] = ej * scale;
+      if (lane == 0) tk.tau[k0 + j] = f > R(0) ? 1.0 : 0.0;
+    }
+    // w_j in place of column j (this CTA's rows of the partition that formed it)
+    for (int idx = tid; idx < 4 * nrows; idx += RT_THREADS) {
+      const int r = rows0 + (idx >> 2), k = idx & 3;
+      if (r <= j) continue;
+      R* dst = reinterpret_cast<R*>((k < 2 ? A : B) + r + (int64_t)j * ld);
+      dst[k & 1] = r == j + 1 ? s_head[1 + k] : own_x[idx] * f;
+    }
+    if (!barrier()) return false;
+    // ------------------------------------------------ rows: g and c
+    const int p = j + 1;
+    partition(p);
+    {
+      constexpr int RPW = 32 / LPR;               // rows per warp and pass
+      const int sl = lane & (LPR - 1);
+      const int k = sl / (LPR / 4);               // component this lane ends with
+      const bool rep = (sl & (LPR / 4 - 1)) == 0;  // one lane of those holding it
+      double cp = 0.0;
+      for (int i0 = warp * RPW; i0 < nrows; i0 += RT_WARPS * RPW) {
+        const int i = i0 + lane / LPR;
+        const bool in = i < nrows;
+        const int r = rows0 + (in ? i : 0);
+        R s[4] = {R(0), R(0), R(0), R(0)};
+        R x = R(0);
+        if (in) {
+          x = __ldcg(reinterpret_cast<const R*>(gr.x + r) + k);
+#pragma unroll 4
+          for (int b = Jlo + sl; b < nt; b += LPR) {
+            const Q4<R> t = q_ldcg(gr.part + (size_t)b * m + r);
+            s[0] += t.ax; s[1] += t.ay; s[2] += t.bx; s[3] += t.by;
+          }
+        }
+        scatter_sum<4, LPR / 2, LPR / 4, R>(s, lane);
+#pragma unroll
+        for (int o = LPR / 8; o > 0; o >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
+        if (in && rep) {
+          const R w = r == p ? s_head[1 + k] : x * f;
+          own_g[4 * i + k] = s[0];
+          own_w[4 * i + k] = w;
+          cp += (double)(w * s[0]);
+        }
+      }
+      const double c = cta_sum(cp, nrows * LPR);
+      if (tid == 0 && rank < NR) gr.cpart[rank] = c;
+    }
+    if (rank == 0) {
+      __syncthreads();
+      if (tid < 4) reinterpret_cast<R*>(gr.g1)[tid] = own_g[tid];
+    }
+    if (!barrier()) return false;
+    // ------------------------------------------------ column j + 1
+    {
+      double ss = 0.0;
+      R xfirst = R(0);
+      const int k = tid & 3;
+      R col = R(0), g1 = R(0);
+      if (nrows > 0) {
+        g1 = __ldcg(reinterpret_cast<const R*>(gr.g1) + k);
+        if (tid < 4 * nrows) col = __ldcg(reinterpret_cast<const R*>(gr.col + rows0) + tid);
+        if (warp == 0) {
+          const double c = warp_gather(gr.cpart, NR, lane);
+          if (lane == 0) s_c = c;
+        }
+      }
+      __syncthreads();
+      if (nrows > 0) {
+        const R hc = (R)(0.5 * s_c);
+        const R wk1 = s_head[1 + k];
+        const R yk1 = g1 - hc * wk1;
+        // this lane's signs of the structured products
+        const bool n1 = k & 1, n2 = k == 1 || k == 2, n3 = k >= 2;
+        R wc[4], yc[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          wc[q] = __shfl_sync(0xffffffffu, wk1, q);
+          yc[q] = __shfl_sync(0xffffffffu, yk1, q);
+        }
+        if (n1) { wc[1] = -wc[1]; yc[1] = -yc[1]; }
+        if (n2) { wc[2] = -wc[2]; yc[2] = -yc[2]; }
+        if (n3) { wc[3] = -wc[3]; yc[3] = -yc[3]; }
+        for (int idx = tid; idx < ((4 * nrows + 31) & ~31); idx += RT_THREADS) {
+          const bool in = idx < 4 * nrows;
+          const int r = rows0 + (idx >> 2);
+          if (in && idx != tid) col = __ldcg(reinterpret_cast<const R*>(gr.col + rows0) + idx);
+          const R w = in ? own_w[idx] : R(0), g = in ? own_g[idx] : R(0);
+          const R y = g - hc * w;
+          R u = w * yc[0], t = y * wc[0];
+#pragma unroll
+          for (int q = 1; q < 4; ++q) {
+            u = fma(__shfl_xor_sync(0xffffffffu, w, q), yc[q], u);
+            t = fma(__shfl_xor_sync(0xffffffffu, y, q), wc[q], t);
+          }
+          R x = R(0);
+          if (in) {
+            x = col - (u + t);
+            if (r == p) { if (k) x = R(0); else tk.d[k0 + p] = (double)x * scale; }
+            own_x[idx] = x;
+            reinterpret_cast<R*>(gr.x)[4 * r + k] = x;
+            reinterpret_cast<R*>(gr.y)[4 * r + k] = y;
+            if (r > p) ss += (double)x * (double)x;
+          }
+          if (idx == tid) xfirst = x;
+        }
+      }
+      publish_norms(p, xfirst, tid, ss);
+    }
+    if (!barrier()) return false;
+  }
+  if (rank == 0 && tid == 0 && m > 0) {
+    double* e = tk.e + 4 * (size_t)(n - 1);
+    e[0] = e[1] = e[2] = e[3] = 0.0;
+    tk.tau[n - 1] = 0.0;
+  }
+  return true;
+}
+
+template <typename R, int T, bool CL>
+__global__ void __launch_bounds__(RT_THREADS, 1) k_tri_resident(const TriArgs<R> a) {
+  extern __shared__ __align__(16) unsigned char rt_smem[];
+  __shared__ int s_task;
+  __shared__ int s_ok;
+  const int group = blockIdx.x / a.G, rank = blockIdx.x % a.G;
+  const TriGroup<R> gr = tri_group<R>(a.ws + (size_t)group * a.ws_stride, a.G, a.m_max, T);
+  unsigned target = 0;
+  bool ok = true;
+  if (!a.tasks) {
+    ok = reduce_matrix<R, T, sizeof(R) == 8 ? 32 : 8, CL>(a.one, gr, rank, a.G, rt_smem, target, a.err, a.limit);
+    if (!ok && rank == 0 && threadIdx.x == 0) a.one.d[a.one.k0] = __longlong_as_double(0x7ff8000000000000ll);
+    return;
+  }
+  // a queue of matrices: the group's first CTA takes one for all of them
+  for (int it = 0;; ++it) {
+    if (rank == 0 && threadIdx.x == 0) gr.slot[it & 1] = atomicAdd(a.queue, 1);
+    if constexpr (CL) cluster_barrier();
+    else if (!group_barrier(gr.counter, target, a.G, gr.abort, a.err, a.limit, &s_ok)) return;
+    if (threadIdx.x == 0) s_task = __ldcg(gr.slot + (it & 1));
+    __syncthreads();
+    const int t = s_task;
+    if (t >= a.ntasks) return;
+    const TriTask<R> tk = a.tasks[t];
+    if (tk.n > 0) {
+      ok = reduce_matrix<R, T, sizeof(R) == 8 ? 32 : 8, CL>(tk, gr, rank, a.G, rt_smem, target, a.err, a.limit);
+      if (!ok) {
+        if (rank == 0 && threadIdx.x == 0) tk.d[0] = __longlong_as_double(0x7ff8000000000000ll);
+        return;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+template <typename R>
+size_t rt_smem_bytes(int m, int T, int G) {
+  const int nt = (m + T - 1) / T, ntiles = nt * (nt + 1) / 2;
+  const size_t cap = (size_t)((ntiles + G - 1) / G);
+  const int NR = row_ctas<R>(G);
+  return cap * T * T * 4 * sizeof(R) + sizeof(Q4<R>) * (3 * (size_t)m + 3 * (size_t)((m + NR - 1) / NR)) + (size_t)nt + 16;
+}
+
+// shared-memory opt-in (and clusters above eight CTAs), once per device and kernel
+template <typename R, int T, bool CL>
+int rt_attr() {
+  static std::atomic<unsigned long long> set{0};
+  int dev = 0;
+  ZQ_CUDA(cudaGetDevice(&dev));
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (!(set.load() & bit)) {
+    ZQ_CUDA(cudaFuncSetAttribute(k_tri_resident<R, T, CL>, cudaFuncAttributeMaxDynamicSharedMemorySize, RT_SMEM_MAX));
+    if (CL) ZQ_CUDA(cudaFuncSetAttribute(k_tri_resident<R, T, CL>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    set.fetch_or(bit);
+  }
+  return ZQ_OK;
+}
+
+template <typename R, int T, bool CL>
+int rt_launch(const TriArgs<R>& a, int ctas, size_t smem, cudaStream_t st) {
+  if (int rc = rt_attr<R, T, CL>()) return rc;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)ctas);
+  cfg.blockDim = dim3(RT_THREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  if (CL) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)a.G;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+  } else {
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  ZQ_CUDA(cudaLaunchKernelEx(&cfg, k_tri_resident<R, T, CL>, a));
+  ZQ_LAUNCH_CHECK();
+  return ZQ_OK;
+}
+
+// whether a full cluster with all of the shared memory can run on this device
+template <typename R, int T>
+bool cluster_available() {
+  static std::atomic<int> known[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+  int k = known[dev].load();
+  if (k == 0) {
+    k = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(RT_THREADS);
+    cfg.dynamicSmemBytes = RT_SMEM_MAX;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 16;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (rt_attr<R, T, true>() == ZQ_OK &&
+        cudaOccupancyMaxActiveClusters(&clusters, k_tri_resident<R, T, true>, &cfg) == cudaSuccess && clusters > 0)
+      k = 2;
+    else
+      (void)cudaGetLastError();
+    known[dev].store(k);
+  }
+  return k == 2;
+}
+
+}  // namespace
+
+namespace {
+// Tile edge: FP64 sweeps are bound by the FP64 pipe (an instruction holds its SM
+// quadrant for 64 cycles), so small tiles spread them over more warps (n = 750:
+// 24.0 ms with 8, 28.5 ms with 16); FP32 sweeps at 16 (n = 1023: 16.6 ms, 17.6
+// with 8, 18.6 with 32).
+template <typename R> constexpr int rt_tile_edge() { return sizeof(R) == 8 ? 8 : 16; }
+constexpr int RT_CLUSTER = 16;
+// Up to this order one cluster of 16 CTAs does the reduction: its hardware
+// barrier takes ~1000 cycles against ~2400 through L2, which outweighs having
+// fewer SMs for the tiles (FP32, n = 300: 8.0 against 8.6 ms for the whole
+// solve; FP64, n = 64: 4.85 against 4.99 ms), and matrices of different streams
+// reduce side by side.
+template <typename R> constexpr int rt_cluster_max() { return sizeof(R) == 8 ? 64 : 448; }
+}  // namespace
+
+int sm_count() {
+  static std::atomic<int> sms[64];
+  int dev = 0, v = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if ((v = sms[dev].load())) return v;
+  int coop = 0;
+  if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) return 0;
+  if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+  sms[dev].store(v);
+  return v;
+}
+
+template <typename R>
+bool resident_fits(int m, int ctas) {
+  if (m < 1 || ctas < 1) return false;
+  constexpr int T = rt_tile_edge<R>();
+  const int nt = (m + T - 1) / T, ntiles = nt * (nt + 1) / 2;
+  return rt_smem_bytes<R>(m, T, ctas < ntiles ? ctas : ntiles) <= (size_t)RT_SMEM_MAX;
+}
+
+template <typename R>
+int resident_max(int ctas) {
+  if (ctas < 1) return 0;
+  int lo = 0, hi = RESIDENT_MMAX;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) / 2;
+    if (resident_fits<R>(mid, ctas)) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+template <typename R>
+int tri_resident(const TridiagView<R>& v, int k0, int ctas, cudaStream_t st) {
+  const int m = v.n - k0;
+  constexpr int T = rt_tile_edge<R>();
+  const int nt = (m + T - 1) / T, ntiles = nt * (nt + 1) / 2;
+  const bool cl = m <= rt_cluster_max<R>() && cluster_available<R, T>();
+  const int most = cl ? RT_CLUSTER : ctas;
+  const int G = most < ntiles ? most : ntiles;
+  TriArgs<R> a{};
+  a.one = TriTask<R>{v.M, v.n, k0, v.ld, v.d, v.e, v.tau};
+  a.G = G; a.m_max = m;
+  a.ws = reinterpret_cast<unsigned char*>(v.rws);
+  a.ws_stride = 0;
+  a.err = v.tc_err;
+  a.limit = pipeline_wait_cycles();
+  ZQ_CUDA(cudaMemsetAsync(v.rws, 0, 64, st));  // counter, abort flag
+  const size_t smem = rt_smem_bytes<R>(m, T, G);
+  return cl ? rt_launch<R, T, true>(a, G, smem, st) : rt_launch<R, T, false>(a, G, smem, st);
+}
+
+int resident_ctas(int n, bool alone) {
+  const int sms = sm_count();
+  // beside other solves: a quarter of the SMs where that is enough
+  return !alone && n <= resident_max<float>(sms / 4) && n <= resident_max<double>(sms / 4) ? sms / 4 : sms;
+}
+
+size_t resident_workspace_bytes(int n, size_t real_bytes) {
+  const int m = n < RESIDENT_MMAX ? n : RESIDENT_MMAX;
+  return tri_group_bytes(1024, m, 8, real_bytes);
+}
+
+template bool resident_fits<float>(int, int);
+template bool resident_fits<double>(int, int);
+template int resident_max<float>(int);
+template int resident_max<double>(int);
+template int tri_resident<float>(const TridiagView<float>&, int, int, cudaStream_t);
+template int tri_resident<double>(const TridiagView<double>&, int, int, cudaStream_t);
+
+}  // namespace zq

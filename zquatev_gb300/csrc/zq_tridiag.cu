@@ -46,6 +46,7 @@
 // and reflector scalars are still formed in double.
 #include "zq_common.cuh"
 #include "zq_kernels.h"
+#include "zq_resident.h"
 #include "zq_tc32.h"
 
 #include <cuda.h>
@@ -1261,7 +1262,11 @@ int tridiagonalize(TridiagView<R> v, int nb, cudaStream_t st) {
   }
   int ncp = 0;  // number of c partials of the previous column
   const int pgrid = (use_tma && v.coop) ? panel_persist_grid() : 0;
+  // the last columns (all of them for orders that fit) run with the trailing
+  // block held in shared memory
+  const int rmax = pgrid > 0 ? 0 : resident_max<R>(v.ctas);
   for (int p = 0; p < n; p += nb) {
+    if (n - p <= rmax) return tri_resident<R>(v, p, v.ctas, st);
     const int nbp = (nb < n - p) ? nb : (n - p);
     if constexpr (std::is_same<R, float>::value) if (pgrid > 0) {
       // the panel's columns in one cooperative launch
@@ -1357,7 +1362,8 @@ size_t tridiag_workspace_bytes(int n, int nbmax) {
   b += sizeof(double) * (2 * hblk + 16);              // npart (2 hblk), scal
   b += sizeof(double) * ((size_t)ceil_div(n > 0 ? n : 1, HRB) + 1);  // cpart (one per hreduce CTA)
   b += sizeof(unsigned) * 8;                          // counters (colupd, dots, grid barrier, abort)
-  return b + 16 * 256;
+  b += resident_workspace_bytes(n, sizeof(R));
+  return b + 17 * 256;
 }
 
 template <typename R>
@@ -1379,6 +1385,8 @@ TridiagView<R> tridiag_bind(void* ws, cplx<R>* M, int n, int64_t ld, int nbmax, 
   v.cpart = reinterpret_cast<double*>(take(sizeof(double) * ((size_t)ceil_div(n > 0 ? n : 1, HRB) + 1)));
   v.scal = reinterpret_cast<double*>(take(sizeof(double) * 16));
   v.counter = reinterpret_cast<unsigned*>(take(sizeof(unsigned) * 8));
+  v.rws = take(resident_workspace_bytes(n, sizeof(R)));
+  v.ctas = resident_ctas(n, true);
   v.coop = 1;
   v.d = d; v.e = e; v.tau = tau;
   return v;
