@@ -20,6 +20,7 @@
 #include "zq_common.cuh"
 #include "zq_kernels.h"
 #include "zq_context.h"
+#include "zq_applyq.h"
 #include "zq_resident.h"
 #include "../../include/zquatev_gb300.h"
 
@@ -295,7 +296,18 @@ int solve_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, bool
   if (int rc = phase_reduce(e, n, offd, phi, c->st)) return rc;
   tm.mark("tridiag", c->st);
 
-  if (vectors) {
+  if (vectors && n <= APPLYQ_MAX) {
+    // each column takes the reflectors directly (zq_applyq.cu)
+    double* Z = nullptr;
+    prof_begin(PC_STEDC, c->st);
+    if (int rc = c->dc.run(d, offd, lam, Z, c->st)) return rc;
+    prof_end(PC_STEDC, c->st);
+    tm.mark("stedc", c->st);
+    prof_begin(PC_APPLYZ, c->st);
+    if (int rc = apply_q(nullptr, nullptr, ApplyQTask{dD, phi, Z, ldd, n, n, 0}, n, n, c->st)) return rc;
+    prof_end(PC_APPLYZ, c->st);
+    tm.mark("apply_q", c->st);
+  } else if (vectors) {
     // Q Phi on the second stream, overlapping the tridiagonal solve
     ZQ_CUDA(cudaEventRecord(c->ev_fork, c->st));
     ZQ_CUDA(cudaStreamWaitEvent(c->st2, c->ev_fork, 0));
