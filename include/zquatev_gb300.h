@@ -83,9 +83,10 @@ int zq_set_path(int path);
 
 /* FP64-accurate complex product C = op(A) op(B) (m x n, inner k; op 0 = N,
  * 1 = T, 2 = conjugate transpose, 3 = conjugate) on the bf16 tensor cores with
- * Ozaki slicing and exact accumulation (the engine of the refinement). All
- * pointers are device memory (interleaved complex, column-major); allocates
- * its scratch with cudaMallocAsync on `stream`. No reference counterpart. */
+ * the Ozaki scheme and exact accumulation (the engine of the refinement). All
+ * pointers are device memory (interleaved complex, column-major); takes its
+ * scratch in stream order from a pool of the library that keeps up to 4 GB
+ * between calls (zq_release_workspace returns them). No reference counterpart. */
 int zq_zgemm_accurate(int opa, int opb, int m, int n, int k, const double* A, int lda, const double* B, int ldb,
                       double* C, int ldc, void* stream);
 
@@ -110,8 +111,10 @@ int zq_get_block_size(void);
  * zq_zgemm_accurate: 0 = mma.sync (bf16 m16n8k16, 64 x 64 tiles), 1 = tcgen05
  * (TMEM accumulators, TMA-fed 128 x 256 MMAs, one CTA per tile), 2 = tcgen05 in
  * clusters of two CTAs that share the B operand by TMA multicast, 3 = 2-SM
- * tcgen05 MMAs (cta_group::2, 256 x 256 per CTA pair; the default). Same
- * arithmetic and results. */
+ * tcgen05 MMAs (cta_group::2, 256 x 256 per CTA pair; the default). 0 to 2
+ * multiply digit slices; 3 does products of 28 bits and more on integer
+ * residues (the Ozaki scheme II), at least as accurate, with a third of the
+ * tensor work for FP64. */
 int zq_set_ozaki_kernel(int which);
 int zq_get_ozaki_kernel(void);
 
@@ -192,8 +195,9 @@ int zq_profile_flops(int cls, double* flops);
  * entry points; every launch is counted on the host right after it is made). */
 long long zq_launch_count(void);
 
-/* Frees the cached device workspace of the current device, and the device copy
- * of D that the host-memory entry points keep between calls (n2^2 complex). */
+/* Frees the cached device workspace of the current device, the device copy of D
+ * that the host-memory entry points keep between calls (n2^2 complex), and the
+ * scratch pool's idle memory. */
 int zq_release_workspace(void);
 
 /* ---------------------------------------------------------------- serving

@@ -188,6 +188,34 @@ static int get_context(Context** out) {
   return ZQ_OK;
 }
 
+static std::mutex g_pool_mu;
+static cudaMemPool_t g_pool[64];
+int scratch_pool(cudaMemPool_t* pool) {
+  int dev = 0;
+  ZQ_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= 64) { set_msg("device ordinal out of range"); return ZQ_ERR_ARG; }
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if (!g_pool[dev]) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t p;
+    ZQ_CUDA(cudaMemPoolCreate(&p, &props));
+    uint64_t keep = SCRATCH_KEEP;
+    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    g_pool[dev] = p;
+  }
+  *pool = g_pool[dev];
+  return ZQ_OK;
+}
+void scratch_pool_trim() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  if (g_pool[dev]) cudaMemPoolTrimTo(g_pool[dev], 0);
+}
+
 static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
 // workspace layout for one solve of quaternion size n (excluding the output D)
@@ -776,6 +804,7 @@ long long zq_launch_count(void) { return zq::g_launches.load(std::memory_order_r
 int zq_release_workspace(void) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return ZQ_ERR_CUDA;
+  scratch_pool_trim();
   std::lock_guard<std::mutex> lk(g_ctx_mu);
   Context* c = g_ctx[dev];
   if (!c) return ZQ_OK;

@@ -116,6 +116,8 @@ struct DcPlan {
   float* Zf[2] = {nullptr, nullptr};
   float* Mbf = nullptr;
   DgemmDescT<float>* fdescs_dev = nullptr;
+  double* crt_ws = nullptr;  // scratch of the residue-arithmetic merges (orders from DC_CRT_MIN)
+  int* err = nullptr;        // raised when one of their pipeline waits ran out: the eigenvalues become NaN
   int* tc_err = nullptr;  // run_single: merges of large nodes on the tensor cores (timeout flag) when set
 
   static size_t workspace_doubles(int n);
@@ -190,10 +192,20 @@ struct OzOpts {
   int structured;  // 0 general; +1 Hermitian / -1 antisymmetric square output (lower tiles computed)
   int reuse_a;     // 1: the A operand is the same as in the previous call (slices kept)
   int nofill;      // structured: leave the upper triangle to the caller (who fills it with structured_fill)
+  int prev_slices; // reuse_a: the slices of the previous call
+  int* err;        // device flag a pipeline timeout raises, cleared and read by the caller (null: here, with a wait)
 };
 int zgemm_ozaki(int opa1, int opb1, int opa2, int opb2, const ZgemmArgs& g, void* ws, size_t ws_bytes, cudaStream_t st,
                 const OzOpts& opt);
+// workspace of one product (K = the complex inner dimension of all segments)
+size_t zgemm_ozaki_bytes(int m, int n, int64_t K, int slices);
 size_t ozaki_workspace_bytes(int n);
+// the current device's pool for the scratch of single calls: stream-ordered,
+// keeps up to SCRATCH_KEEP bytes mapped between calls (zq_release_workspace
+// returns them)
+constexpr unsigned long long SCRATCH_KEEP = 4ull << 30;
+int scratch_pool(cudaMemPool_t* pool);
+void scratch_pool_trim();
 // limit of every mbarrier wait in the tensor-core pipelines, SM clock cycles
 // (<= 0: the default, about 2 s); a test hook for the timeout path
 void set_pipeline_wait_cycles(long long cycles);

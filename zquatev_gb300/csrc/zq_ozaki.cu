@@ -29,7 +29,9 @@
 // tiles, cp.async double buffering.
 #include "zq_common.cuh"
 #include "zq_kernels.h"
+#include "zq_crt.h"
 
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
@@ -541,14 +543,39 @@ int oz_umma_gemm(const __nv_bfloat16* As, const __nv_bfloat16* Brs, const __nv_b
                  int m, int n, int nsl, int lower, const int* ea, const int* eb, double2* C, int64_t ldc, int* err,
                  cudaStream_t st, int variant);
 
-// workspace for products with m, n <= 2 * nq and Kp <= 4 * nq + 64
+// Whether a product with this many slices' accuracy runs on residues (zq_crt.cu)
+// instead of digit slices, and with how many moduli: the default kernel, from
+// four slices (28 bits) up, where the residue products are fewer (four slices:
+// 9 moduli x 3 real products against 10 digit products x 4; three: 8 x 3 against
+// 6 x 4, no gain for the reconstruction's cost).
+static int crt_bits(int slices) { return OZ_BETA * slices - 1; }
+static int use_crt(int slices, int64_t K) {
+  return ozaki_kernel() == 3 && slices >= 4 ? crt_moduli(crt_bits(slices), 2.0 * (double)K) : 0;
+}
+
+size_t zgemm_ozaki_bytes(int m, int n, int64_t K, int slices) {
+  if (const int L = use_crt(slices, K)) {
+    const CrtShape s = crt_shape(m, n, (int)K, L, true);
+    return s.a_bytes + s.b_bytes + s.r_bytes + sizeof(int) * (size_t)(s.mp + s.np + 64) + 9 * 256;
+  }
+  const int64_t mp = rup(m, OZ_PAD), np = rup(n, OZ_PAD), Kp = rup(2 * K, OZ_TK);
+  return sizeof(__nv_bfloat16) * (size_t)OZ_SMAX * (mp + 2 * np) * Kp + sizeof(int) * (size_t)(mp + np + 64) + 9 * 256;
+}
+
+// workspace of the refinement's products, (m, n, K) = (2 nq, nq, nq) and
+// (nq, nq, 2 nq), at any slice count and with any product kernel
 size_t ozaki_workspace_bytes(int nq) {
-  const int64_t mp = rup(2 * (int64_t)nq, OZ_PAD), np = rup(2 * (int64_t)nq, OZ_PAD), Kp = rup(4 * (int64_t)nq, 64);
-  size_t b = 0;
-  b += sizeof(__nv_bfloat16) * (size_t)OZ_SMAX * mp * Kp;       // A slices
-  b += sizeof(__nv_bfloat16) * (size_t)OZ_SMAX * np * Kp * 2;   // B slices (re / im forms)
-  b += sizeof(int) * (size_t)(mp + np + 64);
-  return b + 9 * 256;
+  size_t most = 0;
+  const int64_t shapes[2][3] = {{2 * (int64_t)nq, nq, nq}, {nq, nq, 2 * (int64_t)nq}};
+  for (const auto& q : shapes) {
+    const int64_t mp = rup(q[0], OZ_PAD), np = rup(q[1], OZ_PAD), Kp = rup(2 * q[2], OZ_TK);
+    const size_t digits = sizeof(__nv_bfloat16) * (size_t)OZ_SMAX * (mp + 2 * np) * Kp + sizeof(int) * (size_t)(mp + np + 64);
+    const int L = crt_moduli(crt_bits(OZ_SMAX), 2.0 * (double)q[2]);
+    const CrtShape s = crt_shape((int)q[0], (int)q[1], (int)q[2], L > 0 ? L : 1, true);
+    const size_t residues = s.a_bytes + s.b_bytes + s.r_bytes + sizeof(int) * (size_t)(s.mp + s.np + 64);
+    most = std::max(most, std::max(digits, residues));
+  }
+  return most + 9 * 256;
 }
 
 // structured square outputs: fill the upper triangle from the lower one
@@ -641,9 +668,8 @@ int zgemm_ozaki(int opa1, int opb1, int opa2, int opb2, const ZgemmArgs& g, void
   b.X2 = two ? g.B2 : nullptr; b.ld2 = g.ldb2; b.op2 = opb2; b.K2 = two ? g.k2 : 0; b.s2 = 1.0;
   const int64_t Kp = rup(2 * ((int64_t)g.k1 + (two ? g.k2 : 0)), OZ_TK);
   const int64_t mp = rup(m, OZ_PAD), np = rup(n, OZ_PAD);
-  size_t need = sizeof(__nv_bfloat16) * ((size_t)OZ_SMAX * mp * Kp + 2 * (size_t)OZ_SMAX * np * Kp) +
-                sizeof(int) * (size_t)(mp + np + 64) + 9 * 256;
-  if (need > ws_bytes) { set_error_message("zgemm_ozaki: workspace too small"); return ZQ_ERR_LIMIT; }
+  const int64_t Kc = (int64_t)g.k1 + (two ? g.k2 : 0);
+  if (zgemm_ozaki_bytes(m, n, Kc, nsl) > ws_bytes) { set_error_message("zgemm_ozaki: workspace too small"); return ZQ_ERR_LIMIT; }
   if (g.alpha.x != 1.0 || g.alpha.y != 0.0 || g.beta.x != 0.0 || g.beta.y != 0.0) {
     set_error_message("zgemm_ozaki: only C = op(A) op(B) (alpha 1, beta 0)");
     return ZQ_ERR_ARG;
@@ -651,45 +677,83 @@ int zgemm_ozaki(int opa1, int opb1, int opa2, int opb2, const ZgemmArgs& g, void
   if (opt.structured != 0 && m != n) { set_error_message("zgemm_ozaki: structured output must be square"); return ZQ_ERR_ARG; }
   char* p = reinterpret_cast<char*>(ws);
   auto take = [&](size_t bytes) { char* q = p; p += (bytes + 255) & ~(size_t)255; return q; };
-  // fixed carve-up (sized for the largest shapes) so the A slices of one call can be reused by the next
-  const int64_t cap = (int64_t)(ws_bytes / 8);
-  (void)cap;
-  __nv_bfloat16* As = reinterpret_cast<__nv_bfloat16*>(take(sizeof(__nv_bfloat16) * OZ_SMAX * mp * Kp));
-  __nv_bfloat16* Brs = reinterpret_cast<__nv_bfloat16*>(take(sizeof(__nv_bfloat16) * OZ_SMAX * np * Kp));
-  __nv_bfloat16* Bis = reinterpret_cast<__nv_bfloat16*>(take(sizeof(__nv_bfloat16) * OZ_SMAX * np * Kp));
-  int* ea = reinterpret_cast<int*>(take(sizeof(int) * mp));
-  int* eb = reinterpret_cast<int*>(take(sizeof(int) * np));
-  int* errf = reinterpret_cast<int*>(take(sizeof(int) * 4));
-  auto grid = [](int64_t total) { int64_t x = (total + 255) / 256; return (int)(x > 16384 ? 16384 : x); };
-  if (!opt.reuse_a) {
-    const bool cm = (opa1 == OP_N || opa1 == OP_R) && (!two || opa2 == OP_N || opa2 == OP_R);
+  // exponents of the rows of op(A) (rows that are strided in memory: column-wise passes with coalesced reads)
+  const bool cm = (opa1 == OP_N || opa1 == OP_R) && (!two || opa2 == OP_N || opa2 == OP_R);
+  auto row_exponents = [&](int* ea) -> int {
+    k_oz_exp_init<<<ceil_div(m, 256), 256, 0, st>>>(ea, m);
+    ZQ_LAUNCH_CHECK();
     if (cm) {
-      // rows of op(A) are strided: column-wise passes (coalesced reads)
-      k_oz_exp_init<<<ceil_div(m, 256), 256, 0, st>>>(ea, m);
-      ZQ_LAUNCH_CHECK();
-      const int Kc = g.k1 + (two ? g.k2 : 0);  // complex columns of op(A)
-      k_oz_exp_cm<<<dim3((unsigned)ceil_div(m, 32), (unsigned)ceil_div(Kc, 256)), dim3(32, 8), 0, st>>>(a, m, Kc, ea);
-      ZQ_LAUNCH_CHECK();
-      k_oz_slice_cm<<<dim3((unsigned)(mp / 32), (unsigned)ceil_div((int)Kp, 32)), dim3(32, 8), 0, st>>>(a, m, (int)Kp, ea,
-                                                                                                        nsl, As, mp * Kp);
-      ZQ_LAUNCH_CHECK();
+      k_oz_exp_cm<<<dim3((unsigned)ceil_div(m, 32), (unsigned)ceil_div((int)Kc, 256)), dim3(32, 8), 0, st>>>(a, m, (int)Kc, ea);
     } else {
       const int parts = oz_exp_parts(m, a);
-      k_oz_exp_init<<<ceil_div(m, 256), 256, 0, st>>>(ea, m);
-      ZQ_LAUNCH_CHECK();
       k_oz_exp<<<ceil_div(m * parts * 32, 256), 256, 0, st>>>(a, true, m, parts, ea);
-      ZQ_LAUNCH_CHECK();
-      k_oz_slice<<<grid(mp * Kp / 8), 256, 0, st>>>(a, true, m, (int)mp, (int)Kp, ea, nsl, As, nullptr, mp * Kp);
-      ZQ_LAUNCH_CHECK();
     }
-  }
-  {
+    ZQ_LAUNCH_CHECK();
+    return ZQ_OK;
+  };
+  auto col_exponents = [&](int* eb) -> int {
     const int parts = oz_exp_parts(n, b);
     k_oz_exp_init<<<ceil_div(n, 256), 256, 0, st>>>(eb, n);
     ZQ_LAUNCH_CHECK();
     k_oz_exp<<<ceil_div(n * parts * 32, 256), 256, 0, st>>>(b, false, n, parts, eb);
     ZQ_LAUNCH_CHECK();
+    return ZQ_OK;
+  };
+  // the pipeline's timeout flag: the caller's, or one read here
+  auto check_flag = [&](int* errf) -> int {
+    if (opt.err) return ZQ_OK;
+    int herr = 0;
+    ZQ_CUDA(cudaMemcpyAsync(&herr, errf, sizeof(int), cudaMemcpyDeviceToHost, st));
+    ZQ_CUDA(cudaStreamSynchronize(st));
+    if (herr) {
+      set_error_message("tensor-core product: a pipeline wait ran out of time (kernel stopped)");
+      return ZQ_ERR_TIMEOUT;
+    }
+    return ZQ_OK;
+  };
+  const int L = use_crt(nsl, Kc);
+  const bool reuse_a = opt.reuse_a && (L > 0) == (use_crt(opt.prev_slices, Kc) > 0) && (L == 0 || opt.prev_slices == nsl);
+  if (L > 0) {
+    const CrtShape sh = crt_shape(m, n, (int)Kc, L, true);
+    const int bits = crt_bits(nsl);
+    void* As = take(sh.a_bytes);
+    int* ea = reinterpret_cast<int*>(take(sizeof(int) * sh.mp));
+    void* Bs = take(sh.b_bytes);
+    int* eb = reinterpret_cast<int*>(take(sizeof(int) * sh.np));
+    void* Rs = take(sh.r_bytes);
+    int* errf = opt.err ? opt.err : reinterpret_cast<int*>(take(sizeof(int) * 4));
+    CrtSide ca{a.X1, a.ld1, a.op1, a.K1, a.X2, a.ld2, a.op2, a.K2, a.s2};
+    CrtSide cb{b.X1, b.ld1, b.op1, b.K1, b.X2, b.ld2, b.op2, b.K2, b.s2};
+    if (!reuse_a) {
+      if (int rc = row_exponents(ea)) return rc;
+      if (int rc = crt_split(ca, true, m, sh.mp, sh.Kp, ea, bits, L, As, st)) return rc;
+    }
+    if (int rc = col_exponents(eb)) return rc;
+    if (int rc = crt_split(cb, false, n, sh.np, sh.Kp, eb, bits, L, Bs, st)) return rc;
+    if (!opt.err) ZQ_CUDA(cudaMemsetAsync(errf, 0, sizeof(int), st));
+    if (int rc = crt_multiply(sh, As, Bs, Rs, opt.structured != 0, errf, st)) return rc;
+    if (int rc = crt_join(sh, Rs, m, n, bits, ea, eb, opt.structured != 0, g.C, g.ldc, st)) return rc;
+    if (int rc = check_flag(errf)) return rc;
+    if (opt.structured != 0 && !opt.nofill) return structured_fill(g.C, g.ldc, m, opt.structured, st);
+    return ZQ_OK;
   }
+  __nv_bfloat16* As = reinterpret_cast<__nv_bfloat16*>(take(sizeof(__nv_bfloat16) * OZ_SMAX * mp * Kp));
+  __nv_bfloat16* Brs = reinterpret_cast<__nv_bfloat16*>(take(sizeof(__nv_bfloat16) * OZ_SMAX * np * Kp));
+  __nv_bfloat16* Bis = reinterpret_cast<__nv_bfloat16*>(take(sizeof(__nv_bfloat16) * OZ_SMAX * np * Kp));
+  int* ea = reinterpret_cast<int*>(take(sizeof(int) * mp));
+  int* eb = reinterpret_cast<int*>(take(sizeof(int) * np));
+  int* errf = opt.err ? opt.err : reinterpret_cast<int*>(take(sizeof(int) * 4));
+  auto grid = [](int64_t total) { int64_t x = (total + 255) / 256; return (int)(x > 16384 ? 16384 : x); };
+  if (!reuse_a) {
+    if (int rc = row_exponents(ea)) return rc;
+    if (cm)
+      k_oz_slice_cm<<<dim3((unsigned)(mp / 32), (unsigned)ceil_div((int)Kp, 32)), dim3(32, 8), 0, st>>>(a, m, (int)Kp, ea,
+                                                                                                        nsl, As, mp * Kp);
+    else
+      k_oz_slice<<<grid(mp * Kp / 8), 256, 0, st>>>(a, true, m, (int)mp, (int)Kp, ea, nsl, As, nullptr, mp * Kp);
+    ZQ_LAUNCH_CHECK();
+  }
+  if (int rc = col_exponents(eb)) return rc;
   k_oz_slice<<<grid(np * Kp / 8), 256, 0, st>>>(b, false, n, (int)np, (int)Kp, eb, nsl, Brs, Bis, np * Kp);
   ZQ_LAUNCH_CHECK();
   OzGemmArgs og{};
@@ -704,18 +768,13 @@ int zgemm_ozaki(int opa1, int opb1, int opa2, int opb2, const ZgemmArgs& g, void
     const double pairs = (double)nsl * (nsl + 1) / 2.0;
     const double tiles = lower ? (double)tm * (tm + 1) / 2.0 : (double)tm * tn;
     prof_add_flops(PC_OZAKI, pairs * 2.0 * tiles * 128.0 * 128.0 * (double)Kp * 2.0);
+    if (!opt.err) ZQ_CUDA(cudaMemsetAsync(errf, 0, sizeof(int), st));
     prof_begin(PC_OZAKI, st);
     if (int rc = oz_umma_gemm(As, Brs, Bis, (int)mp, (int)np, (int)Kp, m, n, nsl, lower ? 1 : 0, ea, eb, g.C, g.ldc, errf,
                               st, ozaki_kernel() - 1))
       return rc;
     prof_end(PC_OZAKI, st);
-    int herr = 0;
-    ZQ_CUDA(cudaMemcpyAsync(&herr, errf, sizeof(int), cudaMemcpyDeviceToHost, st));
-    ZQ_CUDA(cudaStreamSynchronize(st));
-    if (herr) {
-      set_error_message("k_oz_umma: a pipeline wait ran out of time (kernel stopped)");
-      return ZQ_ERR_TIMEOUT;
-    }
+    if (int rc = check_flag(errf)) return rc;
   } else {
     const int smem = 2 * 3 * OZ_TM * OZ_LDS * (int)sizeof(__nv_bfloat16);
     {
@@ -767,11 +826,12 @@ extern "C" int zq_zgemm_accurate(int opa, int opb, int m, int n, int k, const do
   using namespace zq;
   if (m < 0 || n < 0 || k < 0 || opa < 0 || opa > 3 || opb < 0 || opb > 3) return ZQ_ERR_ARG;
   if (m == 0 || n == 0) return ZQ_OK;
-  const int q = (m > n ? m : n) / 2 + 1 > (k + 1) / 2 + 16 ? (m > n ? m : n) / 2 + 1 : (k + 1) / 2 + 16;
-  const size_t bytes = ozaki_workspace_bytes(q);
+  const size_t bytes = zgemm_ozaki_bytes(m, n, k, 8);
   void* ws = nullptr;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  ZQ_CUDA(cudaMallocAsync(&ws, bytes, st));
+  cudaMemPool_t pool = nullptr;
+  if (int rc = scratch_pool(&pool)) return rc;
+  ZQ_CUDA(cudaMallocFromPoolAsync(&ws, bytes, pool, st));
   ZgemmArgs g{};
   g.m = m; g.n = n; g.k1 = k;
   g.A1 = reinterpret_cast<const double2*>(A); g.lda1 = lda;

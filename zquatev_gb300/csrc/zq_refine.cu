@@ -455,14 +455,17 @@ size_t refine_workspace_bytes(int n, int nbq) {
 // structured from their lower triangles, so that the symmetric part of E is R
 // exactly and the orthogonality of the update does not depend on eigenvalue gaps.
 // structured: 0 general; +-1 Hermitian / antisymmetric square output (lower
-// tiles computed, upper filled); +-2 the lower triangle only, the caller fills
+// tiles computed, upper filled); +-2 the lower triangle only, the caller fills.
+// prev_slices > 0: the A operand is the previous call's, cut into that many slices.
+// err: device flag of the tensor-core pipelines' timeouts, read once per step.
 static int zgemm_acc(int mode, int opa1, int opb1, int opa2, int opb2, const ZgemmArgs& g, void* ows, size_t ows_bytes,
-                     cudaStream_t st, int slices, int structured, int reuse_a) {
+                     cudaStream_t st, int slices, int structured, int prev_slices, int* err) {
   const int sym = structured > 0 ? 1 : (structured < 0 ? -1 : 0);
   const bool fill = structured == 1 || structured == -1;
   if (mode == 1) {
     OzOpts o{};
-    o.slices = slices; o.structured = sym; o.reuse_a = reuse_a; o.nofill = fill ? 0 : 1;
+    o.slices = slices; o.structured = sym; o.reuse_a = prev_slices > 0; o.prev_slices = prev_slices; o.nofill = fill ? 0 : 1;
+    o.err = err;
     return zgemm_ozaki(opa1, opb1, opa2, opb2, g, ows, ows_bytes, st, o);
   }
   if (int rc = zgemm<double>(opa1, opb1, opa2, opb2, g, 1, st)) return rc;
@@ -582,6 +585,11 @@ static int resolve_clusters(RefineArgs& ra, double2* X, int64_t ldd, double2* S1
   return ZQ_OK;
 }
 
+static int oz_timeout() {
+  set_error_message("tensor-core product: a pipeline wait ran out of time (kernel stopped)");
+  return ZQ_ERR_TIMEOUT;
+}
+
 int refined_solve(RefineArgs& ra) {
   const int n = ra.n;
   const int n2 = 2 * n;
@@ -605,6 +613,7 @@ int refined_solve(RefineArgs& ra) {
   double* sm = reinterpret_cast<double*>(take(sizeof(double) * (46 * (size_t)n + 3 * 8192 + 8192 + 2048 + 64)));
   int* rank = reinterpret_cast<int*>(take(sizeof(int) * (size_t)n));
   int* tc_err = reinterpret_cast<int*>(take(256));
+  int* oz_err = tc_err + 1;
   double* d = sm; sm += n;
   double* e = sm; sm += 4 * (size_t)n;
   double* tau = sm; sm += n;
@@ -634,7 +643,7 @@ int refined_solve(RefineArgs& ra) {
                             cudaMemcpyDeviceToDevice, st));
   k_c128_to_c64<<<grid_for((int64_t)n2 * n), 256, 0, st>>>(H0, n2, Mf, n2, n2, n);
   ZQ_LAUNCH_CHECK();
-  ZQ_CUDA(cudaMemsetAsync(tc_err, 0, sizeof(int), st));
+  ZQ_CUDA(cudaMemsetAsync(tc_err, 0, 2 * sizeof(int), st));
   TridiagView<float> vf = tridiag_bind<float>(tri_ws, Mf, n, n2, NBMAX, d, e, tau);
   vf.tc_err = tc_err;  // tensor-core products where fp32_products_on_tensor_cores allows them
   vf.coop = ra.coop;
@@ -701,9 +710,9 @@ int refined_solve(RefineArgs& ra) {
     g = ZgemmArgs{};
     g.m = n2; g.n = n; g.k1 = n; g.A1 = H0; g.lda1 = n2; g.B1 = U; g.ldb1 = ldd;
     g.alpha = one; g.beta = zero; g.C = P1; g.ldc = n2;
-    if (int rc = zgemm_acc(ra.mode, OP_N, OP_N, OP_N, OP_N, g, ra.ows, ra.ows_bytes, st, sl, 0, 0)) return rc;
+    if (int rc = zgemm_acc(ra.mode, OP_N, OP_N, OP_N, OP_N, g, ra.ows, ra.ows_bytes, st, sl, 0, 0, oz_err)) return rc;
     g.B1 = V; g.C = P2;
-    if (int rc = zgemm_acc(ra.mode, OP_N, OP_R, OP_N, OP_N, g, ra.ows, ra.ows_bytes, st, sl, 0, 1)) return rc;
+    if (int rc = zgemm_acc(ra.mode, OP_N, OP_R, OP_N, OP_N, g, ra.ows, ra.ows_bytes, st, sl, 0, sl, oz_err)) return rc;
     // R = HX - X diag(lamr), lamr the current eigenvalue estimates (the
     // divide-and-conquer values, then the previous step's Rayleigh quotients).
     // S = X^H H X = X^H R + G diag(lamr) for any diagonal lamr; with R small
@@ -716,17 +725,17 @@ int refined_solve(RefineArgs& ra) {
     g = ZgemmArgs{};
     g.m = n; g.n = n; g.k1 = n2; g.A1 = X; g.lda1 = ldd; g.B1 = X; g.ldb1 = ldd;
     g.alpha = one; g.beta = zero; g.C = G1; g.ldc = n;
-    if (int rc = zgemm_acc(ra.mode, OP_C, OP_N, OP_N, OP_N, g, ra.ows, ra.ows_bytes, st, sl, 1, 0)) return rc;
+    if (int rc = zgemm_acc(ra.mode, OP_C, OP_N, OP_N, OP_N, g, ra.ows, ra.ows_bytes, st, sl, 1, 0, oz_err)) return rc;
     g.B1 = HX; g.ldb1 = n2; g.C = S1;
-    if (int rc = zgemm_acc(ra.mode, OP_C, OP_N, OP_N, OP_N, g, ra.ows, ra.ows_bytes, st, ss_slices, 2, 1)) return rc;
+    if (int rc = zgemm_acc(ra.mode, OP_C, OP_N, OP_N, OP_N, g, ra.ows, ra.ows_bytes, st, ss_slices, 2, sl, oz_err)) return rc;
     // G2 = U^T V - V^T U ; S2 = U^T R_bot - V^T R_top + G2 Lambda
     g = ZgemmArgs{};
     g.m = n; g.n = n; g.k1 = n; g.k2 = n;
     g.A1 = U; g.lda1 = ldd; g.B1 = V; g.ldb1 = ldd; g.A2 = V; g.lda2 = ldd; g.B2 = U; g.ldb2 = ldd; g.s2 = -1.0;
     g.alpha = one; g.beta = zero; g.C = G2; g.ldc = n;
-    if (int rc = zgemm_acc(ra.mode, OP_T, OP_N, OP_T, OP_N, g, ra.ows, ra.ows_bytes, st, sl, -1, 0)) return rc;
+    if (int rc = zgemm_acc(ra.mode, OP_T, OP_N, OP_T, OP_N, g, ra.ows, ra.ows_bytes, st, sl, -1, 0, oz_err)) return rc;
     g.B1 = HX + n; g.ldb1 = n2; g.B2 = HX; g.ldb2 = n2; g.C = S2;
-    if (int rc = zgemm_acc(ra.mode, OP_T, OP_N, OP_T, OP_N, g, ra.ows, ra.ows_bytes, st, ss_slices, -2, 1)) return rc;
+    if (int rc = zgemm_acc(ra.mode, OP_T, OP_N, OP_T, OP_N, g, ra.ows, ra.ows_bytes, st, ss_slices, -2, sl, oz_err)) return rc;
     k_add_glam<<<grid_for((int64_t)nn), 256, 0, st>>>(S1, G1, n, lamr);
     ZQ_LAUNCH_CHECK();
     k_add_glam<<<grid_for((int64_t)nn), 256, 0, st>>>(S2, G2, n, lamr);
@@ -737,7 +746,7 @@ int refined_solve(RefineArgs& ra) {
     // test are grouped into clusters, rotated (Rayleigh-Ritz on the current
     // basis, S and G carried along), and E is rebuilt in the rotated basis
     double em = 0.0, cm = 0.0;
-    int hcount = 0, clusters = 0;
+    int hcount = 0, clusters = 0, herr = 0;
     for (int pass = 0; pass < 2; ++pass) {
       k_oa_lambda<<<ceil_div(n, 256), 256, 0, st>>>(S1, G1, n, n, lam);
       ZQ_LAUNCH_CHECK();
@@ -749,7 +758,9 @@ int refined_solve(RefineArgs& ra) {
       ZQ_LAUNCH_CHECK();
       ZQ_CUDA(cudaMemcpyAsync(hemax.data(), emax, sizeof(double) * 2 * ne, cudaMemcpyDeviceToHost, st));
       ZQ_CUDA(cudaMemcpyAsync(&hcount, pair_count, sizeof(int), cudaMemcpyDeviceToHost, st));
+      ZQ_CUDA(cudaMemcpyAsync(&herr, oz_err, sizeof(int), cudaMemcpyDeviceToHost, st));
       ZQ_CUDA(cudaStreamSynchronize(st));
+      if (herr) return oz_timeout();
       em = 0.0; cm = 0.0;
       for (int q = 0; q < ne; ++q) { em = hemax[q] > em ? hemax[q] : em; cm = hemax[ne + q] > cm ? hemax[ne + q] : cm; }
       if (pass == 1 || !(cm > ra.cluster_tol)) break;
@@ -767,9 +778,9 @@ int refined_solve(RefineArgs& ra) {
     g.m = n; g.n = n; g.k1 = n; g.k2 = n;
     g.A1 = U; g.lda1 = ldd; g.B1 = Et; g.ldb1 = n; g.A2 = V; g.lda2 = ldd; g.B2 = Eb; g.ldb2 = n; g.s2 = -1.0;
     g.alpha = one; g.beta = zero; g.C = P1; g.ldc = n2;
-    if (int rc = zgemm_acc(ra.mode, OP_N, OP_N, OP_R, OP_N, g, ra.ows, ra.ows_bytes, st, sl_upd, 0, 0)) return rc;
+    if (int rc = zgemm_acc(ra.mode, OP_N, OP_N, OP_R, OP_N, g, ra.ows, ra.ows_bytes, st, sl_upd, 0, 0, oz_err)) return rc;
     g.A1 = V; g.A2 = U; g.s2 = 1.0; g.C = P1 + n;
-    if (int rc = zgemm_acc(ra.mode, OP_N, OP_N, OP_R, OP_N, g, ra.ows, ra.ows_bytes, st, sl_upd, 0, 0)) return rc;
+    if (int rc = zgemm_acc(ra.mode, OP_N, OP_N, OP_R, OP_N, g, ra.ows, ra.ows_bytes, st, sl_upd, 0, 0, oz_err)) return rc;
     k_add_c128<<<grid_for((int64_t)n2 * n), 256, 0, st>>>(P1, n2, X, ldd, n2, n);
     ZQ_LAUNCH_CHECK();
     ra.iters = it + 1;
@@ -797,6 +808,13 @@ int refined_solve(RefineArgs& ra) {
             "d&c done %.2f | apply_z done %.2f | step0 %.2f step1 %.2f step2 %.2f | end %.2f\n",
             t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8]);
     for (auto& e : tev) cudaEventDestroy(e);
+  }
+  {
+    // the last update's products
+    int herr = 0;
+    ZQ_CUDA(cudaMemcpyAsync(&herr, oz_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    ZQ_CUDA(cudaStreamSynchronize(st));
+    if (herr) return oz_timeout();
   }
   // ascending order
   k_rank<<<ceil_div(n, 128), 128, 0, st>>>(lam, n, rank);
