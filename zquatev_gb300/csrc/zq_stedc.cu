@@ -25,6 +25,7 @@
 //       gemm     - Z_node = blockdiag(Z1, Z2) * M  (grouped DGEMM).
 #include "zq_common.cuh"
 #include "zq_kernels.h"
+#include "zq_crt.h"
 #include "zq_tc32.h"
 
 #include <algorithm>
@@ -156,6 +157,8 @@ __global__ void __launch_bounds__(256) k_dc_prepare(DcNode* nodes, DcWork w, con
     }
     __syncthreads();
     if (!s_flag) {
+      // rho z^2 for the secular equation (the staging area is free now)
+      for (int q = tid; q < Ktot; q += blockDim.x) w.sz[a + q] = rho2 * w.nd_z[a + q] * w.nd_z[a + q];
       if (tid == 0) { nd.K = Ktot; nd.ndefl = m - Ktot; nd.nrot = 0; nd.rho2 = rho2; }
       return;
     }
@@ -190,8 +193,10 @@ __global__ void __launch_bounds__(256) k_dc_prepare(DcNode* nodes, DcWork w, con
     if (pj >= 0) { w.nd_val[a + K] = D[pj]; w.nd_z[a + K] = Zs[pj]; w.nd_col[a + K] = P[pj]; ++K; }
     nd.K = K; nd.ndefl = nd_; nd.nrot = nr; nd.rho2 = rho2;
     s_cnt[0] = nd_;
+    s_cnt[1] = K;
   }
   __syncthreads();
+  for (int q = tid; q < s_cnt[1]; q += blockDim.x) w.sz[a + q] = rho2 * w.nd_z[a + q] * w.nd_z[a + q];
   // sort the deflated list (values, columns) by rank; ties by index
   const int nd_ = s_cnt[0];
   const double* fv = w.df_val + a;
@@ -215,6 +220,18 @@ __global__ void __launch_bounds__(256) k_dc_prepare(DcNode* nodes, DcWork w, con
 // secular equation: one warp per root; the lanes split the sums over the
 // poles (butterfly reductions leave identical totals on every lane, so the
 // iteration's control flow stays warp-uniform)
+//
+// FP64 instructions bound it (K^2 poles and roots, ~7 iterations), so each pole
+// takes ten: the products rho z^2 are formed once (w.sz), the reciprocal is
+// 1/del from the approximate instruction and one cubically convergent Newton
+// step (relative error below 2^-52), and the two sides of the root share one
+// accumulation loop each.
+__device__ __forceinline__ double dc_recip(double d) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+  const double e = fma(-d, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
 __global__ void __launch_bounds__(128) k_dc_secular(const DcNode* nodes, int cnt, DcWork w) {
   const int pos = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
@@ -225,15 +242,17 @@ __global__ void __launch_bounds__(128) k_dc_secular(const DcNode* nodes, int cnt
   const int i = pos - a;
   if (i >= K) return;
   const double* D = w.nd_val + a;
-  const double* z = w.nd_z + a;
+  const double* rz = w.sz + a;  // rho z_k^2
   const double rho = nd.rho2;
+  // the lane's poles up to the root's own, and the first one above
+  const int above = lane + ((i + 32 - lane) & ~31);
   int o;
   double lo, hi;
   if (i < K - 1) {
     const double gap = D[i + 1] - D[i];
     const double mid = 0.5 * gap;
     double fs = 0.0;
-    for (int k = lane; k < K; k += 32) fs += rho * z[k] * z[k] / ((D[k] - D[i]) - mid);
+    for (int k = lane; k < K; k += 32) fs = fma(rz[k], dc_recip((D[k] - D[i]) - mid), fs);
     const double f = 1.0 + warp_sum(fs);
     if (f >= 0.0) { o = i; lo = 0.0; hi = mid; }
     else { o = i + 1; lo = -mid; hi = 0.0; }
@@ -244,11 +263,19 @@ __global__ void __launch_bounds__(128) k_dc_secular(const DcNode* nodes, int cnt
   double tau = 0.5 * (lo + hi);
   for (int it = 0; it < 200; ++it) {
     double psi = 0.0, phi = 0.0, dpsi = 0.0, dphi = 0.0;
-    for (int k = lane; k < K; k += 32) {
-      const double del = (D[k] - Do) - tau;
-      const double inv = 1.0 / del;
-      const double t = rho * z[k] * z[k] * inv;
-      if (k <= i) { psi += t; dpsi += t * inv; } else { phi += t; dphi += t * inv; }
+#pragma unroll 4
+    for (int k = lane; k <= i; k += 32) {
+      const double inv = dc_recip((D[k] - Do) - tau);
+      const double t = rz[k] * inv;
+      psi += t;
+      dpsi = fma(t, inv, dpsi);
+    }
+#pragma unroll 4
+    for (int k = above; k < K; k += 32) {
+      const double inv = dc_recip((D[k] - Do) - tau);
+      const double t = rz[k] * inv;
+      phi += t;
+      dphi = fma(t, inv, dphi);
     }
     psi = warp_sum(psi); phi = warp_sum(phi); dpsi = warp_sum(dpsi); dphi = warp_sum(dphi);
     const double f = 1.0 + psi + phi;
@@ -316,10 +343,11 @@ __global__ void __launch_bounds__(128) k_dc_zhat(const DcNode* nodes, int cnt, D
   const double* T = w.r_tau + a;
   // (lambda_{K-1} - D_k) / rho
   double prod = (lane == 0) ? ((D[O[K - 1]] - Dk) + T[K - 1]) / nd.rho2 : 1.0;
+#pragma unroll 4
   for (int j = lane; j < K - 1; j += 32) {
     const double num = (D[O[j]] - Dk) + T[j];  // lambda_j - D_k
     const double den = (j < k) ? (D[j] - Dk) : (D[j + 1] - Dk);
-    prod *= num / den;
+    prod *= num * dc_recip(den);
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) prod *= __shfl_xor_sync(0xffffffffu, prod, off);
@@ -366,7 +394,7 @@ __global__ void __launch_bounds__(128) k_dc_vectors(const DcNode* nodes, int cnt
     double ss = 0.0;
     for (int k = tid; k < K; k += blockDim.x) {
       const double del = (D[k] - Do) - t;
-      const double vk = w.zhat[a + k] / del;
+      const double vk = w.zhat[a + k] * dc_recip(del);
       ss += vk * vk;
     }
     ss = warp_sum(ss);
@@ -376,7 +404,7 @@ __global__ void __launch_bounds__(128) k_dc_vectors(const DcNode* nodes, int cnt
     const double inv = 1.0 / nrm;
     for (int k = tid; k < K; k += blockDim.x) {
       const double del = (D[k] - Do) - t;
-      col[w.nd_col[a + k]] = (ZT)(w.zhat[a + k] / del * inv);
+      col[w.nd_col[a + k]] = (ZT)(w.zhat[a + k] * dc_recip(del) * inv);
     }
   } else {
     if (tid == 0) col[w.df_scol[a + (s - K)]] = (ZT)1;
@@ -424,9 +452,10 @@ __global__ void k_dc_maxabs(const double* d, const double* e, int n, double* out
   if (threadIdx.x == 0) out[0] = m;
 }
 
-__global__ void k_dc_unscale(double* lam, int n, const double* scal) {
+__global__ void k_dc_unscale(double* lam, int n, const double* scal, const int* err) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n && scal[0] > 0.0) lam[i] *= scal[0];
+  if (i < n && *err) lam[i] = __longlong_as_double(0x7ff8000000000000ll);
 }
 
 __global__ void k_dc_setrho(DcNode* nodes, int cnt, const double* es) {
@@ -437,10 +466,22 @@ __global__ void k_dc_setrho(DcNode* nodes, int cnt, const double* es) {
 // ----------------------------------------------------------------------------
 // host side: plan (tree, descriptors) and execution
 // ----------------------------------------------------------------------------
+// FP64 merges of nodes from this order up run on the tensor cores as residue
+// products (zq_crt.cu; FP64-accurate): GB300's FP64 pipe gives 1.25 TFLOP/s, the
+// residue product ~25 TFLOP/s of FP64-equivalent work at n = 3000. Below it
+// the products are too small for their six launches (a depth of eight
+// nodes of 375: 0.34 ms on the FP64 pipe, 0.8 ms as sixteen residue products).
+constexpr int DC_CRT_MIN = 600;
+static size_t dc_crt_doubles(int n) {
+  if (n < DC_CRT_MIN) return 0;
+  const int h = (n + 1) / 2;
+  return crt_dgemm_workspace(h, n, h) / sizeof(double) + 64;
+}
+
 size_t DcPlan::workspace_doubles(int n) {
   // Z x2, M, lam x2, dmod, es, scal + the per-position DcWork arrays
   const size_t nn = (size_t)n * n;
-  return 3 * nn + 2 * (size_t)n + 2 * (size_t)n + 8 + 16 * (size_t)n;
+  return 3 * nn + 2 * (size_t)n + 2 * (size_t)n + 8 + 16 * (size_t)n + dc_crt_doubles(n);
 }
 
 int DcPlan::build(int n_) {
@@ -543,6 +584,9 @@ int DcPlan::upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t s
   int* ip = reinterpret_cast<int*>(p);
   w.perm = ip; ip += n; w.nd_col = ip; ip += n; w.df_col = ip; ip += n; w.df_scol = ip; ip += n;
   w.rot_p = ip; ip += n; w.rot_j = ip; ip += n; w.r_orig = ip; ip += n;
+  err = reinterpret_cast<int*>(scal + 4);
+  // after 16 n doubles of position arrays, on a 256-byte boundary of the workspace
+  crt_ws = n >= DC_CRT_MIN ? ws + ((3 * nn + 20 * (size_t)n + 8 + 31) & ~(size_t)31) : nullptr;
   nodes_dev = dnodes;
   descs_dev = ddescs;
   // bind pointers: at depth t, A (children) lives in Z[(t+1)&1], output in Z[t&1]
@@ -593,6 +637,7 @@ template <typename ZT>
 static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, ZT* const Zb[2], ZT* Mb,
                   const DgemmDescT<ZT>* descs, cudaStream_t st) {
   const int n = P.n;
+  ZQ_CUDA(cudaMemsetAsync(P.err, 0, sizeof(int), st));
   // scale, tear
   k_dc_maxabs<<<1, 1024, 0, st>>>(d, e, n, P.scal);
   ZQ_LAUNCH_CHECK();
@@ -663,13 +708,24 @@ static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, 
           done = true;
         }
       }
+      if constexpr (std::is_same<ZT, double>::value) {
+        if (P.crt_ws && P.depth_mmax[t] >= DC_CRT_MIN) {
+          for (int q = 0; q < 2 * cnt; ++q) {
+            const DgemmDesc& h = P.gemm_host[P.gemm_off[t] + q];
+            if (int rc = crt_dgemm(h.m, h.n, h.k, Zi + h.off_a, h.lda, Mb + h.off_b, h.ldb, Zo + h.off_c, h.ldc, P.crt_ws,
+                                   P.err, st))
+              return rc;
+          }
+          done = true;
+        }
+      }
       if (!done) {
         grouped_launch<ZT>(descs + P.gemm_off[t], 2 * cnt, P.gemm_tiles[t], st);
         ZQ_LAUNCH_CHECK();
       }
     }
   }
-  k_dc_unscale<<<ceil_div(n, 256), 256, 0, st>>>(P.lam[0], n, P.scal);
+  k_dc_unscale<<<ceil_div(n, 256), 256, 0, st>>>(P.lam[0], n, P.scal, P.err);
   ZQ_LAUNCH_CHECK();
   ZQ_CUDA(cudaMemcpyAsync(lam_out, P.lam[0], sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
   return ZQ_OK;
