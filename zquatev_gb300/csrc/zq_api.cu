@@ -332,7 +332,7 @@ int solve_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, bool
     prof_end(PC_STEDC, c->st);
     tm.mark("stedc", c->st);
     prof_begin(PC_APPLYZ, c->st);
-    if (int rc = apply_q(nullptr, nullptr, ApplyQTask{dD, phi, Z, ldd, n, n, 0}, n, n, c->st)) return rc;
+    if (int rc = apply_q(nullptr, nullptr, ApplyQTask{dD, phi, Z, ldd, n, n, 0, 0}, 0, n, n, c->st)) return rc;
     prof_end(PC_APPLYZ, c->st);
     tm.mark("apply_q", c->st);
   } else if (vectors) {
@@ -574,13 +574,29 @@ static int batched_solve(int count, const int* n2s, const int* ld2s, const long 
   std::lock_guard<std::mutex> lk(c->mu);
   const int nmax = batched_max_n();
   // small tasks, largest first (longest-processing-time order)
-  std::vector<int> small, large;
+  std::vector<int> small, mid, large;
   for (int b = 0; b < count; ++b) {
     if (n2s[b] == 0) continue;
-    ((n2s[b] / 2 <= nmax) ? small : large).push_back(b);
+    const int n = n2s[b] / 2;
+    (n < FOREST_MIN ? small : (n <= nmax ? mid : large)).push_back(b);
   }
-  std::stable_sort(small.begin(), small.end(), [&](int x, int y) { return n2s[x] > n2s[y]; });
+  const auto larger = [&](int x, int y) { return n2s[x] > n2s[y]; };
+  std::stable_sort(small.begin(), small.end(), larger);
+  std::stable_sort(mid.begin(), mid.end(), larger);
   int info_max = 0;
+  if (!mid.empty()) {
+    std::vector<ForestItem> items;
+    for (int b : mid) items.push_back(ForestItem{n2s[b] / 2, ld2s[b], offs[b], eoffs[b]});
+    if (!c->forest.matches(items))
+      if (int rc = c->forest.build(items, c->st)) return rc;
+    ZQ_CUDA(cudaEventRecord(c->ev_fork, st));
+    ZQ_CUDA(cudaStreamWaitEvent(c->st, c->ev_fork, 0));
+    if (int rc = c->forest.run(dD, deig, c->st)) return rc;
+    int herr = 0;
+    ZQ_CUDA(cudaMemcpyAsync(&herr, c->forest.error_flag(), sizeof(int), cudaMemcpyDeviceToHost, c->st));
+    ZQ_CUDA(cudaStreamSynchronize(c->st));
+    if (herr) { set_msg("batch: a device-side wait ran out of time"); return ZQ_ERR_TIMEOUT; }
+  }
   if (!small.empty()) {
     int sms = 0;
     ZQ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
@@ -818,6 +834,7 @@ int zq_release_workspace(void) {
   if (c->hbuf) cudaFree(c->hbuf);
   c->hbuf = nullptr;
   c->hbuf_bytes = 0;
+  c->forest.release();
   return ZQ_OK;
 }
 

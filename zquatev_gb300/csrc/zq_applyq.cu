@@ -110,15 +110,16 @@ __device__ __forceinline__ void aq_segment(ColState<NW, NR>& s, int j, double (*
 }
 
 template <int NW, int NR>
-__global__ void __launch_bounds__(32 * NW) k_apply_q(const ApplyQTask* tasks, const int* task_of, ApplyQTask one) {
+__global__ void __launch_bounds__(32 * NW) k_apply_q(const ApplyQTask* tasks, const int* task_of, ApplyQTask one, int first) {
   constexpr int RP = 8 * NW;  // rows per pass
   extern __shared__ __align__(16) unsigned char aq_smem[];
   __shared__ double s_red[2][NW][4];
   const int tid = threadIdx.x;
   ApplyQTask t = one;
-  int col = blockIdx.x;
+  int col = first + blockIdx.x;
   if (tasks) {
-    t = tasks[task_of[blockIdx.x]];
+    t = tasks[task_of[col]];
+    if (!t.D) t.D = one.D + t.off;
     col -= t.col0;
   }
   const int n = t.n;
@@ -147,12 +148,125 @@ __global__ void __launch_bounds__(32 * NW) k_apply_q(const ApplyQTask* tasks, co
   }
 }
 
+// ------------------------------------------------------- one warp per column
+// With enough columns to fill the GPU a warp takes a whole column, eight rows a
+// pass: the products meet inside the warp (6 FP64 instructions per reflector
+// instead of 9, against 8 per pass), four columns share each reflector in
+// shared memory. NP passes; segments of U passes.
+template <int NP>
+struct WarpState {
+  double x[NP];
+  const double* wsrc;  // this thread's component of w: wsrc[2 (r + j ld)]
+  double* ring;
+  int n, rl, k, buf;
+  int64_t ld;
+  unsigned cs, us;
+};
+constexpr int AW = 4;  // warps (columns) per CTA
+template <int NP>
+__device__ __forceinline__ void aw_fetch(const WarpState<NP>& s, int j, double (&wn)[(NP + AW - 1) / AW]) {
+  const int r0 = threadIdx.x >> 2;
+  const double* a = s.wsrc + 2 * (int64_t)(j >= 0 ? j : 0) * s.ld;
+#pragma unroll
+  for (int i = 0; i < (NP + AW - 1) / AW; ++i) {
+    const int r = r0 + 8 * AW * i;
+    wn[i] = (j >= 0 && r > j && r < s.n) ? __ldg(a + 2 * r) : 0.0;
+  }
+}
+template <int NP>
+__device__ __forceinline__ void aw_stage(const WarpState<NP>& s, int buf, const double (&wn)[(NP + AW - 1) / AW]) {
+  double* w = s.ring + (size_t)buf * (32 * NP) + threadIdx.x;
+#pragma unroll
+  for (int i = 0; i < (NP + AW - 1) / AW; ++i)
+    if ((threadIdx.x >> 2) + 8 * AW * i < 8 * NP) w[32 * AW * i] = wn[i];
+}
+template <int NP, int U, int S>
+__device__ __forceinline__ void aw_segment(WarpState<NP>& s, int j, double (&wn)[(NP + AW - 1) / AW]) {
+  constexpr int I0 = S * U;  // first pass of this segment's reflectors
+  for (; j >= 0 && j >= 8 * I0 - 1; --j) {
+    const W4* w = reinterpret_cast<const W4*>(s.ring + (size_t)s.buf * (32 * NP)) + s.rl;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int i = I0; i < NP; ++i) {
+      const W4 wv = w[8 * i];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) acc[q] = fma(wv.v[q], s.x[i], acc[q]);
+    }
+    double c = signed_by(acc[0], s.cs & 1u);
+#pragma unroll
+    for (int q = 1; q < 4; ++q) c += signed_by(__shfl_xor_sync(0xffffffffu, acc[q], q), (s.cs >> q) & 1u);
+#pragma unroll
+    for (int o = 16; o >= 4; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    const int nb = s.buf == 2 ? 0 : s.buf + 1;
+    aw_stage<NP>(s, nb, wn);
+    aw_fetch<NP>(s, j - 2, wn);
+    double u[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) u[q] = signed_by(__shfl_xor_sync(0xffffffffu, c, q), ((s.us >> q) & 1u) ^ 1u);
+#pragma unroll
+    for (int i = I0; i < NP; ++i) {
+      const W4 wv = w[8 * i];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) s.x[i] = fma(wv.v[q], u[q], s.x[i]);
+    }
+    __syncthreads();  // the next reflector is staged; buffer nb + 1 is free in every warp
+    s.buf = nb;
+  }
+  if constexpr (S > 0) aw_segment<NP, U, S - 1>(s, j, wn);
+}
+
+// CTA: four consecutive columns of one matrix (the last CTA of a matrix may
+// have idle warps, which still take part in the staging)
+template <int NP, int U>
+__global__ void __launch_bounds__(32 * AW) k_apply_q_warp(const ApplyQTask* tasks, const int2* blocks, double2* base) {
+  extern __shared__ __align__(16) unsigned char aq_smem[];
+  const int2 bl = blocks[blockIdx.x];  // (task, first column)
+  ApplyQTask t = tasks[bl.x];
+  if (!t.D) t.D = base + t.off;
+  const int n = t.n, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int col = bl.y + warp;
+  const bool live = col < n;
+  WarpState<NP> s;
+  s.n = n; s.ld = t.ld; s.k = lane & 3; s.rl = lane >> 2; s.buf = 0;
+  s.cs = c_signs(s.k); s.us = u_signs(s.k);
+  s.ring = reinterpret_cast<double*>(aq_smem);
+  s.wsrc = reinterpret_cast<const double*>(t.D + (s.k < 2 ? 0 : n)) + (s.k & 1);
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const int r = s.rl + 8 * i;
+    s.x[i] = live && r < n ? t.phi[4 * r + s.k] * t.Z[r + (int64_t)col * t.ldz] : 0.0;
+  }
+  double wn[(NP + AW - 1) / AW];
+  aw_fetch<NP>(s, n - 3, wn);
+  aw_stage<NP>(s, 0, wn);
+  aw_fetch<NP>(s, n - 4, wn);
+  __syncthreads();
+  aw_segment<NP, U, (NP - 1) / U>(s, n - 3, wn);
+  if (!live) return;
+  double* X = reinterpret_cast<double*>(t.D + (s.k < 2 ? 0 : n) + (int64_t)(n + col) * t.ld) + (s.k & 1);
+#pragma unroll
+  for (int i = 0; i < NP; ++i) {
+    const int r = s.rl + 8 * i;
+    if (r < n) X[2 * r] = s.x[i];
+  }
+}
+
+template <int NP, int U>
+int launch_warp(const ApplyQTask* tasks, const int2* blocks, double2* base, int count, cudaStream_t st) {
+  constexpr int smem = 3 * (int)sizeof(W4) * 8 * NP;
+  static_assert(smem <= 47 * 1024, "shared memory");
+  k_apply_q_warp<NP, U><<<count, 32 * AW, smem, st>>>(tasks, blocks, base);
+  ZQ_LAUNCH_CHECK();
+  return ZQ_OK;
+}
+
 // (U; V) from the right half into the left half, (-conj V; conj U) in its place
-__global__ void k_apply_q_finish(const ApplyQTask* tasks, const int* task_of, ApplyQTask one) {
+__global__ void k_apply_q_finish(const ApplyQTask* tasks, const int* task_of, ApplyQTask one, int first) {
   ApplyQTask t = one;
-  int col = blockIdx.x;
+  int col = first + blockIdx.x;
   if (tasks) {
-    t = tasks[task_of[blockIdx.x]];
+    t = tasks[task_of[col]];
+    if (!t.D) t.D = one.D + t.off;
     col -= t.col0;
   }
   double2* L = t.D + (int64_t)col * t.ld;
@@ -167,7 +281,8 @@ __global__ void k_apply_q_finish(const ApplyQTask* tasks, const int* task_of, Ap
 }
 
 template <int NW, int NR>
-int launch(const ApplyQTask* tasks, const int* task_of, const ApplyQTask& one, int cols, cudaStream_t st) {
+int launch(const ApplyQTask* tasks, const int* task_of, const ApplyQTask& one, int first, int cols,
+           cudaStream_t st) {
   constexpr int smem = 3 * (int)sizeof(W4) * 8 * NW * NR;
   if (smem > 47 * 1024) {
     static std::atomic<unsigned long long> set{0};
@@ -179,34 +294,52 @@ int launch(const ApplyQTask* tasks, const int* task_of, const ApplyQTask& one, i
       set.fetch_or(bit);
     }
   }
-  k_apply_q<NW, NR><<<cols, 32 * NW, smem, st>>>(tasks, task_of, one);
+  k_apply_q<NW, NR><<<cols, 32 * NW, smem, st>>>(tasks, task_of, one, first);
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }
 
 }  // namespace
 
-int apply_q(const ApplyQTask* tasks, const int* task_of, const ApplyQTask& one, int cols, int nmax, cudaStream_t st) {
+int apply_q(const ApplyQTask* tasks, const int* task_of, const ApplyQTask& one, int first, int cols, int nmax,
+            cudaStream_t st) {
   if (cols <= 0 || nmax <= 0) return ZQ_OK;
   int rc;
   // rows in registers: the smallest count that holds the largest order. One
   // warp per column up to 64 rows (no block barrier), four above
-  if (nmax <= 16) rc = launch<1, 2>(tasks, task_of, one, cols, st);
-  else if (nmax <= 32) rc = launch<1, 4>(tasks, task_of, one, cols, st);
-  else if (nmax <= 64) rc = launch<4, 2>(tasks, task_of, one, cols, st);
-  else if (nmax <= 96) rc = launch<4, 3>(tasks, task_of, one, cols, st);
-  else if (nmax <= 128) rc = launch<4, 4>(tasks, task_of, one, cols, st);
-  else if (nmax <= 192) rc = launch<4, 6>(tasks, task_of, one, cols, st);
-  else if (nmax <= 256) rc = launch<4, 8>(tasks, task_of, one, cols, st);
-  else if (nmax <= 320) rc = launch<4, 10>(tasks, task_of, one, cols, st);
-  else if (nmax <= 384) rc = launch<4, 12>(tasks, task_of, one, cols, st);
-  else if (nmax <= 448) rc = launch<4, 14>(tasks, task_of, one, cols, st);
-  else if (nmax <= 512) rc = launch<4, 16>(tasks, task_of, one, cols, st);
-  else if (nmax <= 640) rc = launch<4, 20>(tasks, task_of, one, cols, st);
-  else if (nmax <= APPLYQ_MAX) rc = launch<4, 25>(tasks, task_of, one, cols, st);
+  if (nmax <= 16) rc = launch<1, 2>(tasks, task_of, one, first, cols, st);
+  else if (nmax <= 32) rc = launch<1, 4>(tasks, task_of, one, first, cols, st);
+  else if (nmax <= 64) rc = launch<4, 2>(tasks, task_of, one, first, cols, st);
+  else if (nmax <= 96) rc = launch<4, 3>(tasks, task_of, one, first, cols, st);
+  else if (nmax <= 128) rc = launch<4, 4>(tasks, task_of, one, first, cols, st);
+  else if (nmax <= 192) rc = launch<4, 6>(tasks, task_of, one, first, cols, st);
+  else if (nmax <= 256) rc = launch<4, 8>(tasks, task_of, one, first, cols, st);
+  else if (nmax <= 320) rc = launch<4, 10>(tasks, task_of, one, first, cols, st);
+  else if (nmax <= 384) rc = launch<4, 12>(tasks, task_of, one, first, cols, st);
+  else if (nmax <= 448) rc = launch<4, 14>(tasks, task_of, one, first, cols, st);
+  else if (nmax <= 512) rc = launch<4, 16>(tasks, task_of, one, first, cols, st);
+  else if (nmax <= 640) rc = launch<4, 20>(tasks, task_of, one, first, cols, st);
+  else if (nmax <= APPLYQ_MAX) rc = launch<4, 25>(tasks, task_of, one, first, cols, st);
   else return ZQ_ERR_ARG;
   if (rc) return rc;
-  k_apply_q_finish<<<cols, nmax <= 64 ? 64 : 128, 0, st>>>(tasks, task_of, one);
+  return apply_q_finish(tasks, task_of, one, first, cols, nmax, st);
+}
+
+int apply_q_warp(const ApplyQTask* tasks, const int2* blocks, int count, double2* base, int nmax, cudaStream_t st) {
+  if (count <= 0) return ZQ_OK;
+  if (nmax <= 64) return launch_warp<8, 1>(tasks, blocks, base, count, st);
+  if (nmax <= 96) return launch_warp<12, 1>(tasks, blocks, base, count, st);
+  if (nmax <= 128) return launch_warp<16, 1>(tasks, blocks, base, count, st);
+  if (nmax <= 160) return launch_warp<20, 2>(tasks, blocks, base, count, st);
+  if (nmax <= 192) return launch_warp<24, 2>(tasks, blocks, base, count, st);
+  if (nmax <= 224) return launch_warp<28, 2>(tasks, blocks, base, count, st);
+  if (nmax <= 256) return launch_warp<32, 2>(tasks, blocks, base, count, st);
+  return ZQ_ERR_ARG;
+}
+
+int apply_q_finish(const ApplyQTask* tasks, const int* task_of, const ApplyQTask& one, int first, int cols, int nmax,
+                   cudaStream_t st) {
+  k_apply_q_finish<<<cols, nmax <= 64 ? 64 : 128, 0, st>>>(tasks, task_of, one, first);
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }

@@ -61,12 +61,20 @@ __device__ __forceinline__ Quat qunit_of(const double* e, int k, double& nrm) {
   else { u.a0 = 1.0; u.a1 = 0.0; u.b0 = 0.0; u.b1 = 0.0; u.reset = 1; }
   return u;
 }
-constexpr int PH_T = 1024;
-__global__ void __launch_bounds__(PH_T) k_phase(const double* e, int n, double* offd, double* phi) {
+// Few threads: an FP64 instruction holds its SM quadrant for 64 cycles a warp, so
+// the scan's steps cost by the warps that take part (1024 threads at any order:
+// 59 us at n = 23, 78 us at n = 750; now 8 and 41 us).
+constexpr int PH_T = 256;
+__global__ void __launch_bounds__(PH_T) k_phase(const double* e, int n, double* offd, double* phi, const DcMat* mats) {
   __shared__ Quat s_q[PH_T];
-  const int t = threadIdx.x;
+  if (mats) {
+    const DcMat mt = mats[blockIdx.x];
+    n = mt.n;
+    e += 4 * (int64_t)mt.p; offd += mt.p; phi += 4 * (int64_t)mt.p;
+  }
+  const int t = threadIdx.x, T = blockDim.x;
   const int m = n - 1;                      // number of u_k
-  const int per = (m + PH_T - 1) / PH_T;
+  const int per = (m + T - 1) / T;
   const int k0 = t * per, k1 = (k0 + per < m) ? k0 + per : m;
   Quat acc{1.0, 0.0, 0.0, 0.0, 0};
   for (int k = k0; k < k1; ++k) {
@@ -76,7 +84,7 @@ __global__ void __launch_bounds__(PH_T) k_phase(const double* e, int n, double* 
   }
   s_q[t] = acc;
   __syncthreads();
-  for (int off = 1; off < PH_T; off <<= 1) {
+  for (int off = 1; off < T && off * per < m; off <<= 1) {
     Quat v = s_q[t];
     if (t >= off) v = qcombine(v, s_q[t - off]);
     __syncthreads();
@@ -97,9 +105,19 @@ __global__ void __launch_bounds__(PH_T) k_phase(const double* e, int n, double* 
   }
 }
 
+static int phase_threads(int n) { return n <= 32 ? 32 : (n <= 256 ? 64 : (n <= 1024 ? 128 : PH_T)); }
+
 int phase_reduce(const double* e, int n, double* offd, double* phi, cudaStream_t st) {
   if (n <= 0) return ZQ_OK;
-  k_phase<<<1, PH_T, 0, st>>>(e, n, offd, phi);
+  k_phase<<<1, phase_threads(n), 0, st>>>(e, n, offd, phi, nullptr);
+  ZQ_LAUNCH_CHECK();
+  return ZQ_OK;
+}
+
+int phase_reduce_forest(const double* e, const DcMat* mats, int count, int nmax, double* offd, double* phi,
+                        cudaStream_t st) {
+  if (count <= 0) return ZQ_OK;
+  k_phase<<<count, phase_threads(nmax), 0, st>>>(e, nmax, offd, phi, mats);
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }

@@ -10,6 +10,7 @@
 #include <mutex>
 #include <vector>
 
+#include "zq_forest.h"
 #include "zq_kernels.h"
 
 namespace zq {
@@ -40,6 +41,7 @@ struct Context {
   DcPlan dc;
   RefineBuffers rb;
   BatchBuffers bb;
+  BatchForest forest;  // layout and scratch of the last batch's mid-size matrices, rebuilt when the layout changes
   // solves of this context may use cooperative launches (off for the
   // server's lanes, whose solves run beside each other)
   bool coop = true;

@@ -85,17 +85,29 @@ void grouped_launch(const DgemmDescT<R>* dev_descs, int count, int tiles, cudaSt
 int dgemm_tiles(int m, int n);
 
 // ------------------------------------------------------------------ D&C (c)
+// A node covers positions [a, b) (children [a, c) and [c, b)); position r, c of
+// its matrix lie at zoff + r + c ld of the eigenvector buffers.
 struct DcNode {
   int a, c, b;
   int K, ndefl, nrot;
   double rho, rho2;
+  long long zoff;
+  int ld, pad;
+};
+// one matrix of a forest: positions [p, p + n), eigenvalues at eig + eoff
+struct DcMat {
+  int p, n;
+  long long eoff;
 };
 struct DcWork {
   double *sd, *sz, *nd_val, *nd_z, *df_val, *df_sval, *rot_c, *rot_s, *r_tau, *r_lam, *zhat;
   int *perm, *nd_col, *df_col, *df_scol, *rot_p, *rot_j, *r_orig;
 };
 struct DcPlan {
-  int n = 0;
+  int n = 0;           // positions (the order, or the sum of the orders of a forest)
+  size_t nn = 0;       // elements of one eigenvector buffer (the sum of the squares)
+  std::vector<DcMat> mats_host;
+  std::vector<long long> zoff;  // per matrix: element (0, 0) of its block in the eigenvector buffers
   int max_depth = 0;
   std::vector<DcNode> nodes_host;
   std::vector<int> depth_off, depth_cnt, leaf_off, leaf_cnt;
@@ -107,7 +119,8 @@ struct DcPlan {
   double* Z[2] = {nullptr, nullptr};
   double* Mb = nullptr;
   double* lam[2] = {nullptr, nullptr};
-  double *dmod = nullptr, *es = nullptr, *scal = nullptr;
+  double *dmod = nullptr, *es = nullptr, *scal = nullptr;  // scal: one scale per matrix
+  DcMat* mats_dev = nullptr;
   DcWork w{};
   DcNode* nodes_dev = nullptr;
   DgemmDesc* descs_dev = nullptr;
@@ -121,12 +134,22 @@ struct DcPlan {
   int* tc_err = nullptr;  // run_single: merges of large nodes on the tensor cores (timeout flag) when set
 
   static size_t workspace_doubles(int n);
+  size_t forest_doubles() const;  // the same for a built plan of several matrices
   int build(int n);
+  // several tridiagonals at once: orders ns, eigenvalues at eoffs of the
+  // array given to run_forest
+  int build(const std::vector<int>& ns, const std::vector<long long>& eoffs);
   size_t num_nodes() const { return nodes_host.size(); }
   size_t num_descs() const { return gemm_host.size(); }
+  int gemm_cnt(int t) const {  // descriptors of depth t
+    return (t + 1 < (int)gemm_off.size() ? gemm_off[t + 1] : (int)gemm_host.size()) - gemm_off[t];
+  }
   int upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t st);
   // d (n), e (n-1) on device; lam_out (n) on device; z_out points into the workspace
   int run(const double* d, const double* e, double* lam_out, double*& z_out, cudaStream_t st);
+  // a forest: d, e indexed by position (e of a matrix's last position unused),
+  // eigenvalues to eig + eoff of each matrix, eigenvectors in Z[0]
+  int run_forest(const double* d, const double* e, double* eig, cudaStream_t st);
   // same tree with Z and the merge products in FP32 (eigenvalues and the
   // secular equation stay FP64): the refined path's decomposition
   int run_single(const double* d, const double* e, double* lam_out, float*& z_out, cudaStream_t st);
@@ -140,6 +163,9 @@ struct DcPlan {
 // phase reduction of the quaternion tridiagonal: e (4 doubles per entry) ->
 // real off-diagonal |e_k| and unit quaternions phi_k = (alpha_k, beta_k)
 int phase_reduce(const double* e, int n, double* offd, double* phi, cudaStream_t st);
+// the same for each matrix of a forest (arrays indexed by position)
+int phase_reduce_forest(const double* e, const DcMat* mats, int count, int nmax, double* offd, double* phi,
+                        cudaStream_t st);
 // X = [diag(alpha); diag(beta)] (2n x n complex, ld), then Q X by blocked reflectors
 // tc_err (FP32 only, may be null): with it, the large products run on the
 // tensor cores (zq_tc32.cu) and a pipeline-wait timeout raises *tc_err

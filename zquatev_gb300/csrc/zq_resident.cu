@@ -47,13 +47,18 @@
 #include "zq_kernels.h"
 #include "zq_resident.h"
 
+#include <algorithm>
 #include <atomic>
+#include <functional>
+#include <queue>
+#include <vector>
 
 namespace zq {
 namespace {
 
 constexpr int RT_THREADS = 256;
 constexpr int RT_WARPS = RT_THREADS / 32;
+constexpr int RT_CLUSTER = 16;  // largest cluster
 constexpr int RT_SMEM_MAX = 227 * 1024 - 1024;  // dynamic shared memory per CTA (static part below 1 KB)
 
 template <typename R> __device__ __forceinline__ Q4<R> q_zero() { return Q4<R>{R(0), R(0), R(0), R(0)}; }
@@ -638,7 +643,8 @@ __global__ void __launch_bounds__(RT_THREADS, 1) k_tri_resident(const TriArgs<R>
     __syncthreads();
     const int t = s_task;
     if (t >= a.ntasks) return;
-    const TriTask<R> tk = a.tasks[t];
+    TriTask<R> tk = a.tasks[t];
+    if (!tk.M) tk.M = a.base + tk.off;
     if (tk.n > 0) {
       ok = reduce_matrix<R, T, sizeof(R) == 8 ? 32 : 8, CL>(tk, gr, rank, a.G, rt_smem, target, a.err, a.limit);
       if (!ok) {
@@ -698,35 +704,35 @@ int rt_launch(const TriArgs<R>& a, int ctas, size_t smem, cudaStream_t st) {
   return ZQ_OK;
 }
 
-// whether a full cluster with all of the shared memory can run on this device
+// clusters of G CTAs with all of the shared memory that run at once on this device
 template <typename R, int T>
-bool cluster_available() {
-  static std::atomic<int> known[64];
+int clusters_at_once(int G) {
+  static std::atomic<int> known[64][RT_CLUSTER + 1];
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
-  int k = known[dev].load();
+  if (G < 1 || G > RT_CLUSTER || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int k = known[dev][G].load();
   if (k == 0) {
-    k = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(16);
+    cfg.gridDim = dim3((unsigned)G);
     cfg.blockDim = dim3(RT_THREADS);
     cfg.dynamicSmemBytes = RT_SMEM_MAX;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 16;
+    attr[0].val.clusterDim.x = (unsigned)G;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int clusters = 0;
-    if (rt_attr<R, T, true>() == ZQ_OK &&
-        cudaOccupancyMaxActiveClusters(&clusters, k_tri_resident<R, T, true>, &cfg) == cudaSuccess && clusters > 0)
-      k = 2;
-    else
+    if (rt_attr<R, T, true>() != ZQ_OK ||
+        cudaOccupancyMaxActiveClusters(&clusters, k_tri_resident<R, T, true>, &cfg) != cudaSuccess) {
       (void)cudaGetLastError();
-    known[dev].store(k);
+      clusters = 0;
+    }
+    k = clusters + 1;
+    known[dev][G].store(k);
   }
-  return k == 2;
+  return k - 1;
 }
 
 }  // namespace
@@ -737,7 +743,6 @@ namespace {
 // 24.0 ms with 8, 28.5 ms with 16); FP32 sweeps at 16 (n = 1023: 16.6 ms, 17.6
 // with 8, 18.6 with 32).
 template <typename R> constexpr int rt_tile_edge() { return sizeof(R) == 8 ? 8 : 16; }
-constexpr int RT_CLUSTER = 16;
 // Up to this order one cluster of 16 CTAs does the reduction: its hardware
 // barrier takes ~1000 cycles against ~2400 through L2, which outweighs having
 // fewer SMs for the tiles (FP32, n = 300: 8.0 against 8.6 ms for the whole
@@ -782,11 +787,11 @@ int tri_resident(const TridiagView<R>& v, int k0, int ctas, cudaStream_t st) {
   const int m = v.n - k0;
   constexpr int T = rt_tile_edge<R>();
   const int nt = (m + T - 1) / T, ntiles = nt * (nt + 1) / 2;
-  const bool cl = m <= rt_cluster_max<R>() && cluster_available<R, T>();
+  const bool cl = m <= rt_cluster_max<R>() && clusters_at_once<R, T>(RT_CLUSTER) > 0;
   const int most = cl ? RT_CLUSTER : ctas;
   const int G = most < ntiles ? most : ntiles;
   TriArgs<R> a{};
-  a.one = TriTask<R>{v.M, v.n, k0, v.ld, v.d, v.e, v.tau};
+  a.one = TriTask<R>{v.M, v.n, k0, v.ld, v.d, v.e, v.tau, 0};
   a.G = G; a.m_max = m;
   a.ws = reinterpret_cast<unsigned char*>(v.rws);
   a.ws_stride = 0;
@@ -806,6 +811,67 @@ int resident_ctas(int n, bool alone) {
 size_t resident_workspace_bytes(int n, size_t real_bytes) {
   const int m = n < RESIDENT_MMAX ? n : RESIDENT_MMAX;
   return tri_group_bytes(1024, m, 8, real_bytes);
+}
+
+// Time of a queue (largest order first) on clusters of G, in clock cycles: per
+// column ~12000 outside the sweep, and the sweep's tiles in rounds of one per SM
+// quadrant at 9700 (146 FP64 instructions of 64 cycles and latencies); each
+// matrix goes to the cluster that is free first. 0: G cannot hold the largest.
+static double tri_queue_cycles(const int* orders, int count, int G) {
+  constexpr int T = rt_tile_edge<double>();
+  const int clusters = clusters_at_once<double, T>(G);
+  if (count < 1 || clusters < 1 || rt_smem_bytes<double>(orders[0], T, G) > (size_t)RT_SMEM_MAX) return 0.0;
+  std::priority_queue<double, std::vector<double>, std::greater<double>> free_at;
+  for (int q = 0; q < clusters; ++q) free_at.push(0.0);
+  double end = 0.0, cost = 0.0;
+  for (int i = 0; i < count; ++i) {
+    if (i == 0 || orders[i] != orders[i - 1]) {
+      cost = 0.0;
+      for (int a = (orders[i] + T - 1) / T; a > 0; --a) {
+        const int tiles = a * (a + 1) / 2;
+        cost += T * (12000.0 + 9700.0 * ((tiles + 4 * G - 1) / (4 * G)));
+      }
+    }
+    const double t = free_at.top() + cost;
+    free_at.pop();
+    free_at.push(t);
+    end = std::max(end, t);
+  }
+  return end;
+}
+
+int tri_queue_cluster(const int* orders, int count, double* cycles) {
+  int best = 0;
+  double least = 0.0;
+  for (int G = 1; G <= RT_CLUSTER; ++G) {
+    const double c = tri_queue_cycles(orders, count, G);
+    if (c > 0.0 && (best == 0 || c < least)) { best = G; least = c; }
+  }
+  if (cycles) *cycles = least;
+  return best;
+}
+
+static size_t tri_queue_stride(int G, int m_max) {
+  return (tri_group_bytes(G, m_max, rt_tile_edge<double>(), sizeof(double)) + 255) & ~(size_t)255;
+}
+static int tri_queue_groups(int G) { return std::max(1, clusters_at_once<double, rt_tile_edge<double>()>(G)); }
+
+size_t tri_queue_bytes(int G, int m_max) { return tri_queue_stride(G, m_max) * tri_queue_groups(G); }
+
+int tri_queue(const TriTask<double>* tasks, int ntasks, double2* base, int m_max, int G, void* ws, int* queue, int* err,
+              cudaStream_t st) {
+  if (ntasks <= 0) return ZQ_OK;
+  constexpr int T = rt_tile_edge<double>();
+  TriArgs<double> a{};
+  a.tasks = tasks; a.ntasks = ntasks; a.base = base; a.queue = queue;
+  a.G = G; a.m_max = m_max;
+  a.ws = reinterpret_cast<unsigned char*>(ws);
+  a.ws_stride = tri_queue_stride(G, m_max);
+  a.err = err;
+  a.limit = pipeline_wait_cycles();
+  const int groups = std::min(ntasks, tri_queue_groups(G));
+  ZQ_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), st));
+  return rt_launch<double, T, true>(a, groups * G, rt_smem_bytes<double>(m_max, T, G), st);
 }
 
 template bool resident_fits<float>(int, int);

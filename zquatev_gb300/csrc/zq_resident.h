@@ -13,10 +13,11 @@ constexpr int RESIDENT_MMAX = 2048;  // bound of the search for the largest orde
 // one matrix: columns k0.. of an order-n reduction whose trailing block is up to date
 template <typename R>
 struct TriTask {
-  cplx<R>* M;  // [A; B], 2n x n, column-major
+  cplx<R>* M;  // [A; B], 2n x n, column-major (in a queue: null, at off from the queue's base, or a pointer)
   int n, k0;
   int64_t ld;
   double *d, *e, *tau;
+  long long off;
 };
 
 // exchange area of one group of CTAs (device memory)
@@ -55,7 +56,8 @@ __device__ __forceinline__ TriGroup<R> tri_group(unsigned char* base, int G, int
 template <typename R>
 struct TriArgs {
   TriTask<R> one;              // tasks == null: this matrix
-  const TriTask<R>* tasks;     // or a queue of them
+  const TriTask<R>* tasks;     // or a queue of them, matrices at base + off
+  cplx<R>* base;
   int ntasks;
   int* queue;                  // zeroed before the launch
   int G, m_max;                // CTAs per group; largest trailing order
@@ -64,6 +66,15 @@ struct TriArgs {
   int* err;                    // raised when a wait ran out (may be null: NaN in d only)
   long long limit;
 };
+
+// A queue of FP64 matrices (device arrays; orders at most m_max), each reduced by
+// a cluster of G CTAs; ws as tri_queue_bytes(G, m_max), queue one int.
+int tri_queue(const TriTask<double>* tasks, int ntasks, double2* base, int m_max, int G, void* ws, int* queue, int* err,
+              cudaStream_t st);
+size_t tri_queue_bytes(int G, int m_max);
+// cluster size that finishes a queue of these orders (largest first) soonest, and
+// the estimated time in clock cycles; 0: no cluster holds the largest
+int tri_queue_cluster(const int* orders, int count, double* cycles);
 
 // CTAs of a cooperative launch with one CTA per SM (0: not available)
 int sm_count();

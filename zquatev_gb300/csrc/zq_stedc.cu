@@ -49,11 +49,11 @@ __device__ __forceinline__ int dc_find_node(const DcNode* nodes, int cnt, int po
 }
 
 template <typename ZT>
-__global__ void k_dc_leaf(const DcNode* nodes, int cnt, const double* dmod, ZT* Zout, double* lamout, int n) {
+__global__ void k_dc_leaf(const DcNode* nodes, int cnt, const double* dmod, ZT* Zout, double* lamout) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= cnt) return;
   const int a = nodes[i].a;
-  Zout[a + (int64_t)a * n] = (ZT)1;
+  Zout[nodes[i].zoff + a + (int64_t)a * nodes[i].ld] = (ZT)1;
   lamout[a] = dmod[a];
 }
 
@@ -65,12 +65,14 @@ __global__ void k_dc_leaf(const DcNode* nodes, int cnt, const double* dmod, ZT* 
 // the deflated list is ranked from shared memory.
 constexpr int DC_SCAP = 8192;  // largest node staged in shared memory (20 bytes per pole)
 template <typename ZT>
-__global__ void __launch_bounds__(256) k_dc_prepare(DcNode* nodes, DcWork w, const ZT* Zin, const double* lamin, int n,
+__global__ void __launch_bounds__(256) k_dc_prepare(DcNode* nodes, DcWork w, const ZT* Zin, const double* lamin,
                                                     int scap) {
   extern __shared__ double dc_sm[];
   DcNode& nd = nodes[blockIdx.x];
   const int a = nd.a, c = nd.c, b = nd.b;
   const int m = b - a, n1 = c - a, n2 = b - c;
+  const int64_t n = nd.ld;
+  Zin += nd.zoff;
   const int tid = threadIdx.x;
   const double rho2 = 2.0 * nd.rho;
   const double rs2 = 0.70710678118654752440;
@@ -360,7 +362,7 @@ __global__ void __launch_bounds__(128) k_dc_zhat(const DcNode* nodes, int cnt, D
 
 // one CTA per column slot of every internal node: writes a full column of M
 template <typename ZT>
-__global__ void __launch_bounds__(128) k_dc_vectors(const DcNode* nodes, int cnt, DcWork w, ZT* Mb, double* lamout, int n) {
+__global__ void __launch_bounds__(128) k_dc_vectors(const DcNode* nodes, int cnt, DcWork w, ZT* Mb, double* lamout) {
   const int pos = blockIdx.x;
   const int ni = dc_find_node(nodes, cnt, pos);
   if (ni < 0) return;
@@ -383,7 +385,7 @@ __global__ void __launch_bounds__(128) k_dc_vectors(const DcNode* nodes, int cnt
     while (lo < hi) { const int mid = (lo + hi) >> 1; if (w.r_lam[a + mid] <= val) lo = mid + 1; else hi = mid; }
     outpos = i + lo;
   }
-  ZT* col = Mb + a + (int64_t)(a + outpos) * n;
+  ZT* col = Mb + nd.zoff + a + (int64_t)(a + outpos) * nd.ld;
   for (int r = tid; r < m; r += blockDim.x) col[r] = (ZT)0;
   __syncthreads();
   if (s < K) {
@@ -414,14 +416,14 @@ __global__ void __launch_bounds__(128) k_dc_vectors(const DcNode* nodes, int cnt
 
 // apply the deflation rotations (in reverse order) to every column of M
 template <typename ZT>
-__global__ void k_dc_rotate(const DcNode* nodes, int cnt, DcWork w, ZT* Mb, int n) {
+__global__ void k_dc_rotate(const DcNode* nodes, int cnt, DcWork w, ZT* Mb) {
   const int pos = blockIdx.x * blockDim.x + threadIdx.x;
   const int ni = dc_find_node(nodes, cnt, pos);
   if (ni < 0) return;
   const DcNode nd = nodes[ni];
   if (nd.nrot == 0) return;
   const int a = nd.a;
-  ZT* col = Mb + a + (int64_t)pos * n;
+  ZT* col = Mb + nd.zoff + a + (int64_t)pos * nd.ld;
   for (int r = nd.nrot - 1; r >= 0; --r) {
     const int P = w.rot_p[a + r], J = w.rot_j[a + r];
     const double c = w.rot_c[a + r], s = w.rot_s[a + r];
@@ -431,31 +433,63 @@ __global__ void k_dc_rotate(const DcNode* nodes, int cnt, DcWork w, ZT* Mb, int 
   }
 }
 
-__global__ void k_dc_scale_in(const double* d, const double* e, int n, double* dmod, double* es, const double* scal) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const double inv = (scal[0] > 0.0) ? 1.0 / scal[0] : 1.0;
-  const double el = (i > 0) ? e[i - 1] * inv : 0.0;
-  const double er = (i < n - 1) ? e[i] * inv : 0.0;
-  dmod[i] = d[i] * inv - el - er;
-  if (i < n - 1) es[i] = er;
-}
-
-__global__ void k_dc_maxabs(const double* d, const double* e, int n, double* out) {
+// Scale and tear, one block per matrix: the largest |entry| becomes 1, the
+// off-diagonals leave the diagonal.
+__global__ void k_dc_scale(const double* d, const double* e, const DcMat* mats, double* dmod, double* es, double* scal) {
   __shared__ double sh[32];
-  double m = 0.0;
+  const DcMat mt = mats[blockIdx.x];
+  const int n = mt.n;
+  d += mt.p; e += mt.p; dmod += mt.p; es += mt.p;
+  unsigned long long mb = 0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    m = fmax(m, fabs(d[i]));
-    if (i < n - 1) m = fmax(m, fabs(e[i]));
+    mb = max(mb, abs_bits(d[i]));
+    if (i < n - 1) mb = max(mb, abs_bits(e[i]));
   }
-  m = block_max(m, sh);
-  if (threadIdx.x == 0) out[0] = m;
+  const double m = block_max(bits_to_double(mb), sh);
+  if (threadIdx.x == 0) scal[blockIdx.x] = m;
+  const double inv = (m > 0.0) ? 1.0 / m : 1.0;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    const double el = (i > 0) ? e[i - 1] * inv : 0.0;
+    const double er = (i < n - 1) ? e[i] * inv : 0.0;
+    dmod[i] = d[i] * inv - el - er;
+    if (i < n - 1) es[i] = er;
+  }
 }
 
-__global__ void k_dc_unscale(double* lam, int n, const double* scal, const int* err) {
+// eigenvalues times the scale, into place (NaN when a merge product failed)
+__global__ void k_dc_unscale(const double* lam, const DcMat* mats, const double* scal, double* eig, const int* err) {
+  const DcMat mt = mats[blockIdx.y];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n && scal[0] > 0.0) lam[i] *= scal[0];
-  if (i < n && *err) lam[i] = __longlong_as_double(0x7ff8000000000000ll);
+  if (i >= mt.n) return;
+  const double s = scal[blockIdx.y];
+  const double v = lam[mt.p + i];
+  eig[mt.eoff + i] = *err ? __longlong_as_double(0x7ff8000000000000ll) : (s > 0.0 ? v * s : v);
+}
+
+// Z_node = blockdiag(Z1, Z2) M for small nodes: a thread per entry. The tiled
+// products' 64 x 64 blocks would do mostly padding here.
+template <typename ZT>
+__global__ void __launch_bounds__(256) k_dc_merge(const DcNode* nodes, int cnt, const ZT* Zin, const ZT* Mb, ZT* Zout,
+                                                  int mmax) {
+  const DcNode nd = nodes[blockIdx.x];
+  const int m = nd.b - nd.a;
+  const int64_t ld = nd.ld, o = nd.zoff + nd.a + (int64_t)nd.a * ld;
+  const int n1 = nd.c - nd.a;
+  for (int t = blockIdx.y * blockDim.x + threadIdx.x; t < m * m; t += gridDim.y * blockDim.x) {
+    const int r = t % m, c = t / m;
+    const int k0 = r < n1 ? 0 : n1, k1 = r < n1 ? n1 : m;
+    const ZT* z = Zin + o + r;
+    const ZT* mm = Mb + o + (int64_t)c * ld;
+    ZT s0 = 0, s1 = 0;
+    int k = k0;
+#pragma unroll 4
+    for (; k + 1 < k1; k += 2) {
+      s0 = fma(z[(int64_t)k * ld], mm[k], s0);
+      s1 = fma(z[(int64_t)(k + 1) * ld], mm[k + 1], s1);
+    }
+    if (k < k1) s0 = fma(z[(int64_t)k * ld], mm[k], s0);
+    Zout[o + r + (int64_t)c * ld] = s0 + s1;
+  }
 }
 
 __global__ void k_dc_setrho(DcNode* nodes, int cnt, const double* es) {
@@ -472,6 +506,10 @@ __global__ void k_dc_setrho(DcNode* nodes, int cnt, const double* es) {
 // the products are too small for their six launches (a depth of eight
 // nodes of 375: 0.34 ms on the FP64 pipe, 0.8 ms as sixteen residue products).
 constexpr int DC_CRT_MIN = 600;
+// Depths whose nodes all have at most this order: one thread per entry of the
+// merged vectors instead of the tiled products (n = 127: a tile's product took
+// 40 us on one SM; an entry takes m / 2 multiply-adds).
+constexpr int DC_MERGE_MAX = 128;
 static size_t dc_crt_doubles(int n) {
   if (n < DC_CRT_MIN) return 0;
   const int h = (n + 1) / 2;
@@ -479,23 +517,40 @@ static size_t dc_crt_doubles(int n) {
 }
 
 size_t DcPlan::workspace_doubles(int n) {
-  // Z x2, M, lam x2, dmod, es, scal + the per-position DcWork arrays
+  // Z x2, M, lam x2, dmod, es, scal + the per-position DcWork arrays, the matrix table
   const size_t nn = (size_t)n * n;
-  return 3 * nn + 2 * (size_t)n + 2 * (size_t)n + 8 + 16 * (size_t)n + dc_crt_doubles(n);
+  return 3 * nn + 2 * (size_t)n + 2 * (size_t)n + 8 + 16 * (size_t)n + 64 + dc_crt_doubles(n);
 }
 
-int DcPlan::build(int n_) {
-  n = n_;
+size_t DcPlan::forest_doubles() const {
+  return 3 * nn + 20 * (size_t)n + (1 + sizeof(DcMat) / sizeof(double)) * mats_host.size() + 72;
+}
+
+int DcPlan::build(int n_) { return build(std::vector<int>{n_}, std::vector<long long>{0}); }
+
+int DcPlan::build(const std::vector<int>& ns, const std::vector<long long>& eoffs) {
+  n = 0;
+  nn = 0;
+  mats_host.clear();
+  zoff.clear();
   nodes_host.clear();
   depth_off.clear();
   depth_cnt.clear();
   leaf_off.clear();
   leaf_cnt.clear();
-  if (n <= 0) return ZQ_OK;
-  // recursive halving, breadth first
-  struct Tmp { int a, b, depth; };
+  // recursive halving, breadth first over all trees
+  struct Tmp { int a, b, depth, mat; };
   std::vector<Tmp> all;
-  std::vector<Tmp> cur = {{0, n, 0}};
+  std::vector<Tmp> cur;
+  for (size_t q = 0; q < ns.size(); ++q) {
+    if (ns[q] <= 0) continue;
+    cur.push_back({n, n + ns[q], 0, (int)mats_host.size()});
+    mats_host.push_back(DcMat{n, ns[q], eoffs[q]});
+    zoff.push_back((long long)nn);
+    n += ns[q];
+    nn += (size_t)ns[q] * ns[q];
+  }
+  if (n <= 0) return ZQ_OK;
   int depth = 0;
   while (!cur.empty()) {
     std::vector<Tmp> nxt;
@@ -503,26 +558,35 @@ int DcPlan::build(int n_) {
       all.push_back(t);
       if (t.b - t.a > 1) {
         const int c = t.a + (t.b - t.a) / 2;
-        nxt.push_back({t.a, c, depth + 1});
-        nxt.push_back({c, t.b, depth + 1});
+        nxt.push_back({t.a, c, depth + 1, t.mat});
+        nxt.push_back({c, t.b, depth + 1, t.mat});
       }
     }
     cur.swap(nxt);
     ++depth;
   }
   max_depth = depth - 1;
-  // group by depth: internal nodes and leaves separately, each sorted by a
+  auto node = [&](const Tmp& x) {
+    DcNode nd{};
+    const DcMat& m = mats_host[x.mat];
+    nd.a = x.a; nd.b = x.b;
+    nd.c = x.b - x.a > 1 ? x.a + (x.b - x.a) / 2 : x.a;
+    nd.ld = m.n;
+    nd.zoff = zoff[x.mat] - m.p - (long long)m.p * m.n;  // positions count from the first matrix
+    return nd;
+  };
+  // group by depth (the order of `all`): internal nodes and leaves separately, each sorted by a
   depth_mmax.clear();
+  std::vector<size_t> first(max_depth + 2, all.size());
+  for (size_t q = all.size(); q-- > 0;) first[all[q].depth] = q;
   for (int t = 0; t <= max_depth; ++t) {
     depth_off.push_back((int)nodes_host.size());
     int cnt = 0, mmax = 0;
-    for (auto& x : all)
-      if (x.depth == t && x.b - x.a > 1) {
-        DcNode nd{};
-        nd.a = x.a; nd.b = x.b; nd.c = x.a + (x.b - x.a) / 2;
-        nodes_host.push_back(nd);
+    for (size_t q = first[t]; q < first[t + 1]; ++q)
+      if (all[q].b - all[q].a > 1) {
+        nodes_host.push_back(node(all[q]));
         ++cnt;
-        mmax = std::max(mmax, x.b - x.a);
+        mmax = std::max(mmax, all[q].b - all[q].a);
       }
     depth_cnt.push_back(cnt);
     depth_mmax.push_back(mmax);
@@ -530,11 +594,9 @@ int DcPlan::build(int n_) {
   for (int t = 0; t <= max_depth; ++t) {
     leaf_off.push_back((int)nodes_host.size());
     int cnt = 0;
-    for (auto& x : all)
-      if (x.depth == t && x.b - x.a == 1) {
-        DcNode nd{};
-        nd.a = x.a; nd.b = x.b; nd.c = x.a;
-        nodes_host.push_back(nd);
+    for (size_t q = first[t]; q < first[t + 1]; ++q)
+      if (all[q].b - all[q].a == 1) {
+        nodes_host.push_back(node(all[q]));
         ++cnt;
       }
     leaf_cnt.push_back(cnt);
@@ -546,17 +608,19 @@ int DcPlan::build(int n_) {
   for (int t = 0; t <= max_depth; ++t) {
     gemm_off.push_back((int)gemm_host.size());
     int tiles = 0;
-    for (int q = 0; q < depth_cnt[t]; ++q) {
+    // depths of small nodes run on k_dc_merge, without descriptors
+    for (int q = 0; q < depth_cnt[t] && depth_mmax[t] > DC_MERGE_MAX; ++q) {
       const DcNode& nd = nodes_host[depth_off[t] + q];
       const int m = nd.b - nd.a, n1 = nd.c - nd.a, n2 = nd.b - nd.c;
+      const int64_t ld = nd.ld;
       DgemmDesc top{}, bot{};
       top.m = n1; top.n = m; top.k = n1; top.alpha = 1.0; top.beta = 0.0;
       // offsets stored as element indices; converted to pointers in run()
-      top.off_a = nd.a + (int64_t)nd.a * n; top.off_b = nd.a + (int64_t)nd.a * n; top.off_c = nd.a + (int64_t)nd.a * n;
+      top.off_a = top.off_b = top.off_c = nd.zoff + nd.a + nd.a * ld;
       bot.m = n2; bot.n = m; bot.k = n2; bot.alpha = 1.0; bot.beta = 0.0;
-      bot.off_a = nd.c + (int64_t)nd.c * n; bot.off_b = nd.c + (int64_t)nd.a * n; bot.off_c = nd.c + (int64_t)nd.a * n;
-      top.lda = top.ldb = top.ldc = n;
-      bot.lda = bot.ldb = bot.ldc = n;
+      bot.off_a = nd.zoff + nd.c + nd.c * ld; bot.off_b = nd.zoff + nd.c + nd.a * ld; bot.off_c = bot.off_b;
+      top.lda = top.ldb = top.ldc = ld;
+      bot.lda = bot.ldb = bot.ldc = ld;
       top.tile0 = tiles; tiles += ceil_div(top.m, 64) * ceil_div(top.n, 64);
       bot.tile0 = tiles; tiles += ceil_div(bot.m, 64) * ceil_div(bot.n, 64);
       gemm_host.push_back(top);
@@ -570,12 +634,13 @@ int DcPlan::build(int n_) {
 // Binds device pointers into the descriptor copies and uploads everything.
 int DcPlan::upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t st) {
   base = ws;
-  const size_t nn = (size_t)n * n;
   Z[0] = ws; Z[1] = ws + nn; Mb = ws + 2 * nn;
   double* p = ws + 3 * nn;
   lam[0] = p; p += n; lam[1] = p; p += n;
   dmod = p; p += n; es = p; p += n;
-  scal = p; p += 8;
+  err = reinterpret_cast<int*>(p); p += 8;
+  scal = p; p += mats_host.size();
+  mats_dev = reinterpret_cast<DcMat*>(p); p += sizeof(DcMat) / sizeof(double) * mats_host.size();
   w.sd = p; p += n; w.sz = p; p += n;
   w.nd_val = p; p += n; w.nd_z = p; p += n;
   w.df_val = p; p += n; w.df_sval = p; p += n;
@@ -584,15 +649,14 @@ int DcPlan::upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t s
   int* ip = reinterpret_cast<int*>(p);
   w.perm = ip; ip += n; w.nd_col = ip; ip += n; w.df_col = ip; ip += n; w.df_scol = ip; ip += n;
   w.rot_p = ip; ip += n; w.rot_j = ip; ip += n; w.r_orig = ip; ip += n;
-  err = reinterpret_cast<int*>(scal + 4);
-  // after 16 n doubles of position arrays, on a 256-byte boundary of the workspace
-  crt_ws = n >= DC_CRT_MIN ? ws + ((3 * nn + 20 * (size_t)n + 8 + 31) & ~(size_t)31) : nullptr;
+  // a single matrix: after the position arrays, on a 256-byte boundary of the workspace
+  crt_ws = mats_host.size() == 1 && n >= DC_CRT_MIN ? ws + ((3 * nn + 20 * (size_t)n + 24 + 31) & ~(size_t)31) : nullptr;
   nodes_dev = dnodes;
   descs_dev = ddescs;
   // bind pointers: at depth t, A (children) lives in Z[(t+1)&1], output in Z[t&1]
   std::vector<DgemmDesc> bound = gemm_host;
   for (int t = 0; t <= max_depth; ++t) {
-    for (int q = 0; q < 2 * depth_cnt[t]; ++q) {
+    for (int q = 0; q < gemm_cnt(t); ++q) {
       DgemmDesc& d = bound[gemm_off[t] + q];
       d.A = Z[(t + 1) & 1] + d.off_a;
       d.B = Mb + d.off_b;
@@ -614,13 +678,15 @@ int DcPlan::upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t s
     f.alpha = 1.f; f.beta = 0.f;
   }
   for (int t = 0; t <= max_depth; ++t) {
-    for (int q = 0; q < 2 * depth_cnt[t]; ++q) {
+    for (int q = 0; q < gemm_cnt(t); ++q) {
       DgemmDescT<float>& d = fbound[gemm_off[t] + q];
       d.A = Zf[(t + 1) & 1] + d.off_a;
       d.B = Mbf + d.off_b;
       d.C = Zf[t & 1] + d.off_c;
     }
   }
+  if (!mats_host.empty())
+    ZQ_CUDA(cudaMemcpyAsync(mats_dev, mats_host.data(), sizeof(DcMat) * mats_host.size(), cudaMemcpyHostToDevice, st));
   if (!nodes_host.empty())
     ZQ_CUDA(cudaMemcpyAsync(dnodes, nodes_host.data(), sizeof(DcNode) * nodes_host.size(), cudaMemcpyHostToDevice, st));
   if (!bound.empty())
@@ -636,12 +702,11 @@ int DcPlan::upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t s
 template <typename ZT>
 static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, ZT* const Zb[2], ZT* Mb,
                   const DgemmDescT<ZT>* descs, cudaStream_t st) {
-  const int n = P.n;
+  const int n = P.n, nmat = (int)P.mats_host.size();
+  int nmax = 0;
+  for (const DcMat& m : P.mats_host) nmax = std::max(nmax, m.n);
   ZQ_CUDA(cudaMemsetAsync(P.err, 0, sizeof(int), st));
-  // scale, tear
-  k_dc_maxabs<<<1, 1024, 0, st>>>(d, e, n, P.scal);
-  ZQ_LAUNCH_CHECK();
-  k_dc_scale_in<<<ceil_div(n, 256), 256, 0, st>>>(d, e, n, P.dmod, P.es, P.scal);
+  k_dc_scale<<<nmat, nmax <= 256 ? 64 : 256, 0, st>>>(d, e, P.mats_dev, P.dmod, P.es, P.scal);
   ZQ_LAUNCH_CHECK();
   if (!P.nodes_host.empty()) {
     k_dc_setrho<<<ceil_div((int)P.nodes_host.size(), 256), 256, 0, st>>>(P.nodes_dev, (int)P.nodes_host.size(), P.es);
@@ -656,7 +721,7 @@ static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, 
     const double* li = P.lam[(t + 1) & 1];
     if (P.leaf_cnt[t] > 0) {
       k_dc_leaf<ZT><<<ceil_div(P.leaf_cnt[t], 128), 128, 0, st>>>(P.nodes_dev + P.leaf_off[t], P.leaf_cnt[t], P.dmod, Zo,
-                                                                    lo, n);
+                                                                    lo);
       ZQ_LAUNCH_CHECK();
     }
     const int cnt = P.depth_cnt[t];
@@ -676,23 +741,28 @@ static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, 
           attr_set.fetch_or(bit);
         }
       }
-      k_dc_prepare<ZT><<<cnt, 256, smem, st>>>(nd, P.w, Zi, li, n, scap);
+      k_dc_prepare<ZT><<<cnt, 256, smem, st>>>(nd, P.w, Zi, li, scap);
       ZQ_LAUNCH_CHECK();
     }
     k_dc_secular<<<ceil_div(n, 4), 128, 0, st>>>(nd, cnt, P.w);
     ZQ_LAUNCH_CHECK();
     k_dc_zhat<<<ceil_div(n, 4), 128, 0, st>>>(nd, cnt, P.w);
     ZQ_LAUNCH_CHECK();
-    k_dc_vectors<ZT><<<n, 128, 0, st>>>(nd, cnt, P.w, Mb, lo, n);
+    k_dc_vectors<ZT><<<n, 128, 0, st>>>(nd, cnt, P.w, Mb, lo);
     ZQ_LAUNCH_CHECK();
-    k_dc_rotate<ZT><<<ceil_div(n, 128), 128, 0, st>>>(nd, cnt, P.w, Mb, n);
+    k_dc_rotate<ZT><<<ceil_div(n, 128), 128, 0, st>>>(nd, cnt, P.w, Mb);
     ZQ_LAUNCH_CHECK();
-    if (P.gemm_tiles[t] > 0) {
+    if (P.depth_mmax[t] <= DC_MERGE_MAX) {
+      const int mm = P.depth_mmax[t];
+      const dim3 grid((unsigned)cnt, (unsigned)std::min(64, ceil_div(mm * mm, 256)));
+      k_dc_merge<ZT><<<grid, mm <= 8 ? 64 : 256, 0, st>>>(nd, cnt, Zi, Mb, Zo, mm);
+      ZQ_LAUNCH_CHECK();
+    } else if (P.gemm_tiles[t] > 0) {
       bool done = false;
       if constexpr (std::is_same<ZT, float>::value) {
         // FP32 merges of large nodes on the tensor cores (TF32 x3), one product per child
         if (P.tc_err && P.depth_mmax[t] >= 512 && fp32_products_on_tensor_cores(TC_USE_DC)) {
-          for (int q = 0; q < 2 * cnt; ++q) {
+          for (int q = 0; q < P.gemm_cnt(t); ++q) {
             const DgemmDesc& h = P.gemm_host[P.gemm_off[t] + q];
             Tc32Args g{};
             g.cplx = 0; g.m = h.m; g.n = h.n; g.nseg = 1;
@@ -710,7 +780,7 @@ static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, 
       }
       if constexpr (std::is_same<ZT, double>::value) {
         if (P.crt_ws && P.depth_mmax[t] >= DC_CRT_MIN) {
-          for (int q = 0; q < 2 * cnt; ++q) {
+          for (int q = 0; q < P.gemm_cnt(t); ++q) {
             const DgemmDesc& h = P.gemm_host[P.gemm_off[t] + q];
             if (int rc = crt_dgemm(h.m, h.n, h.k, Zi + h.off_a, h.lda, Mb + h.off_b, h.ldb, Zo + h.off_c, h.ldc, P.crt_ws,
                                    P.err, st))
@@ -720,15 +790,20 @@ static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, 
         }
       }
       if (!done) {
-        grouped_launch<ZT>(descs + P.gemm_off[t], 2 * cnt, P.gemm_tiles[t], st);
+        grouped_launch<ZT>(descs + P.gemm_off[t], P.gemm_cnt(t), P.gemm_tiles[t], st);
         ZQ_LAUNCH_CHECK();
       }
     }
   }
-  k_dc_unscale<<<ceil_div(n, 256), 256, 0, st>>>(P.lam[0], n, P.scal, P.err);
+  k_dc_unscale<<<dim3((unsigned)ceil_div(nmax, 128), (unsigned)nmat), 128, 0, st>>>(P.lam[0], P.mats_dev, P.scal, lam_out,
+                                                                                    P.err);
   ZQ_LAUNCH_CHECK();
-  ZQ_CUDA(cudaMemcpyAsync(lam_out, P.lam[0], sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
   return ZQ_OK;
+}
+
+int DcPlan::run_forest(const double* d, const double* e, double* eig, cudaStream_t st) {
+  if (n <= 0) return ZQ_OK;
+  return dc_run<double>(*this, d, e, eig, Z, Mb, descs_dev, st);
 }
 
 int DcPlan::run(const double* d, const double* e, double* lam_out, double*& z_out, cudaStream_t st) {

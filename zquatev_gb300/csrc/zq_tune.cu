@@ -112,7 +112,8 @@ struct zq_batch_plan {
   double tune_ms[4] = {0, 0, 0, 0};
   int warp_max = -1;               // switch size of the warp variant (tuned)
   double variant_ms[4] = {0, 0, 0, 0};
-  long long extent = 0;            // complex elements of D the batch touches
+  long long extent = 0;            // complex elements of D the small matrices touch
+  zq::BatchForest forest;              // the mid-size matrices (the tuned kernel solves the small ones)
   void* dev = nullptr;             // tasks | info (+ counter) | per-CTA workspace
   size_t task_bytes = 0, info_bytes = 0;
   cudaStream_t cap = nullptr;      // capture stream
@@ -193,16 +194,18 @@ int plan_capture(zq_batch_plan* p, double2* D, double* E) {
   if (p->exec) { cudaGraphExecDestroy(p->exec); p->exec = nullptr; }
   if (p->graph) { cudaGraphDestroy(p->graph); p->graph = nullptr; }
   const int ctas = std::min(p->ntask, p->ctas_per_sm * p->sms);
+  const long long before = zq_launch_count();
   ZQ_CUDA(cudaStreamBeginCapture(p->cap, cudaStreamCaptureModeThreadLocal));
-  int rc = plan_launch_direct(p, D, E, ctas, p->cap, p->warp_max);
+  int rc = p->forest.run(D, E, p->cap);
+  if (rc == ZQ_OK) rc = plan_launch_direct(p, D, E, ctas, p->cap, p->warp_max);
   cudaGraph_t g = nullptr;
   const cudaError_t ce = cudaStreamEndCapture(p->cap, &g);
-  count_launch(-1);  // capturing ran nothing; replays are counted
+  count_launch((int)(before - zq_launch_count()));  // capturing ran nothing; replays are counted
   if (rc != ZQ_OK) { if (g) cudaGraphDestroy(g); return rc; }
   if (ce != cudaSuccess) { set_last_error(ce, "cudaStreamEndCapture", __FILE__, __LINE__); return ZQ_ERR_CUDA; }
   p->graph = g;
   ZQ_CUDA(cudaGraphInstantiate(&p->exec, p->graph, 0));
-  p->gD = D; p->gE = E; p->gctas = ctas;
+  p->gD = D; p->gE = E; p->gctas = std::max(1, ctas);
   return ZQ_OK;
 }
 
@@ -253,6 +256,7 @@ zq_batch_plan* zq_batch_plan_create(int count, const int* n2s, const int* ld2s, 
   }
   const int nmax = batched_max_n();
   std::vector<int> order;
+  std::vector<int> mid;
   long long extent = 0;
   for (int b = 0; b < count; ++b) {
     const int n2 = n2s[b];
@@ -262,10 +266,13 @@ zq_batch_plan* zq_batch_plan_create(int count, const int* n2s, const int* ld2s, 
     }
     if (n2 / 2 > nmax) { set_error_message("zq_batch_plan_create: every n2 must be <= 512"); return nullptr; }
     if (n2 == 0) continue;
+    if (n2 / 2 >= FOREST_MIN) { mid.push_back(b); continue; }
     order.push_back(b);
     extent = std::max(extent, offs[b] + (long long)ld2s[b] * n2);
   }
-  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return n2s[x] > n2s[y]; });
+  const auto larger = [&](int x, int y) { return n2s[x] > n2s[y]; };
+  std::stable_sort(order.begin(), order.end(), larger);
+  std::stable_sort(mid.begin(), mid.end(), larger);
   zq_batch_plan* p = new zq_batch_plan();
   cudaGetDevice(&p->device);
   cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device);
@@ -273,7 +280,8 @@ zq_batch_plan* zq_batch_plan_create(int count, const int* n2s, const int* ld2s, 
   p->ntask = (int)order.size();
   p->extent = extent;
   p->ctas_per_sm = ctas_per_sm;
-  p->tuned = ctas_per_sm > 0;
+  p->tuned = ctas_per_sm > 0 || order.empty();
+  if (order.empty() && ctas_per_sm == 0) p->ctas_per_sm = 1;
   const size_t tb = batched_task_bytes();
   p->task_bytes = (tb * std::max(1, p->ntask) + 255) & ~(size_t)255;
   p->info_bytes = (sizeof(int) * (p->ntask + 1) + 255) & ~(size_t)255;
@@ -294,6 +302,12 @@ zq_batch_plan* zq_batch_plan_create(int count, const int* n2s, const int* ld2s, 
     delete p;
     return nullptr;
   }
+  std::vector<ForestItem> items;
+  for (int b : mid) items.push_back(ForestItem{n2s[b] / 2, ld2s[b], offs[b], eoffs[b]});
+  if (p->forest.build(items, p->cap) != ZQ_OK) {
+    zq_batch_plan_destroy(p);
+    return nullptr;
+  }
   return p;
 }
 
@@ -312,7 +326,7 @@ int zq_set_batch_warp_max(int n) {
 
 int zq_batch_plan_run(zq_batch_plan* p, double* dD, double* deig, void* stream) {
   if (!p || !dD || !deig) { set_error_message("zq_batch_plan_run: null argument"); return ZQ_ERR_ARG; }
-  if (p->ntask == 0) return ZQ_OK;
+  if (p->ntask == 0 && p->forest.empty()) return ZQ_OK;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   double2* D = reinterpret_cast<double2*>(dD);
   if (!p->tuned) {
@@ -329,11 +343,16 @@ int zq_batch_plan_run(zq_batch_plan* p, double* dD, double* deig, void* stream) 
 
 int zq_batch_plan_info(zq_batch_plan* p, void* stream) {
   if (!p) return ZQ_ERR_ARG;
-  if (p->ntask == 0) return ZQ_OK;
+  if (p->ntask == 0 && p->forest.empty()) return ZQ_OK;
   std::vector<int> h(p->ntask);
+  int herr = 0;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  ZQ_CUDA(cudaMemcpyAsync(h.data(), plan_info(p), sizeof(int) * p->ntask, cudaMemcpyDeviceToHost, st));
+  if (p->ntask > 0)
+    ZQ_CUDA(cudaMemcpyAsync(h.data(), plan_info(p), sizeof(int) * p->ntask, cudaMemcpyDeviceToHost, st));
+  if (!p->forest.empty())
+    ZQ_CUDA(cudaMemcpyAsync(&herr, p->forest.error_flag(), sizeof(int), cudaMemcpyDeviceToHost, st));
   ZQ_CUDA(cudaStreamSynchronize(st));
+  if (herr) { set_error_message("batch: a device-side wait ran out of time"); return ZQ_ERR_TIMEOUT; }
   int m = 0;
   for (int v : h) m = v > m ? v : m;
   return m;
@@ -352,7 +371,9 @@ int zq_batch_plan_destroy(zq_batch_plan* p) {
   if (p->cap) cudaStreamSynchronize(p->cap);
   if (p->exec) cudaGraphExecDestroy(p->exec);
   if (p->graph) cudaGraphDestroy(p->graph);
-  if (p->dev) { cudaDeviceSynchronize(); cudaFree(p->dev); }
+  cudaDeviceSynchronize();
+  p->forest.release();
+  if (p->dev) cudaFree(p->dev);
   if (p->cap) cudaStreamDestroy(p->cap);
   delete p;
   return ZQ_OK;
