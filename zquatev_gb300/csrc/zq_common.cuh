@@ -99,16 +99,19 @@ __device__ __forceinline__ unsigned long long absmax_bits(double2 x) {
   return a > b ? a : b;
 }
 __device__ __forceinline__ double bits_to_double(unsigned long long b) { return __longlong_as_double((long long)b); }
-// Sum over the block; every thread gets the result. `sh` needs blockDim/32 slots.
+// Sum over the block (at most 32 warps); every thread gets the result. `sh`
+// needs blockDim/32 slots. The warps' sums meet by shuffles: an FP64 add holds
+// its SM quadrant for 64 cycles, so a loop over them costs more than the steps.
 template <typename T> __device__ T block_sum(T v, T* sh) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
   v = warp_sum(v);
   __syncthreads();
   if (lane == 0) sh[wid] = v;
   __syncthreads();
-  T r = 0;
-  for (int i = 0; i < nw; ++i) r += sh[i];
-  return r;
+  T r = lane < nw ? sh[lane] : T(0);
+  for (int o = 16; o > 0; o >>= 1)
+    if (o < nw) r += __shfl_xor_sync(0xffffffffu, r, o);
+  return __shfl_sync(0xffffffffu, r, 0);
 }
 template <typename T> __device__ T block_max(T v, T* sh) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
@@ -116,9 +119,10 @@ template <typename T> __device__ T block_max(T v, T* sh) {
   __syncthreads();
   if (lane == 0) sh[wid] = v;
   __syncthreads();
-  T r = sh[0];
-  for (int i = 1; i < nw; ++i) r = fmax(r, sh[i]);
-  return r;
+  T r = sh[lane < nw ? lane : 0];
+  for (int o = 16; o > 0; o >>= 1)
+    if (o < nw) r = fmax(r, __shfl_xor_sync(0xffffffffu, r, o));
+  return __shfl_sync(0xffffffffu, r, 0);
 }
 
 // ----------------------------------------------------------------------------

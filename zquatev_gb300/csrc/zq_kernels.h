@@ -24,7 +24,7 @@ struct TridiagView {
   int nbmax;
   cplx<R>* ga;     // g of the current column (n)
   cplx<R>* gb;
-  cplx<R>* hpart;  // hemv tile partials: hblk x hblk x 64 x 4
+  cplx<R>* hpart;  // hemv tile partials: hblk x hblk x 32 x 2
   int hblk;
   cplx<R>* dpart;  // panel dot partials, one set per 128 rows: hblk x nbmax x 4 (room for 4x that)
   cplx<R>* dots;   // the summed panel dot products: 4 * nbmax
@@ -38,7 +38,6 @@ struct TridiagView {
   int* tc_err;     // FP32: tensor-core products allowed (their timeout flag); null: CUDA cores only
   void* rws;       // exchange area of the resident reduction (zq_resident.cu)
   int ctas;        // CTAs it may use (0: the per-column kernels only)
-  int coop;        // 1: the FP32 panels may run as one cooperative launch each (no other solve runs beside it)
 };
 
 template <typename R>
@@ -200,7 +199,7 @@ struct RefineArgs {
   double pair_eps_late;        // the same bound in the later steps
   int slices0;                 // Ozaki slices of the first step's products
   int slices_res;              // Ozaki slices of the products with the residual R = HX - X Lambda
-  int coop;                    // the FP32 reduction may use cooperative panel launches
+  int coop;                    // no other solve runs beside this one: the FP32 reduction may take every SM
   cudaStream_t st;
   cudaStream_t st2;            // second stream: Q formation overlaps the tridiagonal solve
   cudaEvent_t ev_fork, ev_join;

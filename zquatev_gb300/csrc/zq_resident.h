@@ -2,11 +2,9 @@
 #pragma once
 
 #include "zq_kernels.h"
+#include "zq_quat.cuh"
 
 namespace zq {
-
-// four reals: (a.x, a.y, b.x, b.y) of a quaternion entry
-template <typename R> struct alignas(16) Q4 { R ax, ay, bx, by; };
 
 constexpr int RESIDENT_MMAX = 2048;  // bound of the search for the largest order that fits
 

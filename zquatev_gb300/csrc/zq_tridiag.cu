@@ -134,12 +134,6 @@ template <typename R>
 __device__ void head_write(const TridiagView<R>& v, int j, double f, const double (&m)[4], const double (&ee)[4]) {
   v.scal[4] = f;
   for (int q = 0; q < 4; ++q) v.scal[5 + q] = m[q] * f;
-  // the same head rounded to R once (scal[12..15] as floats): the FP32 kernels
-  // then read it without double-precision conversions
-  float* hf = reinterpret_cast<float*>(v.scal + 12);
-  hf[0] = (float)f;
-  for (int q = 0; q < 4; ++q) hf[1 + q] = (float)(m[q] * f);
-  hf[5] = (f > 0.0) ? 1.f : 0.f;
   for (int q = 0; q < 4; ++q) v.e[4 * j + q] = ee[q];
   v.tau[j] = (f > 0.0) ? 1.0 : 0.0;
 }
@@ -150,6 +144,57 @@ __device__ void reflector_head(const TridiagView<R>& v, int j, int nnp) {
   if (head_math(v, j, nnp, f, m, ee)) head_write(v, j, f, m, ee);
 }
 
+// FP32 columns: squares of floats neither overflow nor vanish in double, so the
+// partials are plain sums of squares, and the scalars come from two reciprocal
+// square roots (with ss = |x|^2, q2 = |x_1|^2: g = sqrt(ss q2) = |x||x_1|,
+// s = |x|/|x_1| = ss / g, f = 1 / sqrt(ss + g)): ~25 dependent FP64 instructions
+// instead of ~130, each ~75 cycles here. The four components of m and e are
+// formed by four lanes.
+template <>
+__device__ void reflector_head<float>(const TridiagView<float>& v, int j, int nnp) {
+  const int lane = threadIdx.x;
+  const int L = v.n - 1 - j;
+  if (lane >= 32 || L < 1) return;  // the last column has no subdiagonal entry
+  const double x1 = __ldcg(v.scal + (lane & 3));
+  double ss = 0.0;
+  for (int i = lane; i < nnp; i += 128) {  // four loads in flight
+    double p[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) p[u] = i + 32 * u < nnp ? __ldcg(v.npart + 2 * (i + 32 * u) + 1) : 0.0;
+    ss += (p[0] + p[1]) + (p[2] + p[3]);
+  }
+  double q2 = x1 * x1;
+  q2 += __shfl_xor_sync(0xffffffffu, q2, 1);
+  q2 += __shfl_xor_sync(0xffffffffu, q2, 2);
+  ss = warp_sum(ss);
+  double f = 0.0, m = 0.0, ee = x1;   // L == 1: the entry itself is e_j
+  if (L >= 2) {
+    const double t = ss * q2;
+    if (t > 0.0) {
+      const double rg = rsqrt(t);
+      const double s = ss * rg;
+      f = rsqrt(fma(t, rg, ss));
+      m = x1 * fma(f, s, f);
+      ee = -s * x1;
+    } else if (ss > 0.0) {           // x_1 = 0
+      f = rsqrt(ss);
+      m = (lane & 3) == 0 ? 1.0 : 0.0;
+      ee = (lane & 3) == 0 ? -ss * f : 0.0;
+    } else {
+      ee = ss == 0.0 ? 0.0 : ss;     // nothing to reduce (or not a number: keep it visible)
+    }
+  }
+  if (lane >= 4) return;
+  float* hf = reinterpret_cast<float*>(v.scal + 12);
+  hf[1 + lane] = (float)m;
+  v.e[4 * j + lane] = ee;
+  if (lane == 0) {
+    hf[0] = (float)f;
+    hf[5] = (f > 0.0) ? 1.f : 0.f;
+    v.tau[j] = (f > 0.0) ? 1.0 : 0.0;
+  }
+}
+
 // the reflector head in the kernel's precision: f, f m (4 reals), and whether
 // a reflector exists (f > 0)
 template <typename R>
@@ -157,20 +202,6 @@ struct WHead {
   R f, m[4];
   bool live;
 };
-
-// The FP32 head of column j formed by warp 0 of every CTA of the persistent
-// panel kernel from the norm partials (the same arithmetic as reflector_head,
-// so every CTA gets the same bits); CTA 0 also writes it to memory (the
-// subdiagonal entry and tau are used after the reduction). Lane 0 stores the
-// head in *out.
-__device__ void reflector_head_all(const TridiagView<float>& v, int j, int nnp, WHead<float>* out, bool write) {
-  double f, m[4], ee[4];
-  if (!head_math(v, j, nnp, f, m, ee)) return;
-  if (write) head_write(v, j, f, m, ee);
-  out->f = (float)f;
-  for (int q = 0; q < 4; ++q) out->m[q] = (float)(m[q] * f);
-  out->live = f > 0.0;
-}
 
 __device__ __forceinline__ void load_head(const TridiagView<float>& v, WHead<float>& h) {
   const float* hf = reinterpret_cast<const float*>(v.scal + 12);
@@ -199,10 +230,9 @@ __device__ __forceinline__ void w_from_x(const WHead<R>& h, int r, int j, cplx<R
 // ----------------------------------------------------------------------------
 // colupd: rows [j, n) of column j
 // ----------------------------------------------------------------------------
-// Row block `bid` (rows j + RB bid ..) of column j with NTH threads; writes
-// the block's norm partials npart[2 bid], npart[2 bid + 1]. Returns false when
-// do_update is 0 (only y_{k-1} finished). Used by k_colupd (one CTA per row
-// block) and by the persistent panel kernel.
+// Row block `bid` (rows j + RB bid ..) of column j; writes the block's norm
+// partials npart[2 bid], npart[2 bid + 1]. Returns false when do_update is 0
+// (only y_{k-1} finished).
 template <typename R, int NTH>
 __device__ bool colupd_block(const TridiagView<R>& v, int p, int j, int k, int ncp, int do_update, int bid) {
   constexpr int NGR = NTH / RB;  // reflector groups
@@ -298,7 +328,6 @@ __device__ bool colupd_block(const TridiagView<R>& v, int p, int j, int k, int n
   s_red[grp][row][1] = db;
   __syncthreads();
 
-  double sc = 0.0;  // local max-abs of x (rows >= j+1)
   Z xa = czero<Z>(), xb = czero<Z>();
   if (grp == 0 && r < n) {
     Z ta = s_red[0][row][0], tb = s_red[0][row][1];
@@ -313,22 +342,35 @@ __device__ bool colupd_block(const TridiagView<R>& v, int p, int j, int k, int n
       v.scal[2] = (double)xb.x; v.scal[3] = (double)xb.y;
       __threadfence();  // before this CTA's arrival is counted
     }
-    if (r > j) {
-      sc = fmax(fmax(fabs((double)xa.x), fabs((double)xa.y)), fmax(fabs((double)xb.x), fabs((double)xb.y)));
+  }
+  if constexpr (std::is_same<R, float>::value) {
+    // the rows lie in warp 0; plain squares (see reflector_head<float>)
+    if (tid < 32) {
+      double ss = 0.0;
+      if (r < n && r > j) {
+        const double a0 = xa.x, a1 = xa.y, b0 = xb.x, b1 = xb.y;
+        ss = fma(a0, a0, a1 * a1) + fma(b0, b0, b1 * b1);
+      }
+      ss = warp_sum(ss);
+      if (tid == 0) v.npart[2 * bid + 1] = ss;
     }
-  }
-  // scaled sum of squares (LAPACK lassq style, combined across CTAs in reflect)
-  const double bmax = block_max(sc, s_red_d[0]);
-  double ss = 0.0;
-  if (grp == 0 && r < n && r > j && bmax > 0.0) {
-    const double inv = 1.0 / bmax;
-    const double a0 = xa.x * inv, a1 = xa.y * inv, b0 = xb.x * inv, b1 = xb.y * inv;
-    ss = a0 * a0 + a1 * a1 + b0 * b0 + b1 * b1;
-  }
-  const double bss = block_sum(ss, s_red_d[1]);
-  if (tid == 0) {
-    v.npart[2 * bid + 0] = bmax;
-    v.npart[2 * bid + 1] = bss;
+  } else {
+    double sc = 0.0;  // local max-abs of x (rows >= j+1)
+    if (grp == 0 && r < n && r > j)
+      sc = fmax(fmax(fabs((double)xa.x), fabs((double)xa.y)), fmax(fabs((double)xb.x), fabs((double)xb.y)));
+    // scaled sum of squares (LAPACK lassq style, combined across CTAs in reflect)
+    const double bmax = block_max(sc, s_red_d[0]);
+    double ss = 0.0;
+    if (grp == 0 && r < n && r > j && bmax > 0.0) {
+      const double inv = 1.0 / bmax;
+      const double a0 = xa.x * inv, a1 = xa.y * inv, b0 = xb.x * inv, b1 = xb.y * inv;
+      ss = a0 * a0 + a1 * a1 + b0 * b0 + b1 * b1;
+    }
+    const double bss = block_sum(ss, s_red_d[1]);
+    if (tid == 0) {
+      v.npart[2 * bid + 0] = bmax;
+      v.npart[2 * bid + 1] = bss;
+    }
   }
   return true;
 }
@@ -359,8 +401,7 @@ __global__ void __launch_bounds__(NT) k_colupd(TridiagView<R> v, int p, int j, i
 // ----------------------------------------------------------------------------
 constexpr int DR = 128;       // rows per dot-partial CTA
 template <typename R>
-__device__ void panel_dots(const TridiagView<R>& v, int p, int j, int k, int b, int ndot, cplx<R>* scratch,
-                           const WHead<R>* hd = nullptr) {
+__device__ void panel_dots(const TridiagView<R>& v, int p, int j, int k, int b, int ndot, cplx<R>* scratch) {
   using Z = cplx<R>;
   const int n = v.n;
   const int64_t ld = v.ld;
@@ -372,7 +413,7 @@ __device__ void panel_dots(const TridiagView<R>& v, int p, int j, int k, int b, 
   WHead<R> h;
   Z xa = czero<Z>(), xb = czero<Z>();
   if (live) {
-    if (hd) h = *hd; else load_head(v, h);
+    load_head(v, h);
     xa = A[gr + (int64_t)j * ld];
     xb = B[gr + (int64_t)j * ld];
   }
@@ -453,331 +494,141 @@ __device__ void panel_dots(const TridiagView<R>& v, int p, int j, int k, int b, 
 
 // ----------------------------------------------------------------------------
 // hemv: quaternion Hermitian mat-vec of the panel-start trailing matrix.
-//   Region rows/cols [r0, n); lower-triangle 32x32 tiles, one CTA per tile
-//   after the first ndot CTAs, which form the panel dot partials.
-//   The A and B tiles are staged in shared memory (padded, conflict-free for
-//   both row and column sweeps) and four warps each own one product:
-//     warp 0: rows,  A x and A z          warp 2: columns, A^H x and A^H z
-//     warp 1: rows,  B x and B z          warp 3: columns, -B^T x and -B^T z
-//   (x = wa, z = conj(wb)), so every lower-triangle element is read once from
-//   HBM and used for its row and its (conjugate-)transposed column without any
-//   cross-thread reduction: all FP64 work is DFMA. Per T-row block R and source
-//   block S the CTA stores the partial sums of v0 = A x, v1 = A z, v2 = B x,
-//   v3 = B z.
+//   Region rows/cols [b0, n); lower-triangle 32x32 tiles, one warp per tile,
+//   after the first ndot CTAs, which form the panel dot partials. b0 is j + 1,
+//   or the even row below it where pairs of rows are read at once (PAIR: FP32,
+//   even n, 16-byte loads); row b0 < j + 1 then carries w = 0 and its output is
+//   not read.
+//   Lane (tr, tc) = (lane & 7, lane >> 3) owns four rows and eight columns of
+//   the tile, read straight into registers; each element is used for its row
+//   and its (conjugate-)transposed column, and the lanes' sums meet by halving
+//   exchanges. Per row block and source block one partial (ga, gb) per row is
+//   stored. A diagonal tile reads both triangles from the lower one and forms row
+//   products only.
+//   Bound: the matrix is read once per column (HBM above ~n = 3600, L2 below);
+//   n = 4096, cold: column 0 134 MB in 31.8 us, column 2400 25 MB in 11.6 us. The
+//   earlier form (tile in shared memory by TMA, a warp per product, products not
+//   yet combined) was issue-bound at 1780 instructions of each of four warps per
+//   tile against ~1300 of one here: 36.2 and 11.4 us, with twice the partial sums
+//   for k_hreduce to read. Four CTAs per SM: 128 registers with a few spills in
+//   the edge tiles beat 156 without (51.9 against 53.7 ms over the reduction).
 // ----------------------------------------------------------------------------
 constexpr int HT = 32;        // hemv tile edge
-constexpr int HLD = HT + 1;   // padded shared leading dimension
-template <typename R>
-__global__ void __launch_bounds__(128) k_hemv(TridiagView<R> v, int p, int j, int k, int ndot) {
+constexpr int HW = 4;         // tiles (warps) per CTA
+template <typename R, bool PAIR>
+__global__ void __launch_bounds__(32 * HW, sizeof(R) == 4 ? 4 : 2) k_hemv(TridiagView<R> v, int p, int j, int k, int ndot, int b0, int ntiles) {
   pdl_wait();  // launched with launch_pdl: the previous kernel's results first
   using Z = cplx<R>;
-  const int n = v.n;
-  const int64_t ld = v.ld;
-  const Z* A = v.M;
-  const Z* B = v.M + n;
-  const int r0 = j + 1;
-  __shared__ Z sAB[2 * HT * HLD];   // the A and B tiles (also the dot CTAs' scratch: 4 warps x 128 x 4)
-  Z* sA = sAB;
-  Z* sB = sAB + HT * HLD;
-  __shared__ Z sx[2][HT], sz[2][HT];   // [0]: rows of block I, [1]: rows of block J
-  __shared__ Z sout[HT][4];
-  // the first ndot CTAs form the panel dot partials (they start first and run
-  // beside the tiles); sAB (2 HT HLD >= 4 warps x 128 x 4) is their scratch
+  // scratch of the dot CTAs (4 warps x k <= NBMAX x 4); the tile CTAs keep w of
+  // their rows and columns there
+  __shared__ __align__(16) Z s_buf[4 * NBMAX * 4];
   if ((int)blockIdx.x < ndot) {
-    panel_dots(v, p, j, k, blockIdx.x, ndot, sA);
+    panel_dots(v, p, j, k, blockIdx.x, ndot, s_buf);
     return;
   }
-  const int t = blockIdx.x - ndot;
-  int I, J;
-  tri_tile(t, I, J);
-  const bool diag = (I == J);
-  const int tid = threadIdx.x;
-  const int rbase = r0 + I * HT, cbase = r0 + J * HT;
-  // all of this thread's loads are issued before any is used: 8 elements of
-  // each tile (one column of 32 rows per warp and step: coalesced), the two
-  // w segments and the reflector head
-  constexpr int PER = HT * HT / 128;
-  Z ta[PER], tb[PER];
-#pragma unroll
-  for (int u = 0; u < PER; ++u) {
-    const int e = tid + 128 * u;
-    const int r = e & (HT - 1), c = e >> 5;
-    const int gr = rbase + r, gc = cbase + c;
-    ta[u] = czero<Z>(); tb[u] = czero<Z>();
-    if (gr < n && gc < n && (!diag || r >= c)) {
-      // streaming loads (evict first): the trailing matrix passes through L2
-      // once per column, the tile partials written below are read next
-      ta[u] = __ldcs(A + gr + (int64_t)gc * ld);
-      tb[u] = __ldcs(B + gr + (int64_t)gc * ld);
-    }
-  }
-  const int ws = tid >> 5, wq = tid & (HT - 1);
-  const int wg = (ws == 0 ? rbase : cbase) + wq;
-  const bool wrow = tid < 2 * HT && wg < n;
-  Z x = czero<Z>(), z = czero<Z>();
-  WHead<R> h;
-  if (wrow) {
-    load_head(v, h);
-    x = A[wg + (int64_t)j * ld];
-    z = B[wg + (int64_t)j * ld];
-  }
-#pragma unroll
-  for (int u = 0; u < PER; ++u) {
-    const int e = tid + 128 * u;
-    const int r = e & (HT - 1), c = e >> 5;
-    if (diag && r == c) { ta[u].y = 0; tb[u] = czero<Z>(); }
-    sA[r + c * HLD] = ta[u];
-    sB[r + c * HLD] = tb[u];
-  }
-  if (tid < 2 * HT) {
-    if (wrow) {
-      w_from_x<R>(h, wg, j, x, z);
-      z = cconj(z);
-    }
-    sx[ws][wq] = x;
-    sz[ws][wq] = z;
-  }
-  __syncthreads();
-  const int role = tid >> 5, q = tid & (HT - 1);
-  // two accumulators per product (even / odd k) for independent FMA chains
-  Z p0 = czero<Z>(), p1 = czero<Z>(), p2 = czero<Z>(), p3 = czero<Z>();
-  if (role < 2) {
-    const Z* S = role == 0 ? sA : sB;
-#pragma unroll 8
-    for (int c = 0; c < HT; c += 2) {
-      const Z m0 = S[q + c * HLD], m1 = S[q + (c + 1) * HLD];
-      cfma(p0, m0, sx[1][c]); cfma(p1, m0, sz[1][c]);
-      cfma(p2, m1, sx[1][c + 1]); cfma(p3, m1, sz[1][c + 1]);
-    }
-  } else if (role == 2) {
-    // column q: rows above q are zero in a diagonal tile; the diagonal itself
-    // belongs to the row products
-#pragma unroll
-    for (int r = 0; r < HT; r += 2) {
-      Z m0 = sA[r + q * HLD], m1 = sA[r + 1 + q * HLD];
-      if (diag && r == q) m0 = czero<Z>();
-      if (diag && r + 1 == q) m1 = czero<Z>();
-      cfmac(p0, m0, sx[0][r]); cfmac(p1, m0, sz[0][r]);
-      cfmac(p2, m1, sx[0][r + 1]); cfmac(p3, m1, sz[0][r + 1]);
-    }
-  } else {
-#pragma unroll
-    for (int r = 0; r < HT; r += 2) {
-      Z m0 = sB[r + q * HLD], m1 = sB[r + 1 + q * HLD];
-      if (diag && r == q) m0 = czero<Z>();
-      if (diag && r + 1 == q) m1 = czero<Z>();
-      cfma(p0, m0, sx[0][r]); cfma(p1, m0, sz[0][r]);
-      cfma(p2, m1, sx[0][r + 1]); cfma(p3, m1, sz[0][r + 1]);
-    }
-    p0 = cneg(p0); p1 = cneg(p1); p2 = cneg(p2); p3 = cneg(p3);
-  }
-  const Z u0 = cadd(p0, p2), u1 = cadd(p1, p3);   // this warp's two products
-  const int nbm = v.hblk;
-  if (role >= 2) {
-    if (diag) { sout[q][2 * (role - 2)] = u0; sout[q][2 * (role - 2) + 1] = u1; }
-    else {
-      Z* o = v.hpart + (((int64_t)J * nbm + I) * HT + q) * 4 + 2 * (role - 2);
-      o[0] = u0; o[1] = u1;
-    }
-  }
-  if (diag) __syncthreads();
-  if (role < 2) {
-    Z a0 = u0, a1 = u1;
-    if (diag) { a0 = cadd(a0, sout[q][2 * role]); a1 = cadd(a1, sout[q][2 * role + 1]); }
-    Z* o = v.hpart + (((int64_t)I * nbm + J) * HT + q) * 4 + 2 * role;
-    o[0] = a0; o[1] = a1;
-  }
-}
-
-// ----------------------------------------------------------------------------
-// hemv, FP32 with TMA staging (even n): the same products and partial layout
-// as k_hemv, but
-//   * the A and B tiles arrive by cp.async.bulk.tensor: each 32 x 32 complex
-//     tile is two 16-row boxes (128 bytes of rows, 128-byte swizzle, zeros
-//     outside the matrix) issued by one thread, completed on an mbarrier;
-//   * the tile grid starts at the even row b0 = r0 - (r0 & 1), as a TMA box
-//     must start on a 16-byte boundary; row / column b0 < r0 carries w = 0 and
-//     its output is not read (k_hreduce is told the shift);
-//   * a complex multiply-add m v is two packed FP32 FMAs on the natural pair
-//     (m.x, m.y): P += (m.x, m.y) (v.x, v.x), Q += (m.x, m.y) (v.y, v.y), and
-//     m v = (P.x - Q.y, P.y + Q.x), conj(m) v = (P.x + Q.y, Q.x - P.y), so the
-//     vectors are kept in shared memory as (v.x, v.x, v.y, v.y).
-// Warp roles as k_hemv: 0 A rows, 1 B rows, 2 A^H columns, 3 -B^T columns.
-// ----------------------------------------------------------------------------
-constexpr int HM_SMEM = 16384 + 1024;  // two tiles (8 KB each) + alignment
-__device__ __forceinline__ void fma2(float2& acc, float2 a, float2 b) {
-  asm("{\n\t.reg .b64 ra, rb, rc;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\tmov.b64 rc, {%0, %1};\n\t"
-      "fma.rn.f32x2 rc, ra, rb, rc;\n\tmov.b64 {%0, %1}, rc;\n\t}"
-      : "+f"(acc.x), "+f"(acc.y)
-      : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-}
-__device__ __forceinline__ float2 lds2(uint32_t a) {
-  float2 v;
-  asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a));
-  return v;
-}
-
-// One work item of the TMA hemv grid with 128 threads: items < ndot are panel
-// dot partials, the others lower-triangle tiles. `tiles` is a 1024-aligned
-// 16 KB shared buffer, `bar` an initialised mbarrier whose next phase has
-// parity `par`; `hd` the reflector head when the caller holds it. Returns
-// false if the tile copy did not arrive within the wait limit.
-__device__ bool hemv_tma_item(const CUtensorMap* tmp, const TridiagView<float>& v, int p, int j, int k, int ndot, int b0,
-                              int item, uint32_t tiles, unsigned char* tiles_gen, uint32_t bar, uint32_t par,
-                              const WHead<float>* hd) {
-  using Z = float2;
-  __shared__ float4 s_xd[2][HT], s_zd[2][HT];       // [0]: block I rows, [1]: block J rows
-  __shared__ Z sout[HT][4];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int t = (blockIdx.x - ndot) * HW + warp;
+  if (t >= ntiles) return;
   const int n = v.n;
   const int64_t ld = v.ld;
   const Z* A = v.M;
   const Z* B = v.M + n;
-  if (item < ndot) {
-    panel_dots(v, p, j, k, item, ndot, reinterpret_cast<Z*>(tiles_gen), hd);
-    return true;
-  }
-  const int t = item - ndot;
   int I, J;
   tri_tile(t, I, J);
   const bool diag = (I == J);
-  const int tid = threadIdx.x;
   const int rbase = b0 + I * HT, cbase = b0 + J * HT;
-  if (tid == 0) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(16384u) : "memory");
-    const uint64_t tma = reinterpret_cast<uint64_t>(tmp);
+  const int tr = lane & 7, tc = lane >> 3;
+  // row i of this lane's four: pairs of consecutive rows in the PAIR form
+  auto row_of = [&](int i) { return PAIR ? 16 * (i >> 1) + 2 * tr + (i & 1) : tr + 8 * i; };
+  constexpr int CB = sizeof(R) == 4 ? 4 : 2;  // columns whose loads are in flight together
+  Q4<R> m[CB][4];
+  // inside the matrix and off the diagonal: unconditional loads from one base
+  const bool inner = !diag && rbase + HT <= n;
+  const Z* a0 = A + rbase + (int64_t)(cbase + tc) * ld;
+  auto load_inner = [&](int c0) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int x = (q >= 2 ? n : 0) + rbase + 16 * (q & 1);   // row: even (b0, n even)
-      asm volatile(
-          "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
-              tiles + 4096u * q),
-          "l"(tma), "r"(x), "r"(cbase), "r"(bar)
-          : "memory");
-    }
-  }
-  // meanwhile: w on the rows of block I (column products) and block J (row products)
-  if (tid < 2 * HT) {
-    const int ws = tid >> 5, wq = tid & (HT - 1);
-    const int wg = (ws == 0 ? rbase : cbase) + wq;
-    Z x = czero<Z>(), z = czero<Z>();
-    if (wg > j && wg < n) {
-      WHead<float> h;
-      if (hd) h = *hd; else load_head(v, h);
-      x = A[wg + (int64_t)j * ld];
-      z = B[wg + (int64_t)j * ld];
-      w_from_x<float>(h, wg, j, x, z);
-      z = cconj(z);
-    }
-    s_xd[ws][wq] = make_float4(x.x, x.x, x.y, x.y);
-    s_zd[ws][wq] = make_float4(z.x, z.x, z.y, z.y);
-  }
-  __syncthreads();
-  {
-    // bounded wait for the tiles (the copies take microseconds)
-    const long long t0 = clock64();
-    uint32_t ok = 0;
-    while (!ok) {
-      asm volatile(
-          "{\n\t.reg .pred pp;\n\tmbarrier.try_wait.parity.shared::cta.b64 pp, [%1], %2;\n\tselp.u32 %0, 1, 0, pp;\n\t}"
-          : "=r"(ok)
-          : "r"(bar), "r"(par)
-          : "memory");
-      if (!ok && clock64() - t0 > 4000000000LL) break;
-    }
-    if (!__syncthreads_and(ok != 0)) {
-      if (tid == 0 && v.tc_err) atomicExch(v.tc_err, 1);
-      return false;
-    }
-  }
-  const int role = tid >> 5, q = tid & (HT - 1);
-  Z P0 = czero<Z>(), Q0 = czero<Z>(), P1 = czero<Z>(), Q1 = czero<Z>();
-  if (role < 2) {
-    // row q of the tile, all 32 columns: element (q, c) of a swizzled 16-row box
-    // sits at box * 4096 + c * 128 + (((q & 15) >> 1) ^ (c & 7)) * 16 + (q & 1) * 8
-    const uint32_t rowb = tiles + (uint32_t)role * 8192u + (uint32_t)(q >> 4) * 4096u + (uint32_t)(q & 1) * 8u;
-    const int hr = (q & 15) >> 1;
-    if (!diag) {
+    for (int q = 0; q < CB; ++q) {
+      const Z* a = a0 + (int64_t)(4 * (c0 + q)) * ld;
+      if constexpr (PAIR) {
 #pragma unroll
-      for (int c = 0; c < HT; ++c) {
-        const float2 m = lds2(rowb + (uint32_t)c * 128u + (uint32_t)((hr ^ (c & 7)) << 4));
-        const float4 xd = s_xd[1][c], zd = s_zd[1][c];
-        fma2(P0, m, make_float2(xd.x, xd.y)); fma2(Q0, m, make_float2(xd.z, xd.w));
-        fma2(P1, m, make_float2(zd.x, zd.y)); fma2(Q1, m, make_float2(zd.z, zd.w));
-      }
-    } else {
-      for (int c = 0; c <= q; ++c) {
-        float2 m = lds2(rowb + (uint32_t)c * 128u + (uint32_t)((hr ^ (c & 7)) << 4));
-        if (c == q) { if (role == 0) m.y = 0.f; else m = czero<Z>(); }  // real diagonal of A, zero of B
-        const float4 xd = s_xd[1][c], zd = s_zd[1][c];
-        fma2(P0, m, make_float2(xd.x, xd.y)); fma2(Q0, m, make_float2(xd.z, xd.w));
-        fma2(P1, m, make_float2(zd.x, zd.y)); fma2(Q1, m, make_float2(zd.z, zd.w));
-      }
-    }
-  } else {
-    // column q, all 32 rows r: element (r, q) at (r >> 4) * 4096 + q * 128 + (((r & 15) >> 1) ^ (q & 7)) * 16 + (r & 1) * 8
-    const uint32_t colb = tiles + (uint32_t)(role - 2) * 8192u + (uint32_t)q * 128u;
-    const int hq = q & 7;
-    if (!diag) {
+        for (int u = 0; u < 2; ++u) {
+          const float4 x = __ldg(reinterpret_cast<const float4*>(a + 16 * u + 2 * tr));
+          const float4 y = __ldg(reinterpret_cast<const float4*>(a + n + 16 * u + 2 * tr));
+          m[q][2 * u] = Q4<R>{x.x, x.y, y.x, y.y};
+          m[q][2 * u + 1] = Q4<R>{x.z, x.w, y.z, y.w};
+        }
+      } else {
 #pragma unroll
-      for (int r = 0; r < HT; ++r) {
-        const float2 m = lds2(colb + (uint32_t)(r >> 4) * 4096u + (uint32_t)((((r & 15) >> 1) ^ hq) << 4) + (uint32_t)(r & 1) * 8u);
-        const float4 xd = s_xd[0][r], zd = s_zd[0][r];
-        fma2(P0, m, make_float2(xd.x, xd.y)); fma2(Q0, m, make_float2(xd.z, xd.w));
-        fma2(P1, m, make_float2(zd.x, zd.y)); fma2(Q1, m, make_float2(zd.z, zd.w));
+        for (int i = 0; i < 4; ++i) {
+          const Z x = __ldg(a + tr + 8 * i), y = __ldg(a + n + tr + 8 * i);
+          m[q][i] = Q4<R>{x.x, x.y, y.x, y.y};
+        }
       }
-    } else {
-      for (int r = q + 1; r < HT; ++r) {  // diagonal tile: strictly below the diagonal
-        const float2 m = lds2(colb + (uint32_t)(r >> 4) * 4096u + (uint32_t)((((r & 15) >> 1) ^ hq) << 4) + (uint32_t)(r & 1) * 8u);
-        const float4 xd = s_xd[0][r], zd = s_zd[0][r];
-        fma2(P0, m, make_float2(xd.x, xd.y)); fma2(Q0, m, make_float2(xd.z, xd.w));
-        fma2(P1, m, make_float2(zd.x, zd.y)); fma2(Q1, m, make_float2(zd.z, zd.w));
+    }
+  };
+  // elements of the diagonal tiles (above the diagonal from below it) and of the last row block
+  auto load_edge = [&](int c0) {
+#pragma unroll
+    for (int q = 0; q < CB; ++q) {
+      const int gc = cbase + tc + 4 * (c0 + q);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int gr = rbase + row_of(i);
+        const int r = min(gr, n - 1), c = min(gc, n - 1);
+        const bool low = r >= c;
+        const int64_t o = low ? r + (int64_t)c * ld : c + (int64_t)r * ld;
+        const Z x = __ldg(A + o), y = __ldg(B + o);
+        // selects, not branches: the loads are in flight together
+        const bool in = gr < n && gc < n, off = in && r != c;
+        m[q][i].ax = in ? x.x : R(0);
+        m[q][i].ay = off ? (low ? x.y : -x.y) : R(0);
+        m[q][i].bx = off ? (low ? y.x : -y.x) : R(0);
+        m[q][i].by = off ? (low ? y.y : -y.y) : R(0);
+      }
+    }
+  };
+  if (inner) load_inner(0); else load_edge(0);
+  // w on the tile's rows and columns: one of each per lane, shared in the warp
+  Q4<R>* sw = reinterpret_cast<Q4<R>*>(s_buf) + warp * 2 * HT;
+  WHead<R> h;
+  load_head(v, h);
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int g = (q ? cbase : rbase) + lane, gl = g < n ? g : n - 1;
+    Z wa = A[gl + (int64_t)j * ld], wb = B[gl + (int64_t)j * ld];
+    w_from_x<R>(h, g, j, wa, wb);
+    if (g <= j || g >= n) { wa = czero<Z>(); wb = czero<Z>(); }
+    q_store(sw + q * HT + lane, Q4<R>{wa.x, wa.y, wb.x, wb.y});
+  }
+  __syncwarp();
+  R rs[16], cs[32];
+#pragma unroll
+  for (int q = 0; q < 16; ++q) rs[q] = R(0);
+#pragma unroll
+  for (int q = 0; q < 32; ++q) cs[q] = R(0);
+#pragma unroll
+  for (int c0 = 0; c0 < 8; c0 += CB) {
+    if (c0 > 0) {
+      if (inner) load_inner(c0); else load_edge(c0);
+    }
+#pragma unroll
+    for (int q = 0; q < CB; ++q) {
+      const Q4<R> wc = sw[HT + tc + 4 * (c0 + q)];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        row_prod(rs + 4 * i, m[q][i], wc);
+        col_prod(cs + 4 * (c0 + q), m[q][i], sw[row_of(i)]);
       }
     }
   }
-  // this warp's two products
-  Z u0, u1;
-  if (role < 2) {            // m v
-    u0 = mk(P0.x - Q0.y, P0.y + Q0.x); u1 = mk(P1.x - Q1.y, P1.y + Q1.x);
-  } else if (role == 2) {    // conj(m) v
-    u0 = mk(P0.x + Q0.y, Q0.x - P0.y); u1 = mk(P1.x + Q1.y, Q1.x - P1.y);
-  } else {                   // -m v
-    u0 = mk(Q0.y - P0.x, -(P0.y + Q0.x)); u1 = mk(Q1.y - P1.x, -(P1.y + Q1.x));
+  Q4<R>* part = reinterpret_cast<Q4<R>*>(v.hpart);
+  scatter_sum<16, 16, 8, R>(rs, lane);   // over the column lanes: lane tc is left with row tc
+  q_store(part + ((int64_t)I * v.hblk + J) * HT + row_of(tc), Q4<R>{rs[0], rs[1], rs[2], rs[3]});
+  if (!diag) {
+    scatter_sum<32, 4, 1, R>(cs, lane);  // over the row lanes: lane tr is left with column tr
+    q_store(part + ((int64_t)J * v.hblk + I) * HT + tc + 4 * tr, Q4<R>{cs[0], cs[1], cs[2], cs[3]});
   }
-  const int nbm = v.hblk;
-  if (role >= 2) {
-    if (diag) { sout[q][2 * (role - 2)] = u0; sout[q][2 * (role - 2) + 1] = u1; }
-    else {
-      Z* o = v.hpart + (((int64_t)J * nbm + I) * HT + q) * 4 + 2 * (role - 2);
-      o[0] = u0; o[1] = u1;
-    }
-  }
-  if (diag) __syncthreads();
-  if (role < 2) {
-    Z a0 = u0, a1 = u1;
-    if (diag) { a0 = cadd(a0, sout[q][2 * role]); a1 = cadd(a1, sout[q][2 * role + 1]); }
-    Z* o = v.hpart + (((int64_t)I * nbm + J) * HT + q) * 4 + 2 * role;
-    o[0] = a0; o[1] = a1;
-  }
-  return true;
 }
-
-__global__ void __launch_bounds__(128) k_hemv_tma(const __grid_constant__ CUtensorMap tm, TridiagView<float> v, int p,
-                                                  int j, int k, int ndot, int b0) {
-  pdl_wait();  // launched with launch_pdl: the previous kernel's results first
-  extern __shared__ __align__(1024) unsigned char hm_raw[];
-  const uint32_t raw = (uint32_t)__cvta_generic_to_shared(hm_raw);
-  const uint32_t tiles = (raw + 1023u) & ~1023u;    // A tile at +0, B tile at +8192
-  __shared__ __align__(8) unsigned long long s_bar;
-  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_bar);
-  if ((int)blockIdx.x >= ndot && threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  }
-  hemv_tma_item(&tm, v, p, j, k, ndot, b0, (int)blockIdx.x, tiles, hm_raw + (tiles - raw), bar, 0u, nullptr);
-}
-
-
 
 // ----------------------------------------------------------------------------
 // hreduce: g = H_panelstart w - corrections, for rows [j+1, n); c partials;
@@ -789,13 +640,13 @@ __global__ void __launch_bounds__(128) k_hemv_tma(const __grid_constant__ CUtens
 //   depend on one another are issued before the first is used.
 // ----------------------------------------------------------------------------
 constexpr int HRB = 8;                 // rows per CTA
-// Row block `bid` (rows j + 1 + HRB bid ..) with NTH threads; `hd` is the
-// reflector head when the caller holds it (null: read from scal).
-template <typename R, int NTH>
-__device__ void hreduce_block(const TridiagView<R>& v, int p, int j, int k, int T, int nblk, int zero_mode, int sh,
-                              int bid, const WHead<R>* hd) {
-  constexpr int HNG = NTH / HRB;          // reflector groups for the corrections
-  constexpr int NSPL = NTH / (4 * HRB);   // threads per (row, product) for the tile partials
+template <typename R>
+__global__ void __launch_bounds__(NT) k_hreduce(TridiagView<R> v, int p, int j, int k, int T, int nblk, int zero_mode,
+                                                int sh) {
+  pdl_wait();  // launched with launch_pdl: the previous kernel's results first
+  constexpr int HNG = NT / HRB;           // reflector groups for the corrections
+  constexpr int NSPL = NT / (2 * HRB);    // threads per (row, part) for the tile partials
+  const int bid = (int)blockIdx.x;        // rows j + 1 + HRB bid ..
   using Z = cplx<R>;
   const int n = v.n;
   const int64_t ld = v.ld;
@@ -805,16 +656,15 @@ __device__ void hreduce_block(const TridiagView<R>& v, int p, int j, int k, int 
   const int tid = threadIdx.x;
   const int row = tid & (HRB - 1), grp = tid / HRB;
   const int r = r0 + bid * HRB + row;
-  __shared__ Z s_v[HRB][4];
+  __shared__ Z s_v[HRB][2];
   __shared__ Z s_dots[4 * NBMAX];
-  __shared__ Z s_part[NSPL][4 * HRB];
+  __shared__ Z s_part[NSPL][2 * HRB];
   __shared__ Z s_red[HNG][HRB][2];
-  __shared__ double s_redd[NTH / 32];
   // this row's x and the reflector head (w = f x is written in place at the end)
   WHead<R> h;
   Z xa = czero<Z>(), xb = czero<Z>();
   if (grp == 0 && r < n) {
-    if (hd) h = *hd; else load_head(v, h);
+    load_head(v, h);
     xa = A[r + (int64_t)j * ld];
     xb = B[r + (int64_t)j * ld];
   }
@@ -826,14 +676,14 @@ __device__ void hreduce_block(const TridiagView<R>& v, int p, int j, int k, int 
       cya = v.Ya[r + (int64_t)grp * v.ldy]; cyb = v.Yb[r + (int64_t)grp * v.ldy];
     }
     if (tid < 4 * k) dt = v.dots[tid];
-    // tile partials: output o = (row, product); split sp sums blocks S = sp, sp + NSPL, ...
-    const int o = tid & (4 * HRB - 1), sp = tid / (4 * HRB);
-    const int lr = bid * HRB + (o >> 2);
+    // tile partials: output o = (row, ga or gb); split sp sums blocks S = sp, sp + NSPL, ...
+    const int o = tid & (2 * HRB - 1), sp = tid / (2 * HRB);
+    const int lr = bid * HRB + (o >> 1);
     Z s0 = czero<Z>(), s1 = czero<Z>(), s2 = czero<Z>(), s3 = czero<Z>();
     if (r0 + lr < n) {
       const int Rb = (lr + sh) / T, off = (lr + sh) % T;  // the hemv tile grid starts sh rows above r0
-      const Z* base = v.hpart + (((int64_t)Rb * v.hblk) * T + off) * 4 + (o & 3);
-      const int64_t stride = (int64_t)T * 4;
+      const Z* base = v.hpart + (((int64_t)Rb * v.hblk) * T + off) * 2 + (o & 1);
+      const int64_t stride = (int64_t)T * 2;
       int S = sp;
 #pragma unroll 2
       for (; S + 3 * NSPL < nblk; S += 4 * NSPL) {
@@ -845,14 +695,14 @@ __device__ void hreduce_block(const TridiagView<R>& v, int p, int j, int k, int 
     }
     s_part[sp][o] = cadd(cadd(s0, s2), cadd(s1, s3));
     if (tid < 4 * k) s_dots[tid] = dt;
-    for (int q = tid + NTH; q < 4 * k; q += NTH) s_dots[q] = v.dots[q];  // wide panels
+    for (int q = tid + NT; q < 4 * k; q += NT) s_dots[q] = v.dots[q];  // wide panels
   }
   __syncthreads();
-  if (!zero_mode && tid < 4 * HRB) {
+  if (!zero_mode && tid < 2 * HRB) {
     Z t = s_part[0][tid];
 #pragma unroll
     for (int u = 1; u < NSPL; ++u) t = cadd(t, s_part[u][tid]);
-    s_v[tid >> 2][tid & 3] = t;
+    s_v[tid >> 1][tid & 1] = t;
   }
   // deferred-update corrections, reflectors split over the groups
   Z ta = czero<Z>(), tb = czero<Z>();
@@ -881,9 +731,8 @@ __device__ void hreduce_block(const TridiagView<R>& v, int p, int j, int k, int 
     B[r + (int64_t)j * ld] = wb;
     Z ga = czero<Z>(), gb = czero<Z>();
     if (!zero_mode) {
-      // ha = A x - conj(B z), hb = B x + conj(A z)
-      ga = csub(s_v[row][0], cconj(s_v[row][3]));
-      gb = cadd(s_v[row][2], cconj(s_v[row][1]));
+      ga = s_v[row][0];
+      gb = s_v[row][1];
       const int ng = k < HNG ? k : HNG;   // groups that hold a correction
       for (int g2 = 0; g2 < ng; ++g2) { ga = csub(ga, s_red[g2][row][0]); gb = csub(gb, s_red[g2][row][1]); }
       cp = (double)(wa.x * ga.x + wa.y * ga.y + wb.x * gb.x + wb.y * gb.y);
@@ -891,15 +740,11 @@ __device__ void hreduce_block(const TridiagView<R>& v, int p, int j, int k, int 
     v.ga[r] = ga;
     v.gb[r] = gb;
   }
-  const double bs = block_sum(cp, s_redd);
-  if (tid == 0) v.cpart[bid] = bs;
-}
-
-template <typename R>
-__global__ void __launch_bounds__(NT) k_hreduce(TridiagView<R> v, int p, int j, int k, int T, int nblk, int zero_mode,
-                                                int sh) {
-  pdl_wait();  // launched with launch_pdl: the previous kernel's results first
-  hreduce_block<R, NT>(v, p, j, k, T, nblk, zero_mode, sh, (int)blockIdx.x, nullptr);
+  if (tid < 32) {  // the rows lie in the first eight lanes
+#pragma unroll
+    for (int o = HRB / 2; o > 0; o >>= 1) cp += __shfl_xor_sync(0xffffffffu, cp, o);
+    if (tid == 0) v.cpart[bid] = cp;
+  }
 }
 
 // ----------------------------------------------------------------------------
@@ -1042,16 +887,6 @@ __global__ void __launch_bounds__(NT) k_trail(TridiagView<R> v, int p, int nbp, 
   }
 }
 
-// TMA-staged FP32 hemv on (default) or the register-staged k_hemv (environment
-// ZQ_HEMV=ldg)
-static bool hemv_tma_enabled() {
-  static const bool on = [] {
-    const char* e = getenv("ZQ_HEMV");
-    return !(e && !strcmp(e, "ldg"));
-  }();
-  return on;
-}
-
 // The same trailing update on the tensor cores (zq_tc32.cu), FP32 path, used
 // only where ZQ_TC32_USES names it: the lower triangles of the (n - t0)^2
 // trailing blocks of A and B take one rank-4 nbp product each,
@@ -1104,135 +939,6 @@ static int trail_tc32(const TridiagView<float>& v, int p, int nbp, int t0, cudaS
 
 
 // ----------------------------------------------------------------------------
-// Persistent panel kernel (FP32 with the TMA mat-vec; opt-in, ZQ_TRIDIAG=persist):
-// the columns of one panel in a single cooperative launch. Per column the
-// three phases of the kernel sequence above (colupd row blocks, hemv items,
-// hreduce row blocks) run as loops over the resident CTAs with a grid barrier
-// after each, and every CTA forms the reflector head itself after the first
-// barrier: 3 nb barriers instead of 3 nb launches. Measured slower than the
-// launches at every size (FP32 reduction at n2 = 1024 / 4096 / 8192: 12.6-14.3
-// / 64-69 / 198-265 ms with 1-6 CTAs per SM, against 11.6 / 53.2 / 156.4 ms):
-// a grid barrier costs about what a dependent launch does, and a fixed grid
-// streams the mat-vec tiles more slowly than thousands of one-tile CTAs.
-// ----------------------------------------------------------------------------
-constexpr int PT = 128;  // threads per CTA of the persistent panel kernel
-constexpr int PT_SMEM = 1024 + 16384;  // 1024-aligned 16 KB tile buffer
-
-// Grid barrier of the persistent kernel (cooperative launch: every CTA is
-// resident). counter[2] counts arrivals, counter[3] is the generation,
-// counter[4] the abort flag. A wait longer than `limit` cycles raises the
-// abort flag and tc_err, after which every barrier returns at once (false).
-__device__ bool grid_barrier(const TridiagView<float>& v, long long limit) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    volatile unsigned* gen = v.counter + 3;
-    volatile unsigned* abt = v.counter + 4;
-    int ok = *abt == 0u;
-    if (ok) {
-      const unsigned g0 = *gen;  // read before arriving: it cannot advance until this CTA arrives
-      __threadfence();
-      if (atomicAdd(v.counter + 2, 1u) == gridDim.x - 1) {
-        atomicExch(v.counter + 2, 0u);
-        __threadfence();
-        atomicAdd(v.counter + 3, 1u);
-      } else {
-        const long long t0 = clock64();
-        while (*gen == g0) {
-          __nanosleep(64);  // back off: hundreds of CTAs poll the same line
-          if (*abt) { ok = 0; break; }
-          if (clock64() - t0 > limit) {
-            atomicExch(v.counter + 4, 1u);
-            if (v.tc_err) atomicExch(v.tc_err, 1);
-            ok = 0;
-            break;
-          }
-        }
-      }
-      __threadfence();
-    }
-    s_ok = ok;
-  }
-  __syncthreads();
-  return s_ok != 0;
-}
-
-__global__ void __launch_bounds__(PT, 4) k_panel_persist(const __grid_constant__ CUtensorMap tm, TridiagView<float> v,
-                                                      int p, int nbp, long long limit) {
-  extern __shared__ __align__(1024) unsigned char pp_raw[];
-  const uint32_t raw = (uint32_t)__cvta_generic_to_shared(pp_raw);
-  const uint32_t tiles = (raw + 1023u) & ~1023u;
-  __shared__ __align__(8) unsigned long long s_bar;
-  __shared__ WHead<float> s_head;
-  const uint32_t bar = (uint32_t)__cvta_generic_to_shared(&s_bar);
-  if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  uint32_t par = 0;  // parity of the tile barrier's next phase
-  const int n = v.n, G = (int)gridDim.x, cta = (int)blockIdx.x;
-  int ncp = 0;
-  for (int k = 0; k < nbp; ++k) {
-    const int j = p + k, L = n - 1 - j;
-    const int ncta1 = ceil_div(n - j, RB);
-    for (int rb = cta; rb < ncta1; rb += G) colupd_block<float, PT>(v, p, j, k, ncp, 1, rb);
-    if (!grid_barrier(v, limit)) return;
-    if (L < 1) { ncp = 0; continue; }
-    reflector_head_all(v, j, ncta1, &s_head, cta == 0);
-    __syncthreads();
-    const int b0 = (j + 1) & ~1, sh = (j + 1) - b0;
-    const int nblk = ceil_div(n - b0, HT);
-    if (L >= 2) {
-      const int ndot = (k > 0) ? ceil_div(L, DR) : 0;
-      const int items = ndot + nblk * (nblk + 1) / 2;
-      for (int it = cta; it < items; it += G) {
-        // the tile buffer was read by this CTA's threads (generic proxy) before
-        // the copy of this item writes it (async proxy)
-        if (threadIdx.x == 0) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        const bool ok = hemv_tma_item(&tm, v, p, j, k, ndot, b0, it, tiles, pp_raw + (tiles - raw), bar, par, &s_head);
-        if (it >= ndot) par ^= 1u;
-        __syncthreads();
-        if (!ok) {
-          if (threadIdx.x == 0) atomicExch(v.counter + 4, 1u);
-          return;
-        }
-      }
-      if (!grid_barrier(v, limit)) return;
-    }
-    const int nhr = ceil_div(L, HRB);
-    for (int rb = cta; rb < nhr; rb += G)
-      hreduce_block<float, PT>(v, p, j, k, HT, nblk, L < 2 ? 1 : 0, sh, rb, &s_head);
-    if (!grid_barrier(v, limit)) return;
-    ncp = nhr;
-  }
-}
-
-// CTAs of the persistent panel kernel (0: use the per-column kernels). Only
-// with ZQ_TRIDIAG=persist; the grid is every SM times min(occupancy,
-// ZQ_PANEL_CTAS_PER_SM, default 4).
-static int panel_persist_grid() {
-  static int grid = -1;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    grid = 0;
-    const char* m = getenv("ZQ_TRIDIAG");
-    if (!m || strcmp(m, "persist")) return;
-    int dev = 0, sms = 0, coop = 0, occ = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return;
-    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) return;
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return;
-    if (cudaFuncSetAttribute(k_panel_persist, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM) != cudaSuccess) return;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_panel_persist, PT, PT_SMEM) != cudaSuccess) return;
-    int per = 4;
-    if (const char* e = getenv("ZQ_PANEL_CTAS_PER_SM")) per = atoi(e);
-    if (per > occ) per = occ;
-    grid = per > 0 ? per * sms : 0;
-  });
-  return grid;
-}
-
-// ----------------------------------------------------------------------------
 // host driver
 // ----------------------------------------------------------------------------
 template <typename R>
@@ -1241,52 +947,19 @@ int tridiagonalize(TridiagView<R> v, int nb, cudaStream_t st) {
   if (n <= 0) return ZQ_OK;
   if (nb > v.nbmax) nb = v.nbmax;
   if (nb < 1) nb = 1;
-  ZQ_CUDA(cudaMemsetAsync(v.counter, 0, 5 * sizeof(unsigned), st));
-  // FP32 with even n: the hemv tiles come by TMA from one tensor map over [A; B]
-  // (2n x n, 8-byte elements, 16 x 32 boxes, 128-byte swizzle, zeros outside)
-  bool use_tma = false;
-  CUtensorMap hemv_map;
-  if (std::is_same<R, float>::value && (n % 2) == 0 && n >= 4 && hemv_tma_enabled()) {
-    using Enc = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                             const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                             CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-    auto enc = reinterpret_cast<Enc>(tensor_map_encode_fn());
-    const cuuint64_t dims[2] = {(cuuint64_t)2 * n, (cuuint64_t)n};
-    const cuuint64_t strides[1] = {(cuuint64_t)v.ld * 8};
-    const cuuint32_t box[2] = {16u, (cuuint32_t)HT};
-    const cuuint32_t es[2] = {1u, 1u};
-    use_tma = enc && (reinterpret_cast<uintptr_t>(v.M) % 16) == 0 && (v.ld % 2) == 0 &&
-              enc(&hemv_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 2, const_cast<void*>(reinterpret_cast<const void*>(v.M)),
-                  dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-  }
+  ZQ_CUDA(cudaMemsetAsync(v.counter, 0, 2 * sizeof(unsigned), st));
+  // FP32 with even n: rows are read in aligned pairs (A and B both start on a
+  // 16-byte boundary in every column)
+  const bool pair = std::is_same<R, float>::value && (n % 2) == 0 && (v.ld % 2) == 0 &&
+                    (reinterpret_cast<uintptr_t>(v.M) % 16) == 0;
   int ncp = 0;  // number of c partials of the previous column
-  const int pgrid = (use_tma && v.coop) ? panel_persist_grid() : 0;
   // the last columns (all of them for orders that fit) run with the trailing
   // block held in shared memory
-  const int rmax = pgrid > 0 ? 0 : resident_max<R>(v.ctas);
+  const int rmax = resident_max<R>(v.ctas);
   for (int p = 0; p < n; p += nb) {
     if (n - p <= rmax) return tri_resident<R>(v, p, v.ctas, st);
     const int nbp = (nb < n - p) ? nb : (n - p);
-    if constexpr (std::is_same<R, float>::value) if (pgrid > 0) {
-      // the panel's columns in one cooperative launch
-      cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3((unsigned)pgrid);
-      cfg.blockDim = dim3(PT);
-      cfg.dynamicSmemBytes = PT_SMEM;
-      cfg.stream = st;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeCooperative;
-      attr[0].val.cooperative = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      const long long limit = pipeline_wait_cycles();
-      ZQ_CUDA(cudaLaunchKernelEx(&cfg, k_panel_persist, hemv_map, v, p, nbp, limit));
-      count_launch();
-      const int jl = p + nbp - 1, Ll = n - 1 - jl;
-      ncp = Ll >= 1 ? ceil_div(Ll, HRB) : 0;
-    }
-    for (int k = 0; k < nbp && pgrid == 0; ++k) {
+    for (int k = 0; k < nbp; ++k) {
       const int j = p + k;
       const int L = n - 1 - j;
       const int ncta1 = ceil_div(n - j, RB);
@@ -1295,8 +968,7 @@ int tridiagonalize(TridiagView<R> v, int nb, cudaStream_t st) {
       count_launch();
       if (L < 1) { prof_end(PC_PANEL, st); ncp = 0; continue; }
       const int T = HT;
-      // TMA-staged FP32 hemv: its tile grid starts at the even row below r0
-      const int b0 = use_tma ? ((j + 1) & ~1) : (j + 1);
+      const int b0 = pair ? ((j + 1) & ~1) : (j + 1);  // first row of the tile grid
       const int sh = (j + 1) - b0;
       const int nblk = ceil_div(n - b0, T);
       const int ndot = (k > 0 && L >= 2) ? ceil_div(L, DR) : 0;  // dot-partial CTAs of the hemv grid
@@ -1304,14 +976,12 @@ int tridiagonalize(TridiagView<R> v, int nb, cudaStream_t st) {
       if (L >= 2) {
         prof_begin(PC_HEMV, st);
         const int ntiles = nblk * (nblk + 1) / 2;
+        const dim3 grid(ceil_div(ntiles, HW) + ndot);
         if constexpr (std::is_same<R, float>::value) {
-          if (use_tma) {
-            ZQ_CUDA(launch_pdl_smem(k_hemv_tma, dim3(ntiles + ndot), dim3(128), HM_SMEM, st, hemv_map, v, p, j, k, ndot, b0));
-          } else {
-            ZQ_CUDA(launch_pdl(k_hemv<R>, dim3(ntiles + ndot), dim3(128), st, v, p, j, k, ndot));
-          }
+          if (pair) ZQ_CUDA(launch_pdl(k_hemv<R, true>, grid, dim3(32 * HW), st, v, p, j, k, ndot, b0, ntiles));
+          else ZQ_CUDA(launch_pdl(k_hemv<R, false>, grid, dim3(32 * HW), st, v, p, j, k, ndot, b0, ntiles));
         } else {
-          ZQ_CUDA(launch_pdl(k_hemv<R>, dim3(ntiles + ndot), dim3(128), st, v, p, j, k, ndot));
+          ZQ_CUDA(launch_pdl(k_hemv<R, false>, grid, dim3(32 * HW), st, v, p, j, k, ndot, b0, ntiles));
         }
         count_launch();
         prof_end(PC_HEMV, st);
@@ -1356,12 +1026,12 @@ size_t tridiag_workspace_bytes(int n, int nbmax) {
   size_t b = 0;
   b += sizeof(Z) * (2 * (size_t)n * nbmax);          // Ya, Yb
   b += sizeof(Z) * (2 * (size_t)n);                   // ga, gb
-  b += sizeof(Z) * ((hblk + 2) * (hblk + 2) * 32 * 4);  // hpart: 32-tiles, or 64-tiles at the same block stride
+  b += sizeof(Z) * ((hblk + 2) * (hblk + 2) * 32 * 2);  // hpart
   b += sizeof(Z) * (hblk * nbmax * 4);                // dpart
   b += sizeof(Z) * (4 * (size_t)nbmax);               // dots
   b += sizeof(double) * (2 * hblk + 16);              // npart (2 hblk), scal
   b += sizeof(double) * ((size_t)ceil_div(n > 0 ? n : 1, HRB) + 1);  // cpart (one per hreduce CTA)
-  b += sizeof(unsigned) * 8;                          // counters (colupd, dots, grid barrier, abort)
+  b += sizeof(unsigned) * 8;                          // counters (colupd, dots)
   b += resident_workspace_bytes(n, sizeof(R));
   return b + 17 * 256;
 }
@@ -1378,7 +1048,7 @@ TridiagView<R> tridiag_bind(void* ws, cplx<R>* M, int n, int64_t ld, int nbmax, 
   v.Yb = reinterpret_cast<Z*>(take(sizeof(Z) * (size_t)n * nbmax));
   v.ga = reinterpret_cast<Z*>(take(sizeof(Z) * (size_t)n));
   v.gb = reinterpret_cast<Z*>(take(sizeof(Z) * (size_t)n));
-  v.hpart = reinterpret_cast<Z*>(take(sizeof(Z) * (size_t)(hblk + 2) * (hblk + 2) * 32 * 4));
+  v.hpart = reinterpret_cast<Z*>(take(sizeof(Z) * (size_t)(hblk + 2) * (hblk + 2) * 32 * 2));
   v.dpart = reinterpret_cast<Z*>(take(sizeof(Z) * (size_t)hblk * nbmax * 4));
   v.dots = reinterpret_cast<Z*>(take(sizeof(Z) * 4 * (size_t)nbmax));
   v.npart = reinterpret_cast<double*>(take(sizeof(double) * 2 * hblk));
@@ -1387,7 +1057,6 @@ TridiagView<R> tridiag_bind(void* ws, cplx<R>* M, int n, int64_t ld, int nbmax, 
   v.counter = reinterpret_cast<unsigned*>(take(sizeof(unsigned) * 8));
   v.rws = take(resident_workspace_bytes(n, sizeof(R)));
   v.ctas = resident_ctas(n, true);
-  v.coop = 1;
   v.d = d; v.e = e; v.tau = tau;
   return v;
 }
