@@ -76,3 +76,32 @@ def test_fp64_structured_columns(gpu):
     assert (w - torch.linalg.eigvalsh(h)[::2]).abs().max().item() <= TOL
     assert (h @ v - v * torch.cat([w, w])).abs().max().item() <= TOL
     assert (v.mH @ v - torch.eye(2 * n, device="cuda", dtype=v.dtype)).abs().max().item() <= TOL
+
+
+@pytest.mark.parametrize("path", ["fp64", "refined"])
+@pytest.mark.parametrize("tiny", [1e-8, 1e-14, 1e-20, 1e-78, 1e-100, 1e-160])
+def test_weakly_coupled_blocks(gpu, path, tiny):
+    """Two blocks joined by entries far below the matrix's size: the columns at
+    the seam shrink to the coupling, and their reflectors must stay unitary."""
+    import torch
+
+    n = 90
+    a, b = inputs.random_blocks(n, 77)
+    a[:30, 30:] *= tiny
+    a[30:, :30] *= tiny
+    b[:30, 30:] *= tiny
+    b[30:, :30] *= tiny
+    d0 = torch.from_numpy(np.ascontiguousarray(inputs.pack_left_half(a, b).T)).cuda()
+    d, e = d0.clone(), torch.zeros(2 * n, dtype=torch.float64, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    if path == "fp64":
+        rc = gpu.zquatev_fp64_device(2 * n, d.data_ptr(), 2 * n, e.data_ptr(), st)
+    else:
+        rc = gpu.zquatev_refined_device(2 * n, d.data_ptr(), 2 * n, e.data_ptr(), st, 1)
+    torch.cuda.synchronize()
+    assert rc == 0, _lib.last_error()
+    h, v, w = d0.T, d.T, e[:n]
+    norm = w.abs().max()
+    assert ((w - torch.linalg.eigvalsh(h)[::2]).abs().max() / norm).item() <= TOL
+    assert ((h @ v - v * torch.cat([w, w])).abs().max() / norm).item() <= TOL
+    assert (v.mH @ v - torch.eye(2 * n, device="cuda", dtype=v.dtype)).abs().max().item() <= TOL

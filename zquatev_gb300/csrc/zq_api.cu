@@ -397,6 +397,7 @@ struct HostPin {
   }
 };
 
+static int path_single(int n);
 // host-memory drop-in (path: -1 policy, 0 FP64, 1 refined)
 static int zquatev_host(int n2, double2* D, int ld2, double* eig, bool vectors, int path = -1) {
   if (int rc = check_args(n2, D, ld2, eig)) return rc;
@@ -437,7 +438,7 @@ static int zquatev_host(int n2, double2* D, int ld2, double* eig, bool vectors, 
     if (cudaMemcpy2DAsync(dD, sizeof(double2) * n2, D, sizeof(double2) * (size_t)ld2, sizeof(double2) * n2, n,
                           cudaMemcpyHostToDevice, c->st) != cudaSuccess) { rc = ZQ_ERR_CUDA; set_msg("H2D copy failed"); break; }
     phase("h2d");
-    const int p = (path >= 0) ? path : path_for(n);
+    const int p = (path >= 0) ? path : path_single(n);
     cudaEvent_t te[2];
     if (timing) { cudaEventCreate(&te[0]); cudaEventCreate(&te[1]); cudaEventRecord(te[0], c->st); }
     rc = (vectors && p == 1) ? refined_device(c, dD, n2, n, deig, c->st, 1) : solve_device(c, dD, n2, n, deig, vectors, c->st);
@@ -551,13 +552,29 @@ int refined_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, cu
 
 // path policy of the drop-in entry points: 0 FP64, 1 refined, 2 auto
 static int g_path = 2;
-int path_for(int n) {
-  int p = g_path;
+static int path_policy() {
   if (const char* s = getenv("ZQ_PATH")) {
-    if (!strcmp(s, "fp64")) p = 0; else if (!strcmp(s, "refined")) p = 1; else if (!strcmp(s, "auto")) p = 2;
+    if (!strcmp(s, "fp64")) return 0;
+    if (!strcmp(s, "refined")) return 1;
+    if (!strcmp(s, "auto")) return 2;
   }
-  if (p == 2) p = (n >= 48) ? 1 : 0;  // refined measured faster from n = 48 up (2-4x)
-  return p;
+  return g_path;
+}
+int path_for(int n) {
+  const int p = path_policy();
+  return p == 2 ? (n >= 48 ? 1 : 0) : p;
+}
+
+// The same for one solve alone on the GPU: there the FP64 path is the faster one
+// up to order ~160 (its reduction and back-transform spread over the SMs and it
+// needs no refinement): n = 64 1.29 against 2.54 ms, n = 127 2.6 / 3.2, n = 160
+// 3.5 / 3.6, n = 200 4.5 / 4.1. The request server keeps path_for: its lanes run
+// side by side, where the FP64 pipe is shared and the refined path's latencies
+// overlap.
+constexpr int SINGLE_REFINED_MIN = 160;
+static int path_single(int n) {
+  const int p = path_policy();
+  return p == 2 ? (n >= SINGLE_REFINED_MIN ? 1 : 0) : p;
 }
 
 // ----------------------------------------------------------------------------
@@ -661,7 +678,7 @@ int zquatev_device(int n2, double* dD, int ld2, double* deig, void* stream) {
   Context* c = nullptr;
   if (int rc = get_context(&c)) return rc;
   std::lock_guard<std::mutex> lk(c->mu);
-  if (path_for(n2 / 2) == 1)
+  if (path_single(n2 / 2) == 1)
     return refined_device(c, reinterpret_cast<double2*>(dD), ld2, n2 / 2, deig, reinterpret_cast<cudaStream_t>(stream), 1);
   return solve_device(c, reinterpret_cast<double2*>(dD), ld2, n2 / 2, deig, true, reinterpret_cast<cudaStream_t>(stream));
 }

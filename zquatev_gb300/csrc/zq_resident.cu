@@ -7,16 +7,15 @@
 // over the shared memories of a group of G co-resident CTAs, and stay there:
 // per column every tile takes the previous column's rank-2 update and the
 // mat-vec with the current reflector in one sweep, and only vectors travel
-// between the CTAs (through L2), with three group barriers per column:
+// between the CTAs (through L2), with two group barriers per column:
 //
 //   sweep j    tiles -= w_{j-1} y_{j-1}^H + y_{j-1} w_{j-1}^H (structured), then the
-//              tile's products with w_j; column j + 1 is published
+//              tile's products with w_j and their part of c = w_j^H H w_j; column
+//              j + 1 is published
 //      -- barrier --
-//   rows       g = H w_j: each CTA sums the tile partials of its share of the
-//              rows, and its part of c = w_j^H g
-//      -- barrier --
-//   column     y_j = g - (c/2) w_j and column j + 1 brought up to date on the
-//              CTA's rows, with its norm partials
+//   rows       g = H w_j from the tile partials of the CTA's share of the rows,
+//              y_j = g - (c/2) w_j, and column j + 1 brought up to date there,
+//              with its norm partials (every CTA also sums row j + 1 for itself)
 //      -- barrier --
 //              every CTA forms reflector j + 1 from the norm partials
 //
@@ -129,11 +128,112 @@ __device__ __forceinline__ double pow2_biased(int be) {
   return be < 1 ? 0.0 : __longlong_as_double((long long)be << 52);
 }
 
-// Sum of `count` doubles (written by other CTAs) by one warp; every lane gets it.
-__device__ __forceinline__ double warp_gather(const double* p, int count, int lane) {
-  double s = 0.0;
-  for (int i = lane; i < count; i += 32) s += __ldcg(p + i);
-  return warp_sum(s);
+// Sums of the vector phases. FP64 data: doubles. FP32 data: unevaluated pairs of
+// floats (hi + lo, ~48 bits; Dekker/Knuth two-sums and FMA products): the FP64 pipe
+// takes ~75 cycles per dependent instruction here, a pair's sum ~30.
+struct Pair { float hi, lo; };
+__device__ __forceinline__ Pair sum2(Pair a, Pair b) {
+  const float s = a.hi + b.hi, t = s - a.hi;
+  const float e = ((a.hi - (s - t)) + (b.hi - t)) + (a.lo + b.lo);
+  const float h = s + e;
+  return Pair{h, e - (h - s)};
+}
+__device__ __forceinline__ Pair mul2(Pair a, Pair b) {
+  const float p = a.hi * b.hi;
+  const float e = fmaf(a.hi, b.lo, fmaf(a.lo, b.hi, fmaf(a.hi, b.hi, -p)));
+  const float h = p + e;
+  return Pair{h, e - (h - p)};
+}
+// 1 / sqrt(a) by one Newton step from the approximate instruction
+__device__ __forceinline__ Pair rsqrt2(Pair a) {
+  const float y = rsqrtf(a.hi), p = y * y;
+  const Pair u = mul2(a, Pair{p, fmaf(y, y, -p)});
+  const float d = (1.f - u.hi) - u.lo;
+  return Pair{y, 0.5f * y * d};
+}
+template <typename R> struct AccOf { using type = double; };
+template <> struct AccOf<float> { using type = Pair; };
+template <typename R> using Acc = typename AccOf<R>::type;
+__device__ __forceinline__ double acc_add(double a, double b) { return a + b; }
+__device__ __forceinline__ Pair acc_add(Pair a, Pair b) { return sum2(a, b); }
+__device__ __forceinline__ double acc_shfl(double v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
+__device__ __forceinline__ Pair acc_shfl(Pair v, int o) {
+  return Pair{__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o)};
+}
+__device__ __forceinline__ void acc_square(double& s, double x) { s = fma(x, x, s); }
+__device__ __forceinline__ void acc_square(Pair& s, float x) {
+  const float p = x * x;
+  s = sum2(s, Pair{p, fmaf(x, x, -p)});
+}
+__device__ __forceinline__ double acc_value(double x) { return x; }
+__device__ __forceinline__ Pair acc_value(float x) { return Pair{x, 0.f}; }
+__device__ __forceinline__ double acc_double(double v) { return v; }
+__device__ __forceinline__ double acc_double(Pair v) { return (double)v.hi + (double)v.lo; }
+__device__ __forceinline__ double acc_half(double v) { return 0.5 * v; }
+__device__ __forceinline__ float acc_half(Pair v) { return 0.5f * (v.hi + v.lo); }
+__device__ __forceinline__ void acc_store(double* p, double v) { *p = v; }
+__device__ __forceinline__ void acc_store(double* p, Pair v) { *reinterpret_cast<float2*>(p) = make_float2(v.hi, v.lo); }
+__device__ __forceinline__ void acc_load(const double* p, double& v) { v = __ldcg(p); }
+__device__ __forceinline__ void acc_load(const double* p, Pair& v) {
+  const float2 t = __ldcg(reinterpret_cast<const float2*>(p));
+  v = Pair{t.x, t.y};
+}
+template <int FROM, int TO, typename V> __device__ __forceinline__ V acc_lanes(V v) {
+#pragma unroll
+  for (int o = FROM; o >= TO; o >>= 1) v = acc_add(v, acc_shfl(v, o));
+  return v;
+}
+// Sum of `count` accumulators written by other CTAs, by one warp; every lane gets it.
+template <typename R>
+__device__ __forceinline__ Acc<R> warp_gather(const double* p, int count, int lane) {
+  Acc<R> s{};
+  for (int i = lane; i < count; i += 128) {  // four loads in flight
+    Acc<R> v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      v[u] = Acc<R>{};
+      if (i + 32 * u < count) acc_load(p + i + 32 * u, v[u]);
+    }
+    s = acc_add(s, acc_add(acc_add(v[0], v[1]), acc_add(v[2], v[3])));
+  }
+  return acc_lanes<16, 1>(s);
+}
+
+// The reflector's scalars from ss = |x|^2 and q2 = |x_1|^2 (in units of the scaled
+// matrix): g = sqrt(ss q2) = |x||x_1|, s = |x| / |x_1| = ss / g, f = 1 / sqrt(ss + g),
+// h = f (1 + s). False: |x_1| is too small beside |x| to matter (below 1e-75, FP32
+// 1e-15), the head is taken as 1 and f = 1 / |x|.
+// Columns below tiny_column (|x| under 1e-75 of the matrix, FP32 1e-14) are left as
+// they are (f = 0, e = 0), so no product here leaves the range of normal numbers.
+__device__ __forceinline__ bool tiny_column(double ss) { return ss < 1e-150; }
+__device__ __forceinline__ bool tiny_column(Pair ss) { return ss.hi < 1e-28f; }
+__device__ __forceinline__ bool reflector_scalars(double ss, double q2, double& f, double& h, double& s) {
+  const double t = ss * q2;
+  if (!(t > 1e-300)) { f = rsqrt(ss); return false; }
+  const double rg = rsqrt(t);
+  s = ss * rg;
+  f = rsqrt(fma(t, rg, ss));
+  h = fma(f, s, f);
+  return true;
+}
+__device__ __forceinline__ bool reflector_scalars(Pair ss, Pair q2, float& f, float& h, Pair& s) {
+  // an even power of two brings ss into [1, 4): q2 <= ss keeps its bits
+  const int e = ((int)(__float_as_uint(ss.hi) >> 23) - 127) & ~1;
+  const float sc = __uint_as_float((unsigned)(127 - e) << 23), sr = __uint_as_float((unsigned)(127 - e / 2) << 23);
+  const Pair a{ss.hi * sc, ss.lo * sc};
+  const Pair t = mul2(a, Pair{q2.hi * sc, q2.lo * sc});
+  if (!(t.hi > 1e-30f)) {
+    const Pair r = rsqrt2(a);
+    f = (r.hi + r.lo) * sr;
+    return false;
+  }
+  const Pair rg = rsqrt2(t);
+  s = mul2(a, rg);
+  const Pair r = rsqrt2(sum2(mul2(t, rg), a));
+  const Pair hh = sum2(mul2(r, s), r);
+  f = (r.hi + r.lo) * sr;
+  h = (hh.hi + hh.lo) * sr;
+  return true;
 }
 __device__ __forceinline__ unsigned mag_bits(float v) { return __float_as_uint(v) & 0x7fffffffu; }
 __device__ __forceinline__ unsigned long long mag_bits(double v) { return abs_bits(v); }
@@ -152,11 +252,9 @@ template <typename R> __host__ __device__ __forceinline__ int row_ctas(int G) {
 //
 // An FP64 instruction holds its SM quadrant's pipe for 64 cycles whatever the
 // number of lanes, so the vector phases keep one real component per lane (the
-// four lanes of a row exchange theirs by shuffles) and the reflector's scalars
-// come from two reciprocal square roots: with ss = |x|^2 and q2 = |x_1|^2,
-// g = sqrt(ss q2) = |x||x_1|, s = |x|/|x_1| = ss / g and f = 1 / sqrt(ss + g).
-// The matrix is scaled by a power of two once (largest entry in [1, 2)), so no
-// sum of squares needs a scale of its own.
+// four lanes of a row exchange theirs by shuffles). The matrix is scaled by a
+// power of two once (largest entry in [1, 2)), so no sum of squares needs a scale
+// of its own; FP32 columns whose squares vanish are 1e-19 of the matrix.
 template <typename R, int T, int LPR, bool CL>
 __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int rank, int G, unsigned char* smem,
                               unsigned& target, int* err, long long limit) {
@@ -166,7 +264,8 @@ __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int r
   constexpr int TILE = T * T * 4;                      // reals per tile
   __shared__ R s_head[8];                              // f, f m (4)
   __shared__ double s_red[RT_WARPS];
-  __shared__ double s_c;
+  __shared__ double s_cw[RT_WARPS];                    // the warps' parts of c
+  __shared__ R s_hc;                                   // c / 2
   __shared__ int s_ok;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tr = lane & 7, tc = lane >> 3;
@@ -196,8 +295,8 @@ __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int r
   Q4<R>* ys = wbuf[1] + m;
   const int rmax = (m + NR - 1) / NR;
   R* own_w = reinterpret_cast<R*>(ys + m);
-  R* own_g = own_w + 4 * rmax;
-  R* own_x = own_g + 4 * rmax;
+  R* own_g = own_w + 4 * rmax;          // and g at row j + 1 in the row after the CTA's
+  R* own_x = own_g + 4 * (rmax + 1);
   unsigned char* need = reinterpret_cast<unsigned char*>(own_x + 4 * rmax);
 
   // load the tiles; clear the vectors; mark the row blocks this CTA's tiles touch
@@ -263,38 +362,36 @@ __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int r
     rows0 = j + rank * per;
     nrows = (rank >= NR || rows0 >= m) ? 0 : (rows0 + per < m ? per : m - rows0);
   };
-  // sum over the block of per-lane values, left in thread 0 (ss: one per thread)
-  auto cta_sum = [&](double v, int items) {
-    const int nw = items <= 32 ? 1 : RT_WARPS;
-    if (nw == 1) return warp == 0 ? warp_sum(v) : 0.0;
-    if (warp * 32 < items) v = warp_sum(v);
-    if (lane == 0) s_red[warp] = warp * 32 < items ? v : 0.0;
-    __syncthreads();
-    if (warp == 0) {
-      v = lane < RT_WARPS ? s_red[lane] : 0.0;
-#pragma unroll
-      for (int o = RT_WARPS / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    }
-    return v;
-  };
-  // |x|^2 of the own rows below the diagonal of column j, from the components'
-  // squares, and |x_1|^2 for everybody (row j + 1)
-  auto publish_norms = [&](int j, R x, int idx, double ss) {
+  // |x|^2 of the own rows below the diagonal of column j (ss: a part per thread),
+  // and |x_1|^2 for everybody (row j + 1; x: this thread's first component)
+  auto publish_norms = [&](int j, R x, Acc<R> ss) {
     const int items = 4 * nrows;
-    const double t = cta_sum(ss, items);
-    if (tid == 0 && rank < NR) gr.npart[rank] = t;
-    const int i1 = j + 1 - rows0;  // row j + 1 among the own rows
-    if (nrows > 0 && i1 >= 0 && i1 < nrows && (idx >> 5) == (4 * i1) >> 5 && idx < RT_THREADS) {
-      double q = (double)x * (double)x;   // only the four lanes of row j + 1 are used
-      q += __shfl_xor_sync(0xffffffffu, q, 1);
-      q += __shfl_xor_sync(0xffffffffu, q, 2);
-      if (idx == 4 * i1) *gr.q2 = q;
+    if (warp * 32 < items || warp == 0) ss = acc_lanes<16, 1>(ss);
+    if (items > 32) {
+      if (lane == 0) acc_store(s_red + warp, warp * 32 < items ? ss : Acc<R>{});
+      __syncthreads();
+      if (warp == 0) {
+        ss = Acc<R>{};
+        if (lane < RT_WARPS) {
+          if constexpr (sizeof(R) == 8) ss = s_red[lane];
+          else { const float2 t = reinterpret_cast<const float2*>(s_red)[lane]; ss = Pair{t.x, t.y}; }
+        }
+        ss = acc_lanes<RT_WARPS / 2, 1>(ss);
+      }
+    }
+    if (tid == 0 && rank < NR) acc_store(gr.npart + rank, ss);
+    const int i1 = j + 1 - rows0;  // row j + 1 among the own rows: the first or the second
+    if (warp == 0 && i1 >= 0 && i1 < nrows) {
+      Acc<R> q{};
+      acc_square(q, x);
+      q = acc_lanes<2, 1>(q);
+      if (tid == 4 * i1) acc_store(gr.q2, q);
     }
   };
   // column 0 as it is
   partition(0);
   {
-    double ss = 0.0;
+    Acc<R> ss{};
     R x0 = R(0);
     for (int idx = tid; idx < ((4 * nrows + 31) & ~31); idx += RT_THREADS) {
       R x = R(0);
@@ -305,11 +402,11 @@ __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int r
         if (r == 0) { if (k) x = R(0); else tk.d[k0] = (double)x * scale; }
         own_x[idx] = x;
         reinterpret_cast<R*>(gr.x)[4 * r + k] = x;
-        if (r > 0) ss += (double)x * (double)x;
+        if (r > 0) acc_square(ss, x);
       }
       if (idx == tid) x0 = x;
     }
-    publish_norms(0, x0, tid, ss);
+    publish_norms(0, x0, ss);
   }
   if (!barrier()) return false;
 
@@ -317,52 +414,74 @@ __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int r
     Q4<R>* wp = wbuf[(j & 1) ^ 1];
     Q4<R>* wn = wbuf[j & 1];
     // ------------------------------------------------ reflector j
-    double ej = 0.0;  // component of e_j (lanes 0..3 of warp 0)
+    const bool last = m - 1 - j < 2;  // one row left: the entry itself is e
     if (warp == 0) {
       const R x1 = __ldcg(reinterpret_cast<const R*>(gr.x + j + 1) + (lane & 3));
-      const double q2 = __ldcg(gr.q2);
-      const double ss = warp_gather(gr.npart, NR, lane);
-      double f = 0.0, h = 0.0, s = 0.0;
-      bool unit = false;               // x_1 = 0: the head is 1
-      const bool last = m - 1 - j < 2;  // one row left: the entry itself is e
-      if (!last && ss > 0.0) {
-        const double t = ss * q2;
-        if (t > 0.0) {
-          const double rg = rsqrt(t);
-          s = ss * rg;
-          f = rsqrt(fma(t, rg, ss));
-          h = fma(f, s, f);
-        } else {
-          f = rsqrt(ss);
-          unit = true;
-        }
+      Acc<R> q2;
+      acc_load(gr.q2, q2);
+      const Acc<R> ss = warp_gather<R>(gr.npart, NR, lane);
+      R f = R(0), h = R(0);
+      bool unit = false;  // the head is 1
+      if (!last && !tiny_column(ss)) {
+        Acc<R> s{};
+        unit = !reflector_scalars(ss, q2, f, h, s);
       }
-      ej = last ? (double)x1 : (unit ? ((lane & 3) == 0 ? -ss * f : 0.0) : (ss == 0.0 ? 0.0 : -s * (double)x1));
-      if (!last && !(ss >= 0.0)) ej = ss;  // not a number: keep it visible
-      const double mk_ = unit ? ((lane & 3) == 0 ? 1.0 : 0.0) : (double)x1 * h;
       if (lane < 4) {
-        s_head[1 + lane] = (R)mk_;
-        if (lane == 0) s_head[0] = (R)f;
+        s_head[1 + lane] = unit ? (lane == 0 ? R(1) : R(0)) : x1 * h;
+        if (lane == 0) { s_head[0] = f; s_head[5] = unit ? R(1) : R(0); }
       }
     }
-    // w (as x for now) and y_{j-1} of the blocks this CTA's tiles touch
-    for (int r = tid + (j >= 2 ? j - 2 : 0); r < m; r += RT_THREADS) {
-      if (!need[r / T]) continue;
-      Q4<R> x = q_zero<R>(), y = q_zero<R>();
-      if (r > j) x = q_ldcg(gr.x + r);
-      if (j > 0 && r >= j) y = q_ldcg(gr.y + r);
-      wn[r] = x;
-      ys[r] = y;
+    // w and y_{j-1} of the blocks this CTA's tiles touch: up to RPT rows per thread
+    // are held until the reflector is known
+    constexpr int RPT = 4;
+    const int rfrom = j >= 2 ? j - 2 : 0;
+    Q4<R> xr[RPT];
+#pragma unroll
+    for (int u = 0; u < RPT; ++u) {
+      const int r = rfrom + tid + RT_THREADS * u;
+      xr[u] = q_zero<R>();
+      if (r >= m || !need[r / T]) continue;
+      if (r > j) xr[u] = q_ldcg(gr.x + r);
+      ys[r] = j > 0 && r >= j ? q_ldcg(gr.y + r) : q_zero<R>();
     }
     __syncthreads();
     const R f = s_head[0];
     const Q4<R> w1{s_head[1], s_head[2], s_head[3], s_head[4]};  // w at row j + 1
-    for (int r = tid + (j >= 2 ? j - 2 : 0); r < m; r += RT_THREADS) {
-      if (r <= j || !need[r / T]) continue;
-      const Q4<R> x = wn[r];
+#pragma unroll
+    for (int u = 0; u < RPT; ++u) {
+      const int r = rfrom + tid + RT_THREADS * u;
+      if (r >= m || !need[r / T]) continue;
+      const Q4<R> x = xr[u];
       wn[r] = r == j + 1 ? w1 : Q4<R>{x.ax * f, x.ay * f, x.bx * f, x.by * f};
     }
+    for (int r = rfrom + tid + RT_THREADS * RPT; r < m; r += RT_THREADS) {
+      if (!need[r / T]) continue;
+      Q4<R> x = q_zero<R>();
+      if (r > j) x = q_ldcg(gr.x + r);
+      wn[r] = r == j + 1 ? w1 : Q4<R>{x.ax * f, x.ay * f, x.bx * f, x.by * f};
+      ys[r] = j > 0 && r >= j ? q_ldcg(gr.y + r) : q_zero<R>();
+    }
     __syncthreads();
+    // e_j and tau_j: one warp, beside the sweep
+    if (rank == G - 1 && warp == RT_WARPS - 1) {
+      const R x1 = __ldcg(reinterpret_cast<const R*>(gr.x + j + 1) + (lane & 3));
+      Acc<R> q2a;
+      acc_load(gr.q2, q2a);
+      const double q2 = acc_double(q2a), ss = acc_double(warp_gather<R>(gr.npart, NR, lane));
+      if (lane < 4) {
+        double e = x1;
+        if (!last) {
+          // |x| in the direction the reflector took; not a number stays visible
+          if (!(ss >= 0.0)) e = ss;
+          else if (!(f > R(0))) e = 0.0;
+          else if (s_head[5] != R(0)) e = lane == 0 ? -ss * rsqrt(ss) : 0.0;
+          else e = -ss * rsqrt(ss * q2) * (double)x1;
+        }
+        tk.e[4 * (size_t)(k0 + j) + lane] = e * scale;
+        if (lane == 0) tk.tau[k0 + j] = f > R(0) ? 1.0 : 0.0;
+      }
+    }
+    R cacc = R(0);  // this lane's part of c = w^H H w
     // ------------------------------------------------ sweep
     const int Jlo = (j + 1) / T;                       // first live column block
     const int live = (nt - Jlo) * (nt - Jlo + 1) / 2;  // tiles in dealing order
@@ -416,8 +535,14 @@ __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int r
         const int r = I * T + tr + 8 * (k / 4);
         if (r < m) {
           R* o = reinterpret_cast<R*>(gr.part + (size_t)J * m + r) + (k & 3);
+          const R* wv = reinterpret_cast<const R*>(wn + r) + (k & 3);
+          R cp = R(0);
 #pragma unroll
-          for (int q2 = 0; q2 < NRV; ++q2) o[q2] = rs[q2];
+          for (int q2 = 0; q2 < NRV; ++q2) {
+            o[q2] = rs[q2];
+            cp = fma(wv[q2], rs[q2], cp);
+          }
+          cacc += diag ? cp : cp + cp;  // an off-diagonal tile stands for its mirror too
         }
       }
       if (!diag) {
@@ -431,10 +556,6 @@ __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int r
         }
       }
     }
-    if (rank == G - 1 && warp == 0 && lane < 4) {
-      tk.e[4 * (size_t)(k0 + j) + lane] = ej * scale;
-      if (lane == 0) tk.tau[k0 + j] = f > R(0) ? 1.0 : 0.0;
-    }
     // w_j in place of column j (this CTA's rows of the partition that formed it)
     for (int idx = tid; idx < 4 * nrows; idx += RT_THREADS) {
       const int r = rows0 + (idx >> 2), k = idx & 3;
@@ -442,24 +563,43 @@ __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int r
       R* dst = reinterpret_cast<R*>((k < 2 ? A : B) + r + (int64_t)j * ld);
       dst[k & 1] = r == j + 1 ? s_head[1 + k] : own_x[idx] * f;
     }
+    // this CTA's part of c
+    {
+      const Acc<R> c = acc_lanes<16, 1>(acc_value(cacc));
+      if (lane == 0) acc_store(s_cw + warp, c);
+      __syncthreads();
+      if (warp == 0) {
+        Acc<R> t{};
+        if (lane < RT_WARPS) {
+          if constexpr (sizeof(R) == 8) t = s_cw[lane];
+          else { const float2 u = reinterpret_cast<const float2*>(s_cw)[lane]; t = Pair{u.x, u.y}; }
+        }
+        t = acc_lanes<RT_WARPS / 2, 1>(t);
+        if (lane == 0) acc_store(gr.cpart + rank, t);
+      }
+    }
     if (!barrier()) return false;
-    // ------------------------------------------------ rows: g and c
+    // ------------------------------------------------ rows: g, y_j and column j + 1
     const int p = j + 1;
     partition(p);
-    {
+    if (nrows > 0) {
+      if (warp == RT_WARPS - 1) {
+        const Acc<R> c = warp_gather<R>(gr.cpart, G, lane);
+        if (lane == 0) s_hc = acc_half(c);
+      }
       constexpr int RPW = 32 / LPR;               // rows per warp and pass
       const int sl = lane & (LPR - 1);
       const int k = sl / (LPR / 4);               // component this lane ends with
       const bool rep = (sl & (LPR / 4 - 1)) == 0;  // one lane of those holding it
-      double cp = 0.0;
-      for (int i0 = warp * RPW; i0 < nrows; i0 += RT_WARPS * RPW) {
+      // the CTA's rows, and row p once more for its own use
+      for (int i0 = warp * RPW; i0 <= nrows; i0 += RT_WARPS * RPW) {
         const int i = i0 + lane / LPR;
-        const bool in = i < nrows;
-        const int r = rows0 + (in ? i : 0);
+        const bool in = i <= nrows;
+        const int r = i < nrows ? rows0 + i : p;
         R s[4] = {R(0), R(0), R(0), R(0)};
         R x = R(0);
         if (in) {
-          x = __ldcg(reinterpret_cast<const R*>(gr.x + r) + k);
+          if (i < nrows) x = __ldcg(reinterpret_cast<const R*>(gr.x + r) + k);
 #pragma unroll 4
           for (int b = Jlo + sl; b < nt; b += LPR) {
             const Q4<R> t = q_ldcg(gr.part + (size_t)b * m + r);
@@ -470,37 +610,21 @@ __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int r
 #pragma unroll
         for (int o = LPR / 8; o > 0; o >>= 1) s[0] += __shfl_xor_sync(0xffffffffu, s[0], o);
         if (in && rep) {
-          const R w = r == p ? s_head[1 + k] : x * f;
           own_g[4 * i + k] = s[0];
-          own_w[4 * i + k] = w;
-          cp += (double)(w * s[0]);
+          if (i < nrows) own_w[4 * i + k] = r == p ? s_head[1 + k] : x * f;
         }
       }
-      const double c = cta_sum(cp, nrows * LPR);
-      if (tid == 0 && rank < NR) gr.cpart[rank] = c;
     }
-    if (rank == 0) {
-      __syncthreads();
-      if (tid < 4) reinterpret_cast<R*>(gr.g1)[tid] = own_g[tid];
-    }
-    if (!barrier()) return false;
-    // ------------------------------------------------ column j + 1
     {
-      double ss = 0.0;
+      Acc<R> ss{};
       R xfirst = R(0);
       const int k = tid & 3;
-      R col = R(0), g1 = R(0);
-      if (nrows > 0) {
-        g1 = __ldcg(reinterpret_cast<const R*>(gr.g1) + k);
-        if (tid < 4 * nrows) col = __ldcg(reinterpret_cast<const R*>(gr.col + rows0) + tid);
-        if (warp == 0) {
-          const double c = warp_gather(gr.cpart, NR, lane);
-          if (lane == 0) s_c = c;
-        }
-      }
+      R col = R(0);
+      if (tid < 4 * nrows) col = __ldcg(reinterpret_cast<const R*>(gr.col + rows0) + tid);
       __syncthreads();
       if (nrows > 0) {
-        const R hc = (R)(0.5 * s_c);
+        const R g1 = own_g[4 * nrows + k];
+        const R hc = s_hc;
         const R wk1 = s_head[1 + k];
         const R yk1 = g1 - hc * wk1;
         // this lane's signs of the structured products
@@ -533,12 +657,12 @@ __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int r
             own_x[idx] = x;
             reinterpret_cast<R*>(gr.x)[4 * r + k] = x;
             reinterpret_cast<R*>(gr.y)[4 * r + k] = y;
-            if (r > p) ss += (double)x * (double)x;
+            if (r > p) acc_square(ss, x);
           }
           if (idx == tid) xfirst = x;
         }
       }
-      publish_norms(p, xfirst, tid, ss);
+      publish_norms(p, xfirst, ss);
     }
     if (!barrier()) return false;
   }
@@ -591,7 +715,7 @@ size_t rt_smem_bytes(int m, int T, int G) {
   const int nt = (m + T - 1) / T, ntiles = nt * (nt + 1) / 2;
   const size_t cap = (size_t)((ntiles + G - 1) / G);
   const int NR = row_ctas<R>(G);
-  return cap * T * T * 4 * sizeof(R) + sizeof(Q4<R>) * (3 * (size_t)m + 3 * (size_t)((m + NR - 1) / NR)) + (size_t)nt + 16;
+  return cap * T * T * 4 * sizeof(R) + sizeof(Q4<R>) * (3 * (size_t)m + 3 * (size_t)((m + NR - 1) / NR) + 1) + (size_t)nt + 16;
 }
 
 // shared-memory opt-in (and clusters above eight CTAs), once per device and kernel
