@@ -566,12 +566,12 @@ int path_for(int n) {
 }
 
 // The same for one solve alone on the GPU: there the FP64 path is the faster one
-// up to order ~160 (its reduction and back-transform spread over the SMs and it
-// needs no refinement): n = 64 1.29 against 2.54 ms, n = 127 2.6 / 3.2, n = 160
-// 3.5 / 3.6, n = 200 4.5 / 4.1. The request server keeps path_for: its lanes run
+// up to order ~200 (its reduction and back-transform spread over the SMs and it
+// needs no refinement): n = 64 1.03 against 2.32 ms, n = 127 1.9 / 2.9, n = 200
+// 3.5 / 3.5, n = 256 4.3 / 4.0. The request server keeps path_for: its lanes run
 // side by side, where the FP64 pipe is shared and the refined path's latencies
 // overlap.
-constexpr int SINGLE_REFINED_MIN = 160;
+constexpr int SINGLE_REFINED_MIN = 200;
 static int path_single(int n) {
   const int p = path_policy();
   return p == 2 ? (n >= SINGLE_REFINED_MIN ? 1 : 0) : p;

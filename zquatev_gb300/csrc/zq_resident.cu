@@ -59,7 +59,7 @@ namespace {
 constexpr int RT_THREADS = 256;
 constexpr int RT_WARPS = RT_THREADS / 32;
 constexpr int RT_CLUSTER = 16;  // largest cluster
-constexpr int RT_SMEM_MAX = 227 * 1024 - 1024;  // dynamic shared memory per CTA (static part below 1 KB)
+constexpr int RT_SMEM_MAX = 227 * 1024 - 3 * 1024;  // dynamic shared memory per CTA (static part below 3 KB)
 
 // a lane's tile slot e: FP32 one 16-byte slot, FP64 two 16-byte planes
 template <int EL> __device__ __forceinline__ Q4<float> t_load(const float* t, int e, int lane) {
@@ -77,6 +77,16 @@ template <int EL> __device__ __forceinline__ Q4<double> t_load(const double* t, 
 template <int EL> __device__ __forceinline__ void t_store(double* t, int e, int lane, const Q4<double>& q) {
   reinterpret_cast<double2*>(t)[e * 32 + lane] = make_double2(q.ax, q.ay);
   reinterpret_cast<double2*>(t)[(EL + e) * 32 + lane] = make_double2(q.bx, q.by);
+}
+
+// Signs (bit q set: minus) of the four products that make component k of
+//   the rank-2 term     sum_q w_r[k^q] y_c[q]   + + + + | + - - + | + + - - | + - + -
+//   a row product       sum_q m[k^q] w_c[q]     + - - - | + + + - | + - + + | + + - +
+//   a column product    sum_q m[k^q] w_r[q]     + + + + | - + - + | - + + - | - - + +
+__device__ __forceinline__ unsigned quat_signs(unsigned table, int k) { return (table >> (4 * k)) & 15u; }
+constexpr unsigned SIGNS_RANK2 = 0xAC60u, SIGNS_ROW = 0x428Eu, SIGNS_COL = 0x3950u;
+__device__ __forceinline__ double flip(double v, unsigned neg) {
+  return __longlong_as_double(__double_as_longlong(v) ^ ((long long)(neg & 1u) << 63));
 }
 
 // tile t in dealing order: column blocks from the last one back
@@ -266,6 +276,7 @@ __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int r
   __shared__ double s_red[RT_WARPS];
   __shared__ double s_cw[RT_WARPS];                    // the warps' parts of c
   __shared__ R s_hc;                                   // c / 2
+  __shared__ R s_team[2][4][32];                       // row sums of the warps that share a tile
   __shared__ int s_ok;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tr = lane & 7, tc = lane >> 3;
@@ -485,7 +496,83 @@ __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int r
     // ------------------------------------------------ sweep
     const int Jlo = (j + 1) / T;                       // first live column block
     const int live = (nt - Jlo) * (nt - Jlo + 1) / 2;  // tiles in dealing order
-    for (int q = warp; rank + q * G < live; q += RT_WARPS) {
+    // FP64 with few tiles left for the CTA: four warps share a tile (two columns
+    // each, a component per lane), so that the SM's four quadrants work on it: a
+    // tile takes 41 FP64 instructions of each of four warps instead of 146 of one
+    bool teams = false;
+    if constexpr (sizeof(R) == 8 && T == 8) teams = live <= 3 * G;
+    if constexpr (sizeof(R) == 8 && T == 8) {
+      if (teams) {
+        const int team = warp >> 2, tw = warp & 3;
+        const int r = lane >> 2, k = lane & 3;
+        const unsigned s2 = quat_signs(SIGNS_RANK2, k), sr = quat_signs(SIGNS_ROW, k), sc = quat_signs(SIGNS_COL, k);
+        for (int q = team; rank + q * G < live; q += 2) {
+          int I, J;
+          rt_tile(rank + q * G, nt, I, J);
+          R* tl = tiles + (size_t)q * TILE;
+          const bool diag = I == J;
+          const int gr_ = I * T + r, rl = min(gr_, m - 1);
+          const bool rin = gr_ < m;
+          // row vectors: this lane's components of w and y, all of the new w
+          const R wk = rin ? reinterpret_cast<const R*>(wp + rl)[k] : R(0);
+          const R yk = rin ? reinterpret_cast<const R*>(ys + rl)[k] : R(0);
+          Q4<R> nr = wn[rl];
+          if (!rin) nr = q_zero<R>();
+          R wx[4], yx[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            wx[u] = flip(__shfl_xor_sync(0xffffffffu, wk, u), s2 >> u);
+            yx[u] = flip(__shfl_xor_sync(0xffffffffu, yk, u), s2 >> u);
+          }
+          const R nw[4] = {flip(nr.ax, sc), flip(nr.ay, sc >> 1), flip(nr.bx, sc >> 2), flip(nr.by, sc >> 3)};
+          R rsum = R(0), csum[2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const int c = 2 * tw + u, gc = J * T + c, cl = min(gc, m - 1);
+            Q4<R> wc = wp[cl], yc = ys[cl], nc = wn[cl];
+            if (gc >= m) { wc = q_zero<R>(); yc = q_zero<R>(); nc = q_zero<R>(); }
+            // the slot of (r, c) in the lanes' layout (t_load)
+            R* e = tl + 2 * (((k >> 1) * EL + (c >> 2)) * 32 + r + 8 * (c & 3)) + (k & 1);
+            R t0 = wx[0] * yc.ax, t1 = yx[0] * wc.ax;
+            t0 = fma(wx[1], yc.ay, t0); t1 = fma(yx[1], wc.ay, t1);
+            t0 = fma(wx[2], yc.bx, t0); t1 = fma(yx[2], wc.bx, t1);
+            t0 = fma(wx[3], yc.by, t0); t1 = fma(yx[3], wc.by, t1);
+            R v = *e - (t0 + t1);
+            if (diag && r == c && k != 0) v = R(0);
+            *e = v;
+            if (gc == j + 1 && gr_ > j && rin) reinterpret_cast<R*>(gr.col + gr_)[k] = v;
+            const R nq[4] = {flip(nc.ax, sr), flip(nc.ay, sr >> 1), flip(nc.bx, sr >> 2), flip(nc.by, sr >> 3)};
+            R cs = R(0);
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+              const R mq = __shfl_xor_sync(0xffffffffu, v, w);
+              rsum = fma(mq, nq[w], rsum);
+              cs = fma(mq, nw[w], cs);
+            }
+            csum[u] = cs;
+          }
+          s_team[team][tw][lane] = rsum;
+          if (!diag) {
+            // over the rows: lanes below 16 keep the first column, the others the second
+            const bool up = lane & 16;
+            R cs = (up ? csum[1] : csum[0]) + __shfl_xor_sync(0xffffffffu, up ? csum[0] : csum[1], 16);
+            cs += __shfl_xor_sync(0xffffffffu, cs, 8);
+            cs += __shfl_xor_sync(0xffffffffu, cs, 4);
+            const int gc = J * T + 2 * tw + (lane >> 4);
+            if ((lane & 12) == 0 && gc < m) reinterpret_cast<R*>(gr.part + (size_t)I * m + gc)[k] = cs;
+          }
+          asm volatile("bar.sync %0, 128;" ::"r"(1 + team) : "memory");
+          if (tw == 0) {
+            const R sum = (s_team[team][0][lane] + s_team[team][1][lane]) + (s_team[team][2][lane] + s_team[team][3][lane]);
+            if (rin) reinterpret_cast<R*>(gr.part + (size_t)J * m + gr_)[k] = sum;
+            const R nk = rin ? reinterpret_cast<const R*>(wn + rl)[k] : R(0);
+            cacc = fma(diag ? nk : nk + nk, sum, cacc);  // an off-diagonal tile stands for its mirror too
+          }
+          asm volatile("bar.sync %0, 128;" ::"r"(1 + team) : "memory");  // the sums are read
+        }
+      }
+    }
+    for (int q = warp; !teams && rank + q * G < live; q += RT_WARPS) {
       int I, J;
       rt_tile(rank + q * G, nt, I, J);
       R* tl = tiles + (size_t)q * TILE;

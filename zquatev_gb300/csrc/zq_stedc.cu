@@ -50,11 +50,27 @@ __device__ __forceinline__ int dc_find_node(const DcNode* nodes, int cnt, int po
 
 template <typename ZT>
 __global__ void k_dc_leaf(const DcNode* nodes, int cnt, const double* dmod, ZT* Zout, double* lamout) {
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= cnt) return;
   const int a = nodes[i].a;
   Zout[nodes[i].zoff + a + (int64_t)a * nodes[i].ld] = (ZT)1;
   lamout[a] = dmod[a];
+}
+
+// What the secular equation reads of the kept poles: rho z^2, and float copies for
+// its first iterations (pole as a pair hi + lo, rho z^2), in areas whose staged
+// contents are no longer needed.
+__device__ __forceinline__ float2* dc_pole_pairs(const DcWork& w) { return reinterpret_cast<float2*>(w.sd); }
+__device__ __forceinline__ float* dc_pole_weights(const DcWork& w) { return reinterpret_cast<float*>(w.perm); }
+__device__ __forceinline__ void dc_publish_poles(const DcWork& w, int a, int K, double rho2) {
+  for (int q = threadIdx.x; q < K; q += blockDim.x) {
+    const double d = w.nd_val[a + q], z = w.nd_z[a + q], rz = rho2 * z * z;
+    const float hi = (float)d;
+    w.sz[a + q] = rz;
+    dc_pole_pairs(w)[a + q] = make_float2(hi, (float)(d - (double)hi));
+    dc_pole_weights(w)[a + q] = (float)rz;
+  }
 }
 
 // one CTA per internal node. The merged poles (value, z, source column) are
@@ -67,6 +83,7 @@ constexpr int DC_SCAP = 8192;  // largest node staged in shared memory (20 bytes
 template <typename ZT>
 __global__ void __launch_bounds__(256) k_dc_prepare(DcNode* nodes, DcWork w, const ZT* Zin, const double* lamin,
                                                     int scap) {
+  pdl_wait();
   extern __shared__ double dc_sm[];
   DcNode& nd = nodes[blockIdx.x];
   const int a = nd.a, c = nd.c, b = nd.b;
@@ -159,8 +176,8 @@ __global__ void __launch_bounds__(256) k_dc_prepare(DcNode* nodes, DcWork w, con
     }
     __syncthreads();
     if (!s_flag) {
-      // rho z^2 for the secular equation (the staging area is free now)
-      for (int q = tid; q < Ktot; q += blockDim.x) w.sz[a + q] = rho2 * w.nd_z[a + q] * w.nd_z[a + q];
+      __syncthreads();
+      dc_publish_poles(w, a, Ktot, rho2);
       if (tid == 0) { nd.K = Ktot; nd.ndefl = m - Ktot; nd.nrot = 0; nd.rho2 = rho2; }
       return;
     }
@@ -198,7 +215,7 @@ __global__ void __launch_bounds__(256) k_dc_prepare(DcNode* nodes, DcWork w, con
     s_cnt[1] = K;
   }
   __syncthreads();
-  for (int q = tid; q < s_cnt[1]; q += blockDim.x) w.sz[a + q] = rho2 * w.nd_z[a + q] * w.nd_z[a + q];
+  dc_publish_poles(w, a, s_cnt[1], rho2);
   // sort the deflated list (values, columns) by rank; ties by index
   const int nd_ = s_cnt[0];
   const double* fv = w.df_val + a;
@@ -227,14 +244,85 @@ __global__ void __launch_bounds__(256) k_dc_prepare(DcNode* nodes, DcWork w, con
 // takes ten: the products rho z^2 are formed once (w.sz), the reciprocal is
 // 1/del from the approximate instruction and one cubically convergent Newton
 // step (relative error below 2^-52), and the two sides of the root share one
-// accumulation loop each.
+// accumulation loop each. The root is first approached in FP32 (dc_approach),
+// whose instructions cost a sixteenth, so that two or three FP64 iterations remain.
 __device__ __forceinline__ double dc_recip(double d) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
   const double e = fma(-d, y, 1.0);
   return fma(y, fma(e, e, e), y);
 }
+// The step of the two-pole rational model around tau, for root i between the
+// poles at distances di, dj (i = K - 1: one pole): f the function's value, dpsi,
+// dphi the derivatives of its two sums. False: no step.
+template <typename T>
+__device__ __forceinline__ bool dc_model_step(bool inner, T di, T dj, T f, T dpsi, T dphi, T& eta) {
+  if (inner) {
+    const T B1 = di * di * dpsi, B2 = dj * dj * dphi;
+    const T qa = f - B1 / di - B2 / dj;
+    const T qb = qa * (di + dj) + B1 + B2;
+    const T qc = qa * di * dj + B1 * dj + B2 * di;
+    // roots of qa x^2 - qb x + qc = 0
+    if (qa == T(0)) {
+      if (qb == T(0)) return false;
+      eta = qc / qb;
+      return true;
+    }
+    const T disc = qb * qb - T(4) * qa * qc;
+    if (!(disc >= T(0))) return false;
+    const T sq = sqrt(disc);
+    const T den = (qb >= T(0)) ? (qb + sq) : (qb - sq);
+    const T r1 = den / (T(2) * qa);
+    const T r2 = (den != T(0)) ? T(2) * qc / den : r1;
+    if (r2 > di && r2 < dj) { eta = r2; return true; }
+    if (r1 > di && r1 < dj) { eta = r1; return true; }
+    return false;
+  }
+  const T B1 = di * di * dpsi;
+  const T c = f - B1 / di;
+  if (!(c > T(0))) return false;
+  eta = di + B1 / c;
+  return true;
+}
+// A first value for root i (origin o, tau in (lo, hi)): the same iteration in
+// FP32, on pole distances taken from the pairs. A guess only: the FP64 iteration
+// starts from it with its own bracket.
+__device__ float dc_approach(const float2* D, const float* rz, int K, int i, int o, int lane, int above, float lo,
+                             float hi) {
+  const float2 Do = D[o];
+  auto dist = [&](int k) { const float2 d = D[k]; return (d.x - Do.x) + (d.y - Do.y); };
+  float tau = 0.5f * (lo + hi);
+  for (int it = 0; it < 24; ++it) {
+    float psi = 0.f, phi = 0.f, dpsi = 0.f, dphi = 0.f;
+#pragma unroll 4
+    for (int k = lane; k <= i; k += 32) {
+      const float inv = __frcp_rn(dist(k) - tau), t = rz[k] * inv;
+      psi += t;
+      dpsi = fmaf(t, inv, dpsi);
+    }
+#pragma unroll 4
+    for (int k = above; k < K; k += 32) {
+      const float inv = __frcp_rn(dist(k) - tau), t = rz[k] * inv;
+      phi += t;
+      dphi = fmaf(t, inv, dphi);
+    }
+    psi = warp_sum(psi); phi = warp_sum(phi); dpsi = warp_sum(dpsi); dphi = warp_sum(dphi);
+    const float f = 1.f + psi + phi;
+    if (f < 0.f) lo = tau; else hi = tau;
+    if (!(fabsf(f) > 1e-6f * (1.f + fabsf(psi) + fabsf(phi)))) break;  // (also when not a number)
+    float eta, tn = 0.5f * (lo + hi);
+    if (dc_model_step(i < K - 1, dist(i) - tau, i < K - 1 ? dist(i + 1) - tau : 0.f, f, dpsi, dphi, eta)) {
+      const float t = tau + eta;
+      if (t > lo && t < hi) tn = t;
+    }
+    const bool done = fabsf(tn - tau) <= 1e-6f * fabsf(tn);
+    tau = tn;
+    if (done) break;
+  }
+  return tau;
+}
 __global__ void __launch_bounds__(128) k_dc_secular(const DcNode* nodes, int cnt, DcWork w) {
+  pdl_wait();
   const int pos = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   const int ni = dc_find_node(nodes, cnt, pos);
@@ -263,6 +351,10 @@ __global__ void __launch_bounds__(128) k_dc_secular(const DcNode* nodes, int cnt
   }
   const double Do = D[o];
   double tau = 0.5 * (lo + hi);
+  {
+    const double t = (double)dc_approach(dc_pole_pairs(w) + a, dc_pole_weights(w) + a, K, i, o, lane, above, (float)lo, (float)hi);
+    if (t > lo && t < hi) tau = t;
+  }
   for (int it = 0; it < 200; ++it) {
     double psi = 0.0, phi = 0.0, dpsi = 0.0, dphi = 0.0;
 #pragma unroll 4
@@ -286,36 +378,8 @@ __global__ void __launch_bounds__(128) k_dc_secular(const DcNode* nodes, int cnt
     const double errb = 8.0 * DEPS * (1.0 + fabs(psi) + fabs(phi)) + DEPS * fabs(tau) * (dpsi + dphi);
     if (fabs(f) <= errb) break;
     if (hi - lo <= 2.0 * DEPS * fmax(fabs(lo), fabs(hi))) break;
-    // two-pole rational model around the current point
-    const double di = (D[i] - Do) - tau;
-    double eta;
-    bool ok = false;
-    if (i < K - 1) {
-      const double dj = (D[i + 1] - Do) - tau;
-      const double B1 = di * di * dpsi, B2 = dj * dj * dphi;
-      const double cc0 = f - B1 / di - B2 / dj;
-      const double qa = cc0;
-      const double qb = cc0 * (di + dj) + B1 + B2;
-      const double qc = cc0 * di * dj + B1 * dj + B2 * di;
-      // roots of qa x^2 - qb x + qc = 0
-      if (qa == 0.0) {
-        if (qb != 0.0) { eta = qc / qb; ok = true; }
-      } else {
-        const double disc = qb * qb - 4.0 * qa * qc;
-        if (disc >= 0.0) {
-          const double sq = sqrt(disc);
-          const double den = (qb >= 0.0) ? (qb + sq) : (qb - sq);
-          const double r1 = den / (2.0 * qa);
-          const double r2 = (den != 0.0) ? 2.0 * qc / den : r1;
-          const bool in1 = (r1 > di && r1 < dj), in2 = (r2 > di && r2 < dj);
-          if (in2) { eta = r2; ok = true; } else if (in1) { eta = r1; ok = true; }
-        }
-      }
-    } else {
-      const double B1 = di * di * dpsi;
-      const double cc0 = f - B1 / di;
-      if (cc0 > 0.0) { eta = di + B1 / cc0; ok = true; }
-    }
+    double eta = 0.0;
+    const bool ok = dc_model_step(i < K - 1, (D[i] - Do) - tau, i < K - 1 ? (D[i + 1] - Do) - tau : 0.0, f, dpsi, dphi, eta);
     double tn = ok ? tau + eta : 0.5 * (lo + hi);
     if (!(tn > lo && tn < hi)) tn = 0.5 * (lo + hi);
     if (tn == tau) break;
@@ -331,6 +395,7 @@ __global__ void __launch_bounds__(128) k_dc_secular(const DcNode* nodes, int cnt
 // Gu-Eisenstat: zhat_k from the computed roots; one warp per k, the product
 // over the roots split over the lanes
 __global__ void __launch_bounds__(128) k_dc_zhat(const DcNode* nodes, int cnt, DcWork w) {
+  pdl_wait();
   const int pos = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   const int ni = dc_find_node(nodes, cnt, pos);
@@ -363,6 +428,7 @@ __global__ void __launch_bounds__(128) k_dc_zhat(const DcNode* nodes, int cnt, D
 // one CTA per column slot of every internal node: writes a full column of M
 template <typename ZT>
 __global__ void __launch_bounds__(128) k_dc_vectors(const DcNode* nodes, int cnt, DcWork w, ZT* Mb, double* lamout) {
+  pdl_wait();
   const int pos = blockIdx.x;
   const int ni = dc_find_node(nodes, cnt, pos);
   if (ni < 0) return;
@@ -417,6 +483,7 @@ __global__ void __launch_bounds__(128) k_dc_vectors(const DcNode* nodes, int cnt
 // apply the deflation rotations (in reverse order) to every column of M
 template <typename ZT>
 __global__ void k_dc_rotate(const DcNode* nodes, int cnt, DcWork w, ZT* Mb) {
+  pdl_wait();
   const int pos = blockIdx.x * blockDim.x + threadIdx.x;
   const int ni = dc_find_node(nodes, cnt, pos);
   if (ni < 0) return;
@@ -436,6 +503,7 @@ __global__ void k_dc_rotate(const DcNode* nodes, int cnt, DcWork w, ZT* Mb) {
 // Scale and tear, one block per matrix: the largest |entry| becomes 1, the
 // off-diagonals leave the diagonal.
 __global__ void k_dc_scale(const double* d, const double* e, const DcMat* mats, double* dmod, double* es, double* scal) {
+  pdl_wait();
   __shared__ double sh[32];
   const DcMat mt = mats[blockIdx.x];
   const int n = mt.n;
@@ -458,6 +526,7 @@ __global__ void k_dc_scale(const double* d, const double* e, const DcMat* mats, 
 
 // eigenvalues times the scale, into place (NaN when a merge product failed)
 __global__ void k_dc_unscale(const double* lam, const DcMat* mats, const double* scal, double* eig, const int* err) {
+  pdl_wait();
   const DcMat mt = mats[blockIdx.y];
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= mt.n) return;
@@ -471,6 +540,7 @@ __global__ void k_dc_unscale(const double* lam, const DcMat* mats, const double*
 template <typename ZT>
 __global__ void __launch_bounds__(256) k_dc_merge(const DcNode* nodes, int cnt, const ZT* Zin, const ZT* Mb, ZT* Zout,
                                                   int mmax) {
+  pdl_wait();
   const DcNode nd = nodes[blockIdx.x];
   const int m = nd.b - nd.a;
   const int64_t ld = nd.ld, o = nd.zoff + nd.a + (int64_t)nd.a * ld;
@@ -493,6 +563,7 @@ __global__ void __launch_bounds__(256) k_dc_merge(const DcNode* nodes, int cnt, 
 }
 
 __global__ void k_dc_setrho(DcNode* nodes, int cnt, const double* es) {
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < cnt && nodes[i].b - nodes[i].a > 1) nodes[i].rho = es[nodes[i].c - 1];
 }
@@ -706,10 +777,10 @@ static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, 
   int nmax = 0;
   for (const DcMat& m : P.mats_host) nmax = std::max(nmax, m.n);
   ZQ_CUDA(cudaMemsetAsync(P.err, 0, sizeof(int), st));
-  k_dc_scale<<<nmat, nmax <= 256 ? 64 : 256, 0, st>>>(d, e, P.mats_dev, P.dmod, P.es, P.scal);
+  ZQ_CUDA(launch_pdl_smem(k_dc_scale, dim3(nmat), dim3(nmax <= 256 ? 64 : 256), 0, st, d, e, P.mats_dev, P.dmod, P.es, P.scal));
   ZQ_LAUNCH_CHECK();
   if (!P.nodes_host.empty()) {
-    k_dc_setrho<<<ceil_div((int)P.nodes_host.size(), 256), 256, 0, st>>>(P.nodes_dev, (int)P.nodes_host.size(), P.es);
+    ZQ_CUDA(launch_pdl_smem(k_dc_setrho, dim3(ceil_div((int)P.nodes_host.size(), 256)), dim3(256), 0, st, P.nodes_dev, (int)P.nodes_host.size(), P.es));
     ZQ_LAUNCH_CHECK();
   }
   // Z buffers need zeros outside the diagonal blocks only where they are read:
@@ -720,8 +791,8 @@ static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, 
     double* lo = P.lam[t & 1];
     const double* li = P.lam[(t + 1) & 1];
     if (P.leaf_cnt[t] > 0) {
-      k_dc_leaf<ZT><<<ceil_div(P.leaf_cnt[t], 128), 128, 0, st>>>(P.nodes_dev + P.leaf_off[t], P.leaf_cnt[t], P.dmod, Zo,
-                                                                    lo);
+      ZQ_CUDA(launch_pdl_smem(k_dc_leaf<ZT>, dim3(ceil_div(P.leaf_cnt[t], 128)), dim3(128), 0, st, P.nodes_dev + P.leaf_off[t], P.leaf_cnt[t], P.dmod, Zo,
+                                                                    lo));
       ZQ_LAUNCH_CHECK();
     }
     const int cnt = P.depth_cnt[t];
@@ -741,21 +812,21 @@ static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, 
           attr_set.fetch_or(bit);
         }
       }
-      k_dc_prepare<ZT><<<cnt, 256, smem, st>>>(nd, P.w, Zi, li, scap);
+      ZQ_CUDA(launch_pdl_smem(k_dc_prepare<ZT>, dim3(cnt), dim3(256), smem, st, nd, P.w, Zi, li, scap));
       ZQ_LAUNCH_CHECK();
     }
-    k_dc_secular<<<ceil_div(n, 4), 128, 0, st>>>(nd, cnt, P.w);
+    ZQ_CUDA(launch_pdl_smem(k_dc_secular, dim3(ceil_div(n, 4)), dim3(128), 0, st, nd, cnt, P.w));
     ZQ_LAUNCH_CHECK();
-    k_dc_zhat<<<ceil_div(n, 4), 128, 0, st>>>(nd, cnt, P.w);
+    ZQ_CUDA(launch_pdl_smem(k_dc_zhat, dim3(ceil_div(n, 4)), dim3(128), 0, st, nd, cnt, P.w));
     ZQ_LAUNCH_CHECK();
-    k_dc_vectors<ZT><<<n, 128, 0, st>>>(nd, cnt, P.w, Mb, lo);
+    ZQ_CUDA(launch_pdl_smem(k_dc_vectors<ZT>, dim3(n), dim3(128), 0, st, nd, cnt, P.w, Mb, lo));
     ZQ_LAUNCH_CHECK();
-    k_dc_rotate<ZT><<<ceil_div(n, 128), 128, 0, st>>>(nd, cnt, P.w, Mb);
+    ZQ_CUDA(launch_pdl_smem(k_dc_rotate<ZT>, dim3(ceil_div(n, 128)), dim3(128), 0, st, nd, cnt, P.w, Mb));
     ZQ_LAUNCH_CHECK();
     if (P.depth_mmax[t] <= DC_MERGE_MAX) {
       const int mm = P.depth_mmax[t];
       const dim3 grid((unsigned)cnt, (unsigned)std::min(64, ceil_div(mm * mm, 256)));
-      k_dc_merge<ZT><<<grid, mm <= 8 ? 64 : 256, 0, st>>>(nd, cnt, Zi, Mb, Zo, mm);
+      ZQ_CUDA(launch_pdl_smem(k_dc_merge<ZT>, grid, dim3(mm <= 8 ? 64 : 256), 0, st, nd, cnt, Zi, Mb, Zo, mm));
       ZQ_LAUNCH_CHECK();
     } else if (P.gemm_tiles[t] > 0) {
       bool done = false;
@@ -795,8 +866,8 @@ static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, 
       }
     }
   }
-  k_dc_unscale<<<dim3((unsigned)ceil_div(nmax, 128), (unsigned)nmat), 128, 0, st>>>(P.lam[0], P.mats_dev, P.scal, lam_out,
-                                                                                    P.err);
+  ZQ_CUDA(launch_pdl_smem(k_dc_unscale, dim3((unsigned)ceil_div(nmax, 128), (unsigned)nmat), dim3(128), 0, st, P.lam[0], P.mats_dev, P.scal, lam_out,
+                                                                                    P.err));
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }
