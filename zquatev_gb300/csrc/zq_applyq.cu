@@ -111,6 +111,7 @@ __device__ __forceinline__ void aq_segment(ColState<NW, NR>& s, int j, double (*
 
 template <int NW, int NR>
 __global__ void __launch_bounds__(32 * NW) k_apply_q(const ApplyQTask* tasks, const int* task_of, ApplyQTask one, int first) {
+  pdl_wait();
   constexpr int RP = 8 * NW;  // rows per pass
   extern __shared__ __align__(16) unsigned char aq_smem[];
   __shared__ double s_red[2][NW][4];
@@ -219,6 +220,7 @@ __device__ __forceinline__ void aw_segment(WarpState<NP>& s, int j, double (&wn)
 // have idle warps, which still take part in the staging)
 template <int NP, int U>
 __global__ void __launch_bounds__(32 * AW) k_apply_q_warp(const ApplyQTask* tasks, const int2* blocks, double2* base) {
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char aq_smem[];
   const int2 bl = blocks[blockIdx.x];  // (task, first column)
   ApplyQTask t = tasks[bl.x];
@@ -255,13 +257,14 @@ template <int NP, int U>
 int launch_warp(const ApplyQTask* tasks, const int2* blocks, double2* base, int count, cudaStream_t st) {
   constexpr int smem = 3 * (int)sizeof(W4) * 8 * NP;
   static_assert(smem <= 47 * 1024, "shared memory");
-  k_apply_q_warp<NP, U><<<count, 32 * AW, smem, st>>>(tasks, blocks, base);
+  ZQ_CUDA(launch_pdl_smem(k_apply_q_warp<NP, U>, dim3(count), dim3(32 * AW), smem, st, tasks, blocks, base));
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }
 
 // (U; V) from the right half into the left half, (-conj V; conj U) in its place
 __global__ void k_apply_q_finish(const ApplyQTask* tasks, const int* task_of, ApplyQTask one, int first) {
+  pdl_wait();
   ApplyQTask t = one;
   int col = first + blockIdx.x;
   if (tasks) {
@@ -294,7 +297,7 @@ int launch(const ApplyQTask* tasks, const int* task_of, const ApplyQTask& one, i
       set.fetch_or(bit);
     }
   }
-  k_apply_q<NW, NR><<<cols, 32 * NW, smem, st>>>(tasks, task_of, one, first);
+  ZQ_CUDA(launch_pdl_smem(k_apply_q<NW, NR>, dim3(cols), dim3(32 * NW), smem, st, tasks, task_of, one, first));
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }
@@ -339,7 +342,7 @@ int apply_q_warp(const ApplyQTask* tasks, const int2* blocks, int count, double2
 
 int apply_q_finish(const ApplyQTask* tasks, const int* task_of, const ApplyQTask& one, int first, int cols, int nmax,
                    cudaStream_t st) {
-  k_apply_q_finish<<<cols, nmax <= 64 ? 64 : 128, 0, st>>>(tasks, task_of, one, first);
+  ZQ_CUDA(launch_pdl_smem(k_apply_q_finish, dim3(cols), dim3(nmax <= 64 ? 64 : 128), 0, st, tasks, task_of, one, first));
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }

@@ -66,6 +66,7 @@ __device__ __forceinline__ Quat qunit_of(const double* e, int k, double& nrm) {
 // 59 us at n = 23, 78 us at n = 750; now 8 and 41 us).
 constexpr int PH_T = 256;
 __global__ void __launch_bounds__(PH_T) k_phase(const double* e, int n, double* offd, double* phi, const DcMat* mats) {
+  pdl_wait();
   __shared__ Quat s_q[PH_T];
   if (mats) {
     const DcMat mt = mats[blockIdx.x];
@@ -109,7 +110,7 @@ static int phase_threads(int n) { return n <= 32 ? 32 : (n <= 256 ? 64 : (n <= 1
 
 int phase_reduce(const double* e, int n, double* offd, double* phi, cudaStream_t st) {
   if (n <= 0) return ZQ_OK;
-  k_phase<<<1, phase_threads(n), 0, st>>>(e, n, offd, phi, nullptr);
+  ZQ_CUDA(launch_pdl_smem(k_phase, dim3(1), dim3(phase_threads(n)), 0, st, e, n, offd, phi, nullptr));
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }
@@ -117,7 +118,7 @@ int phase_reduce(const double* e, int n, double* offd, double* phi, cudaStream_t
 int phase_reduce_forest(const double* e, const DcMat* mats, int count, int nmax, double* offd, double* phi,
                         cudaStream_t st) {
   if (count <= 0) return ZQ_OK;
-  k_phase<<<count, phase_threads(nmax), 0, st>>>(e, nmax, offd, phi, mats);
+  ZQ_CUDA(launch_pdl_smem(k_phase, dim3(count), dim3(phase_threads(nmax)), 0, st, e, nmax, offd, phi, mats));
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }
@@ -125,6 +126,7 @@ int phase_reduce_forest(const double* e, const DcMat* mats, int count, int nmax,
 // X = [diag(alpha); diag(beta)]
 template <typename Z>
 __global__ void k_init_x(Z* X, int64_t ldx, int n, const double* phi) {
+  pdl_wait();
   const int64_t total = (int64_t)2 * n * n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int r = (int)(t % (2 * n));
@@ -139,6 +141,7 @@ __global__ void k_init_x(Z* X, int64_t ldx, int n, const double* phi) {
 // pack the block's reflectors: Wa[r, i] = A(p+1+r, p+i) for r >= i, else 0 (same for B)
 template <typename Z>
 __global__ void k_pack_w(const Z* M, int64_t ldm, int n, int p, int kb, int L, Z* Wa, Z* Wb) {
+  pdl_wait();
   const int64_t total = (int64_t)L * kb;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int r = (int)(t % L), i = (int)(t / L);
@@ -160,6 +163,7 @@ __global__ void k_pack_w(const Z* M, int64_t ldm, int n, int p, int kb, int L, Z
 constexpr int BT_G = 16;
 template <typename Z>
 __global__ void __launch_bounds__(1024) k_build_t(const Z* G1, const Z* G2, int kb, Z* Ta, Z* Tb) {
+  pdl_wait();
   const int tid = threadIdx.x;
   const int i = tid & 63, g = tid >> 6;
   __shared__ Z red[BT_G][64][2];
@@ -201,6 +205,7 @@ __global__ void __launch_bounds__(1024) k_build_t(const Z* G1, const Z* G2, int 
 // a shared-memory load away instead of an L2 round trip.
 __global__ void __launch_bounds__(1024) k_build_t_sm(const float2* G1, const float2* G2, int kb, float2* Ta,
                                                      float2* Tb) {
+  pdl_wait();
   extern __shared__ float2 bt_sm[];
   float2* g1 = bt_sm;
   float2* g2 = g1 + kb * kb;
@@ -287,7 +292,7 @@ int form_q(const cplx<R>* M, int64_t ldm, int n, const double* phi, cplx<R>* X, 
   const bool fp32 = std::is_same<R, float>::value && tc_err != nullptr;
   const bool use_tc = fp32 && fp32_products_on_tensor_cores(TC_USE_FORMQ);     // C1 = W^H X (inner L)
   const bool use_tc_x = fp32 && fp32_products_on_tensor_cores(TC_USE_FORMQ_X); // X -= W C2 (inner nbq)
-  k_init_x<Z><<<ceil_div(2 * n * n, 256) > 4096 ? 4096 : ceil_div(2 * n * n, 256), 256, 0, st>>>(X, ldx, n, phi);
+  ZQ_CUDA(launch_pdl_smem(k_init_x<Z>, dim3(ceil_div(2 * n * n, 256) > 4096 ? 4096 : ceil_div(2 * n * n, 256)), dim3(256), 0, st, X, ldx, n, phi));
   ZQ_LAUNCH_CHECK();
   const int nref = n - 2;  // reflectors exist for columns 0..n-3
   if (nref <= 0) return ZQ_OK;
@@ -329,8 +334,7 @@ int form_q(const cplx<R>* M, int64_t ldm, int n, const double* phi, cplx<R>* X, 
     const int pb = bi * nbq;
     const int kb = (nbq < nref - pb) ? nbq : (nref - pb);
     const int L = n - 1 - pb;
-    k_pack_w<Z><<<ceil_div(L * kb, 256) > 2048 ? 2048 : ceil_div(L * kb, 256), 256, 0, sp>>>(M, ldm, n, pb, kb, L, s.Wa,
-                                                                                           s.Wb);
+    ZQ_CUDA(launch_pdl_smem(k_pack_w<Z>, dim3(ceil_div(L * kb, 256) > 2048 ? 2048 : ceil_div(L * kb, 256)), dim3(256), 0, sp, M, ldm, n, pb, kb, L, s.Wa, s.Wb));
     ZQ_LAUNCH_CHECK();
     // G1 = Wa^H Wa + Wb^H Wb ; G2 = Wa^T Wb - Wb^T Wa   (kb x kb, inner L)
     Args g{};
@@ -353,9 +357,9 @@ int form_q(const cplx<R>* M, int64_t ldm, int n, const double* phi, cplx<R>* X, 
         ZQ_CUDA(cudaFuncSetAttribute(k_build_t_sm, cudaFuncAttributeMaxDynamicSharedMemorySize, 4 * 64 * 64 * 8));
         attr_set.fetch_or(bit);
       }
-      k_build_t_sm<<<1, 1024, sm, sp>>>(s.G1, s.G2, kb, s.Ta, s.Tb);
+      ZQ_CUDA(launch_pdl_smem(k_build_t_sm, dim3(1), dim3(1024), sm, sp, s.G1, s.G2, kb, s.Ta, s.Tb));
     } else {
-      k_build_t<Z><<<1, 1024, 0, sp>>>(s.G1, s.G2, kb, s.Ta, s.Tb);
+      ZQ_CUDA(launch_pdl_smem(k_build_t<Z>, dim3(1), dim3(1024), 0, sp, s.G1, s.G2, kb, s.Ta, s.Tb));
     }
     ZQ_LAUNCH_CHECK();
     return ZQ_OK;
@@ -563,6 +567,7 @@ template int apply_z<double>(const cplx<double>*, int64_t, const double*, int64_
 template int apply_z<float>(const cplx<float>*, int64_t, const float*, int64_t, int, cplx<float>*, int64_t, DgemmDescT<float>*, cudaStream_t, int*);
 
 __global__ void k_symfill(double2* D, int64_t ld, int n) {
+  pdl_wait();
   const int64_t total = (int64_t)n * n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int j = (int)(t % n), i = (int)(t / n);
@@ -577,7 +582,7 @@ int symmetry_fill(double2* D, int64_t ld, int n, cudaStream_t st) {
   if (n <= 0) return ZQ_OK;
   const int64_t total = (int64_t)n * n;
   const int blocks = (int)((total + 255) / 256 > 8192 ? 8192 : (total + 255) / 256);
-  k_symfill<<<blocks, 256, 0, st>>>(D, ld, n);
+  ZQ_CUDA(launch_pdl_smem(k_symfill, dim3(blocks), dim3(256), 0, st, D, ld, n));
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }

@@ -120,6 +120,7 @@ template <bool CPLX>
 __global__ void __launch_bounds__(256) k_crt_split(CrtSide s, bool is_a, int count, int count_pad, int Kp,
                                                    const int* __restrict__ exps, int bits, int moduli,
                                                    __nv_bfloat16* __restrict__ out) {
+  pdl_wait();
   using E = typename std::conditional<CPLX, double2, double>::type;
   __shared__ E tile[32][65];  // padded: a column of the tile is read and written without conflicts too
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -202,11 +203,13 @@ __global__ void __launch_bounds__(256) k_crt_split(CrtSide s, bool is_a, int cou
 
 // exponents (2^e above the largest magnitude) of a real operand's rows (A) or columns (B)
 __global__ void k_crt_exp_init(int* e, int n) {
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) e[i] = -1100;
 }
 __global__ void __launch_bounds__(256) k_crt_exp_real(const double* __restrict__ X, int64_t ld, int count, int K, bool is_a,
                                                       int* __restrict__ exps) {
+  pdl_wait();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   unsigned long long mb = 0;
   if (is_a) {  // rows: 32 per block column, 256 columns per block row
@@ -260,6 +263,7 @@ __device__ __forceinline__ int crt_mod(int v, int p, float ip) {
 
 __global__ void __launch_bounds__(CB_THREADS, 1)
     k_crt_mma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const CrtMma g) {
+  pdl_wait();
   extern __shared__ __align__(1024) unsigned char cb_raw[];
   const uint32_t raw = su32(cb_raw);
   const uint32_t ring = (raw + 1023u) & ~1023u;
@@ -454,6 +458,7 @@ __global__ void __launch_bounds__(256) k_crt_join(const uint8_t* __restrict__ R,
                                                   int m, int n, int bits, const int* __restrict__ ea,
                                                   const int* __restrict__ eb, int lower, double* __restrict__ C,
                                                   int64_t ldc) {
+  pdl_wait();
   constexpr int PR = CPLX ? 3 : 1;
   const int m4 = (m + 3) / 4;
   const int64_t total = (int64_t)m4 * n;
@@ -580,8 +585,7 @@ CrtShape crt_shape(int m, int n, int K, int moduli, bool cplx) {
 
 int crt_split(const CrtSide& s, bool is_a, int count, int count_pad, int Kp, const int* exps, int bits, int moduli,
               void* out, cudaStream_t st) {
-  k_crt_split<true><<<dim3((unsigned)(count_pad / 32), (unsigned)(Kp / 64)), 256, 0, st>>>(
-      s, is_a, count, count_pad, Kp, exps, bits, moduli, reinterpret_cast<__nv_bfloat16*>(out));
+  ZQ_CUDA(launch_pdl_smem(k_crt_split<true>, dim3((unsigned)(count_pad / 32), (unsigned)(Kp / 64)), dim3(256), 0, st, s, is_a, count, count_pad, Kp, exps, bits, moduli, reinterpret_cast<__nv_bfloat16*>(out)));
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }
@@ -616,13 +620,15 @@ int crt_multiply(const CrtShape& sh, const void* a, const void* b, void* r, bool
   cfg.blockDim = dim3(CB_THREADS);
   cfg.dynamicSmemBytes = CB_SMEM;
   cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = 2;
   prof_add_flops(PC_OZAKI, 2.0 * g.jobs * CB_M * CB_N * (double)sh.Kp);
   prof_begin(PC_OZAKI, st);
   ZQ_CUDA(cudaLaunchKernelEx(&cfg, k_crt_mma, ta, tb, g));
@@ -638,11 +644,9 @@ int crt_join(const CrtShape& sh, const void* r, int m, int n, int bits, const in
   const CrtJoin cj = crt_constants(sh.moduli);
   const uint8_t* R = reinterpret_cast<const uint8_t*>(r);
   if (sh.prods == 3)
-    k_crt_join<true><<<grid, 256, 0, st>>>(R, sh.mp, sh.np, sh.moduli, cj, m, n, bits, ea, eb, lower ? 1 : 0,
-                                           reinterpret_cast<double*>(C), ldc);
+    ZQ_CUDA(launch_pdl_smem(k_crt_join<true>, dim3(grid), dim3(256), 0, st, R, sh.mp, sh.np, sh.moduli, cj, m, n, bits, ea, eb, lower ? 1 : 0, reinterpret_cast<double*>(C), ldc));
   else
-    k_crt_join<false><<<grid, 256, 0, st>>>(R, sh.mp, sh.np, sh.moduli, cj, m, n, bits, ea, eb, lower ? 1 : 0,
-                                            reinterpret_cast<double*>(C), ldc);
+    ZQ_CUDA(launch_pdl_smem(k_crt_join<false>, dim3(grid), dim3(256), 0, st, R, sh.mp, sh.np, sh.moduli, cj, m, n, bits, ea, eb, lower ? 1 : 0, reinterpret_cast<double*>(C), ldc));
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }
@@ -668,20 +672,18 @@ int crt_dgemm(int m, int n, int k, const double* A, int64_t lda, const double* B
   int* ea = reinterpret_cast<int*>(take(sizeof(int) * sh.mp));
   int* eb = ea + sh.mp;
   take(sizeof(int) * sh.np);
-  k_crt_exp_init<<<ceil_div(sh.mp + sh.np, 256), 256, 0, st>>>(ea, sh.mp + sh.np);
+  ZQ_CUDA(launch_pdl_smem(k_crt_exp_init, dim3(ceil_div(sh.mp + sh.np, 256)), dim3(256), 0, st, ea, sh.mp + sh.np));
   ZQ_LAUNCH_CHECK();
-  k_crt_exp_real<<<dim3((unsigned)ceil_div(m, 32), (unsigned)ceil_div(k, 256)), 256, 0, st>>>(A, lda, m, k, true, ea);
+  ZQ_CUDA(launch_pdl_smem(k_crt_exp_real, dim3((unsigned)ceil_div(m, 32), (unsigned)ceil_div(k, 256)), dim3(256), 0, st, A, lda, m, k, true, ea));
   ZQ_LAUNCH_CHECK();
-  k_crt_exp_real<<<dim3((unsigned)ceil_div(n, 8)), 256, 0, st>>>(B, ldb, n, k, false, eb);
+  ZQ_CUDA(launch_pdl_smem(k_crt_exp_real, dim3((unsigned)ceil_div(n, 8)), dim3(256), 0, st, B, ldb, n, k, false, eb));
   ZQ_LAUNCH_CHECK();
   CrtSide s{};
   s.X1 = reinterpret_cast<const double2*>(A); s.ld1 = lda; s.op1 = OP_N; s.K1 = k;
-  k_crt_split<false><<<dim3((unsigned)(sh.mp / 32), (unsigned)(sh.Kp / 64)), 256, 0, st>>>(
-      s, true, m, sh.mp, sh.Kp, ea, CRT_FP64_BITS, L, reinterpret_cast<__nv_bfloat16*>(a));
+  ZQ_CUDA(launch_pdl_smem(k_crt_split<false>, dim3((unsigned)(sh.mp / 32), (unsigned)(sh.Kp / 64)), dim3(256), 0, st, s, true, m, sh.mp, sh.Kp, ea, CRT_FP64_BITS, L, reinterpret_cast<__nv_bfloat16*>(a)));
   ZQ_LAUNCH_CHECK();
   s.X1 = reinterpret_cast<const double2*>(B); s.ld1 = ldb;
-  k_crt_split<false><<<dim3((unsigned)(sh.np / 32), (unsigned)(sh.Kp / 64)), 256, 0, st>>>(
-      s, false, n, sh.np, sh.Kp, eb, CRT_FP64_BITS, L, reinterpret_cast<__nv_bfloat16*>(b));
+  ZQ_CUDA(launch_pdl_smem(k_crt_split<false>, dim3((unsigned)(sh.np / 32), (unsigned)(sh.Kp / 64)), dim3(256), 0, st, s, false, n, sh.np, sh.Kp, eb, CRT_FP64_BITS, L, reinterpret_cast<__nv_bfloat16*>(b)));
   ZQ_LAUNCH_CHECK();
   if (int rc = crt_multiply(sh, a, b, r, false, err, st)) return rc;
   return crt_join(sh, r, m, n, CRT_FP64_BITS, ea, eb, false, reinterpret_cast<double2*>(C), ldc, st);

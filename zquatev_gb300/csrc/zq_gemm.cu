@@ -40,6 +40,7 @@ __device__ __forceinline__ Z load_op(const Z* X, int64_t ldx, int r, int c) {
 
 template <typename R, int OPA1, int OPB1, int OPA2, int OPB2>
 __global__ void __launch_bounds__(GNT) k_zgemm(ZgemmArgsT<R> g) {
+  pdl_wait();
   using Z = cplx<R>;
   __shared__ R sA[3][GK][GT];
   __shared__ R sB[3][GK][GT];
@@ -148,6 +149,7 @@ __global__ void __launch_bounds__(GNT) k_zgemm(ZgemmArgsT<R> g) {
 
 template <typename R>
 __global__ void k_zsplit_reduce(ZgemmArgsT<R> g, int splits) {
+  pdl_wait();
   using Z = cplx<R>;
   const int64_t total = (int64_t)g.m * g.n;
   const bool use_beta = (g.beta.x != (R)0 || g.beta.y != (R)0);
@@ -275,6 +277,7 @@ __device__ __forceinline__ void cg_segment(float (&re)[4][8], float (&im)[4][8],
 
 template <int OPA1, int OPB1, int OPA2, int OPB2>
 __global__ void __launch_bounds__(CNT) k_cgemm32(ZgemmArgsT<float> g) {
+  pdl_wait();
   __shared__ __align__(16) float2 sA[2][SK][GT];
   __shared__ __align__(16) float2 sB[2][SK][GT];
   const int tr = threadIdx.x & 15, tc = threadIdx.x >> 4;
@@ -338,6 +341,7 @@ __global__ void __launch_bounds__(CNT) k_cgemm32(ZgemmArgsT<float> g) {
 // {4tr..4tr+3, 32+4tr..} and the same pattern of columns
 constexpr int RNT = 64;
 __global__ void __launch_bounds__(RNT) k_sgemm_grouped(const DgemmDescT<float>* __restrict__ descs, int count) {
+  pdl_wait();
   __shared__ __align__(16) float sA[2][SK][GT];
   __shared__ __align__(16) float sB[2][SK][GT];
   const int t = blockIdx.x;
@@ -438,18 +442,18 @@ int zgemm_launch(const ZgemmArgsT<R>& g, int batch, cudaStream_t st) {
   prof_begin(PC_FORMQ_GEMM, st);
   if constexpr (std::is_same<R, float>::value) {
     if (g.A2 == nullptr || g.s2 == 1.f || g.s2 == -1.f)
-      k_cgemm32<OPA1, OPB1, OPA2, OPB2><<<grid, CNT, 0, st>>>(g);
+      ZQ_CUDA(launch_pdl_smem(k_cgemm32<OPA1, OPB1, OPA2, OPB2>, dim3(grid), dim3(CNT), 0, st, g));
     else
-      k_zgemm<R, OPA1, OPB1, OPA2, OPB2><<<grid, GNT, 0, st>>>(g);
+      ZQ_CUDA(launch_pdl_smem(k_zgemm<R, OPA1, OPB1, OPA2, OPB2>, dim3(grid), dim3(GNT), 0, st, g));
   } else {
-    k_zgemm<R, OPA1, OPB1, OPA2, OPB2><<<grid, GNT, 0, st>>>(g);
+    ZQ_CUDA(launch_pdl_smem(k_zgemm<R, OPA1, OPB1, OPA2, OPB2>, dim3(grid), dim3(GNT), 0, st, g));
   }
   prof_end(PC_FORMQ_GEMM, st);
   ZQ_LAUNCH_CHECK();
   if (splits > 1) {
     const int64_t total = (int64_t)g.m * g.n;
     const int blocks = (int)((total + 255) / 256 > 4096 ? 4096 : (total + 255) / 256);
-    k_zsplit_reduce<R><<<blocks, 256, 0, st>>>(g, splits);
+    ZQ_CUDA(launch_pdl_smem(k_zsplit_reduce<R>, dim3(blocks), dim3(256), 0, st, g, splits));
     ZQ_LAUNCH_CHECK();
   }
   return ZQ_OK;
@@ -479,6 +483,7 @@ template int zgemm<float>(int, int, int, int, const ZgemmArgsT<float>&, int, cud
 // ----------------------------------------------------------------------------
 template <typename R>
 __global__ void __launch_bounds__(GNT) k_dgemm_grouped(const DgemmDescT<R>* __restrict__ descs, int count) {
+  pdl_wait();
   __shared__ R sA[GKR][GT];
   __shared__ R sB[GKR][GT + 1];
   // locate descriptor (linear search over prefix offsets; count is small)
@@ -551,9 +556,9 @@ template <typename R>
 void grouped_launch(const DgemmDescT<R>* dev_descs, int count, int tiles, cudaStream_t st) {
   if (tiles <= 0 || count <= 0) return;
   if constexpr (std::is_same<R, float>::value)
-    k_sgemm_grouped<<<tiles, RNT, 0, st>>>(dev_descs, count);
+    (void)launch_pdl_smem(k_sgemm_grouped, dim3(tiles), dim3(RNT), 0, st, dev_descs, count);  // checked by the caller
   else
-    k_dgemm_grouped<R><<<tiles, GNT, 0, st>>>(dev_descs, count);
+    (void)launch_pdl_smem(k_dgemm_grouped<R>, dim3(tiles), dim3(GNT), 0, st, dev_descs, count);
 }
 template void grouped_launch<double>(const DgemmDescT<double>*, int, int, cudaStream_t);
 template void grouped_launch<float>(const DgemmDescT<float>*, int, int, cudaStream_t);

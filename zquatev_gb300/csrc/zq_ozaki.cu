@@ -87,6 +87,7 @@ __device__ __forceinline__ void oz_entry(const OzSide& s, bool is_a, int idx, in
 
 // exponent e with 2^e >= max |entry| of row/column idx (e = -1100 for a zero row)
 __global__ void k_oz_exp(OzSide s, bool is_a, int count, int parts, int* __restrict__ exps) {
+  pdl_wait();
   // The entries of row/column idx over k' are Re x and Im x of each complex x
   // of the row (times s2 in A's second segment), so the maximum is taken over
   // max(|Re x|, |Im x|) with eight loads in flight per lane. One warp per
@@ -180,6 +181,7 @@ __device__ __forceinline__ unsigned long long oz_fixed(double v, int e, int F, b
 __global__ void __launch_bounds__(256, 4)
     k_oz_slice(OzSide s, bool is_a, int count, int count_pad, int Kp, const int* __restrict__ exps, int nsl,
                __nv_bfloat16* __restrict__ out_re, __nv_bfloat16* __restrict__ out_im, int64_t slice_stride) {
+  pdl_wait();
   // eight consecutive k' of one row per thread (Kp is a multiple of 64), each
   // slice written as one 16-byte store
   const int64_t total8 = (int64_t)count_pad * Kp / 8;
@@ -267,11 +269,13 @@ __global__ void __launch_bounds__(256, 4)
 // Column-major A operands (op N or R: a row of op(A) is strided in memory):
 // the exponent pass and the slicing read 32 consecutive rows per warp.
 __global__ void k_oz_exp_init(int* __restrict__ exps, int count) {
+  pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count) exps[i] = -1100;
 }
 // block (32, 8): 32 rows x 256 K terms; the per-row maximum exponent via atomicMax (order-free)
 __global__ void k_oz_exp_cm(OzSide s, int count, int Kc, int* __restrict__ exps) {
+  pdl_wait();
   // rows of a column-major op(A) (OP_N / OP_R): 32 rows x 256 complex columns
   // per CTA, rows on the lanes (coalesced); the maximum of max(|Re x|, |Im x|)
   // (times |s2| in the second segment) over each complex column once, eight
@@ -322,6 +326,7 @@ __global__ void k_oz_exp_cm(OzSide s, int count, int Kc, int* __restrict__ exps)
 // block (32, 8): a 32-row x 32-K tile, digits staged in shared memory, stored along K
 __global__ void k_oz_slice_cm(OzSide s, int count, int Kp, const int* __restrict__ exps, int nsl,
                               __nv_bfloat16* __restrict__ out, int64_t slice_stride) {
+  pdl_wait();
   __shared__ __nv_bfloat16 s_d[OZ_SMAX][32][33];
   const int tx = threadIdx.x, ty = threadIdx.y;
   const int i0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
@@ -392,6 +397,7 @@ __device__ __forceinline__ double pow2i(int E) {
 
 // One CTA per 64x64 tile; loops over all levels and super-chunks.
 __global__ void __launch_bounds__(OZ_THREADS, 3) k_oz_gemm(OzGemmArgs g) {
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char oz_smem[];
   __nv_bfloat16* sm = reinterpret_cast<__nv_bfloat16*>(oz_smem);
   // stage layout: A [64][LDS], Bre [64][LDS], Bim [64][LDS]; two stages
@@ -586,6 +592,7 @@ size_t ozaki_workspace_bytes(int nq) {
 // is transposed through shared memory.
 constexpr int SF_T = 32;
 __global__ void __launch_bounds__(256) k_oz_symfill(double2* __restrict__ C, int64_t ldc, int n, int sym) {
+  pdl_wait();
   const int ti = blockIdx.x, tj = blockIdx.y;
   if (tj > ti) return;
   __shared__ double2 sl[SF_T][SF_T + 1];  // sl[r][c] = C(i0 + r, j0 + c)
@@ -641,7 +648,7 @@ __global__ void __launch_bounds__(256) k_oz_symfill(double2* __restrict__ C, int
 int structured_fill(double2* C, int64_t ldc, int n, int sym, cudaStream_t st) {
   if (n <= 0) return ZQ_OK;
   const unsigned nt = (unsigned)ceil_div(n, SF_T);
-  k_oz_symfill<<<dim3(nt, nt), dim3(SF_T, 8), 0, st>>>(C, ldc, n, sym);
+  ZQ_CUDA(launch_pdl_smem(k_oz_symfill, dim3(nt, nt), dim3(SF_T, 8), 0, st, C, ldc, n, sym));
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }
@@ -680,22 +687,22 @@ int zgemm_ozaki(int opa1, int opb1, int opa2, int opb2, const ZgemmArgs& g, void
   // exponents of the rows of op(A) (rows that are strided in memory: column-wise passes with coalesced reads)
   const bool cm = (opa1 == OP_N || opa1 == OP_R) && (!two || opa2 == OP_N || opa2 == OP_R);
   auto row_exponents = [&](int* ea) -> int {
-    k_oz_exp_init<<<ceil_div(m, 256), 256, 0, st>>>(ea, m);
+    ZQ_CUDA(launch_pdl_smem(k_oz_exp_init, dim3(ceil_div(m, 256)), dim3(256), 0, st, ea, m));
     ZQ_LAUNCH_CHECK();
     if (cm) {
-      k_oz_exp_cm<<<dim3((unsigned)ceil_div(m, 32), (unsigned)ceil_div((int)Kc, 256)), dim3(32, 8), 0, st>>>(a, m, (int)Kc, ea);
+      ZQ_CUDA(launch_pdl_smem(k_oz_exp_cm, dim3((unsigned)ceil_div(m, 32), (unsigned)ceil_div((int)Kc, 256)), dim3(32, 8), 0, st, a, m, (int)Kc, ea));
     } else {
       const int parts = oz_exp_parts(m, a);
-      k_oz_exp<<<ceil_div(m * parts * 32, 256), 256, 0, st>>>(a, true, m, parts, ea);
+      ZQ_CUDA(launch_pdl_smem(k_oz_exp, dim3(ceil_div(m * parts * 32, 256)), dim3(256), 0, st, a, true, m, parts, ea));
     }
     ZQ_LAUNCH_CHECK();
     return ZQ_OK;
   };
   auto col_exponents = [&](int* eb) -> int {
     const int parts = oz_exp_parts(n, b);
-    k_oz_exp_init<<<ceil_div(n, 256), 256, 0, st>>>(eb, n);
+    ZQ_CUDA(launch_pdl_smem(k_oz_exp_init, dim3(ceil_div(n, 256)), dim3(256), 0, st, eb, n));
     ZQ_LAUNCH_CHECK();
-    k_oz_exp<<<ceil_div(n * parts * 32, 256), 256, 0, st>>>(b, false, n, parts, eb);
+    ZQ_CUDA(launch_pdl_smem(k_oz_exp, dim3(ceil_div(n * parts * 32, 256)), dim3(256), 0, st, b, false, n, parts, eb));
     ZQ_LAUNCH_CHECK();
     return ZQ_OK;
   };
@@ -747,14 +754,13 @@ int zgemm_ozaki(int opa1, int opb1, int opa2, int opb2, const ZgemmArgs& g, void
   if (!reuse_a) {
     if (int rc = row_exponents(ea)) return rc;
     if (cm)
-      k_oz_slice_cm<<<dim3((unsigned)(mp / 32), (unsigned)ceil_div((int)Kp, 32)), dim3(32, 8), 0, st>>>(a, m, (int)Kp, ea,
-                                                                                                        nsl, As, mp * Kp);
+      ZQ_CUDA(launch_pdl_smem(k_oz_slice_cm, dim3((unsigned)(mp / 32), (unsigned)ceil_div((int)Kp, 32)), dim3(32, 8), 0, st, a, m, (int)Kp, ea, nsl, As, mp * Kp));
     else
-      k_oz_slice<<<grid(mp * Kp / 8), 256, 0, st>>>(a, true, m, (int)mp, (int)Kp, ea, nsl, As, nullptr, mp * Kp);
+      ZQ_CUDA(launch_pdl_smem(k_oz_slice, dim3(grid(mp * Kp / 8)), dim3(256), 0, st, a, true, m, (int)mp, (int)Kp, ea, nsl, As, nullptr, mp * Kp));
     ZQ_LAUNCH_CHECK();
   }
   if (int rc = col_exponents(eb)) return rc;
-  k_oz_slice<<<grid(np * Kp / 8), 256, 0, st>>>(b, false, n, (int)np, (int)Kp, eb, nsl, Brs, Bis, np * Kp);
+  ZQ_CUDA(launch_pdl_smem(k_oz_slice, dim3(grid(np * Kp / 8)), dim3(256), 0, st, b, false, n, (int)np, (int)Kp, eb, nsl, Brs, Bis, np * Kp));
   ZQ_LAUNCH_CHECK();
   OzGemmArgs og{};
   og.A = As; og.Bre = Brs; og.Bim = Bis; og.sa = mp * Kp; og.sb = np * Kp;
@@ -797,7 +803,7 @@ int zgemm_ozaki(int opa1, int opb1, int opa2, int opb2, const ZgemmArgs& g, void
       prof_add_flops(PC_OZAKI, pairs * 2.0 * tiles * OZ_TM * OZ_TN * (double)Kp * 2.0);
     }
     prof_begin(PC_OZAKI, st);
-    k_oz_gemm<<<gg, OZ_THREADS, smem, st>>>(og);
+    ZQ_CUDA(launch_pdl_smem(k_oz_gemm, dim3(gg), dim3(OZ_THREADS), smem, st, og));
     prof_end(PC_OZAKI, st);
     ZQ_LAUNCH_CHECK();
   }

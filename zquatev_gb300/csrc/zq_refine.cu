@@ -39,6 +39,7 @@ namespace zq {
 // ----------------------------------------------------------------- helpers
 __global__ void k_c128_to_c64(const double2* __restrict__ src, int64_t lds, float2* __restrict__ dst, int64_t ldd,
                               int rows, int cols) {
+  pdl_wait();
   const int64_t total = (int64_t)rows * cols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int r = (int)(t % rows), c = (int)(t / rows);
@@ -48,6 +49,7 @@ __global__ void k_c128_to_c64(const double2* __restrict__ src, int64_t lds, floa
 }
 __global__ void k_c64_to_c128(const float2* __restrict__ src, int64_t lds, double2* __restrict__ dst, int64_t ldd,
                               int rows, int cols) {
+  pdl_wait();
   const int64_t total = (int64_t)rows * cols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int r = (int)(t % rows), c = (int)(t / rows);
@@ -58,6 +60,7 @@ __global__ void k_c64_to_c128(const float2* __restrict__ src, int64_t lds, doubl
 // x += y   (2D, complex FP64)
 __global__ void k_add_c128(const double2* __restrict__ y, int64_t ldy, double2* __restrict__ x, int64_t ldx, int rows,
                            int cols) {
+  pdl_wait();
   const int64_t total = (int64_t)rows * cols;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int r = (int)(t % rows), c = (int)(t / rows);
@@ -73,6 +76,7 @@ __global__ void k_add_c128(const double2* __restrict__ y, int64_t ldy, double2* 
 __global__ void k_hx_combine(const double2* __restrict__ P1, const double2* __restrict__ P2, int64_t ldp, int n,
                              double2* __restrict__ HX, int64_t ldh, const double2* __restrict__ X, int64_t ldx,
                              const double* __restrict__ lam) {
+  pdl_wait();
   // HX (left half) from P1 = [A;B] U and P2 = [A;B] conj(V); with lam given,
   // the residual R = HX - X diag(lam) instead
   const int64_t total = (int64_t)n * n;
@@ -96,6 +100,7 @@ __global__ void k_hx_combine(const double2* __restrict__ P1, const double2* __re
 // S += G diag(lam) (n x n, ld n): S = X^H R + G Lambda (and the same for the
 // antisymmetric pair) recovers X^H H X from the residual products
 __global__ void k_add_glam(double2* __restrict__ S, const double2* __restrict__ G, int n, const double* __restrict__ lam) {
+  pdl_wait();
   const int64_t total = (int64_t)n * n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const double l = lam[t / n];
@@ -109,6 +114,7 @@ __global__ void k_add_glam(double2* __restrict__ S, const double2* __restrict__ 
 // lambda_j = Re S1_jj / Re G1_jj
 __global__ void k_oa_lambda(const double2* __restrict__ S1, const double2* __restrict__ G1, int64_t ld, int n,
                             double* __restrict__ lam) {
+  pdl_wait();
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j < n) lam[j] = S1[j + (int64_t)j * ld].x / G1[j + (int64_t)j * ld].x;
 }
@@ -117,6 +123,7 @@ __global__ void k_oa_lambda(const double2* __restrict__ S1, const double2* __res
 __global__ void k_oa_norms(const double2* __restrict__ S1, const double2* __restrict__ S2, const double2* __restrict__ G1,
                            const double2* __restrict__ G2, int64_t ld, int n, const double* __restrict__ lam,
                            double* __restrict__ part) {
+  pdl_wait();
   __shared__ double sh[32];
   unsigned long long ssb = 0, rrb = 0;  // maxima as bits (integer instructions)
   double lm = 0.0;
@@ -154,6 +161,7 @@ __global__ void k_oa_build_e(const double2* __restrict__ S1, const double2* __re
                              const double* __restrict__ lam, const double* __restrict__ part, int nparts,
                              double2* __restrict__ Et, double2* __restrict__ Eb, int64_t lde, double* __restrict__ emax,
                              int* __restrict__ pair_count, int2* __restrict__ pairs, int pair_cap, double eps_pair) {
+  pdl_wait();
   __shared__ double sh[32];
   __shared__ double s_lm;
   if (threadIdx.x == 0) {
@@ -236,6 +244,7 @@ __global__ void k_cl_gather(const double2* __restrict__ S1, const double2* __res
                             const double* __restrict__ lam, const int* __restrict__ members,
                             const int* __restrict__ cstart, const long long* __restrict__ coff, int ncl,
                             double2* __restrict__ blocks) {
+  pdl_wait();
   __shared__ double sh[32];
   const int c = blockIdx.x;
   if (c >= ncl) return;
@@ -262,6 +271,7 @@ __global__ void k_cl_rotate(double2* __restrict__ X, int64_t ldx, int n, const i
                             const int* __restrict__ cstart, const long long* __restrict__ coff, const long long* __restrict__ eoff,
                             int ncl, const double2* __restrict__ blocks, const double* __restrict__ ceig,
                             double2* __restrict__ tmp, double* __restrict__ lam) {
+  pdl_wait();
   const int c = blockIdx.y;
   if (c >= ncl) return;
   const int b = cstart[c], k = cstart[c + 1] - b;
@@ -289,6 +299,7 @@ __global__ void k_cl_rotate(double2* __restrict__ X, int64_t ldx, int n, const i
 }
 __global__ void k_cl_writeback(double2* __restrict__ X, int64_t ldx, int n, const int* __restrict__ members, int total_m,
                                const double2* __restrict__ tmp) {
+  pdl_wait();
   const int64_t total = (int64_t)2 * n * total_m;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int row = (int)(t % (2 * n)), q = (int)(t / (2 * n));
@@ -307,6 +318,7 @@ __global__ void k_cl_congr_cols(const double2* __restrict__ S1, const double2* _
                                 const int* __restrict__ members, const int* __restrict__ cstart,
                                 const long long* __restrict__ coff, int ncl, const double2* __restrict__ blocks, int m,
                                 double2* __restrict__ tmpS, double2* __restrict__ tmpG) {
+  pdl_wait();
   const int c = blockIdx.y;
   if (c >= ncl) return;
   const double2* M1 = blockIdx.z ? G1 : S1;
@@ -335,6 +347,7 @@ __global__ void k_cl_congr_cols(const double2* __restrict__ S1, const double2* _
 __global__ void k_cl_cols_writeback(double2* __restrict__ S1, double2* __restrict__ S2, double2* __restrict__ G1,
                                     double2* __restrict__ G2, int64_t ld, int n, const int* __restrict__ members, int m,
                                     const double2* __restrict__ tmpS, const double2* __restrict__ tmpG) {
+  pdl_wait();
   double2* M1 = blockIdx.z ? G1 : S1;
   double2* M2 = blockIdx.z ? G2 : S2;
   const double2* T = blockIdx.z ? tmpG : tmpS;
@@ -356,6 +369,7 @@ __global__ void k_cl_congr_rows(const double2* __restrict__ S1, const double2* _
                                 const int* __restrict__ members, const int* __restrict__ cstart,
                                 const long long* __restrict__ coff, int ncl, const double2* __restrict__ blocks,
                                 const int* __restrict__ pos, int m, double2* __restrict__ tmpS, double2* __restrict__ tmpG) {
+  pdl_wait();
   const int c = blockIdx.y;
   if (c >= ncl) return;
   const double2* M1 = blockIdx.z ? G1 : S1;
@@ -393,6 +407,7 @@ __global__ void k_cl_congr_rows(const double2* __restrict__ S1, const double2* _
 __global__ void k_cl_rows_writeback(double2* __restrict__ S1, double2* __restrict__ S2, double2* __restrict__ G1,
                                     double2* __restrict__ G2, int64_t ld, int n, const int* __restrict__ members, int m,
                                     const double2* __restrict__ tmpS, const double2* __restrict__ tmpG) {
+  pdl_wait();
   double2* M1 = blockIdx.z ? G1 : S1;
   double2* M2 = blockIdx.z ? G2 : S2;
   const double2* T = blockIdx.z ? tmpG : tmpS;
@@ -407,6 +422,7 @@ __global__ void k_cl_rows_writeback(double2* __restrict__ S1, double2* __restric
 
 // ascending order after refinement: rank of each eigenvalue
 __global__ void k_rank(const double* __restrict__ lam, int n, int* __restrict__ dst_of) {
+  pdl_wait();
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const double v = lam[k];
@@ -416,6 +432,7 @@ __global__ void k_rank(const double* __restrict__ lam, int n, int* __restrict__ 
 }
 __global__ void k_permute_cols(const double2* __restrict__ X, int64_t ldx, int rows, int n, const int* __restrict__ dst_of,
                                double2* __restrict__ Y, int64_t ldy, const double* __restrict__ lam, double* __restrict__ lam_out) {
+  pdl_wait();
   const int64_t total = (int64_t)rows * n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int r = (int)(t % rows), c = (int)(t / rows);
@@ -559,27 +576,26 @@ static int resolve_clusters(RefineArgs& ra, double2* X, int64_t ldd, double2* S1
   ZQ_CUDA(cudaMemcpyAsync(dco, coff.data(), sizeof(long long) * ncl, cudaMemcpyHostToDevice, st));
   ZQ_CUDA(cudaMemcpyAsync(deo, eoff.data(), sizeof(long long) * ncl, cudaMemcpyHostToDevice, st));
   ZQ_CUDA(cudaMemcpyAsync(dtasks, htasks.data(), tb * ncl, cudaMemcpyHostToDevice, st));
-  k_cl_gather<<<ncl, 256, 0, st>>>(S1, S2, G1, G2, n, lam, dmem, dcs, dco, ncl, blocks);
+  ZQ_CUDA(launch_pdl_smem(k_cl_gather, dim3(ncl), dim3(256), 0, st, S1, S2, G1, G2, n, lam, dmem, dcs, dco, ncl, blocks));
   ZQ_LAUNCH_CHECK();
   // cluster blocks are not queued by size: one CTA per block (no warp variant)
   if (int rc = batched_launch(dtasks, ncl, dinf + ncl, blocks, ceig, bws, ctas, dinf, st, 0)) return rc;
   // X_C (2n x m scratch in tmpa)
   const int gx = ceil_div(2 * n * kmax, 256) > 64 ? 64 : ceil_div(2 * n * kmax, 256);
-  k_cl_rotate<<<dim3(gx, ncl), 256, 0, st>>>(X, ldd, n, dmem, dcs, dco, deo, ncl, blocks, ceig, tmpa, lam);
+  ZQ_CUDA(launch_pdl_smem(k_cl_rotate, dim3(gx, ncl), dim3(256), 0, st, X, ldd, n, dmem, dcs, dco, deo, ncl, blocks, ceig, tmpa, lam));
   ZQ_LAUNCH_CHECK();
-  k_cl_writeback<<<grid_for((int64_t)2 * n * m), 256, 0, st>>>(X, ldd, n, dmem, m, tmpa);
+  ZQ_CUDA(launch_pdl_smem(k_cl_writeback, dim3(grid_for((int64_t)2 * n * m)), dim3(256), 0, st, X, ldd, n, dmem, m, tmpa));
   ZQ_LAUNCH_CHECK();
   // S, G: columns, then rows (2 n m double2 of scratch per pair)
   const int gc = ceil_div(n * kmax, 256) > 64 ? 64 : ceil_div(n * kmax, 256);
   const int gw = grid_for((int64_t)n * m) > 4096 ? 4096 : grid_for((int64_t)n * m);
-  k_cl_congr_cols<<<dim3(gc, ncl, 2), 256, 0, st>>>(S1, S2, G1, G2, n, n, dmem, dcs, dco, ncl, blocks, m, tmpa, tmpb);
+  ZQ_CUDA(launch_pdl_smem(k_cl_congr_cols, dim3(gc, ncl, 2), dim3(256), 0, st, S1, S2, G1, G2, n, n, dmem, dcs, dco, ncl, blocks, m, tmpa, tmpb));
   ZQ_LAUNCH_CHECK();
-  k_cl_cols_writeback<<<dim3(gw, 1, 2), 256, 0, st>>>(S1, S2, G1, G2, n, n, dmem, m, tmpa, tmpb);
+  ZQ_CUDA(launch_pdl_smem(k_cl_cols_writeback, dim3(gw, 1, 2), dim3(256), 0, st, S1, S2, G1, G2, n, n, dmem, m, tmpa, tmpb));
   ZQ_LAUNCH_CHECK();
-  k_cl_congr_rows<<<dim3(gc, ncl, 2), 256, 0, st>>>(S1, S2, G1, G2, n, n, dmem, dcs, dco, ncl, blocks, dpos, m, tmpa,
-                                                    tmpb);
+  ZQ_CUDA(launch_pdl_smem(k_cl_congr_rows, dim3(gc, ncl, 2), dim3(256), 0, st, S1, S2, G1, G2, n, n, dmem, dcs, dco, ncl, blocks, dpos, m, tmpa, tmpb));
   ZQ_LAUNCH_CHECK();
-  k_cl_rows_writeback<<<dim3(gw, 1, 2), 256, 0, st>>>(S1, S2, G1, G2, n, n, dmem, m, tmpa, tmpb);
+  ZQ_CUDA(launch_pdl_smem(k_cl_rows_writeback, dim3(gw, 1, 2), dim3(256), 0, st, S1, S2, G1, G2, n, n, dmem, m, tmpa, tmpb));
   ZQ_LAUNCH_CHECK();
   ZQ_CUDA(cudaFreeAsync(mem, st));
   return ZQ_OK;
@@ -641,7 +657,7 @@ int refined_solve(RefineArgs& ra) {
   mark(0, st);
   ZQ_CUDA(cudaMemcpy2DAsync(H0, sizeof(double2) * n2, ra.dD, sizeof(double2) * ldd, sizeof(double2) * n2, n,
                             cudaMemcpyDeviceToDevice, st));
-  k_c128_to_c64<<<grid_for((int64_t)n2 * n), 256, 0, st>>>(H0, n2, Mf, n2, n2, n);
+  ZQ_CUDA(launch_pdl_smem(k_c128_to_c64, dim3(grid_for((int64_t)n2 * n)), dim3(256), 0, st, H0, n2, Mf, n2, n2, n));
   ZQ_LAUNCH_CHECK();
   ZQ_CUDA(cudaMemsetAsync(tc_err, 0, 2 * sizeof(int), st));
   TridiagView<float> vf = tridiag_bind<float>(tri_ws, Mf, n, n2, NBMAX, d, e, tau);
@@ -665,7 +681,7 @@ int refined_solve(RefineArgs& ra) {
   mark(3, st);
   ZQ_CUDA(cudaStreamWaitEvent(st, ra.ev_join, 0));
   if (int rc = apply_z<float>(XfQ, n2, Zf, n, n, Mf, n2, ra.fdesc, st, tc_err)) return rc;
-  k_c64_to_c128<<<grid_for((int64_t)n2 * n), 256, 0, st>>>(Mf, n2, X, ldd, n2, n);
+  ZQ_CUDA(launch_pdl_smem(k_c64_to_c128, dim3(grid_for((int64_t)n2 * n)), dim3(256), 0, st, Mf, n2, X, ldd, n2, n));
   ZQ_LAUNCH_CHECK();
   {
     // a tensor-core pipeline wait that ran out leaves X0 unusable: report it
@@ -718,7 +734,7 @@ int refined_solve(RefineArgs& ra) {
     // (~ the eigenvector error times ||H||) the products with R need only
     // ss_slices, while G keeps sl.
     ZQ_CUDA(cudaMemcpyAsync(lamr, lam, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
-    k_hx_combine<<<grid_for((int64_t)nn), 256, 0, st>>>(P1, P2, n2, n, HX, n2, X, ldd, lamr);
+    ZQ_CUDA(launch_pdl_smem(k_hx_combine, dim3(grid_for((int64_t)nn)), dim3(256), 0, st, P1, P2, n2, n, HX, n2, X, ldd, lamr));
     ZQ_LAUNCH_CHECK();
     // G1 = X^H X ; S1 = X^H R + G1 Lambda
     g = ZgemmArgs{};
@@ -735,9 +751,9 @@ int refined_solve(RefineArgs& ra) {
     if (int rc = zgemm_acc(ra.mode, OP_T, OP_N, OP_T, OP_N, g, ra.ows, ra.ows_bytes, st, sl, -1, 0, oz_err)) return rc;
     g.B1 = HX + n; g.ldb1 = n2; g.B2 = HX; g.ldb2 = n2; g.C = S2;
     if (int rc = zgemm_acc(ra.mode, OP_T, OP_N, OP_T, OP_N, g, ra.ows, ra.ows_bytes, st, ss_slices, -2, sl, oz_err)) return rc;
-    k_add_glam<<<grid_for((int64_t)nn), 256, 0, st>>>(S1, G1, n, lamr);
+    ZQ_CUDA(launch_pdl_smem(k_add_glam, dim3(grid_for((int64_t)nn)), dim3(256), 0, st, S1, G1, n, lamr));
     ZQ_LAUNCH_CHECK();
-    k_add_glam<<<grid_for((int64_t)nn), 256, 0, st>>>(S2, G2, n, lamr);
+    ZQ_CUDA(launch_pdl_smem(k_add_glam, dim3(grid_for((int64_t)nn)), dim3(256), 0, st, S2, G2, n, lamr));
     ZQ_LAUNCH_CHECK();
     if (int rc = structured_fill(S1, n, n, 1, st)) return rc;
     if (int rc = structured_fill(S2, n, n, -1, st)) return rc;
@@ -747,13 +763,12 @@ int refined_solve(RefineArgs& ra) {
     double em = 0.0, cm = 0.0;
     int hcount = 0, clusters = 0, herr = 0;
     for (int pass = 0; pass < 2; ++pass) {
-      k_oa_lambda<<<ceil_div(n, 256), 256, 0, st>>>(S1, G1, n, n, lam);
+      ZQ_CUDA(launch_pdl_smem(k_oa_lambda, dim3(ceil_div(n, 256)), dim3(256), 0, st, S1, G1, n, n, lam));
       ZQ_LAUNCH_CHECK();
-      k_oa_norms<<<nparts, 256, 0, st>>>(S1, S2, G1, G2, n, n, lam, part);
+      ZQ_CUDA(launch_pdl_smem(k_oa_norms, dim3(nparts), dim3(256), 0, st, S1, S2, G1, G2, n, n, lam, part));
       ZQ_LAUNCH_CHECK();
       ZQ_CUDA(cudaMemsetAsync(pair_count, 0, sizeof(int), st));
-      k_oa_build_e<<<ne, 256, 0, st>>>(S1, S2, G1, G2, n, n, lam, part, nparts, Et, Eb, n, emax, pair_count, pairs,
-                                       pair_cap, it == 0 ? ra.pair_eps : ra.pair_eps_late);
+      ZQ_CUDA(launch_pdl_smem(k_oa_build_e, dim3(ne), dim3(256), 0, st, S1, S2, G1, G2, n, n, lam, part, nparts, Et, Eb, n, emax, pair_count, pairs, pair_cap, it == 0 ? ra.pair_eps : ra.pair_eps_late));
       ZQ_LAUNCH_CHECK();
       ZQ_CUDA(cudaMemcpyAsync(hemax.data(), emax, sizeof(double) * 2 * ne, cudaMemcpyDeviceToHost, st));
       ZQ_CUDA(cudaMemcpyAsync(&hcount, pair_count, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -780,7 +795,7 @@ int refined_solve(RefineArgs& ra) {
     if (int rc = zgemm_acc(ra.mode, OP_N, OP_N, OP_R, OP_N, g, ra.ows, ra.ows_bytes, st, sl_upd, 0, 0, oz_err)) return rc;
     g.A1 = V; g.A2 = U; g.s2 = 1.0; g.C = P1 + n;
     if (int rc = zgemm_acc(ra.mode, OP_N, OP_N, OP_R, OP_N, g, ra.ows, ra.ows_bytes, st, sl_upd, 0, 0, oz_err)) return rc;
-    k_add_c128<<<grid_for((int64_t)n2 * n), 256, 0, st>>>(P1, n2, X, ldd, n2, n);
+    ZQ_CUDA(launch_pdl_smem(k_add_c128, dim3(grid_for((int64_t)n2 * n)), dim3(256), 0, st, P1, n2, X, ldd, n2, n));
     ZQ_LAUNCH_CHECK();
     ra.iters = it + 1;
     if (trace) {
@@ -816,9 +831,9 @@ int refined_solve(RefineArgs& ra) {
     if (herr) return oz_timeout();
   }
   // ascending order
-  k_rank<<<ceil_div(n, 128), 128, 0, st>>>(lam, n, rank);
+  ZQ_CUDA(launch_pdl_smem(k_rank, dim3(ceil_div(n, 128)), dim3(128), 0, st, lam, n, rank));
   ZQ_LAUNCH_CHECK();
-  k_permute_cols<<<grid_for((int64_t)n2 * n), 256, 0, st>>>(X, ldd, n2, n, rank, P1, n2, lam, lam2);
+  ZQ_CUDA(launch_pdl_smem(k_permute_cols, dim3(grid_for((int64_t)n2 * n)), dim3(256), 0, st, X, ldd, n2, n, rank, P1, n2, lam, lam2));
   ZQ_LAUNCH_CHECK();
   ZQ_CUDA(cudaMemcpy2DAsync(X, sizeof(double2) * ldd, P1, sizeof(double2) * n2, sizeof(double2) * n2, n,
                             cudaMemcpyDeviceToDevice, st));

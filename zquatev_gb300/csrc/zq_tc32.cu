@@ -287,6 +287,7 @@ __device__ __forceinline__ void stage_store(const Tc32Args& g, int kbg, int j0, 
 
 template <bool CPLX>
 __global__ void __launch_bounds__(TC_THREADS, 1) k_tc32(const __grid_constant__ Tc32Args g) {
+  pdl_wait();
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
   const uint32_t raw = su32(tc_smem_raw);
   const uint32_t ring = (raw + 1023u) & ~1023u;
@@ -468,6 +469,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc32(const __grid_constant__ 
 
 // C = alpha * sum_z P_z + beta * C (partials column-major m x n)
 __global__ void k_tc32_reduce(const __grid_constant__ Tc32Args g) {
+  pdl_wait();
   const int64_t total = (int64_t)g.m * g.n;
   const bool use_beta = (g.beta.x != 0.f || g.beta.y != 0.f);
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
@@ -579,13 +581,13 @@ int tc32_gemm(const Tc32Args& in, cudaStream_t st) {
   }
   const int tm = ceil_div(g.m, TC_BM), tn = ceil_div(g.n, g.cplx ? 128 : 256);
   const dim3 grid(g.tri ? (unsigned)(tm * (tm + 1) / 2) : (unsigned)(tm * tn), 1, (unsigned)g.splits);
-  if (g.cplx) k_tc32<true><<<grid, TC_THREADS, TC_SMEM, st>>>(g);
-  else k_tc32<false><<<grid, TC_THREADS, TC_SMEM, st>>>(g);
+  if (g.cplx) ZQ_CUDA(launch_pdl_smem(k_tc32<true>, dim3(grid), dim3(TC_THREADS), TC_SMEM, st, g));
+  else ZQ_CUDA(launch_pdl_smem(k_tc32<false>, dim3(grid), dim3(TC_THREADS), TC_SMEM, st, g));
   ZQ_LAUNCH_CHECK();
   if (g.splits > 1) {
     const int64_t total = (int64_t)g.m * g.n;
     const int blocks = (int)((total + 255) / 256 > 4096 ? 4096 : (total + 255) / 256);
-    k_tc32_reduce<<<blocks, 256, 0, st>>>(g);
+    ZQ_CUDA(launch_pdl_smem(k_tc32_reduce, dim3(blocks), dim3(256), 0, st, g));
     ZQ_LAUNCH_CHECK();
   }
   return ZQ_OK;
