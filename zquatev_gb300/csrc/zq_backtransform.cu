@@ -54,11 +54,21 @@ __device__ __forceinline__ Quat qcombine(const Quat& later, const Quat& earlier)
   return r;
 }
 __device__ __forceinline__ Quat qunit_of(const double* e, int k, double& nrm) {
-  const double ea0 = e[4 * k], ea1 = e[4 * k + 1], eb0 = e[4 * k + 2], eb1 = e[4 * k + 3];
+  double ea0 = e[4 * k], ea1 = e[4 * k + 1], eb0 = e[4 * k + 2], eb1 = e[4 * k + 3], back = 1.0;
+  // entries whose squares leave the range of doubles are brought to [1, 2) first
+  const unsigned long long t0 = abs_bits(ea0) > abs_bits(ea1) ? abs_bits(ea0) : abs_bits(ea1);
+  const unsigned long long t1 = abs_bits(eb0) > abs_bits(eb1) ? abs_bits(eb0) : abs_bits(eb1);
+  const int ex = (int)((t0 > t1 ? t0 : t1) >> 52);
+  if (ex > 0 && ex < 2046 && (ex < 1023 - 450 || ex > 1023 + 450)) {
+    const double sc = __hiloint2double((2046 - ex) << 20, 0);
+    back = __hiloint2double(ex << 20, 0);
+    ea0 *= sc; ea1 *= sc; eb0 *= sc; eb1 *= sc;
+  }
   nrm = sqrt(ea0 * ea0 + ea1 * ea1 + eb0 * eb0 + eb1 * eb1);
   Quat u;
   if (nrm > 0.0) { const double s = 1.0 / nrm; u.a0 = ea0 * s; u.a1 = ea1 * s; u.b0 = eb0 * s; u.b1 = eb1 * s; u.reset = 0; }
   else { u.a0 = 1.0; u.a1 = 0.0; u.b0 = 0.0; u.b1 = 0.0; u.reset = 1; }
+  nrm *= back;
   return u;
 }
 // Few threads: an FP64 instruction holds its SM quadrant for 64 cycles a warp, so

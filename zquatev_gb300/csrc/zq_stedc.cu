@@ -99,6 +99,11 @@ __global__ void __launch_bounds__(256) k_dc_prepare(DcNode* nodes, DcWork w, con
   int* P = staged ? reinterpret_cast<int*>(dc_sm + 2 * scap) : w.perm + a;
   __shared__ double s_red[8];
   __shared__ int s_cnt[3];
+  // Values that are not numbers have no place in a sorted order: several may take
+  // one position. Every position starts as a valid entry, so that no index below is
+  // ever out of range.
+  for (int i = tid; i < m; i += blockDim.x) { D[i] = 0.0; Zs[i] = 0.0; P[i] = i; }
+  __syncthreads();
   // merge the two sorted eigenvalue lists; z in sorted order
   double dm = 0.0, zm = 0.0;
   for (int i = tid; i < m; i += blockDim.x) {
@@ -219,6 +224,8 @@ __global__ void __launch_bounds__(256) k_dc_prepare(DcNode* nodes, DcWork w, con
   // sort the deflated list (values, columns) by rank; ties by index
   const int nd_ = s_cnt[0];
   const double* fv = w.df_val + a;
+  for (int i = tid; i < nd_; i += blockDim.x) { w.df_sval[a + i] = fv[i]; w.df_scol[a + i] = w.df_col[a + i]; }
+  __syncthreads();  // (valid entries whatever the ranks of values that are not numbers)
   if (staged) {  // the staged poles are dead now: their space holds the deflated values
     for (int i = tid; i < nd_; i += blockDim.x) dc_sm[i] = w.df_val[a + i];
     __syncthreads();
@@ -521,8 +528,8 @@ __global__ void k_dc_scale(const double* d, const double* e, const DcMat* mats, 
     if (i < n - 1) mb = max(mb, abs_bits(e[i]));
   }
   const double m = block_max(bits_to_double(mb), sh);
-  if (threadIdx.x == 0) scal[blockIdx.x] = m;
-  const double inv = (m > 0.0) ? 1.0 / m : 1.0;
+  if (threadIdx.x == 0) scal[blockIdx.x] = m > 0.0 ? fmax(m, 2.2250738585072014e-308) : m;
+  const double inv = (m > 0.0) ? 1.0 / fmax(m, 2.2250738585072014e-308) : 1.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const double el = (i > 0) ? e[i - 1] * inv : 0.0;
     const double er = (i < n - 1) ? e[i] * inv : 0.0;
