@@ -75,7 +75,7 @@ int zq_refine_stats(int* iters, double* last_correction, int* fell_back);
 /* Explicit paths of the host drop-in: plain FP64, or refined (with the FP64
  * fallback). zquatev_c / ts::zquatev / zquatev_device follow the path policy
  * set by zq_set_path: 0 FP64, 1 refined, 2 auto (default: refined for
- * n2 >= 320, FP64 below; the request server's lanes: n2 >= 96); environment ZQ_PATH=fp64|refined|auto overrides. */
+ * n2 >= 400, FP64 below; the request server's lanes: n2 >= 96); environment ZQ_PATH=fp64|refined|auto overrides. */
 int zquatev_fp64_c(int n2, double* D, int ld2, double* eig);
 int zquatev_refined_c(int n2, double* D, int ld2, double* eig);
 int zquatev_fp64_device(int n2, double* dD, int ld2, double* deig, void* stream);
@@ -167,14 +167,14 @@ int zq_batch_plan_info(zq_batch_plan* p, void* stream);
 /* Chosen CTAs per SM, CTAs of the captured launch, and the tuning times (4 doubles, ms; 0 = not tried). */
 int zq_batch_plan_shape(zq_batch_plan* p, int* ctas_per_sm, int* ctas, double* tune_ms);
 /* The per-size kernel variant the plan's autotuner chose: matrices of order
- * n <= *warp_max_n are solved one per warp (eight per CTA), larger ones one per
- * CTA, in the same persistent launch. ms (4 doubles, may be NULL): the tuning
+ * n <= *warp_max_n are solved one per warp, larger ones one per CTA (orders above
+ * 32, and from 16 where the batch has few of up to 32, all together in any case). ms (4 doubles, may be NULL): the tuning
  * times for the switch sizes 0 (CTA variant only), 16, 24 and 32. No
  * counterpart in the reference (one matrix per call). */
 int zq_batch_plan_variant(zq_batch_plan* p, int* warp_max_n, double* ms);
 /* Switch size of the warp variant for batched launches that are not planned
  * (zquatev_batched_device, the request server): 0..32, or -1 for the default
- * (24; environment ZQ_BATCH_WARP_MAX). */
+ * (32; environment ZQ_BATCH_WARP_MAX). */
 int zq_set_batch_warp_max(int n);
 int zq_batch_plan_destroy(zq_batch_plan* p);
 

@@ -578,8 +578,8 @@ static int path_single(int n) {
 }
 
 // ----------------------------------------------------------------------------
-// batched: small matrices (n <= batched_max_n()) in one persistent kernel,
-// larger ones through the per-matrix path on the same stream
+// batched: small matrices a warp each (zq_small.cu), mid-size ones all together
+// (zq_forest.cu), larger ones through the per-matrix path on the same stream
 // ----------------------------------------------------------------------------
 
 static int g_batch_ctas_per_sm = 2;
@@ -592,10 +592,11 @@ static int batched_solve(int count, const int* n2s, const int* ld2s, const long 
   const int nmax = batched_max_n();
   // small tasks, largest first (longest-processing-time order)
   std::vector<int> small, mid, large;
+  const int few = forest_small_count(count, n2s);
   for (int b = 0; b < count; ++b) {
     if (n2s[b] == 0) continue;
     const int n = n2s[b] / 2;
-    (n < FOREST_MIN ? small : (n <= nmax ? mid : large)).push_back(b);
+    (n > nmax ? large : (forest_takes(n, few) ? mid : small)).push_back(b);
   }
   const auto larger = [&](int x, int y) { return n2s[x] > n2s[y]; };
   std::stable_sort(small.begin(), small.end(), larger);
@@ -645,7 +646,8 @@ static int batched_solve(int count, const int* n2s, const int* ld2s, const long 
     ZQ_CUDA(cudaEventRecord(c->ev_fork, st));
     ZQ_CUDA(cudaStreamWaitEvent(c->st, c->ev_fork, 0));
     ZQ_CUDA(cudaMemcpyAsync(dtasks, bb.host_tasks.data(), tb * small.size(), cudaMemcpyHostToDevice, c->st));
-    if (int rc = batched_launch(dtasks, (int)small.size(), dcounter, dD, deig, dws, ctas, dinfo, c->st)) return rc;
+    const BatchSplit split = batched_split((int)small.size(), batched_warp_max(), [&](int q) { return n2s[small[q]] / 2; });
+    if (int rc = batched_launch(dtasks, split, dcounter, dD, deig, dws, ctas, dinfo, c->st)) return rc;
     std::vector<int> hinfo(small.size());
     ZQ_CUDA(cudaMemcpyAsync(hinfo.data(), dinfo, sizeof(int) * small.size(), cudaMemcpyDeviceToHost, c->st));
     ZQ_CUDA(cudaStreamSynchronize(c->st));

@@ -74,13 +74,21 @@ int path_for(int n);
 void nb_table_set(int prec, int n, int nb);
 int nb_table_get(int prec, int n);
 
-// batched kernel (zq_batched.cu)
+// batched kernels (zq_batched.cu, zq_small.cu)
+// a task table sorted largest first: `large` tasks for a CTA each, then `small`
+// ones, of order at most small_max, for a warp each
+struct BatchSplit { int large = 0, small = 0, small_max = 0; };
+template <typename F> BatchSplit batched_split(int count, int wmax, F&& order_of) {
+  BatchSplit s;
+  while (s.large < count && order_of(s.large) > wmax) ++s.large;
+  s.small = count - s.large;
+  s.small_max = s.small > 0 ? order_of(s.large) : 0;
+  return s;
+}
 long long batched_ws_stride();
 int batched_max_n();
-// wmax: largest order solved by the warp variant (tasks sorted largest first;
-// -1: the current default, 0: CTA variant only)
-int batched_launch(const void* dev_tasks, int count, int* dev_counter, double2* D, double* eig, double* ws,
-                   int ctas, int* dev_info, cudaStream_t st, int wmax = -1);
+int batched_launch(const void* dev_tasks, const BatchSplit& split, int* dev_counter, double2* D, double* eig, double* ws,
+                   int ctas, int* dev_info, cudaStream_t st);
 int batched_warp_max();
 void batched_set_warp_max(int v);
 size_t batched_task_bytes();

@@ -1,4 +1,4 @@
-// Batches of mid-size matrices (order above FOREST_MIN) on all SMs (zq_forest.cu).
+// Batches of mid-size matrices on all SMs (zq_forest.cu).
 #pragma once
 
 #include <vector>
@@ -7,9 +7,22 @@
 
 namespace zq {
 
-// Orders the forest takes: the persistent kernel's one-warp range (zq_batched.cu)
-// stays with it, and above 256 the per-matrix path runs.
-constexpr int FOREST_MIN = 33, FOREST_MAX = 256;
+constexpr int SMALL_MAX = 32;  // largest order a warp solves (zq_small.cu)
+// Which matrices of a batch the forest takes: orders 33 to 256 always (above, the
+// per-matrix path runs). Orders up to 32 have a warp each (zq_small.cu); where a batch
+// has so few of them that a warp's serial chain shows, the forest is sooner from order
+// 16 up: 60 matrices take 0.57 ms here and 1.0 ms there at n = 19, 0.92 and 2.6 ms at
+// n = 32, but 0.28 and 0.26 ms at n = 8, and 2000 of n = 19 take 9.9 and 2.1 ms.
+constexpr int FOREST_FEW = 128;
+inline bool forest_takes(int n, int small_count) {
+  return n > SMALL_MAX || (small_count <= FOREST_FEW && n >= 16);
+}
+// small_count: the matrices of order 1 to SMALL_MAX
+inline int forest_small_count(int count, const int* n2s) {
+  int k = 0;
+  for (int b = 0; b < count; ++b) k += n2s[b] > 0 && n2s[b] / 2 <= SMALL_MAX;
+  return k;
+}
 
 struct ForestItem {
   int n, ld;

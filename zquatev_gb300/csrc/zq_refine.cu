@@ -26,6 +26,7 @@
 //   The iteration stops when max|E| (off the Kramers pairs) is below
 //   tol_converged; the caller gets the number of iterations and that value.
 #include "zq_common.cuh"
+#include "zq_context.h"
 #include "zq_kernels.h"
 #include "zq_resident.h"
 
@@ -493,13 +494,6 @@ static int zgemm_acc(int mode, int opa1, int opb1, int opa2, int opb2, const Zge
 // Eigenvalue clusters (consecutive eigenvalues closer than delta): for each,
 // the quaternion block [S1_CC; S2_CC] is diagonalised by the batched small
 // solver and the cluster's columns are rotated by its eigenvectors.
-long long batched_ws_stride();
-int batched_max_n();
-int batched_launch(const void* dev_tasks, int count, int* dev_counter, double2* D, double* eig, double* ws,
-                   int ctas, int* dev_info, cudaStream_t st, int wmax);
-size_t batched_task_bytes();
-void batched_fill_task(void* dst, long long off, long long eoff, int n, int ld, int slot);
-
 // Rayleigh-Ritz inside each eigenvalue cluster, on the current basis: group the
 // coupled pairs (union-find), solve every cluster's orthogonalised quaternion
 // block with the batched kernel, rotate X_C, and carry the rotation through
@@ -578,8 +572,11 @@ static int resolve_clusters(RefineArgs& ra, double2* X, int64_t ldd, double2* S1
   ZQ_CUDA(cudaMemcpyAsync(dtasks, htasks.data(), tb * ncl, cudaMemcpyHostToDevice, st));
   ZQ_CUDA(launch_pdl_smem(k_cl_gather, dim3(ncl), dim3(256), 0, st, S1, S2, G1, G2, n, lam, dmem, dcs, dco, ncl, blocks));
   ZQ_LAUNCH_CHECK();
-  // cluster blocks are not queued by size: one CTA per block (no warp variant)
-  if (int rc = batched_launch(dtasks, ncl, dinf + ncl, blocks, ceig, bws, ctas, dinf, st, 0)) return rc;
+  // cluster blocks are not queued by size: a warp each if all are small, else a CTA each
+  BatchSplit split;
+  (kmax <= SMALL_MAX ? split.small : split.large) = ncl;
+  split.small_max = kmax;
+  if (int rc = batched_launch(dtasks, split, dinf + ncl, blocks, ceig, bws, ctas, dinf, st)) return rc;
   // X_C (2n x m scratch in tmpa)
   const int gx = ceil_div(2 * n * kmax, 256) > 64 ? 64 : ceil_div(2 * n * kmax, 256);
   ZQ_CUDA(launch_pdl_smem(k_cl_rotate, dim3(gx, ncl), dim3(256), 0, st, X, ldd, n, dmem, dcs, dco, deo, ncl, blocks, ceig, tmpa, lam));

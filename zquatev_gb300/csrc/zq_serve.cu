@@ -260,8 +260,8 @@ void batch_loop(Server* s, Context* c) {
       if (rc == ZQ_OK && cudaMemcpyAsync(b, htasks.data(), tb * k, cudaMemcpyHostToDevice, c->st) != cudaSuccess)
         rc = ZQ_ERR_CUDA;
       if (rc == ZQ_OK)
-        rc = batched_launch(b, k, dinfo + k, nullptr, nullptr, reinterpret_cast<double*>(b + task_bytes + info_bytes),
-                            ctas, dinfo, c->st);
+        rc = batched_launch(b, batched_split(k, batched_warp_max(), [&](int q) { return batch[q]->n; }), dinfo + k, nullptr,
+                            nullptr, reinterpret_cast<double*>(b + task_bytes + info_bytes), ctas, dinfo, c->st);
       if (rc == ZQ_OK && cudaMemcpyAsync(hinfo.data(), dinfo, sizeof(int) * k, cudaMemcpyDeviceToHost, c->st) != cudaSuccess)
         rc = ZQ_ERR_CUDA;
       for (int q = 0; q < k && rc == ZQ_OK; ++q) rc = copy_back(batch[q], c->st);

@@ -114,6 +114,7 @@ struct zq_batch_plan {
   double variant_ms[4] = {0, 0, 0, 0};
   long long extent = 0;            // complex elements of D the small matrices touch
   zq::BatchForest forest;              // the mid-size matrices (the tuned kernel solves the small ones)
+  std::vector<int> orders;         // of the tasks, largest first
   void* dev = nullptr;             // tasks | info (+ counter) | per-CTA workspace
   size_t task_bytes = 0, info_bytes = 0;
   cudaStream_t cap = nullptr;      // capture stream
@@ -134,8 +135,8 @@ int* plan_info(zq_batch_plan* p) { return reinterpret_cast<int*>(reinterpret_cas
 
 int plan_launch_direct(zq_batch_plan* p, double2* D, double* E, int ctas, cudaStream_t st, int wmax) {
   int* info = plan_info(p);
-  return batched_launch(p->dev, p->ntask, info + p->ntask, D, E, reinterpret_cast<double*>(plan_ws(p)), ctas, info, st,
-                        wmax);
+  const BatchSplit split = batched_split(p->ntask, wmax, [&](int q) { return p->orders[q]; });
+  return batched_launch(p->dev, split, info + p->ntask, D, E, reinterpret_cast<double*>(plan_ws(p)), ctas, info, st);
 }
 // candidates of the warp variant's switch size (0: CTA variant for every size)
 constexpr int PLAN_WMAX[4] = {0, 16, 24, 32};
@@ -257,6 +258,7 @@ zq_batch_plan* zq_batch_plan_create(int count, const int* n2s, const int* ld2s, 
   const int nmax = batched_max_n();
   std::vector<int> order;
   std::vector<int> mid;
+  const int few = forest_small_count(count, n2s);
   long long extent = 0;
   for (int b = 0; b < count; ++b) {
     const int n2 = n2s[b];
@@ -266,7 +268,7 @@ zq_batch_plan* zq_batch_plan_create(int count, const int* n2s, const int* ld2s, 
     }
     if (n2 / 2 > nmax) { set_error_message("zq_batch_plan_create: every n2 must be <= 512"); return nullptr; }
     if (n2 == 0) continue;
-    if (n2 / 2 >= FOREST_MIN) { mid.push_back(b); continue; }
+    if (forest_takes(n2 / 2, few)) { mid.push_back(b); continue; }
     order.push_back(b);
     extent = std::max(extent, offs[b] + (long long)ld2s[b] * n2);
   }
@@ -291,6 +293,7 @@ zq_batch_plan* zq_batch_plan_create(int count, const int* n2s, const int* ld2s, 
   for (int q = 0; q < p->ntask; ++q) {
     const int b = order[q];
     batched_fill_task(ht.data() + q * tb, offs[b], eoffs[b], n2s[b] / 2, ld2s[b], q);
+    p->orders.push_back(n2s[b] / 2);
   }
   if (cudaMalloc(&p->dev, need) != cudaSuccess ||
       cudaStreamCreateWithFlags(&p->cap, cudaStreamNonBlocking) != cudaSuccess ||
