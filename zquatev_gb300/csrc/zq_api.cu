@@ -398,6 +398,7 @@ struct HostPin {
 };
 
 static int path_single(int n);
+static int values_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, cudaStream_t st);
 // host-memory drop-in (path: -1 policy, 0 FP64, 1 refined)
 static int zquatev_host(int n2, double2* D, int ld2, double* eig, bool vectors, int path = -1) {
   if (int rc = check_args(n2, D, ld2, eig)) return rc;
@@ -441,7 +442,8 @@ static int zquatev_host(int n2, double2* D, int ld2, double* eig, bool vectors, 
     const int p = (path >= 0) ? path : path_single(n);
     cudaEvent_t te[2];
     if (timing) { cudaEventCreate(&te[0]); cudaEventCreate(&te[1]); cudaEventRecord(te[0], c->st); }
-    rc = (vectors && p == 1) ? refined_device(c, dD, n2, n, deig, c->st, 1) : solve_device(c, dD, n2, n, deig, vectors, c->st);
+    rc = !vectors ? values_device(c, dD, n2, n, deig, c->st)
+                  : (p == 1 ? refined_device(c, dD, n2, n, deig, c->st, 1) : solve_device(c, dD, n2, n, deig, true, c->st));
     if (timing) {
       float gms = 0.f;
       cudaEventRecord(te[1], c->st);
@@ -487,16 +489,28 @@ int ensure_plan(Context* c, int n) {
   return ZQ_OK;
 }
 
-int refined_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, cudaStream_t st, int mode) {
+// `spare`: take the workspace only if that leaves as much free again (else ZQ_ERR_NOMEM)
+static int refined_reserve(Context* c, int n, int mode, bool spare) {
   if (int rc = ensure_plan(c, n)) return rc;
   RefineBuffers& rb = c->rb;
   const size_t need = refine_workspace_bytes(n, g_nbq) + (mode == 1 ? ozaki_workspace_bytes(n) : 0) + 4096;
   if (rb.bytes < need) {
     if (rb.external) { set_msg("bound refinement workspace too small"); return ZQ_ERR_ARG; }
+    if (spare) {
+      size_t free_b = 0, total_b = 0;
+      ZQ_CUDA(cudaMemGetInfo(&free_b, &total_b));
+      if (need > free_b / 2) return ZQ_ERR_NOMEM;
+    }
     if (rb.dev) { cudaStreamSynchronize(c->st); cudaFree(rb.dev); rb.dev = nullptr; rb.bytes = 0; }
     ZQ_CUDA(cudaMalloc(&rb.dev, need));
     rb.bytes = need;
   }
+  return ZQ_OK;
+}
+
+int refined_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, cudaStream_t st, int mode, bool vectors) {
+  if (int rc = refined_reserve(c, n, mode, false)) return rc;
+  RefineBuffers& rb = c->rb;
   Layout L = layout_for(n, NBMAX, g_nbq, c->dc.num_nodes(), c->dc.num_descs());
   DgemmDesc* desc1 = reinterpret_cast<DgemmDesc*>(reinterpret_cast<char*>(c->ws) + L.tri + L.small + L.dc + L.fq + L.nodes) +
                      c->dc.num_descs();
@@ -508,6 +522,7 @@ int refined_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, cu
   ra.ows_bytes = (mode == 1) ? ozaki_workspace_bytes(n) : 0;
   ra.dc = &c->dc;
   ra.coop = c->coop ? 1 : 0;
+  ra.values_only = vectors ? 0 : 1;
   ra.fdesc = reinterpret_cast<DgemmDescT<float>*>(desc1);
   ra.nb = nb_for(n, 1); ra.nbq = g_nbq; ra.mode = mode;
   ra.max_iter = 6;
@@ -543,7 +558,7 @@ int refined_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, cu
     ZQ_CUDA(cudaMemcpy2DAsync(dD, sizeof(double2) * ldd, H0, sizeof(double2) * 2 * n, sizeof(double2) * 2 * n, n,
                               cudaMemcpyDeviceToDevice, c->st));
     rb.last_fallback = 1;
-    if (int rc = solve_device(c, dD, ldd, n, deig, true, c->st)) return rc;
+    if (int rc = solve_device(c, dD, ldd, n, deig, vectors, c->st)) return rc;
   }
   ZQ_CUDA(cudaEventRecord(c->ev_join, c->st));
   ZQ_CUDA(cudaStreamWaitEvent(st, c->ev_join, 0));
@@ -575,6 +590,28 @@ constexpr int SINGLE_REFINED_MIN = 200;
 static int path_single(int n) {
   const int p = path_policy();
   return p == 2 ? (n >= SINGLE_REFINED_MIN ? 1 : 0) : p;
+}
+
+// Eigenvalues only. The FP64 path skips the vectors but reduces in FP64, where the
+// pipe alone takes 64/3 n^3 multiply-adds at 0.63e12 a second; the refined path
+// (without its last update) costs less from n = VALUES_REFINED_MIN up, and its
+// eigenvalues, Rayleigh quotients, are if anything closer to the exact ones.
+// Calls under stream capture stay on the FP64 path, which the host does not
+// wait for; so do those whose refinement workspace would crowd the memory.
+constexpr int VALUES_REFINED_MIN = 384;
+static int values_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, cudaStream_t st) {
+  if (n >= VALUES_REFINED_MIN && path_policy() != 0) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    const cudaError_t ce = cudaStreamIsCapturing(st, &cs);
+    if (ce != cudaSuccess) cudaGetLastError();
+    if (ce == cudaSuccess && cs == cudaStreamCaptureStatusNone) {
+      const int rc = refined_reserve(c, n, 1, true);
+      if (rc == ZQ_OK) return refined_device(c, dD, ldd, n, deig, st, 1, false);
+      if (rc != ZQ_ERR_NOMEM) return rc;
+      cudaGetLastError();
+    }
+  }
+  return solve_device(c, dD, ldd, n, deig, false, st);
 }
 
 // ----------------------------------------------------------------------------
@@ -714,7 +751,7 @@ int zquatev_values_device(int n2, double* dD, int ld2, double* deig, void* strea
   Context* c = nullptr;
   if (int rc = get_context(&c)) return rc;
   std::lock_guard<std::mutex> lk(c->mu);
-  return solve_device(c, reinterpret_cast<double2*>(dD), ld2, n2 / 2, deig, false, reinterpret_cast<cudaStream_t>(stream));
+  return values_device(c, reinterpret_cast<double2*>(dD), ld2, n2 / 2, deig, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int zq_stedc_device(int n, const double* d, const double* e, double* lam, double* Z, int ldz, void* stream) {

@@ -67,7 +67,8 @@ void context_bind(Context* c, void* ws, size_t ws_bytes, void* rws, size_t rws_b
 int ensure_ws(Context* c, size_t bytes);
 int ensure_plan(Context* c, int n);
 int solve_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, bool vectors, cudaStream_t st);
-int refined_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, cudaStream_t st, int mode);
+int refined_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, cudaStream_t st, int mode,
+                   bool vectors = true);
 // drop-in policy: 0 FP64 path, 1 refined path for quaternion size n
 int path_for(int n);
 // tuned panel widths (prec 0: FP64 path, 1: FP32 decomposition), 0 = not tuned

@@ -199,6 +199,7 @@ struct RefineArgs {
   double pair_eps_late;        // the same bound in the later steps
   int slices0;                 // Ozaki slices of the first step's products
   int slices_res;              // Ozaki slices of the products with the residual R = HX - X Lambda
+  int values_only;             // the eigenvalues alone: no last update of X, no vectors in place
   int coop;                    // no other solve runs beside this one: the FP32 reduction may take every SM
   cudaStream_t st;
   cudaStream_t st2;            // second stream: Q formation overlaps the tridiagonal solve

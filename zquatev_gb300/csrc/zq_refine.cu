@@ -783,6 +783,8 @@ int refined_solve(RefineArgs& ra) {
     if (ra.clusters < 0) break;
     ra.last_emax = em;
     ra.last_cluster = cm;
+    const bool last = em <= ra.tol && (ra.mode == 0 || sl == 8) && clusters == 0;
+    if (ra.values_only && last) { ra.iters = it + 1; break; }  // lam is final: its error is of the order of E squared
     // X += X E_top + J conj(X) E_bot with sl_upd slices; FP64 accumulation
     //   P1_top = U E_top - conj(V) E_bot,  P1_bot = V E_top + conj(U) E_bot
     g = ZgemmArgs{};
@@ -804,7 +806,7 @@ int refined_solve(RefineArgs& ra) {
     // on a basis rotated with the previous step's accuracy (seen on a clustered
     // n = 64 input: orthonormality 1.6e-12 when stopping there, 9e-16 after one
     // more step), so the final update is always a plain first-order one.
-    if (em <= ra.tol && (ra.mode == 0 || sl == 8) && clusters == 0) break;
+    if (last) break;
   }
   prof_end(PC_REFINE, st);
   if (trace) {
@@ -830,8 +832,13 @@ int refined_solve(RefineArgs& ra) {
   // ascending order
   ZQ_CUDA(launch_pdl_smem(k_rank, dim3(ceil_div(n, 128)), dim3(128), 0, st, lam, n, rank));
   ZQ_LAUNCH_CHECK();
-  ZQ_CUDA(launch_pdl_smem(k_permute_cols, dim3(grid_for((int64_t)n2 * n)), dim3(256), 0, st, X, ldd, n2, n, rank, P1, n2, lam, lam2));
+  const int rows = ra.values_only ? 1 : n2;
+  ZQ_CUDA(launch_pdl_smem(k_permute_cols, dim3(grid_for((int64_t)rows * n)), dim3(256), 0, st, X, ldd, rows, n, rank, P1, n2, lam, lam2));
   ZQ_LAUNCH_CHECK();
+  if (ra.values_only) {
+    ZQ_CUDA(cudaMemcpyAsync(ra.deig, lam2, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
+    return ZQ_OK;
+  }
   ZQ_CUDA(cudaMemcpy2DAsync(X, sizeof(double2) * ldd, P1, sizeof(double2) * n2, sizeof(double2) * n2, n,
                             cudaMemcpyDeviceToDevice, st));
   ZQ_CUDA(cudaMemcpyAsync(ra.deig, lam2, sizeof(double) * n, cudaMemcpyDeviceToDevice, st));
