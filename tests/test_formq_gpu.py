@@ -1,0 +1,28 @@
+"""GPU tests of the batched Q formation (zq_backtransform.cu) through the refined path:
+orders at the edges of its blocks of 64 reflectors, with even and odd numbers of rows,
+of one chunk of Gram sums and of the scratch it needs (below order ~35 the general
+formation runs).
+
+Tolerance: the parity suite's 1e-12 on the result; and the FP32 start must be good
+enough for the refinement to converge by itself (no FP64 fallback).
+"""
+import numpy as np
+import pytest
+
+from zquatev_gb300 import inputs, metrics, solver
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [3, 20, 34, 40, 65, 66, 67, 68, 129, 130, 131, 194, 255, 256, 257, 322, 515])
+def test_refined_from_its_q(gpu, n):
+    d = inputs.random_matrix(n, 60 + n)
+    out = np.array(d, order="F", copy=True)
+    eig = np.zeros(2 * n)
+    assert solver.zquatev_refined(2 * n, out, 2 * n, eig) == 0
+    assert not solver.refine_stats()[2]
+    h = inputs.full_from_blocks(d[:n, :n], d[n:, :n])
+    ref = np.linalg.eigvalsh(h)[::2]
+    assert metrics.eig_error(eig[:n], ref, metrics.h_norm2(ref)) <= 1e-12
+    assert metrics.residual(h, out, eig[:n]) <= 1e-12
+    assert metrics.orthonormality(out) <= 1e-12

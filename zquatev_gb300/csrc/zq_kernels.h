@@ -170,7 +170,7 @@ int phase_reduce_forest(const double* e, const DcMat* mats, int count, int nmax,
 // tensor cores (zq_tc32.cu) and a pipeline-wait timeout raises *tc_err
 template <typename R>
 int form_q(const cplx<R>* M, int64_t ldm, int n, const double* phi, cplx<R>* X, int64_t ldx,
-           int nbq, void* ws, cudaStream_t st, int* tc_err = nullptr);
+           int nbq, void* ws, cudaStream_t st, int* tc_err = nullptr, void* big = nullptr, size_t big_bytes = 0);
 size_t form_q_workspace_bytes(int n, int nbq);
 // out (2n x n complex, ldo) = X (2n x n complex, ldx) * Z (n x n real, ldz)
 template <typename R>

@@ -667,7 +667,10 @@ int refined_solve(RefineArgs& ra) {
   // Q Phi (FP32) on the second stream while the divide and conquer runs
   ZQ_CUDA(cudaEventRecord(ra.ev_fork, st));
   ZQ_CUDA(cudaStreamWaitEvent(ra.st2, ra.ev_fork, 0));
-  if (int rc = form_q<float>(Mf, n2, n, phi, XfQ, n2, ra.nbq, fq_ws, ra.st2, tc_err)) return rc;
+  // (the buffers from P1 to Eb, one after the other, are free until the refinement)
+  if (int rc = form_q<float>(Mf, n2, n, phi, XfQ, n2, ra.nbq, fq_ws, ra.st2, tc_err, P1,
+                             reinterpret_cast<char*>(Eb + nn) - reinterpret_cast<char*>(P1)))
+    return rc;
   mark(2, ra.st2);
   ZQ_CUDA(cudaEventRecord(ra.ev_join, ra.st2));
   float* Zf = nullptr;  // FP32 divide and conquer: Z in the plan's workspace

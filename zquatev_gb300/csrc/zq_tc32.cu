@@ -331,8 +331,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc32(const __grid_constant__ 
   const int i0 = bi * TC_BM, j0 = bj * bn;
   // this split's K blocks
   const int z = (int)blockIdx.z;
-  const int kb0 = (int)(((int64_t)g.kb_total * z) / g.splits), kb1 = (int)(((int64_t)g.kb_total * (z + 1)) / g.splits);
+  const int half = (int)blockIdx.y;
+  const int hb = half ? g.kb_first[2] : 0;
+  const int kb0 = hb + (int)(((int64_t)g.kb_total * z) / g.splits), kb1 = hb + (int)(((int64_t)g.kb_total * (z + 1)) / g.splits);
   const int nblk = kb1 - kb0;
+  float* const Cout = g.C + (half ? g.chalf : 0);
 
   if (warp == 0) {
     // ------------------------------------------------------------ MMA issuer
@@ -402,8 +405,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc32(const __grid_constant__ 
 #pragma unroll
       for (int c = 0; c < 16; ++c) {
         const int col = j0 + cw * h + 16 * gq + c;
-        if (CPLX) cpre[c] = masked(col) ? make_float2(0.f, 0.f) : reinterpret_cast<const float2*>(g.C)[cidx(col)];
-        else rpre[c] = masked(col) ? 0.f : g.C[cidx(col)];
+        if (CPLX) cpre[c] = masked(col) ? make_float2(0.f, 0.f) : reinterpret_cast<const float2*>(Cout)[cidx(col)];
+        else rpre[c] = masked(col) ? 0.f : Cout[cidx(col)];
       }
     };
     prefetch(0);
@@ -438,7 +441,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc32(const __grid_constant__ 
           if (masked(col)) continue;
           const int64_t o = cidx(col);
           if (CPLX) {
-            float2* C = reinterpret_cast<float2*>(partial ? g.P + (int64_t)2 * z * g.m * g.n : g.C);
+            float2* C = reinterpret_cast<float2*>(partial ? g.P + (int64_t)2 * z * g.m * g.n : Cout);
             const float xr = __uint_as_float(re[c]), xi = __uint_as_float(im[c]);
             if (partial) { C[o] = make_float2(xr, xi); continue; }
             float2 out = make_float2(g.alpha.x * xr - g.alpha.y * xi, g.alpha.x * xi + g.alpha.y * xr);
@@ -448,7 +451,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc32(const __grid_constant__ 
             }
             C[o] = out;
           } else {
-            float* C = partial ? g.P + (int64_t)z * g.m * g.n : g.C;
+            float* C = partial ? g.P + (int64_t)z * g.m * g.n : Cout;
             const float x = __uint_as_float(re[c]);
             if (partial) { C[o] = x; continue; }
             float out = g.alpha.x * x;
@@ -552,6 +555,13 @@ int tc32_gemm(const Tc32Args& in, cudaStream_t st) {
     kb += ceil_div(g.seg[s].k > 0 ? g.seg[s].k : 0, per);
   }
   g.kb_first[g.nseg] = kb;
+  if (g.halves > 1) {
+    if (g.nseg != 4 || kb != 2 * g.kb_first[2] || g.splits > 1 || g.tri) {
+      set_error_message("tc32_gemm: two products need two segments each, of the same inner size");
+      return ZQ_ERR_ARG;
+    }
+    kb /= 2;
+  }
   g.kb_total = kb;
   if (g.splits < 1) g.splits = 1;
   if (g.splits > kb && kb > 0) g.splits = kb;
@@ -580,7 +590,7 @@ int tc32_gemm(const Tc32Args& in, cudaStream_t st) {
     }
   }
   const int tm = ceil_div(g.m, TC_BM), tn = ceil_div(g.n, g.cplx ? 128 : 256);
-  const dim3 grid(g.tri ? (unsigned)(tm * (tm + 1) / 2) : (unsigned)(tm * tn), 1, (unsigned)g.splits);
+  const dim3 grid(g.tri ? (unsigned)(tm * (tm + 1) / 2) : (unsigned)(tm * tn), g.halves > 1 ? 2u : 1u, (unsigned)g.splits);
   if (g.cplx) ZQ_CUDA(launch_pdl_smem(k_tc32<true>, dim3(grid), dim3(TC_THREADS), TC_SMEM, st, g));
   else ZQ_CUDA(launch_pdl_smem(k_tc32<false>, dim3(grid), dim3(TC_THREADS), TC_SMEM, st, g));
   ZQ_LAUNCH_CHECK();

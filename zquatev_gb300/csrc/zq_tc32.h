@@ -34,6 +34,9 @@ struct Tc32Args {
   float2 alpha, beta;    // real products use .x
   float* C;
   int64_t ldc;
+  int halves;            // 2: a second product of the same sizes in the launch, from segments 2 and 3 (0, 1
+                         // are the first's), stored `chalf` floats further; no split K (0 or 1: one product)
+  int64_t chalf;
   int ctrans;            // 1: the product's (i, j) is stored at C[j + i * ldc]
   int tri;               // 0 every tile; 1 lower tiles, elements i >= j; 2 lower tiles, i > j
   float* P;              // split-K partials (splits * m * n elements), or null
