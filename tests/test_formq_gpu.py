@@ -26,3 +26,19 @@ def test_refined_from_its_q(gpu, n):
     assert metrics.eig_error(eig[:n], ref, metrics.h_norm2(ref)) <= 1e-12
     assert metrics.residual(h, out, eig[:n]) <= 1e-12
     assert metrics.orthonormality(out) <= 1e-12
+
+
+@pytest.mark.parametrize("path", ["refined", "auto"])
+def test_uncoupled_equal_eigenvalues(gpu, path):
+    """Equal Rayleigh quotients whose coupling is exactly zero: no correction, no reciprocal of the zero gap."""
+    n = 300
+    lam = np.repeat(np.arange(30.0), 10) - 3.0
+    d = np.zeros((2 * n, 2 * n), np.complex128, order="F")
+    d[:n, :n] = np.diag(np.random.default_rng(2).permutation(lam))
+    h = inputs.full_from_blocks(d[:n, :n], d[n:, :n])
+    eig = np.zeros(2 * n)
+    fn = solver.zquatev_refined if path == "refined" else solver.zquatev
+    assert fn(2 * n, d, 2 * n, eig) == 0
+    assert np.abs(eig[:n] - np.sort(lam)).max() <= 1e-12 * 30
+    assert metrics.residual(h, d, eig[:n]) <= 1e-12
+    assert metrics.orthonormality(d) <= 1e-12

@@ -33,6 +33,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <cstdlib>
+#include <limits>
 #include <vector>
 
 namespace zq {
@@ -149,6 +150,12 @@ __global__ void k_oa_norms(const double2* __restrict__ S1, const double2* __rest
   }
 }
 
+__device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+
 // E_top (n x n) and E_bot (n x n), written as complex64 for the FP32 update.
 // A pair (p, j) is corrected by the first-order formula only when its
 // coupling c = S_pj + lambda_j R_pj is small against its gap,
@@ -157,22 +164,28 @@ __global__ void k_oa_norms(const double2* __restrict__ S1, const double2* __rest
 // recorded, so the host can group the clusters and rotate inside them.
 // Outputs: per-block max |E| (convergence) and max in-cluster coupling
 // relative to max |lambda|.
+//
+// FP64 instructions bound it, so magnitudes are compared as integers (bit patterns
+// without the sign) and the gap's reciprocal is the approximate instruction with one
+// cubic step. max |lambda| is gathered by the whole block: one thread's chain over
+// the 1024 partials took longer than the rest up to n ~ 1000 (n = 750: 182 us a call).
 __global__ void k_oa_build_e(const double2* __restrict__ S1, const double2* __restrict__ S2,
                              const double2* __restrict__ G1, const double2* __restrict__ G2, int64_t ld, int n,
                              const double* __restrict__ lam, const double* __restrict__ part, int nparts,
                              double2* __restrict__ Et, double2* __restrict__ Eb, int64_t lde, double* __restrict__ emax,
                              int* __restrict__ pair_count, int2* __restrict__ pairs, int pair_cap, double eps_pair) {
   pdl_wait();
-  __shared__ double sh[32];
-  __shared__ double s_lm;
-  if (threadIdx.x == 0) {
-    double lm = 0.0;
-    for (int q = 0; q < nparts; ++q) lm = fmax(lm, part[3 * q + 2]);
-    s_lm = lm;
-  }
+  __shared__ unsigned long long s_max[3];
+  if (threadIdx.x < 3) s_max[threadIdx.x] = 0ull;
   __syncthreads();
+  unsigned long long lmb = 0;
+  for (int q = threadIdx.x; q < nparts; q += blockDim.x) lmb = max(lmb, abs_bits(part[3 * q + 2]));
+  lmb = warp_max_bits(lmb);
+  if ((threadIdx.x & 31) == 0) atomicMax(&s_max[0], lmb);
+  __syncthreads();
+  const double s_lm = bits_to_double(s_max[0]);
   const double inv_lm = s_lm > 0.0 ? 1.0 / s_lm : 1.0;
-  double em = 0.0, cm = 0.0;
+  unsigned long long emb = 0, cmb = 0;  // max |E|, max in-cluster coupling
   const int64_t total = (int64_t)n * n;
   for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
     const int i = (int)(t % n), j = (int)(t / n);
@@ -196,26 +209,33 @@ __global__ void k_oa_build_e(const double2* __restrict__ S1, const double2* __re
     // the pair's rotation per step (seen: |E| halving from 2.5e-5 each step).
     const double2 c1t = make_double2(s1.x + li * r1.x, s1.y + li * r1.y);
     const double2 c2t = make_double2(s2.x + li * r2.x, s2.y + li * r2.y);
-    const double a1 = fmax(fmax(fabs(c1.x), fabs(c1.y)), fmax(fabs(c1t.x), fabs(c1t.y)));
-    const double a2 = fmax(fmax(fabs(c2.x), fabs(c2.y)), fmax(fabs(c2t.x), fabs(c2t.y)));
+    const unsigned long long a1 = max(absmax_bits(c1), absmax_bits(c1t));
+    const unsigned long long a2 = max(absmax_bits(c2), absmax_bits(c2t));
+    // (a coupling that is not a number compares above every bound)
+    const unsigned long long bound = abs_bits(eps_pair * gap);
     double2 e1, e2;
     bool cl = false;
-    // one FP64 division per entry instead of four (FP64 divisions bounded this
-    // kernel; E is a correction, its last bit does not matter)
-    const double igap = (i == j) ? 0.0 : 1.0 / gap;
+    // uncoupled equal eigenvalues (0 <= 0) need no correction: no reciprocal of zero
+    double igap = 0.0;
+    if (i != j && gap != 0.0) {
+      double y;
+      asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(gap));
+      const double h = fma(-gap, y, 1.0);
+      igap = fma(y, fma(h, h, h), y);
+    }
     if (i == j) {
       e1 = make_double2(0.5 * r1.x, 0.5 * r1.y);
-    } else if (a1 <= eps_pair * fabs(gap)) {
+    } else if (a1 <= bound) {
       e1 = make_double2(c1.x * igap, c1.y * igap);
     } else {
       e1 = make_double2(0.5 * r1.x, 0.5 * r1.y);
       cl = true;
-      cm = fmax(cm, a1 * inv_lm);
+      cmb = max(cmb, abs_bits(bits_to_double(a1) * inv_lm));
     }
-    if (i == j || a2 > eps_pair * fabs(gap)) {
+    if (i == j || a2 > bound) {
       // i == j: the Kramers partner (same eigenvalue, zero coupling by structure)
       e2 = make_double2(0.5 * r2.x, 0.5 * r2.y);
-      if (i != j) { cl = true; cm = fmax(cm, a2 * inv_lm); }
+      if (i != j) { cl = true; cmb = max(cmb, abs_bits(bits_to_double(a2) * inv_lm)); }
     } else {
       e2 = make_double2(c2.x * igap, c2.y * igap);
     }
@@ -225,12 +245,13 @@ __global__ void k_oa_build_e(const double2* __restrict__ S1, const double2* __re
     }
     Et[i + (int64_t)j * lde] = e1;
     Eb[i + (int64_t)j * lde] = e2;
-    em = fmax(em, fmax(fabs(e1.x), fabs(e1.y)));
-    em = fmax(em, fmax(fabs(e2.x), fabs(e2.y)));
+    emb = max(emb, max(absmax_bits(e1), absmax_bits(e2)));
   }
-  em = block_max(em, sh);
-  cm = block_max(cm, sh);
-  if (threadIdx.x == 0) { emax[blockIdx.x] = em; emax[gridDim.x + blockIdx.x] = cm; }
+  emb = warp_max_bits(emb);
+  cmb = warp_max_bits(cmb);
+  if ((threadIdx.x & 31) == 0) { atomicMax(&s_max[1], emb); atomicMax(&s_max[2], cmb); }
+  __syncthreads();
+  if (threadIdx.x < 2) emax[threadIdx.x * gridDim.x + blockIdx.x] = bits_to_double(s_max[1 + threadIdx.x]);
 }
 
 // ---------------------------------------------------------------- clusters
@@ -421,15 +442,29 @@ __global__ void k_cl_rows_writeback(double2* __restrict__ S1, double2* __restric
   }
 }
 
-// ascending order after refinement: rank of each eigenvalue
-__global__ void k_rank(const double* __restrict__ lam, int n, int* __restrict__ dst_of) {
+// ascending order after refinement: rank of each eigenvalue, ties by index. Compared as
+// integers in the doubles' order, from shared memory (n FP64 comparisons per thread:
+// n = 4096 520 us).
+__device__ __forceinline__ long long order_key(double v) {
+  const long long b = __double_as_longlong(v);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+constexpr int RANK_T = 128;
+__global__ void __launch_bounds__(RANK_T) k_rank(const double* __restrict__ lam, int n, int* __restrict__ dst_of) {
   pdl_wait();
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const double v = lam[k];
+  __shared__ long long key[4 * RANK_T];
+  const int k = blockIdx.x * RANK_T + threadIdx.x;
+  const long long v = order_key(lam[k < n ? k : n - 1]);
   int r = 0;
-  for (int q = 0; q < n; ++q) r += (lam[q] < v) || (lam[q] == v && q < k);
-  dst_of[k] = r;
+  for (int q0 = 0; q0 < n; q0 += 4 * RANK_T) {
+    __syncthreads();
+    for (int q = threadIdx.x; q < 4 * RANK_T && q0 + q < n; q += RANK_T) key[q] = order_key(lam[q0 + q]);
+    __syncthreads();
+    const int cnt = min(4 * RANK_T, n - q0);
+#pragma unroll 8
+    for (int q = 0; q < cnt; ++q) r += (key[q] < v) || (key[q] == v && q0 + q < k);
+  }
+  if (k < n) dst_of[k] = r;
 }
 __global__ void k_permute_cols(const double2* __restrict__ X, int64_t ldx, int rows, int n, const int* __restrict__ dst_of,
                                double2* __restrict__ Y, int64_t ldy, const double* __restrict__ lam, double* __restrict__ lam_out) {
@@ -776,7 +811,13 @@ int refined_solve(RefineArgs& ra) {
       ZQ_CUDA(cudaStreamSynchronize(st));
       if (herr) return oz_timeout();
       em = 0.0; cm = 0.0;
-      for (int q = 0; q < ne; ++q) { em = hemax[q] > em ? hemax[q] : em; cm = hemax[ne + q] > cm ? hemax[ne + q] : cm; }
+      bool nan = false;
+      for (int q = 0; q < ne; ++q) {
+        em = hemax[q] > em ? hemax[q] : em;
+        cm = hemax[ne + q] > cm ? hemax[ne + q] : cm;
+        nan = nan || hemax[q] != hemax[q];
+      }
+      if (nan) em = std::numeric_limits<double>::quiet_NaN();
       if (pass == 1 || !(cm > ra.cluster_tol)) break;
       if (hcount > pair_cap) { ra.clusters = -1; break; }
       if (int rc = resolve_clusters(ra, X, ldd, S1, S2, G1, G2, lam, pairs, hcount, P1, P2)) return rc;
@@ -785,6 +826,7 @@ int refined_solve(RefineArgs& ra) {
     }
     if (ra.clusters < 0) break;
     ra.last_emax = em;
+    if (em != em) break;  // not converged: the caller falls back to the FP64 path
     ra.last_cluster = cm;
     const bool last = em <= ra.tol && (ra.mode == 0 || sl == 8) && clusters == 0;
     if (ra.values_only && last) { ra.iters = it + 1; break; }  // lam is final: its error is of the order of E squared
@@ -833,7 +875,7 @@ int refined_solve(RefineArgs& ra) {
     if (herr) return oz_timeout();
   }
   // ascending order
-  ZQ_CUDA(launch_pdl_smem(k_rank, dim3(ceil_div(n, 128)), dim3(128), 0, st, lam, n, rank));
+  ZQ_CUDA(launch_pdl_smem(k_rank, dim3(ceil_div(n, RANK_T)), dim3(RANK_T), 0, st, lam, n, rank));
   ZQ_LAUNCH_CHECK();
   const int rows = ra.values_only ? 1 : n2;
   ZQ_CUDA(launch_pdl_smem(k_permute_cols, dim3(grid_for((int64_t)rows * n)), dim3(256), 0, st, X, ldd, rows, n, rank, P1, n2, lam, lam2));
