@@ -135,79 +135,24 @@ __device__ __forceinline__ uint32_t swz(int r, int c) {
   return (uint32_t)((r >> 3) * 1024 + (r & 7) * 128 + ((c ^ (r & 7)) << 4));
 }
 
-// Raw loads of one 16-byte chunk (four floats: two complex or four real
-// elements along K) of one operand row. The loads are unconditional and their
-// values untouched here: an element outside [0, rows) x [0, kdim) reads the
-// operand's base address instead and is cleared by its mask bit later, and
-// signs / conjugation are applied when the chunk is stored. So all of a
-// thread's loads of a K block are in flight together; an arithmetic use right
-// after each load (or a branch around it) would make every load wait for the
-// previous one.
-__device__ __forceinline__ uint32_t ld_chunk(const Tc32Src& s, bool cplx, int r, int rows, int k, int kdim, float (&v)[4]) {
-  const int per = cplx ? 2 : 4;        // elements in the chunk
-  const bool row_ok = r < rows;
-  if (s.vec && row_ok && k + per - 1 < kdim) {
-    const int64_t off = cplx ? 2 * (k + (int64_t)r * s.ld) : (k + (int64_t)r * s.ld);
-    const float4 q = __ldg(reinterpret_cast<const float4*>(s.p + off));
-    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
-    return 0xFu;
-  }
-  uint32_t mask = 0;
-  if (cplx) {
-    const float2* p = reinterpret_cast<const float2*>(s.p);
-#pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const bool ok = row_ok && k + e < kdim;
-      const float2* a = ok ? (s.kfast ? p + (k + e) + (int64_t)r * s.ld : p + r + (int64_t)(k + e) * s.ld) : p;
-      const float2 x = __ldg(a);
-      v[2 * e] = x.x; v[2 * e + 1] = x.y;
-      mask |= ok ? (3u << (2 * e)) : 0u;
-    }
-  } else {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const bool ok = row_ok && k + e < kdim;
-      const float* a = ok ? (s.kfast ? s.p + (k + e) + (int64_t)r * s.ld : s.p + r + (int64_t)(k + e) * s.ld) : s.p;
-      v[e] = __ldg(a);
-      mask |= ok ? (1u << e) : 0u;
-    }
-  }
-  return mask;
+// What a producer thread moves: four 16-byte chunks of A and four (real: eight) of B
+// per K block, a chunk being four floats along K (two complex or four real elements)
+// of one operand row. Which chunks these are is fixed for a segment, so their
+// addresses are formed once per segment and advanced per block; rows outside the
+// matrix read row 0 (their outputs are not stored), and only a segment's last,
+// partial block checks its elements. Instructions bound this kernel where a CTA has
+// few K blocks: with the addresses, bounds and signs worked out per chunk a block
+// took ~900 instructions of each producer warp (two CTAs of eight blocks 37 us, now
+// 25; the Q formation and back-transform of n = 4096 32 ms, now 22).
+// Chunk q of thread t -> (row, chunk): K-contiguous sources put eight consecutive
+// threads on one row, row-contiguous ones 32 threads on consecutive rows (both
+// coalesced).
+__device__ __forceinline__ void unit_a(bool kfast, int t, int q, int& r, int& c) {
+  if (kfast) { c = t & 7; r = (t >> 3) + 32 * q; } else { r = t & 127; c = (t >> 7) + 2 * q; }
 }
-// the chunk's values as the product uses them: masked, signed, conjugated
-__device__ __forceinline__ void fix_chunk(const Tc32Src& s, bool cplx, uint32_t mask, const float (&v)[4], float (&o)[4]) {
-  const float si = (cplx && s.conj) ? -s.sign : s.sign;
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const float sg = (cplx && (e & 1)) ? si : s.sign;
-    o[e] = ((mask >> e) & 1u) ? v[e] * sg : 0.f;
-  }
-}
-
-// One producer thread's share of one K block, held in registers between its
-// global loads and its shared-memory stores (complex: 4 A and 4 B chunks;
-// real: 4 A and 8 B chunks), with the chunks' mask bits.
-template <bool CPLX>
-struct TcStage {
-  float a[4][4];
-  float b[CPLX ? 4 : 8][4];
-  uint32_t am, bm;
-};
-
-// unit q of thread t -> (row, 16-byte chunk): K-contiguous sources put eight
-// consecutive threads on one row, row-contiguous ones 32 threads on
-// consecutive rows (both coalesced)
-__device__ __forceinline__ void unit_a(const Tc32Src& s, int t, int q, int& r, int& c) {
-  if (s.kfast) { c = t & 7; r = (t >> 3) + 32 * q; } else { r = t & 127; c = (t >> 7) + 2 * q; }
-}
-__device__ __forceinline__ void unit_b(const Tc32Src& s, bool cplx, int t, int q, int& r, int& c) {
-  if (cplx || s.kfast) unit_a(s, t, q, r, c);
+__device__ __forceinline__ void unit_b(bool kfast, bool cplx, int t, int q, int& r, int& c) {
+  if (cplx || kfast) unit_a(kfast, t, q, r, c);
   else { r = t; c = q; }
-}
-__device__ __forceinline__ int seg_of(const Tc32Args& g, int kbg) {
-  int s = 0;
-  while (s + 1 < g.nseg && kbg >= g.kb_first[s + 1]) ++s;
-  return s;
 }
 // the segment's descriptors copied into registers: each field read at a
 // constant parameter offset, not through a run-time index into parameter space
@@ -219,68 +164,164 @@ __device__ __forceinline__ Tc32Seg seg_copy(const Tc32Args& g, int s) {
     default: return g.seg[3];
   }
 }
-// the B source of output column col (the second source past nsplit)
-__device__ __forceinline__ void b_source(const Tc32Seg& sg, int n, int col, Tc32Src& bs, int& bc, int& bcols) {
-  const bool second = sg.b2.p != nullptr && col >= sg.nsplit;
-  bs = second ? sg.b2 : sg.b;
-  bc = second ? col - sg.nsplit : col;
-  bcols = second ? n - sg.nsplit : (sg.b2.p != nullptr ? sg.nsplit : n);
-}
-
 template <bool CPLX>
-__device__ __forceinline__ void stage_load(const Tc32Args& g, int kbg, int i0, int j0, int t, TcStage<CPLX>& st) {
-  const int s = seg_of(g, kbg);
+struct TcUnits {
+  static constexpr int NB = CPLX ? 4 : 8;  // chunks of B
+  static constexpr int KB = CPLX ? 16 : 32;
+  static constexpr int EW = CPLX ? 2 : 1;  // floats per element
+  static constexpr int NS = CPLX ? 4 : 1;  // signs of B (two column sources: complex only)
+  const float *a[4], *b[NB];
+  int64_t astep, bstep;                    // floats from one K element to the next
+  float ar, ai, br[NS], bi[NS];            // signs of real and imaginary parts
+  int k, kdim, end, seg;                   // next K element, the segment's K, first K block past it
+  bool avec, bvec, akf, bkf;
+};
+// start (or continue, at block kbg of the whole product) with the segment kbg lies in
+template <bool CPLX>
+__device__ __forceinline__ void units_seek(const Tc32Args& g, int kbg, int i0, int j0, int t, TcUnits<CPLX>& u) {
+  using U = TcUnits<CPLX>;
+  int s = 0;
+  while (s + 1 < g.nseg && kbg >= g.kb_first[s + 1]) ++s;
   const Tc32Seg sg = seg_copy(g, s);
-  const int k0 = (kbg - g.kb_first[s]) * (CPLX ? 16 : 32);
-  const int kw = CPLX ? 2 : 4;  // K elements per chunk
-  st.am = 0; st.bm = 0;
+  u.end = s + 1 < g.nseg ? g.kb_first[s + 1] : 0x7fffffff;
+  u.k = (kbg - g.kb_first[s]) * U::KB;
+  u.kdim = sg.k;
+  u.astep = (int64_t)U::EW * (sg.a.kfast ? 1 : sg.a.ld);
+  u.bstep = (int64_t)U::EW * (sg.b.kfast ? 1 : sg.b.ld);
+  u.akf = sg.a.kfast; u.bkf = sg.b.kfast;
+  u.avec = sg.a.vec;
+  u.bvec = sg.b.vec && (sg.b2.p == nullptr || sg.b2.vec);
+  u.ar = sg.a.sign;
+  u.ai = sg.a.conj ? -sg.a.sign : sg.a.sign;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     int r, c;
-    unit_a(sg.a, t, q, r, c);
-    st.am |= ld_chunk(sg.a, CPLX, i0 + r, g.m, k0 + kw * c, sg.k, st.a[q]) << (4 * q);
+    unit_a(u.akf, t, q, r, c);
+    const int row = i0 + r < g.m ? i0 + r : 0;
+    u.a[q] = sg.a.p + U::EW * (int64_t)row * (sg.a.kfast ? sg.a.ld : 1) + (u.k + (4 / U::EW) * c) * u.astep;
   }
 #pragma unroll
-  for (int q = 0; q < (CPLX ? 4 : 8); ++q) {
+  for (int q = 0; q < U::NB; ++q) {
     int r, c;
-    unit_b(sg.b, CPLX, t, q, r, c);
-    Tc32Src bs;
-    int bc, bcols;
-    b_source(sg, g.n, j0 + r, bs, bc, bcols);
-    st.bm |= ld_chunk(bs, CPLX, bc, bcols, k0 + kw * c, sg.k, st.b[q]) << (4 * q);
+    unit_b(u.bkf, CPLX, t, q, r, c);
+    const int col = j0 + r < g.n ? j0 + r : 0;
+    const bool second = sg.b2.p != nullptr && col >= sg.nsplit;
+    const float* p = second ? sg.b2.p : sg.b.p;
+    const int bc = second ? col - sg.nsplit : col;
+    u.b[q] = p + U::EW * (int64_t)bc * (sg.b.kfast ? sg.b.ld : 1) + (u.k + (4 / U::EW) * c) * u.bstep;
+    if (q < U::NS) {
+      u.br[q] = second ? sg.b2.sign : sg.b.sign;
+      u.bi[q] = (second ? sg.b2.conj : sg.b.conj) ? -u.br[q] : u.br[q];
+    }
+  }
+}
+
+// One producer thread's share of one K block, held in registers between its
+// global loads and its shared-memory stores, with its signs.
+template <bool CPLX>
+struct TcStage {
+  static constexpr int NB = TcUnits<CPLX>::NB, NS = TcUnits<CPLX>::NS;
+  float a[4][4], b[NB][4];
+  float ar, ai, br[NS], bi[NS];
+  bool akf, bkf;
+};
+
+template <bool CPLX>
+__device__ __forceinline__ void chunk_load(const float* p, int64_t step, bool vec, float (&v)[4]) {
+  if (vec) {
+    const float4 q = __ldg(reinterpret_cast<const float4*>(p));
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+  } else if constexpr (CPLX) {
+    const float2 x = __ldg(reinterpret_cast<const float2*>(p)), y = __ldg(reinterpret_cast<const float2*>(p + step));
+    v[0] = x.x; v[1] = x.y; v[2] = y.x; v[3] = y.y;
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) v[e] = __ldg(p + e * step);
+  }
+}
+// the same where the segment ends inside the block: elements from `left` on are zero
+template <bool CPLX>
+__device__ __forceinline__ void chunk_load_tail(const float* p, int64_t step, int left, float (&v)[4]) {
+  constexpr int W = CPLX ? 2 : 1;
+#pragma unroll
+  for (int e = 0; e < 4 / W; ++e) {
+    const bool in = e < left;
+#pragma unroll
+    for (int h = 0; h < W; ++h) v[W * e + h] = in ? __ldg(p + e * step + h) : 0.f;
   }
 }
 
 template <bool CPLX>
-__device__ __forceinline__ void stage_store(const Tc32Args& g, int kbg, int j0, int t, uint32_t sa,
-                                            const TcStage<CPLX>& st) {
-  const Tc32Seg sg = seg_copy(g, seg_of(g, kbg));
+__device__ __forceinline__ void stage_load(const Tc32Args& g, int kbg, int i0, int j0, int t, TcUnits<CPLX>& u,
+                                           TcStage<CPLX>& st) {
+  using U = TcUnits<CPLX>;
+  if (kbg >= u.end) units_seek<CPLX>(g, kbg, i0, j0, t, u);
+  if (u.k + U::KB <= u.kdim) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) chunk_load<CPLX>(u.a[q], u.astep, u.avec, st.a[q]);
+#pragma unroll
+    for (int q = 0; q < U::NB; ++q) chunk_load<CPLX>(u.b[q], u.bstep, u.bvec, st.b[q]);
+  } else {
+    const int left = u.kdim - u.k;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      int r, c;
+      unit_a(u.akf, t, q, r, c);
+      chunk_load_tail<CPLX>(u.a[q], u.astep, left - (4 / U::EW) * c, st.a[q]);
+    }
+#pragma unroll
+    for (int q = 0; q < U::NB; ++q) {
+      int r, c;
+      unit_b(u.bkf, CPLX, t, q, r, c);
+      chunk_load_tail<CPLX>(u.b[q], u.bstep, left - (4 / U::EW) * c, st.b[q]);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q) u.a[q] += U::KB * u.astep;
+#pragma unroll
+  for (int q = 0; q < U::NB; ++q) u.b[q] += U::KB * u.bstep;
+  u.k += U::KB;
+  st.ar = u.ar; st.ai = u.ai; st.akf = u.akf; st.bkf = u.bkf;
+#pragma unroll
+  for (int q = 0; q < U::NS; ++q) { st.br[q] = u.br[q]; st.bi[q] = u.bi[q]; }
+}
+
+__device__ __forceinline__ void st_v4(uint32_t dst, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+
+template <bool CPLX>
+__device__ __forceinline__ void stage_store(int t, uint32_t sa, const TcStage<CPLX>& st) {
   const uint32_t sah = sa, sal = sa + TC_A_BYTES, sbh = sa + 2 * TC_A_BYTES, sbl = sbh + TC_B_BYTES;
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     int r, c;
-    unit_a(sg.a, t, q, r, c);
-    float v[4];
-    fix_chunk(sg.a, CPLX, (st.am >> (4 * q)) & 0xFu, st.a[q], v);
+    unit_a(st.akf, t, q, r, c);
     const uint32_t o = swz(r, c);
-    split_store(sah + o, sal + o, v[0], v[1], v[2], v[3]);
+    if (CPLX) split_store(sah + o, sal + o, st.a[q][0] * st.ar, st.a[q][1] * st.ai, st.a[q][2] * st.ar, st.a[q][3] * st.ai);
+    else split_store(sah + o, sal + o, st.a[q][0] * st.ar, st.a[q][1] * st.ar, st.a[q][2] * st.ar, st.a[q][3] * st.ar);
   }
 #pragma unroll
-  for (int q = 0; q < (CPLX ? 4 : 8); ++q) {
+  for (int q = 0; q < TcStage<CPLX>::NB; ++q) {
     int r, c;
-    unit_b(sg.b, CPLX, t, q, r, c);
-    Tc32Src bs;
-    int bc, bcols;
-    b_source(sg, g.n, j0 + r, bs, bc, bcols);
-    float b[4];
-    fix_chunk(bs, CPLX, (st.bm >> (4 * q)) & 0xFu, st.b[q], b);
-    if (CPLX) {  // (re0, im0, re1, im1) -> real-part row (re, -im), imaginary-part row (im, re)
-      const uint32_t ore = swz(r, c), oim = swz(128 + r, c);
-      split_store(sbh + ore, sbl + ore, b[0], -b[1], b[2], -b[3]);
-      split_store(sbh + oim, sbl + oim, b[1], b[0], b[3], b[2]);
+    unit_b(st.bkf, CPLX, t, q, r, c);
+    const uint32_t o = swz(r, c);
+    if (CPLX) {  // (re0, im0, re1, im1) -> real-part row (re, -im), imaginary-part row 128 below (im, re)
+      uint32_t h[4], l[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float v = st.b[q][e] * ((e & 1) ? st.bi[q] : st.br[q]);
+        h[e] = tf32_rna(v);
+        l[e] = tf32_rna(v - __uint_as_float(h[e]));
+      }
+      constexpr uint32_t NEG = 0x80000000u, IM = 16 * 1024;
+      st_v4(sbh + o, h[0], h[1] ^ NEG, h[2], h[3] ^ NEG);
+      st_v4(sbl + o, l[0], l[1] ^ NEG, l[2], l[3] ^ NEG);
+      st_v4(sbh + o + IM, h[1], h[0], h[3], h[2]);
+      st_v4(sbl + o + IM, l[1], l[0], l[3], l[2]);
     } else {
-      const uint32_t o = swz(r, c);
-      split_store(sbh + o, sbl + o, b[0], b[1], b[2], b[3]);
+      split_store(sbh + o, sbl + o, st.b[q][0] * st.br[0], st.b[q][1] * st.br[0], st.b[q][2] * st.br[0],
+                  st.b[q][3] * st.br[0]);
     }
   }
 }
@@ -366,18 +407,20 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc32(const __grid_constant__ 
     // block it is split and stored
     const int t = threadIdx.x - 32;  // 0..255
     TcStage<CPLX> sx, sy;
+    TcUnits<CPLX> un;
+    un.end = -1;
     bool go = true;
     auto step = [&](int it, TcStage<CPLX>& cur, TcStage<CPLX>& nxt) {
-      if (it + 1 < nblk) stage_load<CPLX>(g, kb0 + it + 1, i0, j0, t, nxt);
+      if (it + 1 < nblk) stage_load<CPLX>(g, kb0 + it + 1, i0, j0, t, un, nxt);
       const int stage = it % TC_STAGES, round = it / TC_STAGES;
       if (!__all_sync(0xffffffffu, mbar_wait(empty0 + 8 * stage, (round & 1) ^ 1, abort, g.wait))) { go = false; return; }
-      stage_store<CPLX>(g, kb0 + it, j0, t, ring + stage * TC_STAGE_BYTES, cur);
+      stage_store<CPLX>(t, ring + stage * TC_STAGE_BYTES, cur);
       // generic-proxy stores become visible to the tensor core (async proxy)
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(full0 + 8 * stage);
     };
-    if (nblk > 0) stage_load<CPLX>(g, kb0, i0, j0, t, sx);
+    if (nblk > 0) stage_load<CPLX>(g, kb0, i0, j0, t, un, sx);
     for (int it = 0; it < nblk && go; it += 2) {
       step(it, sx, sy);
       if (go && it + 1 < nblk) step(it + 1, sy, sx);
@@ -392,8 +435,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_tc32(const __grid_constant__ 
     const bool use_beta = !partial && (g.beta.x != 0.f || g.beta.y != 0.f);
     const int64_t ldc = partial ? g.m : g.ldc;
     const int ctr = partial ? 0 : g.ctrans;
-    auto masked = [&](int col) { return col >= g.n || (g.tri && (row < col || (g.tri == 2 && row == col))); };
-    auto cidx = [&](int col) { return ctr ? (col + (int64_t)row * ldc) : (row + (int64_t)col * ldc); };
+    // a tile inside the matrix (and strictly below the diagonal) stores every element
+    const bool whole = i0 + TC_BM <= g.m && j0 + bn <= g.n && (!g.tri || i0 >= j0 + bn);
+    auto masked = [&](int col) {
+      return !whole && (col >= g.n || (g.tri && (row < col || (g.tri == 2 && row == col))));
+    };
+    const int64_t c_row = ctr ? (int64_t)row * ldc : row, c_col = ctr ? 1 : ldc;
+    auto cidx = [&](int col) { return c_row + (int64_t)col * c_col; };
     constexpr int NG = CPLX ? 4 : 8;    // 16-column groups of this thread's half
     const int cw = CPLX ? 64 : 128;     // columns per half
     // beta != 0: the C values of a group are loaded one group ahead (the first
@@ -573,6 +621,13 @@ int tc32_gemm(const Tc32Args& in, cudaStream_t st) {
   g.wait = pipeline_wait_cycles();
   // 16-byte loads where a source is K-contiguous, 16-byte aligned and its rows
   // start on 16-byte boundaries
+  for (int s = 0; s < g.nseg; ++s) {
+    const Tc32Seg& q = g.seg[s];
+    if (q.b2.p != nullptr && (!g.cplx || q.b2.kfast != q.b.kfast || q.b2.ld != q.b.ld)) {
+      set_error_message("tc32_gemm: two column sources only for complex operands of one layout");
+      return ZQ_ERR_ARG;
+    }
+  }
   auto vec_ok = [&](Tc32Src& x) {
     x.vec = (x.p != nullptr && x.kfast && (reinterpret_cast<uintptr_t>(x.p) % 16) == 0 &&
              (g.cplx ? (x.ld % 2) == 0 : (x.ld % 4) == 0)) ? 1 : 0;
