@@ -75,7 +75,7 @@ int zq_refine_stats(int* iters, double* last_correction, int* fell_back);
 /* Explicit paths of the host drop-in: plain FP64, or refined (with the FP64
  * fallback). zquatev_c / ts::zquatev / zquatev_device follow the path policy
  * set by zq_set_path: 0 FP64, 1 refined, 2 auto (default: refined for
- * n2 >= 400, FP64 below; the request server's lanes: n2 >= 96); environment ZQ_PATH=fp64|refined|auto overrides. */
+ * n2 >= 320, FP64 below; the request server's lanes: n2 >= 96); environment ZQ_PATH=fp64|refined|auto overrides. */
 int zquatev_fp64_c(int n2, double* D, int ld2, double* eig);
 int zquatev_refined_c(int n2, double* D, int ld2, double* eig);
 int zquatev_fp64_device(int n2, double* dD, int ld2, double* deig, void* stream);
@@ -112,7 +112,7 @@ int zq_get_block_size(void);
  * (TMEM accumulators, TMA-fed 128 x 256 MMAs, one CTA per tile), 2 = tcgen05 in
  * clusters of two CTAs that share the B operand by TMA multicast, 3 = 2-SM
  * tcgen05 MMAs (cta_group::2, 256 x 256 per CTA pair; the default). 0 to 2
- * multiply digit slices; 3 does products of 28 bits and more on integer
+ * multiply digit slices; 3 does products of 21 bits and more on integer
  * residues (the Ozaki scheme II), at least as accurate, with a third of the
  * tensor work for FP64. */
 int zq_set_ozaki_kernel(int which);

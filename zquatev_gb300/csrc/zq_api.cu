@@ -581,12 +581,12 @@ int path_for(int n) {
 }
 
 // The same for one solve alone on the GPU: there the FP64 path is the faster one
-// up to order ~200 (its reduction and back-transform spread over the SMs and it
-// needs no refinement): n = 64 1.03 against 2.32 ms, n = 127 1.9 / 2.9, n = 200
-// 3.5 / 3.5, n = 256 4.3 / 4.0. The request server keeps path_for: its lanes run
+// up to order ~160 (its reduction and back-transform spread over the SMs and it
+// needs no refinement): n = 110 1.55 against 1.9 ms, n = 140 2.1 / 2.2, n = 160
+// 2.5 / 2.3, n = 200 3.3 / 2.6. The request server keeps path_for: its lanes run
 // side by side, where the FP64 pipe is shared and the refined path's latencies
 // overlap.
-constexpr int SINGLE_REFINED_MIN = 200;
+constexpr int SINGLE_REFINED_MIN = 160;
 static int path_single(int n) {
   const int p = path_policy();
   return p == 2 ? (n >= SINGLE_REFINED_MIN ? 1 : 0) : p;
@@ -594,11 +594,12 @@ static int path_single(int n) {
 
 // Eigenvalues only. The FP64 path skips the vectors but reduces in FP64, where the
 // pipe alone takes 64/3 n^3 multiply-adds at 0.63e12 a second; the refined path
-// (without its last update) costs less from n = VALUES_REFINED_MIN up, and its
+// (without its last update) costs less from n = VALUES_REFINED_MIN up (n = 200 2.6
+// against 2.6 ms, n = 256 3.0 / 3.4, n = 750 9.9 / 18.6, n = 1500 28 / 113), and its
 // eigenvalues, Rayleigh quotients, are if anything closer to the exact ones.
 // Calls under stream capture stay on the FP64 path, which the host does not
 // wait for; so do those whose refinement workspace would crowd the memory.
-constexpr int VALUES_REFINED_MIN = 384;
+constexpr int VALUES_REFINED_MIN = 220;
 static int values_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, cudaStream_t st) {
   if (n >= VALUES_REFINED_MIN && path_policy() != 0) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;

@@ -248,7 +248,9 @@ size_t form_q_workspace_bytes(int n, int nbq) {
 // W and X in 16-byte pieces.
 // ----------------------------------------------------------------------------
 constexpr int FQ_NB = 64;        // reflectors per block
-constexpr int FQ_ROWS = 256;     // rows of W per partial Gram sum
+// rows of W per partial Gram sum: few enough CTAs' worth for small orders (n = 512: 16
+// CTAs of 256 rows took 89 us)
+__host__ __device__ inline int fq_rows(int n) { return n <= 1024 ? 64 : 256; }
 struct FqBlocks {
   const float2* M; int64_t ldm;
   int n, nref, nblocks;
@@ -259,7 +261,7 @@ __host__ __device__ inline int fq_ld(int n, int b) { return (n - FQ_NB * b + 1) 
 __host__ __device__ inline int64_t fq_off(int n, int b) {  // complex elements before block b
   return (int64_t)2 * FQ_NB * ((int64_t)b * fq_ld(n, 0) - (int64_t)FQ_NB * b * (b - 1) / 2);
 }
-__host__ __device__ inline int fq_chunks(int n, int b) { return (n - FQ_NB * b + FQ_ROWS - 1) / FQ_ROWS; }
+__host__ __device__ inline int fq_chunks(int n, int b) { return (n - FQ_NB * b + fq_rows(n) - 1) / fq_rows(n); }
 __host__ __device__ inline int fq_kb(int nref, int b) { return nref - FQ_NB * b < FQ_NB ? nref - FQ_NB * b : FQ_NB; }
 // bytes of W, V, T and the partial sums
 static size_t fq_bytes(int n, int nblocks) {
@@ -291,7 +293,7 @@ __global__ void __launch_bounds__(256) k_fq_gram(FqBlocks q) {
   pdl_wait();
   const int b = blockIdx.y, ch = blockIdx.x;
   const int pb = FQ_NB * b, kb = fq_kb(q.nref, b), ld = fq_ld(q.n, b), rows = q.n - pb;
-  if (ch * FQ_ROWS >= rows) return;
+  if (ch * fq_rows(q.n) >= rows) return;
   __shared__ float4 w[32][FQ_NB + 1];
   const float2* wa = q.W + fq_off(q.n, b);
   const float2* wb = wa + (int64_t)ld * kb;
@@ -301,8 +303,8 @@ __global__ void __launch_bounds__(256) k_fq_gram(FqBlocks q) {
   for (int x = 0; x < 4; ++x)
 #pragma unroll
     for (int y = 0; y < 4; ++y) acc[x][y] = make_float4(0.f, 0.f, 0.f, 0.f);
-  const int r1 = min((ch + 1) * FQ_ROWS, rows);
-  for (int r0 = ch * FQ_ROWS; r0 < r1; r0 += 32) {
+  const int r1 = min((ch + 1) * fq_rows(q.n), rows);
+  for (int r0 = ch * fq_rows(q.n); r0 < r1; r0 += 32) {
     __syncthreads();
 #pragma unroll
     for (int u = 0; u < 8; ++u) {  // a warp per column, a lane per row

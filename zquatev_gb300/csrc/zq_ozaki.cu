@@ -551,12 +551,13 @@ int oz_umma_gemm(const __nv_bfloat16* As, const __nv_bfloat16* Brs, const __nv_b
 
 // Whether a product with this many slices' accuracy runs on residues (zq_crt.cu)
 // instead of digit slices, and with how many moduli: the default kernel, from
-// four slices (28 bits) up, where the residue products are fewer (four slices:
-// 9 moduli x 3 real products against 10 digit products x 4; three: 8 x 3 against
-// 6 x 4, no gain for the reconstruction's cost).
+// three slices (21 bits) up. Four slices: 9 moduli x 3 real products against 10
+// digit products x 4; three: 8 x 3 against 6 x 4, where the shorter preparation
+// decides for small products (the two of a solve at n = 512 0.3 ms on digits, 0.15
+// on residues; n = 4096 the same 9 ms). Two: fewer digit products (12).
 static int crt_bits(int slices) { return OZ_BETA * slices - 1; }
 static int use_crt(int slices, int64_t K) {
-  return ozaki_kernel() == 3 && slices >= 4 ? crt_moduli(crt_bits(slices), 2.0 * (double)K) : 0;
+  return ozaki_kernel() == 3 && slices >= 3 ? crt_moduli(crt_bits(slices), 2.0 * (double)K) : 0;
 }
 
 size_t zgemm_ozaki_bytes(int m, int n, int64_t K, int slices) {

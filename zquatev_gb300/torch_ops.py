@@ -7,7 +7,7 @@ the left half of H = (A -B*; B A*), which is all the reference reads). It
 returns ``(eig, v)``: the n ascending eigenvalues (float64) and the (n2, n2)
 eigenvectors in the (U -V*; V U*) layout, column j of ``v`` belonging to
 ``eig[j % n]``. The solve runs through ``zquatev_device`` (the drop-in's path
-policy: refined from n = 200 up) on torch's current stream, without host
+policy: refined from n = 160 up) on torch's current stream, without host
 synchronisation. ``torch.ops.zquatev_gb300.eigvalsh(h_left)`` returns the
 eigenvalues only (``zquatev_values_device``).
 
