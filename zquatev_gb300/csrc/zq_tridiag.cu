@@ -751,15 +751,7 @@ __global__ void __launch_bounds__(NT) k_hreduce(TridiagView<R> v, int p, int j, 
 // trailing update of the lower triangles of A (incl. diagonal) and B (strict)
 // region [t0, n) x [t0, n), rank-4*nbp structured update.
 // ----------------------------------------------------------------------------
-constexpr int KC = 4;  // reflectors per smem stage
-__device__ __forceinline__ void cp_async8_zfill(void* smem, const void* gmem, bool pred) {
-  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(gmem), "r"(pred ? 8 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
+constexpr int KC = 4;  // reflectors per smem stage (FP64)
 
 // the rank-4 KC products of one K stage into the 4 x 4 complex micro-tiles
 template <typename Z>
@@ -789,6 +781,144 @@ __device__ __forceinline__ void trail_stage(const Z (&sr)[4][KC][TB], const Z (&
   }
 }
 
+// FP32: 64 x 32 tiles, 128 threads of 4 x 4 quaternion entries; packed FP32 instructions
+// on pairs of rows, so that an entry pair's 32 products take 32 issue slots. All of a
+// chunk's reflectors are staged at once (components apart, for the pairs), one barrier
+// on each side; three CTAs per SM cover each other's staging and read-modify-write.
+// Bound: the FP32 pipe (n = 4096: 3.4e11 multiply-adds, 9.3 ms). 64 x 64 tiles of 256
+// threads, one CTA per SM, scalar: 20.5 ms, now 14.5.
+constexpr int TF_R = 64, TF_C = 32, TF_K = 16;
+using F32x2 = unsigned long long;
+__device__ __forceinline__ void fma2(F32x2& acc, F32x2 a, F32x2 b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+__device__ __forceinline__ F32x2 both(float v) {
+  F32x2 r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(v));
+  return r;
+}
+__device__ __forceinline__ float2 halves(F32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void copy_async4(float* smem, const float* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
+}
+__global__ void __launch_bounds__(128, 3) k_trail_f32(TridiagView<float> v, int p, int nbp, int t0) {
+  pdl_wait();
+  // [reflector][component of wa, wb, ya, yb][row or column]
+  __shared__ __align__(16) float sr[TF_K][8][TF_R];
+  __shared__ __align__(16) float sc[TF_K][8][TF_C];
+  const int n = v.n;
+  const int64_t ld = v.ld;
+  float2* A = v.M;
+  float2* B = v.M + n;
+  int I, J;
+  tri_tile((int)(blockIdx.x >> 1), I, J);
+  const int rb = t0 + I * TF_R, cb = t0 + J * TF_R + TF_C * (int)(blockIdx.x & 1);
+  if (cb >= n) return;
+  const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
+  F32x2 acc[4][4][2];  // component, column, pair of rows
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[k][c][0] = acc[k][c][1] = 0ull;
+  for (int k0 = 0; k0 < nbp; k0 += TF_K) {
+    const int kt = min(TF_K, nbp - k0);
+    if (k0) __syncthreads();
+    // rows, then columns, by asynchronous copies of one component each: all in flight
+    // at once (through registers their latency took as long as the products)
+    auto source = [&](int vec, int kk) -> const float* {
+      const int kc = k0 + kk;
+      const float2* q = vec == 0 ? A + (int64_t)(p + kc) * ld : vec == 1 ? B + (int64_t)(p + kc) * ld
+                      : vec == 2 ? v.Ya + (int64_t)kc * v.ldy : v.Yb + (int64_t)kc * v.ldy;
+      return reinterpret_cast<const float*>(q);
+    };
+    {
+      const int row = tid & (TF_R - 1), col = tid & (TF_C - 1);
+      const int gr = 2 * min(rb + row, n - 1), gc = 2 * min(cb + col, n - 1);
+#pragma unroll
+      for (int vec = 0; vec < 4; ++vec) {
+        for (int kk = tid / TF_R; kk < kt; kk += 128 / TF_R) {
+          const float* src = source(vec, kk) + gr;
+          copy_async4(&sr[kk][2 * vec][row], src);
+          copy_async4(&sr[kk][2 * vec + 1][row], src + 1);
+        }
+        for (int kk = tid / TF_C; kk < kt; kk += 128 / TF_C) {
+          const float* src = source(vec, kk) + gc;
+          copy_async4(&sc[kk][2 * vec][col], src);
+          copy_async4(&sc[kk][2 * vec + 1][col], src + 1);
+        }
+      }
+      asm volatile("cp.async.wait_all;" ::: "memory");
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int kk = 0; kk < kt; ++kk) {
+      F32x2 r[8][2];
+      float4 cv[8];
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(&sr[kk][s][4 * tr]);
+        r[s][0] = q.x;
+        r[s][1] = q.y;
+        cv[s] = *reinterpret_cast<const float4*>(&sc[kk][s][4 * tc]);
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        // w of the row with y of the column, then y of the row with w of the column
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          float x[4];
+#pragma unroll
+          for (int s = 0; s < 4; ++s) {
+            const float4 q = cv[4 * (1 - t) + s];
+            x[s] = c == 0 ? q.x : c == 1 ? q.y : c == 2 ? q.z : q.w;
+          }
+          const F32x2 ax = both(x[0]), ay = both(x[1]), bx = both(x[2]), by = both(x[3]);
+          const F32x2 nay = both(-x[1]), nbx = both(-x[2]), nby = both(-x[3]);
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const F32x2 rax = r[4 * t][h], ray = r[4 * t + 1][h], rbx = r[4 * t + 2][h], rby = r[4 * t + 3][h];
+            fma2(acc[0][c][h], rax, ax); fma2(acc[1][c][h], ray, ax); fma2(acc[2][c][h], rbx, ax); fma2(acc[3][c][h], rby, ax);
+            fma2(acc[0][c][h], ray, ay); fma2(acc[1][c][h], rax, nay); fma2(acc[2][c][h], rby, ay); fma2(acc[3][c][h], rbx, nay);
+            fma2(acc[0][c][h], rbx, bx); fma2(acc[1][c][h], rby, nbx); fma2(acc[2][c][h], rax, nbx); fma2(acc[3][c][h], ray, bx);
+            fma2(acc[0][c][h], rby, by); fma2(acc[1][c][h], rbx, by); fma2(acc[2][c][h], ray, nby); fma2(acc[3][c][h], rax, nby);
+          }
+        }
+      }
+    }
+  }
+  const bool whole = rb >= cb + TF_C && rb + TF_R <= n;
+  const int gr = rb + 4 * tr;
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const int gc = cb + 4 * tc + c;
+    if (gc >= n) continue;
+    float2* pa = A + gr + (int64_t)gc * ld;
+    float2* pb = B + gr + (int64_t)gc * ld;
+    const float2 a0x = halves(acc[0][c][0]), a0y = halves(acc[1][c][0]), a1x = halves(acc[0][c][1]), a1y = halves(acc[1][c][1]);
+    const float2 b0x = halves(acc[2][c][0]), b0y = halves(acc[3][c][0]), b1x = halves(acc[2][c][1]), b1y = halves(acc[3][c][1]);
+    const float2 ua[4] = {{a0x.x, a0y.x}, {a0x.y, a0y.y}, {a1x.x, a1y.x}, {a1x.y, a1y.y}};
+    const float2 ub[4] = {{b0x.x, b0y.x}, {b0x.y, b0y.y}, {b1x.x, b1y.x}, {b1x.y, b1y.y}};
+    if (whole) {
+      float2 x[4], y[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) { x[q] = pa[q]; y[q] = pb[q]; }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) { pa[q] = csub(x[q], ua[q]); pb[q] = csub(y[q], ub[q]); }
+    } else {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (gr + q >= n || gr + q < gc) continue;
+        pa[q] = csub(pa[q], ua[q]);
+        if (gr + q > gc) pb[q] = csub(pb[q], ub[q]);
+      }
+    }
+  }
+}
+
 template <typename R>
 __global__ void __launch_bounds__(NT) k_trail(TridiagView<R> v, int p, int nbp, int t0) {
   pdl_wait();  // launched with launch_pdl: the previous kernel's results first
@@ -809,38 +939,7 @@ __global__ void __launch_bounds__(NT) k_trail(TridiagView<R> v, int p, int nbp, 
 #pragma unroll
     for (int c = 0; c < 4; ++c) { accA[q][c] = czero<Z>(); accB[q][c] = czero<Z>(); }
 
-  if constexpr (std::is_same<R, float>::value) {
-    // FP32: the [vector: wa, wb, ya, yb][kk][row] stages double-buffered by
-    // cp.async (zero fill outside the matrix): the next stage's copies are in
-    // flight while this stage's products run, instead of each thread's loads
-    // waiting in turn before every stage
-    __shared__ Z s_r[2][4][KC][TB];
-    __shared__ Z s_c[2][4][KC][TB];
-    auto issue = [&](int k0, int buf) {
-      for (int e = tid; e < 4 * KC * TB; e += NT) {
-        const int row = e % TB, kk = (e / TB) % KC, vec = e / (TB * KC);
-        const int kg = k0 + kk;
-        const bool kok = kg < nbp;
-        const int kc = kok ? kg : 0;
-        const Z* base = vec == 0 ? A + (int64_t)(p + kc) * ld
-                      : vec == 1 ? B + (int64_t)(p + kc) * ld
-                      : vec == 2 ? v.Ya + (int64_t)kc * v.ldy
-                                 : v.Yb + (int64_t)kc * v.ldy;
-        const bool rok = kok && rb + row < n, cok = kok && cb + row < n;
-        cp_async8_zfill(&s_r[buf][vec][kk][row], base + (rok ? rb + row : 0), rok);
-        cp_async8_zfill(&s_c[buf][vec][kk][row], base + (cok ? cb + row : 0), cok);
-      }
-      cp_async_commit();
-    };
-    issue(0, 0);
-    for (int k0 = 0, st = 0; k0 < nbp; k0 += KC, ++st) {
-      const int buf = st & 1;
-      if (k0 + KC < nbp) { issue(k0 + KC, buf ^ 1); cp_async_wait<1>(); } else { cp_async_wait<0>(); }
-      __syncthreads();
-      trail_stage<Z>(s_r[buf], s_c[buf], tr, tc, accA, accB);
-      __syncthreads();  // the buffer is refilled by the issue two stages on
-    }
-  } else {
+  {
     // [vector: wa, wb, ya, yb][kk][row]
     __shared__ Z s_r[4][KC][TB];
     __shared__ Z s_c[4][KC][TB];
@@ -1010,7 +1109,10 @@ int tridiagonalize(TridiagView<R> v, int nb, cudaStream_t st) {
           continue;
         }
       }
-      ZQ_CUDA(launch_pdl(k_trail<R>, dim3(nblk * (nblk + 1) / 2), dim3(NT), st, v, p, nbp, t0));
+      if constexpr (std::is_same<R, float>::value)
+        ZQ_CUDA(launch_pdl(k_trail_f32, dim3(nblk * (nblk + 1)), dim3(128), st, v, p, nbp, t0));
+      else
+        ZQ_CUDA(launch_pdl(k_trail<R>, dim3(nblk * (nblk + 1) / 2), dim3(NT), st, v, p, nbp, t0));
       count_launch();
       prof_end(PC_TRAIL, st);
       ncp = 0;
