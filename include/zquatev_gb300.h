@@ -51,8 +51,8 @@ int zq_stedc_device(int n, const double* d, const double* e, double* lam, double
  * matrix b has order n2s[b] (even), starts at dD + 2*offs[b] doubles
  * (complex offset offs[b]) with leading dimension ld2s[b], and eigenvalues at
  * deig + eoffs[b]. All arrays n2s/ld2s/offs/eoffs are HOST arrays. Matrices
- * with n2 <= 512 run in one persistent kernel launch (one CTA per matrix,
- * largest first); larger ones through the per-matrix path. Ordered after
+ * with n2 <= 512 run together (up to n2 = 64 a warp each, larger ones over all
+ * SMs step by step); larger ones through the per-matrix path. Ordered after
  * `stream`; returns after the batch has finished, with the largest per-matrix
  * info (0 = all converged). The reference solves one matrix per call; this has
  * no counterpart there. */

@@ -96,3 +96,21 @@ def test_special_matrices(gpu, copies, orders):
         mats.append((np.eye(n) + 1e-14 * (u @ u.conj().T), z))
     mats *= copies
     _check(mats, _solve(gpu, mats))
+
+
+@pytest.mark.parametrize("n", range(1, 11))
+def test_single_solve(gpu, n):
+    """One matrix per call around the order up to which a warp solves it."""
+    import torch
+
+    a, b = _random(n, 800 + n)
+    for scale in (1.0, 1e-290, 1e290):
+        half = np.zeros((2 * n + 1, 2 * n), np.complex128)
+        half[:n, :n], half[n:2 * n, :n] = np.tril(a) * scale, np.tril(b) * scale
+        d = torch.from_numpy(np.ascontiguousarray(half.T)).cuda()
+        e = torch.full((2 * n,), -3.0, dtype=torch.float64, device="cuda")
+        rc = gpu.zquatev_device(2 * n, d.data_ptr(), 2 * n + 1, e.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert rc == 0, _lib.last_error()
+        out, e = d.cpu().numpy().T, e.cpu().numpy()
+        assert (e[n:] == -3.0).all() and (out[2 * n] == 0).all()
+        _check([(a * scale, b * scale)], [(e[:n], out[:2 * n])])

@@ -19,6 +19,7 @@
 //   * eig[n..] is left untouched, as in the reference.
 #include "zq_common.cuh"
 #include "zq_kernels.h"
+#include "zq_batched.h"
 #include "zq_context.h"
 #include "zq_applyq.h"
 #include "zq_resident.h"
@@ -279,7 +280,13 @@ struct StageTimer {
   }
 };
 
+// Up to this order one warp solves a single matrix in one launch (zq_small.cu) sooner
+// than the steps of the larger ones do in twenty or more: n = 2 0.029 against 0.083 ms,
+// n = 4 0.075 / 0.145, n = 8 0.193 / 0.215, n = 10 0.280 / 0.263.
+constexpr int SINGLE_SMALL_MAX = 8;
+
 int solve_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, bool vectors, cudaStream_t st) {
+  if (vectors && n <= SINGLE_SMALL_MAX) return small_solve(dD, ldd, n, deig, st);
   const int nb = nb_for(n);
   const char* tenv = getenv("ZQ_TIMING");
   StageTimer tm(tenv && tenv[0] == '1');

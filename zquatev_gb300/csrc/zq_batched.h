@@ -23,4 +23,7 @@ struct BatchTask {
 int small_launch(const BatchTask* tasks, int count, int nmax, int* dev_counter, double2* D, double* eig, int ctas,
                  int* dev_info, cudaStream_t st);
 
+// one matrix of order 1 to 24 (48 KB of shared memory need no opt-in), on the stream
+int small_solve(double2* D, int64_t ld, int n, double* eig, cudaStream_t st);
+
 }  // namespace zq

@@ -1,5 +1,5 @@
-// Batches of mid-size matrices (order 33 to 256, FP64) as a few launches over all
-// matrices at once. Reference: the steps of ts::zquatev (zquatev.cc:42-100) once
+// Batches of mid-size matrices (order 33 to 256, from 16 where a batch has few small
+// ones; FP64) as a few launches over all matrices at once. Reference: the steps of ts::zquatev (zquatev.cc:42-100) once
 // per matrix; it has no batched entry point.
 //
 //   1. the reductions: a queue of matrices, largest first, each taken by a cluster
@@ -13,7 +13,7 @@
 // where the FP64 pipe (2 FMA per clock) alone needs 76 ms and the serial QL
 // iteration as much again: 340 ms, whatever the batch. Here every step spreads
 // over the GPU, bound by the FP64 pipe: 40 matrices each of orders 256, 215,
-// 214, 140, 47, 34, 23 and 13 take 127 ms instead of 338 (reductions 58 ms,
+// 214, 140, 47, 34, 23 and 13 take 120 ms instead of 338 (reductions 58 ms,
 // 27 ms of FP64 pipe time; divide and conquer 12 ms; back-transform 50 ms, 40 ms
 // of pipe time; the small ones 3 ms).
 #include "zq_common.cuh"

@@ -24,10 +24,11 @@
 // at orders where the arithmetic takes a few; and GB300's FP64 pipe (2 FMA per
 // clock per SM) makes the split of the FP64 work over all SMs matter more than
 // operand reuse, hence small tiles. Reduction before and after: FP64 n = 384
-// 29 -> 6.3 ms, n = 750 60 -> 19.6 ms (7.2 ms of FP64 pipe time); FP32 n = 1023
-// 23.5 -> 9.8 ms. What remains per column (FP32, n = 600, cycles): reflector
-// scalars 3100, vectors 1100, sweep 2100, rows 3100, column 3400, barriers
-// 3 x 2500: chains of L2 round trips and dependent FP64 instructions.
+// 29 -> 4.9 ms, n = 750 60 -> 18 ms (7.2 ms of FP64 pipe time); FP32 n = 1023
+// 23.5 -> 8.4 ms. What remains per column (FP32, n = 750, cycles): reflector
+// scalars 1400, vectors 1250, sweep 2400, c 1000, rows 2450, column 860, norms
+// 780, barriers 3100 + 2500 (2540 in isolation): chains of L2 round trips and
+// dependent instructions.
 //
 // Tile work: one warp per tile, lane (tr, tc) = (lane & 7, lane >> 3) owns
 // rows tr + 8 i and columns tc + 4 q of the tile, stored so that a lane only

@@ -390,6 +390,7 @@ struct SmallArgs {
   int* info;     // per task: 0 ok, > 0 QL non-convergence
   SmallOffsets o;
   int nmax;
+  BatchTask one;  // the only task where tasks is null (no counter, no info)
 };
 
 __global__ void __launch_bounds__(SMALL_WARPS * 32, 2) k_small(SmallArgs a) {
@@ -400,16 +401,18 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 2) k_small(SmallArgs a) {
   // CTAs that share an SM run their chains in different quadrants
   const int chain = (int)blockIdx.x % warps;
   double* s = smem + warp * a.o.total;
+  int pass = 0;
   for (;;) {
-    if (threadIdx.x == 0) s_first = atomicAdd(a.counter, warps);
+    if (threadIdx.x == 0 && a.tasks) s_first = atomicAdd(a.counter, warps);
+    if (threadIdx.x == 0 && !a.tasks) s_first = pass++;
     __syncthreads();
     const int t = s_first + warp;
     if (s_first >= a.count) return;
     BatchTask tk{};
-    if (t < a.count) tk = a.tasks[t];
+    if (t < a.count) tk = a.tasks ? a.tasks[t] : a.one;
     int n = tk.n;
     if (n > a.nmax) {  // not within the launch's limit: reported, not solved
-      if (lane == 0) a.info[tk.out_slot] = -1;
+      if (lane == 0 && a.info) a.info[tk.out_slot] = -1;
       n = 0;
     }
     if (lane == 0) s_n[warp] = n;
@@ -460,13 +463,24 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 2) k_small(SmallArgs a) {
       __syncthreads();  // the rotations are read
     }
     __syncwarp();
-    if (own && nl > 0) a.info[a.tasks[s_first + lane].out_slot] = q.bad;
+    if (own && nl > 0 && a.info) a.info[a.tasks[s_first + lane].out_slot] = q.bad;
     if (n > 0) small_back(A, B, gld, tk.Ep ? tk.Ep : a.eig + tk.eoff, n, scale, s, a.o, lane);
     __syncthreads();  // s_first, s_n and the matrices are free
   }
 }
 
 }  // namespace
+
+int small_solve(double2* D, int64_t ld, int n, double* eig, cudaStream_t st) {
+  SmallArgs a{};
+  a.count = 1;
+  a.o = small_offsets(n);
+  a.nmax = n;
+  a.one.Dp = D; a.one.Ep = eig; a.one.n = n; a.one.ld = (int)ld;
+  k_small<<<1, 32, sizeof(double) * (size_t)a.o.total, st>>>(a);
+  ZQ_LAUNCH_CHECK();
+  return ZQ_OK;
+}
 
 int small_launch(const BatchTask* tasks, int count, int nmax, int* dev_counter, double2* D, double* eig, int ctas,
                  int* dev_info, cudaStream_t st) {
