@@ -13,7 +13,7 @@ flush is needed between steps.
           (device-to-device) and solved through the device C ABI; ms per solve.
   e2e     the reference-facing host call (zquatev_c on pinned host arrays): H2D
           of the left half, solve, D2H of all of D and eig, per solve.
-  roofline  the dominant kernel (the Ozaki tensor-core product), timed with
+  roofline  the dominant kernel (the residue tensor-core product), timed with
           CUDA events on its launch stream during the timed region, executed
           bf16 flops against MEASURED_PEAKS.json's sustained bf16 figure; the
           FP64 path's kernels are reported against the FP64 DFMA peak measured
@@ -43,10 +43,10 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 METRIC = "n2=8192 solve ms; mixed-stream solves/s, p99 ms vs plain FP64 at resid≤1e-12"
-# DRAM bytes (read + write) per executed bf16 flop of the Ozaki product kernel,
-# from one ncu capture of k_oz_umma<2> (n2 = 4096, second step's P1, 8 slices:
-# 6.264 + 1.048 GB / 4.95e12 flop)
-OZ_BYTES_PER_FLOP = 7.312e9 / 4.95e12
+# DRAM bytes (read + write) per executed bf16 flop of the residue product kernel,
+# from one ncu capture of k_crt_mma (n2 = 4096, a lower-triangle product of the
+# second step: 0.711 + 0.079 GB / 6.38e11 flop)
+OZ_BYTES_PER_FLOP = 0.7908e9 / 6.38e11
 
 
 def parse():
@@ -910,12 +910,12 @@ def main():
                     "d2h_bytes_per_step": n2 * n2 * 16 + n * 8, "host_memory": "pinned",
                     "samples_ms": [round(x, 1) for x in e2e_ms], "clocks": e2e_clk.summary()},
             "gpu_launches": None,
-            "roofline": {"bound": "tensor", "kernel": "k_oz_umma<2> (bf16 2-SM tcgen05.mma cta_group::2, M=256 N=256 per CTA pair; TMEM accumulators; TMA; Ozaki slices)",
+            "roofline": {"bound": "tensor", "kernel": "k_crt_mma (bf16 2-SM tcgen05.mma cta_group::2, M=256 N=256 per CTA pair; TMEM accumulators; TMA; residues)",
                          "achieved": achieved, "peak": bf16_peak, "unit": "TFLOP/s",
                          "frac": (achieved / bf16_peak) if achieved else None,
                          "traffic": (OZ_BYTES_PER_FLOP * oz_flops / oz_launches
                                      if (oz_launches and OZ_BYTES_PER_FLOP) else None),
-                         "traffic_source": "profiles/k_oz_umma_n2-4096.md: dram read+write per executed flop of one "
+                         "traffic_source": "profiles/k_crt_n2-4096.md: dram read+write per executed flop of one "
                                            "captured launch (n2=4096), scaled by this step's executed flops per launch",
                          "peak_source": peak_src, "launches_per_step": oz_launches, "ms_per_step": oz_ms},
             "stage_ms": {"refine": round(prof["refine"][0] / args.steps, 2), "ozaki": round(oz_ms, 2),
