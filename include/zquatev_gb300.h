@@ -39,7 +39,9 @@ int zquatev_values(int n2, double* D, int ld2, double* eig);
  * call returns without synchronising. */
 int zquatev_device(int n2, double* dD, int ld2, double* deig, void* stream);
 
-/* Device-pointer eigenvalues-only variant. */
+/* Device-pointer eigenvalues-only variant. Above n2 = 438 the refined path forms them
+ * and the call waits for its convergence figure, unless `stream` is capturing or
+ * zq_set_path(0) is in force. */
 int zquatev_values_device(int n2, double* dD, int ld2, double* deig, void* stream);
 
 /* Real symmetric tridiagonal eigensolver (the stage that replaces zhbev at

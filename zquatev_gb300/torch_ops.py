@@ -7,9 +7,10 @@ the left half of H = (A -B*; B A*), which is all the reference reads). It
 returns ``(eig, v)``: the n ascending eigenvalues (float64) and the (n2, n2)
 eigenvectors in the (U -V*; V U*) layout, column j of ``v`` belonging to
 ``eig[j % n]``. The solve runs through ``zquatev_device`` (the drop-in's path
-policy: refined from n = 160 up) on torch's current stream, without host
-synchronisation. ``torch.ops.zquatev_gb300.eigvalsh(h_left)`` returns the
-eigenvalues only (``zquatev_values_device``).
+policy: refined from n = 160 up, where the host waits for the refinement's
+convergence figures) on torch's current stream. ``torch.ops.zquatev_gb300.eigvalsh(h_left)``
+returns the eigenvalues only (``zquatev_values_device``: refined from n = 220 up,
+not while the stream is capturing).
 
 The operators are registered for CUDA only (a CPU tensor raises: there is no
 CPU fallback) and have fake implementations, so they trace under FakeTensor /
