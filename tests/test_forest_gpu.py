@@ -91,3 +91,28 @@ def test_layouts_share_the_workspace(gpu):
         rc = gpu.zquatev_batched_device(len(orders), *(a.ctypes.data for a in args), d.data_ptr(), e.data_ptr(), 0)
         assert rc == 0, _lib.last_error()
         _check(orders, args, d0, d, e)
+
+
+@pytest.mark.parametrize("orders", [[48], [64, 33, 32, 20, 16, 15, 3], [256, 130, 40] + [9] * 130])
+def test_server_batches(gpu, orders):
+    """Requests in allocations of their own, alone, with few and with many small ones beside them."""
+    import torch
+
+    from zquatev_gb300.serve import Server
+
+    with Server(hbm_budget_bytes=4 << 30, batch_max_n2=512) as srv:
+        for _ in range(2):
+            before = [inputs.random_matrix(n, 700 + i) for i, n in enumerate(orders)]
+            work = [np.array(d, order="F", copy=True) for d in before]
+            eigs = [np.zeros(n) for n in orders]
+            ids = [srv.submit(2 * n, d, 2 * n, e) for n, d, e in zip(orders, work, eigs)]
+            for i in ids:
+                info, t = srv.wait(i)
+                assert info == 0 and t["path"] == "batched"
+            for n, d0, d, w in zip(orders, before, work, eigs):
+                h = inputs.full_from_blocks(d0[:n, :n], d0[n:, :n])
+                lam = np.concatenate([w, w])
+                assert (np.diff(w) >= 0).all()
+                assert np.abs(h @ d - d * lam).max() <= TOL * np.abs(w).max()
+                assert np.abs(d.conj().T @ d - np.eye(2 * n)).max() <= TOL
+        assert srv.stats()["peak_reserved_bytes"] <= 4 << 30

@@ -1,7 +1,7 @@
 // Batched solve of quaternion-Hermitian matrices in one persistent kernel, one
 // CTA per matrix, work handed out largest-first through a device counter: the
-// request server's batches above order 32, the plan's variants with a lower switch
-// to the warp-per-matrix kernel (zq_small.cu), and the solve that allocates nothing.
+// plan's variants with a lower switch to the warp-per-matrix kernel (zq_small.cu),
+// the refinement's larger cluster blocks, and the solve that allocates nothing.
 //
 // Reference: the same four steps as ts::zquatev (zquatev.cc:42-100) run once
 // per matrix; the reference has no batched entry point, and below n = nb + 2

@@ -113,7 +113,7 @@ int BatchForest::build(const std::vector<ForestItem>& items, cudaStream_t st) {
     }
     if (one <= split) parts.assign(1, Chunk::TriClass{0, c->count, ns[0], G1, nullptr, nullptr});
     c->tri = parts;
-    for (const Chunk::TriClass& t : c->tri) c->tri_ws_bytes = std::max(c->tri_ws_bytes, tri_queue_bytes(t.G, t.m_max));
+    for (const Chunk::TriClass& t : c->tri) c->tri_ws_bytes = std::max(c->tri_ws_bytes, tri_queue_bytes(t.G, t.m_max, t.count));
     c->tri_ws_bytes = up(c->tri_ws_bytes) + 256;  // and the queue's counter
     // Back-transform: one launch per register class (largest order first). With
     // more columns than the GPU has quadrants several times over, a warp takes a

@@ -998,7 +998,9 @@ static size_t tri_queue_stride(int G, int m_max) {
 }
 static int tri_queue_groups(int G) { return std::max(1, clusters_at_once<double, rt_tile_edge<double>()>(G)); }
 
-size_t tri_queue_bytes(int G, int m_max) { return tri_queue_stride(G, m_max) * tri_queue_groups(G); }
+size_t tri_queue_bytes(int G, int m_max, int ntasks) {
+  return tri_queue_stride(G, m_max) * std::min(ntasks, tri_queue_groups(G));
+}
 
 int tri_queue(const TriTask<double>* tasks, int ntasks, double2* base, int m_max, int G, void* ws, int* queue, int* err,
               cudaStream_t st) {

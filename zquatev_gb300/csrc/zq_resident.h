@@ -69,7 +69,7 @@ struct TriArgs {
 // a cluster of G CTAs; ws as tri_queue_bytes(G, m_max), queue one int.
 int tri_queue(const TriTask<double>* tasks, int ntasks, double2* base, int m_max, int G, void* ws, int* queue, int* err,
               cudaStream_t st);
-size_t tri_queue_bytes(int G, int m_max);
+size_t tri_queue_bytes(int G, int m_max, int ntasks);
 // cluster size that finishes a queue of these orders (largest first) soonest, and
 // the estimated time in clock cycles; 0: no cluster holds the largest
 int tri_queue_cluster(const int* orders, int count, double* cycles);

@@ -10,8 +10,8 @@
 //
 // Admitted requests run as soon as an execution slot is free:
 //  * n2 <= batch_max_n2 (at most 512): batch workers take every such request that is ready
-//    when they become free and solve them in one launch of the persistent
-//    batched kernel (largest first), so the batch size follows the load;
+//    when they become free and solve them together (orders above a warp's as a
+//    forest, the others a warp each), so the batch size follows the load;
 //  * larger ones: lane workers (one host thread, stream pair and context each)
 //    run the drop-in's policy path (refined, FP64 fallback) on workspace taken
 //    from the stream-ordered pool for that request.
@@ -215,13 +215,16 @@ void lane_loop(Server* s, Context* c) {
   }
 }
 
+constexpr size_t FOREST_KEEP = (size_t)64 << 20;  // scratch a batch worker keeps between batches
+
 void batch_loop(Server* s, Context* c) {
   cudaSetDevice(s->device);
   const size_t tb = batched_task_bytes();
   std::vector<char> htasks;
   std::vector<int> hinfo;
+  BatchForest forest;  // the orders above a warp's, all together (a CTA each: 10 ms at n = 48)
   for (;;) {
-    std::vector<Req*> batch;
+    std::vector<Req*> batch, all;
     {
       std::unique_lock<std::mutex> lk(s->mu);
       s->cv_batch.wait(lk, [&] { return s->stop || !s->ready_small.empty(); });
@@ -234,15 +237,30 @@ void batch_loop(Server* s, Context* c) {
       for (Req* r : batch) r->t_start = t;
       ++s->batches;
     }
-    // longest first: the persistent kernel hands out tasks in this order
+    // longest first: the kernels hand out tasks in this order
     std::stable_sort(batch.begin(), batch.end(), [](const Req* a, const Req* b) { return a->n > b->n; });
+    all = batch;
+    int few = 0;
+    for (Req* r : batch) few += r->n > 0 && r->n <= SMALL_MAX;
+    // the matrices lie in allocations of their own: offsets from the first one
+    double2* const D0 = batch[0]->dD;
+    double* const E0 = batch[0]->deig;
+    std::vector<ForestItem> items;
+    std::vector<Req*> rest, joint;
+    for (Req* r : batch) {
+      if (!forest_takes(r->n, few)) { rest.push_back(r); continue; }
+      joint.push_back(r);
+      items.push_back(ForestItem{r->n, r->n2, (long long)(r->dD - D0), (long long)(r->deig - E0)});
+    }
+    batch.swap(rest);
     const int k = (int)batch.size();
-    const int ctas = std::min(k, 2 * s->sms);
+    const int ctas = std::max(1, std::min(k, 2 * s->sms));
     const size_t task_bytes = (tb * k + 255) & ~(size_t)255;
     const size_t info_bytes = (sizeof(int) * (k + 1) + 255) & ~(size_t)255;
     const size_t need = task_bytes + info_bytes + sizeof(double) * (size_t)batched_ws_stride() * ctas;
     htasks.resize(tb * k);
     hinfo.assign(k, 0);
+    int herr = 0;
     for (int q = 0; q < k; ++q) batched_fill_task_ptr(htasks.data() + q * tb, batch[q]->dD, batch[q]->deig, batch[q]->n,
                                                       batch[q]->n2, q);
     int rc = ZQ_OK;
@@ -255,21 +273,32 @@ void batch_loop(Server* s, Context* c) {
     if (rc == ZQ_OK) {
       char* b = reinterpret_cast<char*>(mem);
       int* dinfo = reinterpret_cast<int*>(b + task_bytes);
-      for (Req* r : batch)
+      for (Req* r : all)
         if (cudaStreamWaitEvent(c->st, r->ready, 0) != cudaSuccess) rc = ZQ_ERR_CUDA;
-      if (rc == ZQ_OK && cudaMemcpyAsync(b, htasks.data(), tb * k, cudaMemcpyHostToDevice, c->st) != cudaSuccess)
+      if (rc == ZQ_OK && !items.empty()) {
+        rc = forest.matches(items) ? (int)ZQ_OK : forest.build(items, c->st);
+        if (rc == ZQ_OK) rc = forest.run(D0, E0, c->st);
+        if (rc == ZQ_OK && cudaMemcpyAsync(&herr, forest.error_flag(), sizeof(int), cudaMemcpyDeviceToHost, c->st) != cudaSuccess)
+          rc = ZQ_ERR_CUDA;
+      }
+      if (rc == ZQ_OK && k > 0 && cudaMemcpyAsync(b, htasks.data(), tb * k, cudaMemcpyHostToDevice, c->st) != cudaSuccess)
         rc = ZQ_ERR_CUDA;
-      if (rc == ZQ_OK)
+      if (rc == ZQ_OK && k > 0)
         rc = batched_launch(b, batched_split(k, batched_warp_max(), [&](int q) { return batch[q]->n; }), dinfo + k, nullptr,
                             nullptr, reinterpret_cast<double*>(b + task_bytes + info_bytes), ctas, dinfo, c->st);
-      if (rc == ZQ_OK && cudaMemcpyAsync(hinfo.data(), dinfo, sizeof(int) * k, cudaMemcpyDeviceToHost, c->st) != cudaSuccess)
+      if (rc == ZQ_OK && k > 0 &&
+          cudaMemcpyAsync(hinfo.data(), dinfo, sizeof(int) * k, cudaMemcpyDeviceToHost, c->st) != cudaSuccess)
         rc = ZQ_ERR_CUDA;
-      for (int q = 0; q < k && rc == ZQ_OK; ++q) rc = copy_back(batch[q], c->st);
+      for (size_t q = 0; q < all.size() && rc == ZQ_OK; ++q) rc = copy_back(all[q], c->st);
       cudaFreeAsync(mem, c->st);
     }
-    for (Req* r : batch) cudaFreeAsync(r->dD, c->st);
+    for (Req* r : all) cudaFreeAsync(r->dD, c->st);
     const cudaError_t e = cudaStreamSynchronize(c->st);
     if (rc == ZQ_OK && e != cudaSuccess) { set_last_error(e, "server batch", __FILE__, __LINE__); rc = ZQ_ERR_CUDA; }
+    if (rc == ZQ_OK && herr) { set_error_message("server batch: a device-side wait ran out of time"); rc = ZQ_ERR_TIMEOUT; }
+    // its tables and scratch are within the finished requests' footprints: not kept beyond them
+    if (forest.bytes() > FOREST_KEEP) forest.release();
+    for (Req* r : joint) finish(s, r, rc, 2);
     for (int q = 0; q < k; ++q) finish(s, batch[q], rc != ZQ_OK ? rc : hinfo[q], 2);
   }
 }
@@ -287,7 +316,13 @@ long long zq_solve_footprint(int n2, int path) {
   if (path == -1) path = n <= batched_max_n() ? 2 : path_for(n);
   if (path == 2 && n > batched_max_n()) { set_error_message("batched kernel takes n2 <= 512"); return ZQ_ERR_LIMIT; }
   const size_t mat = sizeof(double2) * (size_t)n2 * n2 + sizeof(double) * (size_t)(n + 32);
-  if (path == 2) return (long long)(mat + sizeof(double) * (size_t)batched_ws_stride() + 256);
+  if (path == 2) {
+    // the CTA kernel's workspace, or a matrix's share of the joint solve's (three n x n
+    // buffers, vectors and tables, and a cluster's exchange buffers)
+    const size_t cta = sizeof(double) * (size_t)batched_ws_stride();
+    const size_t joint = sizeof(double) * (5 * (size_t)n * n + 256 * (size_t)n) + 65536;
+    return (long long)(mat + std::max(cta, joint) + 256);
+  }
   size_t f = 0, r = 0;
   solve_workspace_bytes(n, &f, &r);
   return (long long)(mat + f + (path == 1 ? r : 0));
