@@ -266,6 +266,14 @@ template <typename R> __host__ __device__ __forceinline__ int row_ctas(int G) {
 // four lanes of a row exchange theirs by shuffles). The matrix is scaled by a
 // power of two once (largest entry in [1, 2)), so no sum of squares needs a scale
 // of its own; FP32 columns whose squares vanish are 1e-19 of the matrix.
+//
+// Between two barriers an exchanged array is written or read by other CTAs, never
+// both: a CTA that runs ahead must not overwrite what another has yet to read. The
+// phases and what they touch:
+//   load     writes cpart (largest magnitudes)
+//   column 0 reads cpart; writes x, npart, q2
+//   sweep    reads x, y, npart, q2; writes col, part, cpart (parts of c)
+//   rows     reads col, part, cpart, and x of the CTA's own rows; writes x, y, npart, q2
 template <typename R, int T, int LPR, bool CL>
 __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int rank, int G, unsigned char* smem,
                               unsigned& target, int* err, long long limit) {
@@ -343,13 +351,13 @@ __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int r
   if (tid == 0) {
     unsigned long long b = 0;
     for (int q = 0; q < RT_WARPS; ++q) b = max(b, abs_bits(s_red[q]));
-    gr.npart[rank] = bits_to_double(b);
+    gr.cpart[rank] = bits_to_double(b);
   }
   if (!barrier()) return false;
   double scale = 1.0;
   {
     unsigned long long b = 0;
-    for (int i = lane; i < G; i += 32) b = max(b, abs_bits(__ldcg(gr.npart + i)));
+    for (int i = lane; i < G; i += 32) b = max(b, abs_bits(__ldcg(gr.cpart + i)));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
     const int be = (int)(b >> 52);
