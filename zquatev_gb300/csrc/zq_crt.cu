@@ -317,7 +317,8 @@ __global__ void __launch_bounds__(CB_THREADS, 1)
         }
       }
       // copies in flight finish before the CTA may exit (rank 1 is held at the
-      // final cluster barrier until rank 0, which has the full barriers, is done)
+      // final cluster barrier until rank 0, which has the full barriers, is done;
+      // after an abort abort_hold covers what the peer alone issued)
       if (rank == 0)
         for (int q = (ks > CB_STAGES ? ks - CB_STAGES : 0); q < ks; ++q)
           mbar_drain(full0 + 8 * (q % CB_STAGES), (q / CB_STAGES) & 1, 2000000LL);
@@ -410,6 +411,7 @@ __global__ void __launch_bounds__(CB_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (s_abort) abort_hold();
   cluster_sync();  // both CTAs' MMAs and drains are finished before the collective release
   if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   if (threadIdx.x == 0 && s_abort) atomicExch(g.err, 1);

@@ -227,7 +227,8 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
       // cluster a stage may lack the peer's part and never complete: its own
       // copies land within microseconds, so wait about a millisecond there).
       // In variant 2 only rank 0 holds the full barriers; rank 1 is held at
-      // the final cluster barrier until rank 0 has drained them.
+      // the final cluster barrier until rank 0 has drained them. (What the peer
+      // alone issued is covered by abort_hold.)
       if (V != 2 || rank == 0)
         for (int q = (issued > STAGES ? issued - STAGES : 0); q < issued; ++q)
           mbar_drain(full0 + 8 * (q % STAGES), (q / STAGES) & 1, PAIR ? 2000000LL : UM_WAIT_CYCLES);
@@ -362,6 +363,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (PAIR && s_abort) abort_hold();
   // variant 2: both CTAs' MMAs and drains are finished before the collective release
   if (V == 2) cluster_sync();
   if (warp == 1) {

@@ -53,6 +53,16 @@ __device__ __forceinline__ void mbar_drain(uint32_t bar, uint32_t parity, long l
   }
 }
 
+// After an abort in a pair of CTAs: about a millisecond (copies land within
+// microseconds). A stage that one CTA filled and the other did not never
+// completes, so no barrier says when its copies have landed; neither CTA may pass
+// the final cluster barrier before they have.
+__device__ __forceinline__ void abort_hold() {
+  const long long t0 = clock64();
+  while (clock64() - t0 <= 2000000LL) {
+  }
+}
+
 // the same box written to this CTA and its cluster peer (same shared offsets);
 // complete_tx is signalled on the mbarrier at `bar` in each destination
 __device__ __forceinline__ void tma_2d_mc(uint32_t dst, const CUtensorMap* tm, int x, int y, uint32_t bar, uint16_t mask) {
