@@ -202,7 +202,16 @@ __global__ void __launch_bounds__(256, 3) k_crt_split(CrtSide s, bool is_a, int 
   }
 }
 
-// exponents (2^e above the largest magnitude) of a real operand's rows (A) or columns (B)
+// exponents (2^e above the largest magnitude) of a real operand's rows (A) or columns (B);
+// CRT_NOT_FINITE where one of the values is Inf or NaN, which residues cannot carry: the
+// product's row or column is then NaN (k_crt_join)
+constexpr int CRT_NOT_FINITE = 5000;
+__device__ __forceinline__ int crt_exponent(unsigned long long mb) {
+  if (mb >= (0x7ffull << 52)) return CRT_NOT_FINITE;
+  int e;
+  frexp(bits_to_double(mb), &e);
+  return e;
+}
 __global__ void k_crt_exp_init(int* e, int n) {
   pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -224,7 +233,7 @@ __global__ void __launch_bounds__(256) k_crt_exp_real(const double* __restrict__
     if (warp == 0 && r < count) {
 #pragma unroll
       for (int w = 1; w < 8; ++w) mb = max(mb, s[w][lane]);
-      if (mb) { int e; frexp(bits_to_double(mb), &e); atomicMax(exps + r, e); }
+      if (mb) atomicMax(exps + r, crt_exponent(mb));
     }
   } else {     // columns: one warp each
     const int c = blockIdx.x * 8 + warp;
@@ -233,7 +242,7 @@ __global__ void __launch_bounds__(256) k_crt_exp_real(const double* __restrict__
     for (int k = lane; k < K; k += 32) mb = max(mb, abs_bits(__ldg(X + k + (int64_t)c * ld)));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mb = max(mb, __shfl_xor_sync(0xffffffffu, mb, o));
-    if (lane == 0 && mb) { int e; frexp(bits_to_double(mb), &e); exps[c] = e; }
+    if (lane == 0 && mb) exps[c] = crt_exponent(mb);
   }
 }
 
@@ -508,7 +517,9 @@ __global__ void __launch_bounds__(256) k_crt_join(const uint8_t* __restrict__ R,
                                     d[2][2] - d[0][2] - d[1][2], cj.pm, E);
         reinterpret_cast<double2*>(C)[row + (int64_t)col * ldc] = make_double2(re, im);
       } else {
-        C[row + (int64_t)col * ldc] = crt_value(d[0][0], d[0][1], d[0][2], cj.pm, E);
+        const bool finite = ea[row] != CRT_NOT_FINITE && e_col != CRT_NOT_FINITE;
+        C[row + (int64_t)col * ldc] = finite ? crt_value(d[0][0], d[0][1], d[0][2], cj.pm, E)
+                                             : __longlong_as_double(0x7ff8000000000000ll);
       }
     }
   }

@@ -355,17 +355,22 @@ __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int r
   }
   if (!barrier()) return false;
   double scale = 1.0;
+  bool finite = true;
   {
     unsigned long long b = 0;
     for (int i = lane; i < G; i += 32) b = max(b, abs_bits(__ldcg(gr.cpart + i)));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
     const int be = (int)(b >> 52);
+    finite = be < 2047;
     // FP32 data: the scale and its inverse stay normal numbers of R
     const int lim = sizeof(R) == 8 ? 1022 : 126;
     if (b != 0) scale = pow2_biased(be < 1023 - lim ? 1023 - lim : (be > 1023 + lim ? 1023 + lim : be));
   }
-  const R inv = (R)bits_to_double((2046ull << 52) - (unsigned long long)__double_as_longlong(scale));
+  // (a matrix that holds an Inf or a NaN becomes NaN as a whole: at the scale of its
+  // largest entry its numbers would vanish and leave a finite result)
+  const R inv = (R)(finite ? bits_to_double((2046ull << 52) - (unsigned long long)__double_as_longlong(scale))
+                           : __longlong_as_double(0x7ff8000000000000ll));
   for (int q = warp; q < mine; q += RT_WARPS) {
     R* tl = tiles + (size_t)q * TILE;
 #pragma unroll 4

@@ -111,8 +111,11 @@ __device__ double small_reduce(double2* A, double2* B, int64_t gld, int n, doubl
     top = t > top ? t : top;
   }
   int ex = (int)(top >> 52);
+  const bool finite = ex < 2047;
   ex = ex < 1 ? 1023 : (ex > 2045 ? 2045 : ex);  // zero (or subnormal) matrices stay as they are
-  const double scale = __hiloint2double(ex << 20, 0), inv = __hiloint2double((2046 - ex) << 20, 0);
+  // (a matrix that holds an Inf or a NaN becomes NaN as a whole)
+  const double scale = __hiloint2double(ex << 20, 0);
+  const double inv = finite ? __hiloint2double((2046 - ex) << 20, 0) : __longlong_as_double(0x7ff8000000000000ll);
   __syncwarp();
   for (int t = lane; t < n * ld; t += 32) {
     const double2 a = ma[t], b = mb[t];

@@ -515,7 +515,9 @@ __global__ void k_dc_rotate(const DcNode* nodes, int cnt, DcWork w, ZT* Mb) {
 }
 
 // Scale and tear, one block per matrix: the largest |entry| becomes 1, the
-// off-diagonals leave the diagonal.
+// off-diagonals leave the diagonal. An entry that is Inf or NaN makes the scale and
+// so the whole matrix NaN: deflation compares and sorts, and would pass a part of it
+// off as finite.
 __global__ void k_dc_scale(const double* d, const double* e, const DcMat* mats, double* dmod, double* es, double* scal) {
   pdl_wait();
   __shared__ double sh[32];
@@ -527,9 +529,12 @@ __global__ void k_dc_scale(const double* d, const double* e, const DcMat* mats, 
     mb = max(mb, abs_bits(d[i]));
     if (i < n - 1) mb = max(mb, abs_bits(e[i]));
   }
-  const double m = block_max(bits_to_double(mb), sh);
-  if (threadIdx.x == 0) scal[blockIdx.x] = m > 0.0 ? fmax(m, 2.2250738585072014e-308) : m;
-  const double inv = (m > 0.0) ? 1.0 / fmax(m, 2.2250738585072014e-308) : 1.0;
+  constexpr unsigned long long INF = 0x7ffull << 52;  // (a NaN would get lost in the maximum)
+  const double m = block_max(bits_to_double(min(mb, INF)), sh);
+  const double nan = __longlong_as_double(0x7ff8000000000000ll);
+  const bool finite = abs_bits(m) < INF;
+  if (threadIdx.x == 0) scal[blockIdx.x] = !finite ? nan : (m > 0.0 ? fmax(m, 2.2250738585072014e-308) : m);
+  const double inv = !finite ? nan : ((m > 0.0) ? 1.0 / fmax(m, 2.2250738585072014e-308) : 1.0);
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     const double el = (i > 0) ? e[i - 1] * inv : 0.0;
     const double er = (i < n - 1) ? e[i] * inv : 0.0;
@@ -538,7 +543,7 @@ __global__ void k_dc_scale(const double* d, const double* e, const DcMat* mats, 
   }
 }
 
-// eigenvalues times the scale, into place (NaN when a merge product failed)
+// eigenvalues times the scale, into place (NaN when the scale is, or a merge product failed)
 __global__ void k_dc_unscale(const double* lam, const DcMat* mats, const double* scal, double* eig, const int* err) {
   pdl_wait();
   const DcMat mt = mats[blockIdx.y];
@@ -546,7 +551,7 @@ __global__ void k_dc_unscale(const double* lam, const DcMat* mats, const double*
   if (i >= mt.n) return;
   const double s = scal[blockIdx.y];
   const double v = lam[mt.p + i];
-  eig[mt.eoff + i] = *err ? __longlong_as_double(0x7ff8000000000000ll) : (s > 0.0 ? v * s : v);
+  eig[mt.eoff + i] = *err || s != s ? __longlong_as_double(0x7ff8000000000000ll) : (s > 0.0 ? v * s : v);
 }
 
 // Z_node = blockdiag(Z1, Z2) M for small nodes: a thread per entry. The tiled
