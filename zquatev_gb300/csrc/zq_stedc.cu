@@ -546,10 +546,10 @@ __global__ void k_dc_scale(const double* d, const double* e, const DcMat* mats, 
 // eigenvalues times the scale, into place (NaN when the scale is, or a merge product failed)
 __global__ void k_dc_unscale(const double* lam, const DcMat* mats, const double* scal, double* eig, const int* err) {
   pdl_wait();
-  const DcMat mt = mats[blockIdx.y];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const DcMat mt = mats[blockIdx.x];  // (x: a batch may have more matrices than the other dimensions take)
+  const int i = blockIdx.y * blockDim.x + threadIdx.x;
   if (i >= mt.n) return;
-  const double s = scal[blockIdx.y];
+  const double s = scal[blockIdx.x];
   const double v = lam[mt.p + i];
   eig[mt.eoff + i] = *err || s != s ? __longlong_as_double(0x7ff8000000000000ll) : (s > 0.0 ? v * s : v);
 }
@@ -885,8 +885,8 @@ static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, 
       }
     }
   }
-  ZQ_CUDA(launch_pdl_smem(k_dc_unscale, dim3((unsigned)ceil_div(nmax, 128), (unsigned)nmat), dim3(128), 0, st, P.lam[0], P.mats_dev, P.scal, lam_out,
-                                                                                    P.err));
+  ZQ_CUDA(launch_pdl_smem(k_dc_unscale, dim3((unsigned)nmat, (unsigned)ceil_div(nmax, 128)), dim3(128), 0, st, P.lam[0], P.mats_dev,
+                          P.scal, lam_out, P.err));
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }
