@@ -20,6 +20,7 @@
 #include "zq_forest.h"
 
 #include <algorithm>
+#include <cstdlib>
 #include <cstring>
 
 #include "zq_applyq.h"
@@ -28,12 +29,18 @@
 
 namespace zq {
 
-// elements of one eigenvector buffer of a chunk: positions and tile counts of
-// its divide and conquer stay within 32 bits
+// Elements of one eigenvector buffer of a chunk: positions and tile counts of its
+// divide and conquer stay within 32 bits, and the scratch of the chunks, which run one
+// after another in the same memory, within 6.5 GB (ZQ_FOREST_CHUNK: smaller chunks)
 constexpr size_t FOREST_CHUNK = (size_t)1 << 28;
+static size_t forest_chunk() {
+  const char* s = getenv("ZQ_FOREST_CHUNK");
+  const long long v = s ? atoll(s) : 0;
+  return v > 0 && (size_t)v < FOREST_CHUNK ? (size_t)v : FOREST_CHUNK;
+}
 
-// A part of the batch with its own tables and scratch (batches beyond 2 GiB of
-// eigenvectors have several).
+// A part of the batch with its own tables (batches beyond 2 GiB of eigenvectors have
+// several) and the scratch that all parts share.
 struct BatchForest::Chunk {
   DcPlan dc;
   int count = 0, N = 0;
@@ -53,6 +60,7 @@ struct BatchForest::Chunk {
   double* dcws = nullptr;
   DcNode* nodes = nullptr;
   DgemmDesc* descs = nullptr;
+  DcMat* mats = nullptr;
 };
 
 BatchForest::~BatchForest() { release(); }
@@ -76,14 +84,15 @@ int BatchForest::build(const std::vector<ForestItem>& items, cudaStream_t st) {
   ZQ_CUDA(cudaGetDevice(&dev));
   ZQ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  size_t total = 256;
+  size_t tables = 256, scratch = 0;
+  const size_t limit = forest_chunk();
   for (size_t i0 = 0; i0 < items.size();) {
     Chunk* c = new Chunk();
     chunks_.push_back(c);
     std::vector<int> ns;
     std::vector<long long> eo;
     size_t nn = 0, i1 = i0;
-    while (i1 < items.size() && (i1 == i0 || nn + (size_t)items[i1].n * items[i1].n <= FOREST_CHUNK)) {
+    while (i1 < items.size() && (i1 == i0 || nn + (size_t)items[i1].n * items[i1].n <= limit)) {
       nn += (size_t)items[i1].n * items[i1].n;
       ns.push_back(items[i1].n);
       eo.push_back(items[i1].eoff);
@@ -136,11 +145,13 @@ int BatchForest::build(const std::vector<ForestItem>& items, cudaStream_t st) {
       q = q1;
     }
     const size_t N = (size_t)c->N;
-    total += up(sizeof(TriTask<double>) * c->count) + up(sizeof(ApplyQTask) * c->count) + up(sizeof(int) * N) + up(sizeof(int2) * (c->blocks_host.size() + 1)) +
-             up(sizeof(DcNode) * (c->dc.num_nodes() + 1)) + up(DcPlan::desc_bytes(c->dc.num_descs())) +
-             up(sizeof(double) * 11 * N) + c->tri_ws_bytes + up(sizeof(double) * c->dc.forest_doubles());
+    tables += up(sizeof(TriTask<double>) * c->count) + up(sizeof(ApplyQTask) * c->count) + up(sizeof(int) * N) +
+              up(sizeof(int2) * (c->blocks_host.size() + 1)) + up(sizeof(DcNode) * (c->dc.num_nodes() + 1)) +
+              up(DcPlan::desc_bytes(c->dc.num_descs())) + up(sizeof(DcMat) * c->count);
+    scratch = std::max(scratch, up(sizeof(double) * 11 * N) + c->tri_ws_bytes + up(sizeof(double) * c->dc.forest_doubles()));
     i0 = i1;
   }
+  const size_t total = tables + scratch;
   if (bytes_ < total) {
     if (dev_) cudaFree(dev_);
     dev_ = nullptr;
@@ -166,13 +177,17 @@ int BatchForest::build(const std::vector<ForestItem>& items, cudaStream_t st) {
     c->blocks = reinterpret_cast<int2*>(take(sizeof(int2) * (c->blocks_host.size() + 1)));
     c->nodes = reinterpret_cast<DcNode*>(take(sizeof(DcNode) * (c->dc.num_nodes() + 1)));
     c->descs = reinterpret_cast<DgemmDesc*>(take(DcPlan::desc_bytes(c->dc.num_descs())));
+    c->mats = reinterpret_cast<DcMat*>(take(sizeof(DcMat) * c->count));
+    char* const next = p;
+    p = reinterpret_cast<char*>(dev_) + tables;  // the chunks' common scratch
     double* v = reinterpret_cast<double*>(take(sizeof(double) * 11 * N));
     c->d = v; c->e = v + N; c->tau = v + 5 * N; c->offd = v + 6 * N; c->phi = v + 7 * N;
     int* queue = reinterpret_cast<int*>(take(256));
     void* tri_ws = take(c->tri_ws_bytes - 256);
     for (Chunk::TriClass& t : c->tri) { t.queue = queue; t.ws = tri_ws; }
     c->dcws = reinterpret_cast<double*>(take(sizeof(double) * c->dc.forest_doubles()));
-    if (int rc = c->dc.upload(c->dcws, c->nodes, c->descs, st)) return rc;
+    p = next;
+    if (int rc = c->dc.upload(c->dcws, c->nodes, c->descs, st, c->mats)) return rc;
     std::vector<TriTask<double>> tt(c->count);
     std::vector<ApplyQTask> at(c->count);
     std::vector<int> of(N);

@@ -45,7 +45,7 @@ class BatchForest {
   void release();
 
  private:
-  struct Chunk;                    // a part of the batch whose scratch fits at once
+  struct Chunk;                    // a part of the batch; the parts run one after another on the same scratch
   std::vector<ForestItem> items_;
   std::vector<Chunk*> chunks_;
   void* dev_ = nullptr;

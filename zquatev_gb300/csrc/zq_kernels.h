@@ -133,7 +133,7 @@ struct DcPlan {
   int* tc_err = nullptr;  // run_single: merges of large nodes on the tensor cores (timeout flag) when set
 
   static size_t workspace_doubles(int n);
-  size_t forest_doubles() const;  // the same for a built plan of several matrices
+  size_t forest_doubles() const;  // the same for a built plan of several matrices, without their table
   int build(int n);
   // several tridiagonals at once: orders ns, eigenvalues at eoffs of the
   // array given to run_forest
@@ -143,7 +143,8 @@ struct DcPlan {
   int gemm_cnt(int t) const {  // descriptors of depth t
     return (t + 1 < (int)gemm_off.size() ? gemm_off[t + 1] : (int)gemm_host.size()) - gemm_off[t];
   }
-  int upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t st);
+  // mats: the table's place where the workspace is not the plan's alone (null: in the workspace)
+  int upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t st, DcMat* mats = nullptr);
   // d (n), e (n-1) on device; lam_out (n) on device; z_out points into the workspace
   int run(const double* d, const double* e, double* lam_out, double*& z_out, cudaStream_t st);
   // a forest: d, e indexed by position (e of a matrix's last position unused),

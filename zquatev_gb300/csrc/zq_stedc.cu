@@ -613,7 +613,7 @@ size_t DcPlan::workspace_doubles(int n) {
 }
 
 size_t DcPlan::forest_doubles() const {
-  return 3 * nn + 20 * (size_t)n + (1 + sizeof(DcMat) / sizeof(double)) * mats_host.size() + 72;
+  return 3 * nn + 20 * (size_t)n + mats_host.size() + 72;
 }
 
 int DcPlan::build(int n_) { return build(std::vector<int>{n_}, std::vector<long long>{0}); }
@@ -722,7 +722,7 @@ int DcPlan::build(const std::vector<int>& ns, const std::vector<long long>& eoff
 }
 
 // Binds device pointers into the descriptor copies and uploads everything.
-int DcPlan::upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t st) {
+int DcPlan::upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t st, DcMat* mats) {
   base = ws;
   Z[0] = ws; Z[1] = ws + nn; Mb = ws + 2 * nn;
   double* p = ws + 3 * nn;
@@ -730,7 +730,8 @@ int DcPlan::upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t s
   dmod = p; p += n; es = p; p += n;
   err = reinterpret_cast<int*>(p); p += 8;
   scal = p; p += mats_host.size();
-  mats_dev = reinterpret_cast<DcMat*>(p); p += sizeof(DcMat) / sizeof(double) * mats_host.size();
+  mats_dev = mats;
+  if (!mats) { mats_dev = reinterpret_cast<DcMat*>(p); p += sizeof(DcMat) / sizeof(double) * mats_host.size(); }
   w.sd = p; p += n; w.sz = p; p += n;
   w.nd_val = p; p += n; w.nd_z = p; p += n;
   w.df_val = p; p += n; w.df_sval = p; p += n;
