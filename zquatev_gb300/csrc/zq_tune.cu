@@ -135,7 +135,8 @@ int* plan_info(zq_batch_plan* p) { return reinterpret_cast<int*>(reinterpret_cas
 
 int plan_launch_direct(zq_batch_plan* p, double2* D, double* E, int ctas, cudaStream_t st, int wmax) {
   int* info = plan_info(p);
-  const BatchSplit split = batched_split(p->ntask, wmax, [&](int q) { return p->orders[q]; });
+  // (a plan of fixed launch shape is not tuned: the default switch size)
+  const BatchSplit split = batched_split(p->ntask, wmax < 0 ? batched_warp_max() : wmax, [&](int q) { return p->orders[q]; });
   return batched_launch(p->dev, split, info + p->ntask, D, E, reinterpret_cast<double*>(plan_ws(p)), ctas, info, st);
 }
 // candidates of the warp variant's switch size (0: CTA variant for every size)
