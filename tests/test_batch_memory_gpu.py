@@ -1,4 +1,6 @@
-"""The joint solve's scratch is bounded by its largest part."""
+"""The joint solve's scratch: bounded by its largest part, and done without where
+the device has no room for it."""
+import contextlib
 import gc
 
 import numpy as np
@@ -96,3 +98,38 @@ def test_parts_of_mixed_orders(gpu, monkeypatch, entry):
     if plan:
         plan.close()
     gpu.zq_release_workspace()
+
+
+@contextlib.contextmanager
+def _crowded(leave):
+    """The device's memory taken but for `leave` bytes."""
+    import torch
+
+    ballast = torch.empty(_free() - leave, dtype=torch.uint8, device="cuda")
+    try:
+        yield
+    finally:
+        del ballast
+        _free()
+
+
+def test_batch_without_room(gpu):
+    """Three eigenvector buffers (400 MB) do not fit; the CTA kernel's 140 MB do."""
+    d, e, args = _copies(256, 256)
+    assert _run(gpu, d[:1].clone(), e[:1].clone(), tuple(a[:1] for a in args)) == 0
+    gpu.zq_release_workspace()
+    with _crowded(300 * MB):
+        rc = _run(gpu, d, e, args)
+    assert rc == 0, _lib.last_error()
+    _check(256, d, e)
+
+
+def test_plan_without_room(gpu):
+    d, e, args = _copies(256, 256)
+    gpu.zq_release_workspace()
+    with _crowded(300 * MB):
+        plan = solver.BatchPlan(*args, ctas_per_sm=1)
+        plan.run(d, e)
+        assert plan.info() == 0
+        plan.close()
+    _check(256, d, e)

@@ -644,14 +644,22 @@ static int batched_solve(int count, const int* n2s, const int* ld2s, const long 
     (n > nmax ? large : (forest_takes(n, few) ? mid : small)).push_back(b);
   }
   const auto larger = [&](int x, int y) { return n2s[x] > n2s[y]; };
-  std::stable_sort(small.begin(), small.end(), larger);
   std::stable_sort(mid.begin(), mid.end(), larger);
-  int info_max = 0;
   if (!mid.empty()) {
     std::vector<ForestItem> items;
     for (int b : mid) items.push_back(ForestItem{n2s[b] / 2, ld2s[b], offs[b], eoffs[b]});
-    if (!c->forest.matches(items))
-      if (int rc = c->forest.build(items, c->st)) return rc;
+    if (!c->forest.matches(items)) {
+      const int rc = c->forest.build(items, c->st);
+      if (rc != ZQ_OK && !BatchForest::declined(rc)) return rc;
+      if (rc != ZQ_OK) {
+        small.insert(small.end(), mid.begin(), mid.end());
+        mid.clear();
+      }
+    }
+  }
+  std::stable_sort(small.begin(), small.end(), larger);
+  int info_max = 0;
+  if (!mid.empty()) {
     ZQ_CUDA(cudaEventRecord(c->ev_fork, st));
     ZQ_CUDA(cudaStreamWaitEvent(c->st, c->ev_fork, 0));
     if (int rc = c->forest.run(dD, deig, c->st)) return rc;

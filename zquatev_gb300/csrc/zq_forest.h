@@ -3,6 +3,7 @@
 
 #include <vector>
 
+#include "zq_common.cuh"
 #include "zq_kernels.h"
 
 namespace zq {
@@ -38,6 +39,9 @@ class BatchForest {
   ~BatchForest();
   int build(const std::vector<ForestItem>& items, cudaStream_t st);
   bool matches(const std::vector<ForestItem>& items) const { return items == items_; }
+  // build()'s code where the batch cannot run jointly (no room for its scratch, no cluster
+  // for its largest order) but one matrix per CTA still can (zq_batched.cu)
+  static bool declined(int rc) { return rc == ZQ_ERR_NOMEM || rc == ZQ_ERR_LIMIT; }
   bool empty() const { return items_.empty(); }
   int run(double2* D, double* eig, cudaStream_t st);
   const int* error_flag() const { return err_; }  // device: a bounded wait ran out

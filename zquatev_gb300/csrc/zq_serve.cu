@@ -252,6 +252,16 @@ void batch_loop(Server* s, Context* c) {
       joint.push_back(r);
       items.push_back(ForestItem{r->n, r->n2, (long long)(r->dD - D0), (long long)(r->deig - E0)});
     }
+    int rc = ZQ_OK;
+    if (!items.empty() && !forest.matches(items)) {
+      rc = forest.build(items, c->st);
+      if (BatchForest::declined(rc)) {  // no room for it: a CTA each
+        rc = ZQ_OK;
+        items.clear();
+        joint.clear();
+        rest = batch;
+      }
+    }
     batch.swap(rest);
     const int k = (int)batch.size();
     const int ctas = std::max(1, std::min(k, 2 * s->sms));
@@ -263,9 +273,8 @@ void batch_loop(Server* s, Context* c) {
     int herr = 0;
     for (int q = 0; q < k; ++q) batched_fill_task_ptr(htasks.data() + q * tb, batch[q]->dD, batch[q]->deig, batch[q]->n,
                                                       batch[q]->n2, q);
-    int rc = ZQ_OK;
     void* mem = nullptr;
-    if (cudaMallocAsync(&mem, need, c->st) != cudaSuccess) {
+    if (rc == ZQ_OK && cudaMallocAsync(&mem, need, c->st) != cudaSuccess) {
       cudaGetLastError();
       rc = ZQ_ERR_NOMEM;
       mem = nullptr;
@@ -276,8 +285,7 @@ void batch_loop(Server* s, Context* c) {
       for (Req* r : all)
         if (cudaStreamWaitEvent(c->st, r->ready, 0) != cudaSuccess) rc = ZQ_ERR_CUDA;
       if (rc == ZQ_OK && !items.empty()) {
-        rc = forest.matches(items) ? (int)ZQ_OK : forest.build(items, c->st);
-        if (rc == ZQ_OK) rc = forest.run(D0, E0, c->st);
+        rc = forest.run(D0, E0, c->st);
         if (rc == ZQ_OK && cudaMemcpyAsync(&herr, forest.error_flag(), sizeof(int), cudaMemcpyDeviceToHost, c->st) != cudaSuccess)
           rc = ZQ_ERR_CUDA;
       }

@@ -274,11 +274,27 @@ zq_batch_plan* zq_batch_plan_create(int count, const int* n2s, const int* ld2s, 
     extent = std::max(extent, offs[b] + (long long)ld2s[b] * n2);
   }
   const auto larger = [&](int x, int y) { return n2s[x] > n2s[y]; };
-  std::stable_sort(order.begin(), order.end(), larger);
   std::stable_sort(mid.begin(), mid.end(), larger);
   zq_batch_plan* p = new zq_batch_plan();
   cudaGetDevice(&p->device);
   cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, p->device);
+  if (cudaStreamCreateWithFlags(&p->cap, cudaStreamNonBlocking) != cudaSuccess) {
+    cudaGetLastError();
+    set_error_message("zq_batch_plan_create: stream creation failed");
+    p->cap = nullptr;
+    zq_batch_plan_destroy(p);
+    return nullptr;
+  }
+  std::vector<ForestItem> items;
+  for (int b : mid) items.push_back(ForestItem{n2s[b] / 2, ld2s[b], offs[b], eoffs[b]});
+  if (const int rc = p->forest.build(items, p->cap)) {
+    if (!BatchForest::declined(rc)) { zq_batch_plan_destroy(p); return nullptr; }
+    for (int b : mid) {
+      order.push_back(b);
+      extent = std::max(extent, offs[b] + (long long)ld2s[b] * n2s[b]);
+    }
+  }
+  std::stable_sort(order.begin(), order.end(), larger);
   p->count = count;
   p->ntask = (int)order.size();
   p->extent = extent;
@@ -297,19 +313,10 @@ zq_batch_plan* zq_batch_plan_create(int count, const int* n2s, const int* ld2s, 
     p->orders.push_back(n2s[b] / 2);
   }
   if (cudaMalloc(&p->dev, need) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&p->cap, cudaStreamNonBlocking) != cudaSuccess ||
       cudaMemcpy(p->dev, ht.data(), tb * p->ntask, cudaMemcpyHostToDevice) != cudaSuccess) {
     cudaGetLastError();
-    set_error_message("zq_batch_plan_create: device allocation or upload failed");
-    if (p->dev) cudaFree(p->dev);
-    if (p->cap) cudaStreamDestroy(p->cap);
-    delete p;
-    return nullptr;
-  }
-  std::vector<ForestItem> items;
-  for (int b : mid) items.push_back(ForestItem{n2s[b] / 2, ld2s[b], offs[b], eoffs[b]});
-  if (p->forest.build(items, p->cap) != ZQ_OK) {
     zq_batch_plan_destroy(p);
+    set_error_message("zq_batch_plan_create: device allocation or upload failed");
     return nullptr;
   }
   return p;
