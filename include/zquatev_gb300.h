@@ -56,7 +56,8 @@ int zq_stedc_device(int n, const double* d, const double* e, double* lam, double
  * with n2 <= 512 run together (up to n2 = 64 a warp each, larger ones over all
  * SMs step by step); larger ones through the per-matrix path. Ordered after
  * `stream`; returns after the batch has finished, with the largest per-matrix
- * info (0 = all converged). The reference solves one matrix per call; this has
+ * info (0 = all converged; above 0 the eigenvalues of some matrix that did not, or
+ * that are not finite, as from an input with an Inf or a NaN). The reference solves one matrix per call; this has
  * no counterpart there. */
 int zquatev_batched_device(int count, const int* n2s, const int* ld2s, const long long* offs,
                            const long long* eoffs, double* dD, double* deig, void* stream);

@@ -663,10 +663,10 @@ static int batched_solve(int count, const int* n2s, const int* ld2s, const long 
     ZQ_CUDA(cudaEventRecord(c->ev_fork, st));
     ZQ_CUDA(cudaStreamWaitEvent(c->st, c->ev_fork, 0));
     if (int rc = c->forest.run(dD, deig, c->st)) return rc;
-    int herr = 0;
-    ZQ_CUDA(cudaMemcpyAsync(&herr, c->forest.error_flag(), sizeof(int), cudaMemcpyDeviceToHost, c->st));
+    std::vector<int> hinfo(mid.size());
+    ZQ_CUDA(cudaMemcpyAsync(hinfo.data(), c->forest.info(), sizeof(int) * mid.size(), cudaMemcpyDeviceToHost, c->st));
     ZQ_CUDA(cudaStreamSynchronize(c->st));
-    if (herr) { set_msg("batch: a device-side wait ran out of time"); return ZQ_ERR_TIMEOUT; }
+    for (int v : hinfo) info_max = v > info_max ? v : info_max;
   }
   if (!small.empty()) {
     int sms = 0;

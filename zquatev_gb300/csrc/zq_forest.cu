@@ -84,7 +84,7 @@ int BatchForest::build(const std::vector<ForestItem>& items, cudaStream_t st) {
   ZQ_CUDA(cudaGetDevice(&dev));
   ZQ_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  size_t tables = 256, scratch = 0;
+  size_t tables = up(sizeof(int) * items.size()), scratch = 0;
   const size_t limit = forest_chunk();
   for (size_t i0 = 0; i0 < items.size();) {
     Chunk* c = new Chunk();
@@ -166,8 +166,7 @@ int BatchForest::build(const std::vector<ForestItem>& items, cudaStream_t st) {
   }
   char* p = reinterpret_cast<char*>(dev_);
   auto take = [&](size_t b) { char* q = p; p += up(b); return q; };
-  err_ = reinterpret_cast<int*>(take(256));
-  ZQ_CUDA(cudaMemsetAsync(dev_, 0, 256, st));
+  info_ = reinterpret_cast<int*>(take(sizeof(int) * items.size()));
   size_t base = 0;
   for (Chunk* c : chunks_) {
     const size_t N = (size_t)c->N;
@@ -213,12 +212,14 @@ int BatchForest::build(const std::vector<ForestItem>& items, cudaStream_t st) {
 
 int BatchForest::run(double2* D, double* eig, cudaStream_t st) {
   if (items_.empty()) return ZQ_OK;
-  ZQ_CUDA(cudaMemsetAsync(err_, 0, sizeof(int), st));
+  ZQ_CUDA(cudaMemsetAsync(info_, 0, sizeof(int) * items_.size(), st));
+  int* info = info_;
   for (Chunk* c : chunks_) {
     for (const Chunk::TriClass& t : c->tri)
-      if (int rc = tri_queue(c->tri_tasks + t.first, t.count, D, t.m_max, t.G, t.ws, t.queue, err_, st)) return rc;
+      if (int rc = tri_queue(c->tri_tasks + t.first, t.count, D, t.m_max, t.G, t.ws, t.queue, st)) return rc;
     if (int rc = phase_reduce_forest(c->e, c->dc.mats_dev, c->count, items_.front().n, c->offd, c->phi, st)) return rc;
-    if (int rc = c->dc.run_forest(c->d, c->offd, eig, st)) return rc;
+    if (int rc = c->dc.run_forest(c->d, c->offd, eig, info, st)) return rc;
+    info += c->count;
     ApplyQTask base{};
     base.D = D;
     for (const Chunk::ApplyClass& a : c->apply) {

@@ -44,7 +44,10 @@ class BatchForest {
   static bool declined(int rc) { return rc == ZQ_ERR_NOMEM || rc == ZQ_ERR_LIMIT; }
   bool empty() const { return items_.empty(); }
   int run(double2* D, double* eig, cudaStream_t st);
-  const int* error_flag() const { return err_; }  // device: a bounded wait ran out
+  // device, an int per item in the order given: the last run's count of its eigenvalues that are
+  // not finite (its QL would not have converged)
+  const int* info() const { return info_; }
+  int count() const { return (int)items_.size(); }
   size_t bytes() const { return bytes_; }
   void release();
 
@@ -54,7 +57,7 @@ class BatchForest {
   std::vector<Chunk*> chunks_;
   void* dev_ = nullptr;
   size_t bytes_ = 0;
-  int* err_ = nullptr;
+  int* info_ = nullptr;
 };
 
 }  // namespace zq

@@ -149,7 +149,8 @@ struct DcPlan {
   int run(const double* d, const double* e, double* lam_out, double*& z_out, cudaStream_t st);
   // a forest: d, e indexed by position (e of a matrix's last position unused),
   // eigenvalues to eig + eoff of each matrix, eigenvectors in Z[0]
-  int run_forest(const double* d, const double* e, double* eig, cudaStream_t st);
+  // (info: one int per matrix, zeroed by the caller, counts its eigenvalues that are not finite)
+  int run_forest(const double* d, const double* e, double* eig, int* info, cudaStream_t st);
   // same tree with Z and the merge products in FP32 (eigenvalues and the
   // secular equation stay FP64): the refined path's decomposition
   int run_single(const double* d, const double* e, double* lam_out, float*& z_out, cudaStream_t st);

@@ -1015,7 +1015,7 @@ size_t tri_queue_bytes(int G, int m_max, int ntasks) {
   return tri_queue_stride(G, m_max) * std::min(ntasks, tri_queue_groups(G));
 }
 
-int tri_queue(const TriTask<double>* tasks, int ntasks, double2* base, int m_max, int G, void* ws, int* queue, int* err,
+int tri_queue(const TriTask<double>* tasks, int ntasks, double2* base, int m_max, int G, void* ws, int* queue,
               cudaStream_t st) {
   if (ntasks <= 0) return ZQ_OK;
   constexpr int T = rt_tile_edge<double>();
@@ -1024,8 +1024,6 @@ int tri_queue(const TriTask<double>* tasks, int ntasks, double2* base, int m_max
   a.G = G; a.m_max = m_max;
   a.ws = reinterpret_cast<unsigned char*>(ws);
   a.ws_stride = tri_queue_stride(G, m_max);
-  a.err = err;
-  a.limit = pipeline_wait_cycles();
   const int groups = std::min(ntasks, tri_queue_groups(G));
   ZQ_CUDA(cudaMemsetAsync(queue, 0, sizeof(int), st));
   return rt_launch<double, T, true>(a, groups * G, rt_smem_bytes<double>(m_max, T, G), st);

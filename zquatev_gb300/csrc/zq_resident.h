@@ -67,7 +67,7 @@ struct TriArgs {
 
 // A queue of FP64 matrices (device arrays; orders at most m_max), each reduced by
 // a cluster of G CTAs; ws as tri_queue_bytes(G, m_max), queue one int.
-int tri_queue(const TriTask<double>* tasks, int ntasks, double2* base, int m_max, int G, void* ws, int* queue, int* err,
+int tri_queue(const TriTask<double>* tasks, int ntasks, double2* base, int m_max, int G, void* ws, int* queue,
               cudaStream_t st);
 size_t tri_queue_bytes(int G, int m_max, int ntasks);
 // cluster size that finishes a queue of these orders (largest first) soonest, and

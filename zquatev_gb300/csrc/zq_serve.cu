@@ -270,7 +270,7 @@ void batch_loop(Server* s, Context* c) {
     const size_t need = task_bytes + info_bytes + sizeof(double) * (size_t)batched_ws_stride() * ctas;
     htasks.resize(tb * k);
     hinfo.assign(k, 0);
-    int herr = 0;
+    std::vector<int> jinfo(joint.size());
     for (int q = 0; q < k; ++q) batched_fill_task_ptr(htasks.data() + q * tb, batch[q]->dD, batch[q]->deig, batch[q]->n,
                                                       batch[q]->n2, q);
     void* mem = nullptr;
@@ -286,7 +286,8 @@ void batch_loop(Server* s, Context* c) {
         if (cudaStreamWaitEvent(c->st, r->ready, 0) != cudaSuccess) rc = ZQ_ERR_CUDA;
       if (rc == ZQ_OK && !items.empty()) {
         rc = forest.run(D0, E0, c->st);
-        if (rc == ZQ_OK && cudaMemcpyAsync(&herr, forest.error_flag(), sizeof(int), cudaMemcpyDeviceToHost, c->st) != cudaSuccess)
+        if (rc == ZQ_OK && cudaMemcpyAsync(jinfo.data(), forest.info(), sizeof(int) * jinfo.size(), cudaMemcpyDeviceToHost,
+                                           c->st) != cudaSuccess)
           rc = ZQ_ERR_CUDA;
       }
       if (rc == ZQ_OK && k > 0 && cudaMemcpyAsync(b, htasks.data(), tb * k, cudaMemcpyHostToDevice, c->st) != cudaSuccess)
@@ -303,10 +304,9 @@ void batch_loop(Server* s, Context* c) {
     for (Req* r : all) cudaFreeAsync(r->dD, c->st);
     const cudaError_t e = cudaStreamSynchronize(c->st);
     if (rc == ZQ_OK && e != cudaSuccess) { set_last_error(e, "server batch", __FILE__, __LINE__); rc = ZQ_ERR_CUDA; }
-    if (rc == ZQ_OK && herr) { set_error_message("server batch: a device-side wait ran out of time"); rc = ZQ_ERR_TIMEOUT; }
     // its tables and scratch are within the finished requests' footprints: not kept beyond them
     if (forest.bytes() > FOREST_KEEP) forest.release();
-    for (Req* r : joint) finish(s, r, rc, 2);
+    for (size_t q = 0; q < joint.size(); ++q) finish(s, joint[q], rc != ZQ_OK ? rc : jinfo[q], 2);
     for (int q = 0; q < k; ++q) finish(s, batch[q], rc != ZQ_OK ? rc : hinfo[q], 2);
   }
 }

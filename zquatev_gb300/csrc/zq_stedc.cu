@@ -544,14 +544,18 @@ __global__ void k_dc_scale(const double* d, const double* e, const DcMat* mats, 
 }
 
 // eigenvalues times the scale, into place (NaN when the scale is, or a merge product failed)
-__global__ void k_dc_unscale(const double* lam, const DcMat* mats, const double* scal, double* eig, const int* err) {
+// `info` (may be null): counts, per matrix, the eigenvalues that are not finite
+__global__ void k_dc_unscale(const double* lam, const DcMat* mats, const double* scal, double* eig, const int* err,
+                             int* info) {
   pdl_wait();
   const DcMat mt = mats[blockIdx.x];  // (x: a batch may have more matrices than the other dimensions take)
   const int i = blockIdx.y * blockDim.x + threadIdx.x;
   if (i >= mt.n) return;
   const double s = scal[blockIdx.x];
   const double v = lam[mt.p + i];
-  eig[mt.eoff + i] = *err || s != s ? __longlong_as_double(0x7ff8000000000000ll) : (s > 0.0 ? v * s : v);
+  const double out = *err || s != s ? __longlong_as_double(0x7ff8000000000000ll) : (s > 0.0 ? v * s : v);
+  eig[mt.eoff + i] = out;
+  if (info && abs_bits(out) >= (0x7ffull << 52)) atomicAdd(info + blockIdx.x, 1);
 }
 
 // Z_node = blockdiag(Z1, Z2) M for small nodes: a thread per entry. The tiled
@@ -792,7 +796,7 @@ int DcPlan::upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t s
 
 template <typename ZT>
 static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, ZT* const Zb[2], ZT* Mb,
-                  const DgemmDescT<ZT>* descs, cudaStream_t st) {
+                  const DgemmDescT<ZT>* descs, cudaStream_t st, int* info = nullptr) {
   const int n = P.n, nmat = (int)P.mats_host.size();
   int nmax = 0;
   for (const DcMat& m : P.mats_host) nmax = std::max(nmax, m.n);
@@ -887,14 +891,14 @@ static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, 
     }
   }
   ZQ_CUDA(launch_pdl_smem(k_dc_unscale, dim3((unsigned)nmat, (unsigned)ceil_div(nmax, 128)), dim3(128), 0, st, P.lam[0], P.mats_dev,
-                          P.scal, lam_out, P.err));
+                          P.scal, lam_out, P.err, info));
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }
 
-int DcPlan::run_forest(const double* d, const double* e, double* eig, cudaStream_t st) {
+int DcPlan::run_forest(const double* d, const double* e, double* eig, int* info, cudaStream_t st) {
   if (n <= 0) return ZQ_OK;
-  return dc_run<double>(*this, d, e, eig, Z, Mb, descs_dev, st);
+  return dc_run<double>(*this, d, e, eig, Z, Mb, descs_dev, st, info);
 }
 
 int DcPlan::run(const double* d, const double* e, double* lam_out, double*& z_out, cudaStream_t st) {

@@ -355,15 +355,13 @@ int zq_batch_plan_run(zq_batch_plan* p, double* dD, double* deig, void* stream) 
 int zq_batch_plan_info(zq_batch_plan* p, void* stream) {
   if (!p) return ZQ_ERR_ARG;
   if (p->ntask == 0 && p->forest.empty()) return ZQ_OK;
-  std::vector<int> h(p->ntask);
-  int herr = 0;
+  std::vector<int> h(p->ntask + p->forest.count());
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   if (p->ntask > 0)
     ZQ_CUDA(cudaMemcpyAsync(h.data(), plan_info(p), sizeof(int) * p->ntask, cudaMemcpyDeviceToHost, st));
   if (!p->forest.empty())
-    ZQ_CUDA(cudaMemcpyAsync(&herr, p->forest.error_flag(), sizeof(int), cudaMemcpyDeviceToHost, st));
+    ZQ_CUDA(cudaMemcpyAsync(h.data() + p->ntask, p->forest.info(), sizeof(int) * p->forest.count(), cudaMemcpyDeviceToHost, st));
   ZQ_CUDA(cudaStreamSynchronize(st));
-  if (herr) { set_error_message("batch: a device-side wait ran out of time"); return ZQ_ERR_TIMEOUT; }
   int m = 0;
   for (int v : h) m = v > m ? v : m;
   return m;
