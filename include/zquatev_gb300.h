@@ -11,7 +11,8 @@
  * Return codes: 0 success; -1 bad n2 (odd or negative); -2 null D; -3 ld2 < n2;
  * -4 null eig; -5 other bad argument; -100 CUDA failure; -101 out of device
  * memory; -103 size above the fixed limit of the called entry point; -104 a
- * device-side pipeline wait ran out of time (the kernel stopped and said so).
+ * device-side wait ran out of time (the kernel stopped and said so; where a call
+ * returns before the GPU is done, all eigenvalues are NaN instead).
  * zq_last_error() describes the last failure on the calling thread.
  */
 #ifndef ZQUATEV_GB300_H

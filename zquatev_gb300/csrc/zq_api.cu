@@ -151,6 +151,7 @@ void context_destroy(Context* c) {
   if (c->ws && !c->ws_external) cudaFree(c->ws);
   if (c->rb.dev && !c->rb.external) cudaFree(c->rb.dev);
   if (c->bb.dev) cudaFree(c->bb.dev);
+  if (c->err) cudaFree(c->err);
   if (c->hbuf) cudaFree(c->hbuf);
   if (c->ev_fork) cudaEventDestroy(c->ev_fork);
   if (c->ev_join) cudaEventDestroy(c->ev_join);
@@ -315,6 +316,10 @@ int solve_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, bool
   double* offd = sm; sm += n;
   double* phi = sm; sm += 4 * (size_t)n;
   double* lam = sm; sm += n;
+  if (!c->err) {
+    ZQ_CUDA(cudaMalloc(&c->err, 256));
+    ZQ_CUDA(cudaMemsetAsync(c->err, 0, 256, c->st));
+  }
   void* fq_ws = base + L.tri + L.small + L.dc;
   DgemmDesc* desc1 = reinterpret_cast<DgemmDesc*>(base + L.tri + L.small + L.dc + L.fq + L.nodes) + c->dc.num_descs();
 
@@ -325,6 +330,9 @@ int solve_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, bool
   tm.mark("start", c->st);
   TridiagView<double> v = tridiag_bind<double>(tri_ws, dD, n, ldd, NBMAX, d, e, tau);
   v.ctas = resident_ctas(n, c->coop);
+  v.tc_err = c->err;  // the resident kernel's waits
+  ZQ_CUDA(cudaMemsetAsync(c->err, 0, sizeof(int), c->st));
+  c->err_set = true;
   prof_begin(PC_TRIDIAG, c->st);
   if (int rc = tridiagonalize<double>(v, nb, c->st)) return rc;
   prof_end(PC_TRIDIAG, c->st);
@@ -335,7 +343,7 @@ int solve_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, bool
     // each column takes the reflectors directly (zq_applyq.cu)
     double* Z = nullptr;
     prof_begin(PC_STEDC, c->st);
-    if (int rc = c->dc.run(d, offd, lam, Z, c->st)) return rc;
+    if (int rc = c->dc.run(d, offd, lam, Z, c->st, c->err)) return rc;
     prof_end(PC_STEDC, c->st);
     tm.mark("stedc", c->st);
     prof_begin(PC_APPLYZ, c->st);
@@ -353,7 +361,7 @@ int solve_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, bool
     ZQ_CUDA(cudaEventRecord(c->ev_join, c->st2));
     double* Z = nullptr;
     prof_begin(PC_STEDC, c->st);
-    if (int rc = c->dc.run(d, offd, lam, Z, c->st)) return rc;
+    if (int rc = c->dc.run(d, offd, lam, Z, c->st, c->err)) return rc;
     prof_end(PC_STEDC, c->st);
     tm.mark("stedc", c->st);
     ZQ_CUDA(cudaStreamWaitEvent(c->st, c->ev_join, 0));
@@ -364,11 +372,20 @@ int solve_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, bool
     tm.mark("symfill", c->st);
   } else {
     double* Z = nullptr;
-    if (int rc = c->dc.run(d, offd, lam, Z, c->st)) return rc;
+    if (int rc = c->dc.run(d, offd, lam, Z, c->st, c->err)) return rc;
   }
   ZQ_CUDA(cudaMemcpyAsync(deig, lam, sizeof(double) * n, cudaMemcpyDeviceToDevice, c->st));
   ZQ_CUDA(cudaEventRecord(c->ev_join, c->st));
   ZQ_CUDA(cudaStreamWaitEvent(st, c->ev_join, 0));
+  return ZQ_OK;
+}
+
+int check_timeout(Context* c, int flag) {
+  int raised = 0;
+  if (!c->err || !c->err_set) return ZQ_OK;
+  ZQ_CUDA(cudaMemcpyAsync(&raised, c->err + flag, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+  ZQ_CUDA(cudaStreamSynchronize(c->st));
+  if (raised) { set_msg("FP64 path: a device-side wait ran out of time (kernel stopped)"); return ZQ_ERR_TIMEOUT; }
   return ZQ_OK;
 }
 
@@ -447,6 +464,7 @@ static int zquatev_host(int n2, double2* D, int ld2, double* eig, bool vectors, 
                           cudaMemcpyHostToDevice, c->st) != cudaSuccess) { rc = ZQ_ERR_CUDA; set_msg("H2D copy failed"); break; }
     phase("h2d");
     const int p = (path >= 0) ? path : path_single(n);
+    c->err_set = false;
     cudaEvent_t te[2];
     if (timing) { cudaEventCreate(&te[0]); cudaEventCreate(&te[1]); cudaEventRecord(te[0], c->st); }
     rc = !vectors ? values_device(c, dD, n2, n, deig, c->st)
@@ -470,6 +488,8 @@ static int zquatev_host(int n2, double2* D, int ld2, double* eig, bool vectors, 
     }
     cudaError_t e = cudaStreamSynchronize(c->st);
     if (e != cudaSuccess) { set_last_error(e, "cudaStreamSynchronize", __FILE__, __LINE__); rc = ZQ_ERR_CUDA; break; }
+    // no eigenvalues: a wait that ran out, or an input that is not finite
+    if (eig[0] != eig[0] && (rc = check_timeout(c, 0))) break;
     phase("d2h");
   } while (0);
   cudaStreamSynchronize(c->st);
@@ -706,10 +726,13 @@ static int batched_solve(int count, const int* n2s, const int* ld2s, const long 
     ZQ_CUDA(cudaStreamSynchronize(c->st));
     for (int v : hinfo) info_max = v > info_max ? v : info_max;
   }
+  if (!large.empty() && c->err) ZQ_CUDA(cudaMemsetAsync(c->err + 1, 0, sizeof(int), c->st));
   for (int b : large) {
     if (int rc = solve_device(c, dD + offs[b], ld2s[b], n2s[b] / 2, deig + eoffs[b], true, st)) return rc;
   }
   ZQ_CUDA(cudaStreamSynchronize(st));
+  if (!large.empty())
+    if (int rc = check_timeout(c, 1)) return rc;
   return info_max;
 }
 

@@ -39,6 +39,11 @@ struct Context {
   bool ws_external = false;  // bound by the caller: never freed or grown here
   int dc_n = -1;
   DcPlan dc;
+  // Device flags of the FP64 path (two ints, made by the first solve), raised when a
+  // device-side wait ran out: [0] in the last solve, whose eigenvalues are NaN then,
+  // [1] in any since it was last cleared
+  int* err = nullptr;
+  bool err_set = false;  // the flags are of a solve since the caller reset this
   RefineBuffers rb;
   BatchBuffers bb;
   BatchForest forest;  // layout and scratch of the last batch's mid-size matrices, rebuilt when the layout changes
@@ -66,6 +71,8 @@ void context_bind(Context* c, void* ws, size_t ws_bytes, void* rws, size_t rws_b
 
 int ensure_ws(Context* c, size_t bytes);
 int ensure_plan(Context* c, int n);
+// reads one of the context's flags if a solve has set it, waiting for c->st: ZQ_ERR_TIMEOUT if it is up
+int check_timeout(Context* c, int flag);
 int solve_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, bool vectors, cudaStream_t st);
 int refined_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, cudaStream_t st, int mode,
                    bool vectors = true);

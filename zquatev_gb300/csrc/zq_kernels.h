@@ -35,7 +35,8 @@ struct TridiagView {
   double* d;       // diagonal (n)
   double* e;       // quaternion subdiagonal (4 doubles each, n)
   double* tau;     // 1 if reflector j exists else 0 (n)
-  int* tc_err;     // FP32: tensor-core products allowed (their timeout flag); null: CUDA cores only
+  int* tc_err;     // raised when a bounded wait ran out (null: NaN in d only); FP32: tensor-core products
+                   // allowed where it is set, CUDA cores only where it is null
   void* rws;       // exchange area of the resident reduction (zq_resident.cu)
   int ctas;        // CTAs it may use (0: the per-column kernels only)
 };
@@ -146,7 +147,9 @@ struct DcPlan {
   // mats: the table's place where the workspace is not the plan's alone (null: in the workspace)
   int upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t st, DcMat* mats = nullptr);
   // d (n), e (n-1) on device; lam_out (n) on device; z_out points into the workspace
-  int run(const double* d, const double* e, double* lam_out, double*& z_out, cudaStream_t st);
+  // flags (two ints, null: the plan's own, cleared here): raised when a wait of a residue
+  // product ran out; the eigenvalues become NaN when [0] is up, which then raises [1] too
+  int run(const double* d, const double* e, double* lam_out, double*& z_out, cudaStream_t st, int* flags = nullptr);
   // a forest: d, e indexed by position (e of a matrix's last position unused),
   // eigenvalues to eig + eoff of each matrix, eigenvectors in Z[0]
   // (info: one int per matrix, zeroed by the caller, counts its eigenvalues that are not finite)

@@ -108,11 +108,12 @@ __device__ __forceinline__ bool group_barrier(unsigned* ctr, unsigned& target, i
       asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(ctr) : "memory");
       unsigned v;
       int ok = 1, spins = 0;
+      const int every = limit < 100000 ? 0 : 63;  // polls between looks at the clock, less one
       const long long t0 = clock64();
       for (;;) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
         if ((int)(v - target) >= 0) break;
-        if ((++spins & 63) == 0) {
+        if ((++spins & every) == 0) {
           if (*reinterpret_cast<volatile unsigned*>(abt)) { ok = 0; break; }
           if (clock64() - t0 > limit) {
             atomicExch(abt, 1u);

@@ -200,6 +200,7 @@ void lane_loop(Server* s, Context* c) {
       char* w = reinterpret_cast<char*>(ws);
       context_bind(c, w, r->ws_fp64, p == 1 ? w + r->ws_fp64 : nullptr, p == 1 ? r->ws_ref : 0);
       if (cudaStreamWaitEvent(c->st, r->ready, 0) != cudaSuccess) rc = ZQ_ERR_CUDA;
+      c->err_set = false;
       if (rc == ZQ_OK)
         rc = (p == 1) ? refined_device(c, r->dD, r->n2, r->n, r->deig, c->st, 1)
                       : solve_device(c, r->dD, r->n2, r->n, r->deig, true, c->st);
@@ -211,6 +212,7 @@ void lane_loop(Server* s, Context* c) {
     const cudaError_t e = cudaStreamSynchronize(c->st);
     context_bind(c, nullptr, 0, nullptr, 0);
     if (rc == ZQ_OK && e != cudaSuccess) { set_last_error(e, "server lane", __FILE__, __LINE__); rc = ZQ_ERR_CUDA; }
+    if (rc == ZQ_OK && used != 1 && r->heig[0] != r->heig[0]) rc = check_timeout(c, 0);
     finish(s, r, rc, used);
   }
 }

@@ -545,7 +545,7 @@ __global__ void k_dc_scale(const double* d, const double* e, const DcMat* mats, 
 
 // eigenvalues times the scale, into place (NaN when the scale is, or a merge product failed)
 // `info` (may be null): counts, per matrix, the eigenvalues that are not finite
-__global__ void k_dc_unscale(const double* lam, const DcMat* mats, const double* scal, double* eig, const int* err,
+__global__ void k_dc_unscale(const double* lam, const DcMat* mats, const double* scal, double* eig, int* err,
                              int* info) {
   pdl_wait();
   const DcMat mt = mats[blockIdx.x];  // (x: a batch may have more matrices than the other dimensions take)
@@ -553,7 +553,9 @@ __global__ void k_dc_unscale(const double* lam, const DcMat* mats, const double*
   if (i >= mt.n) return;
   const double s = scal[blockIdx.x];
   const double v = lam[mt.p + i];
-  const double out = *err || s != s ? __longlong_as_double(0x7ff8000000000000ll) : (s > 0.0 ? v * s : v);
+  const bool failed = *err != 0;
+  if (failed && i == 0) err[1] = 1;
+  const double out = failed || s != s ? __longlong_as_double(0x7ff8000000000000ll) : (s > 0.0 ? v * s : v);
   eig[mt.eoff + i] = out;
   if (info && abs_bits(out) >= (0x7ffull << 52)) atomicAdd(info + blockIdx.x, 1);
 }
@@ -796,11 +798,12 @@ int DcPlan::upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t s
 
 template <typename ZT>
 static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, ZT* const Zb[2], ZT* Mb,
-                  const DgemmDescT<ZT>* descs, cudaStream_t st, int* info = nullptr) {
+                  const DgemmDescT<ZT>* descs, cudaStream_t st, int* info = nullptr, int* flags = nullptr) {
   const int n = P.n, nmat = (int)P.mats_host.size();
   int nmax = 0;
   for (const DcMat& m : P.mats_host) nmax = std::max(nmax, m.n);
-  ZQ_CUDA(cudaMemsetAsync(P.err, 0, sizeof(int), st));
+  int* const err = flags ? flags : P.err;
+  if (!flags) ZQ_CUDA(cudaMemsetAsync(err, 0, sizeof(int), st));
   ZQ_CUDA(launch_pdl_smem(k_dc_scale, dim3(nmat), dim3(nmax <= 256 ? 64 : 256), 0, st, d, e, P.mats_dev, P.dmod, P.es, P.scal));
   ZQ_LAUNCH_CHECK();
   if (!P.nodes_host.empty()) {
@@ -878,7 +881,7 @@ static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, 
           for (int q = 0; q < P.gemm_cnt(t); ++q) {
             const DgemmDesc& h = P.gemm_host[P.gemm_off[t] + q];
             if (int rc = crt_dgemm(h.m, h.n, h.k, Zi + h.off_a, h.lda, Mb + h.off_b, h.ldb, Zo + h.off_c, h.ldc, P.crt_ws,
-                                   P.err, st))
+                                   err, st))
               return rc;
           }
           done = true;
@@ -891,7 +894,7 @@ static int dc_run(DcPlan& P, const double* d, const double* e, double* lam_out, 
     }
   }
   ZQ_CUDA(launch_pdl_smem(k_dc_unscale, dim3((unsigned)nmat, (unsigned)ceil_div(nmax, 128)), dim3(128), 0, st, P.lam[0], P.mats_dev,
-                          P.scal, lam_out, P.err, info));
+                          P.scal, lam_out, err, info));
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }
@@ -901,9 +904,9 @@ int DcPlan::run_forest(const double* d, const double* e, double* eig, int* info,
   return dc_run<double>(*this, d, e, eig, Z, Mb, descs_dev, st, info);
 }
 
-int DcPlan::run(const double* d, const double* e, double* lam_out, double*& z_out, cudaStream_t st) {
+int DcPlan::run(const double* d, const double* e, double* lam_out, double*& z_out, cudaStream_t st, int* flags) {
   if (n <= 0) return ZQ_OK;
-  if (int rc = dc_run<double>(*this, d, e, lam_out, Z, Mb, descs_dev, st)) return rc;
+  if (int rc = dc_run<double>(*this, d, e, lam_out, Z, Mb, descs_dev, st, nullptr, flags)) return rc;
   z_out = Z[0];
   return ZQ_OK;
 }
