@@ -113,8 +113,8 @@ int zq_get_block_size(void);
 
 /* Tensor-core kernel of the Ozaki products in the refined path and
  * zq_zgemm_accurate: 0 = mma.sync (bf16 m16n8k16, 64 x 64 tiles), 1 = tcgen05
- * (TMEM accumulators, TMA-fed 128 x 256 MMAs, one CTA per tile), 2 = tcgen05 in
- * clusters of two CTAs that share the B operand by TMA multicast, 3 = 2-SM
+ * (TMEM accumulators, TMA-fed 128 x 256 MMAs, one CTA per tile), 2 = the same as 1
+ * (kept for saved settings), 3 = 2-SM
  * tcgen05 MMAs (cta_group::2, 256 x 256 per CTA pair; the default). 0 to 2
  * multiply digit slices; 3 does products of 21 bits and more on integer
  * residues (the Ozaki scheme II), at least as accurate, with a third of the

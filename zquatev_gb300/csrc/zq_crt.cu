@@ -27,7 +27,7 @@
 // 0.79 ms, 300 x 300 x 300 products of a solve 0.26 -> 0.10 ms each.
 //
 // k_crt_mma is persistent: each pair of CTAs (cta_group::2, 256 x 256 output
-// tiles) takes jobs (modulus and product, tile); the roles of k_oz_umma<2>
+// tiles) takes jobs (modulus and product, tile); the roles of k_oz_umma's pairs
 // (TMA producer, MMA issuer, eight drain warps; 6 stages of 32 KB, two TMEM
 // accumulators) run through the jobs without draining the pipeline between
 // them. All waits are bounded (zq_umma.cuh).

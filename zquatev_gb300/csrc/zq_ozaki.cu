@@ -527,9 +527,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 3) k_oz_gemm(OzGemmArgs g) {
 static int64_t rup(int64_t a, int64_t b) { return (a + b - 1) / b * b; }
 
 // product kernel: 0 mma.sync (k_oz_gemm), 1 tcgen05 (k_oz_umma, one CTA per
-// tile), 2 tcgen05 in two-CTA clusters sharing B by multicast, 3 tcgen05 2-SM
-// MMAs on two-CTA clusters (the default: n2 = 8192 solve 422 ms against 430
-// ms with one CTA per tile and 440 ms with multicast)
+// tile), 2 the same (it was a form whose CTAs shared B by TMA multicast, no faster;
+// the library also runs with one process per GPU, where such loads have no place),
+// 3 tcgen05 2-SM MMAs on two-CTA clusters (the default)
 static std::atomic<int> g_oz_kernel{3};
 int ozaki_kernel() {
   if (const char* s = getenv("ZQ_OZAKI")) {
@@ -547,7 +547,7 @@ int set_ozaki_kernel(int k) {
 }
 int oz_umma_gemm(const __nv_bfloat16* As, const __nv_bfloat16* Brs, const __nv_bfloat16* Bis, int mp, int np, int Kp,
                  int m, int n, int nsl, int lower, const int* ea, const int* eb, double2* C, int64_t ldc, int* err,
-                 cudaStream_t st, int variant);
+                 cudaStream_t st, bool pairs_of_ctas);
 
 // Whether a product with this many slices' accuracy runs on residues (zq_crt.cu)
 // instead of digit slices, and with how many moduli: the default kernel, from
@@ -778,7 +778,7 @@ int zgemm_ozaki(int opa1, int opb1, int opa2, int opb2, const ZgemmArgs& g, void
     if (!opt.err) ZQ_CUDA(cudaMemsetAsync(errf, 0, sizeof(int), st));
     prof_begin(PC_OZAKI, st);
     if (int rc = oz_umma_gemm(As, Brs, Bis, (int)mp, (int)np, (int)Kp, m, n, nsl, lower ? 1 : 0, ea, eb, g.C, g.ldc, errf,
-                              st, ozaki_kernel() - 1))
+                              st, ozaki_kernel() == 3))
       return rc;
     prof_end(PC_OZAKI, st);
     if (int rc = check_flag(errf)) return rc;
@@ -819,7 +819,7 @@ int zgemm_ozaki(int opa1, int opb1, int opa2, int opb2, const ZgemmArgs& g, void
 extern "C" int zq_set_ozaki_kernel(int which) {
   if (zq::set_ozaki_kernel(which)) {
     zq::set_error_message(
-        "kernel must be 0 (mma.sync), 1 (tcgen05), 2 (tcgen05, cluster-multicast B) or 3 (tcgen05 2-SM MMA)");
+        "kernel must be 0 (mma.sync), 1 (tcgen05), 2 (the same as 1) or 3 (tcgen05 2-SM MMA)");
     return zq::ZQ_ERR_ARG;
   }
   return zq::ZQ_OK;

@@ -72,40 +72,33 @@ __device__ __forceinline__ double um_pow2i(int E) {
   return __longlong_as_double((long long)(1023 + E) << 52);
 }
 
-// Variants (template V):
-//   0  one CTA per 128 x 128 tile: A box + Bre box + Bim box per stage (48 KB),
+// Two forms (template PAIR):
+//   one CTA per 128 x 128 tile: A box + Bre box + Bim box per stage (48 KB),
 //      4 stages.
-//   1  clusters of two CTAs on vertically adjacent tiles of the same column
-//      tile, which share B: each CTA loads its own A box and one half of B
-//      (rank 0 Bre, rank 1 Bim) multicast to both, so a CTA reads 32 KB per
-//      stage from L2 instead of 48 KB; still 48 KB of shared memory per stage.
-//      A stage is refilled once both CTAs' MMAs have released it.
-//   2  the same pairs computed by 2-SM MMAs (tcgen05.mma.cta_group::2, M =
-//      256): each CTA stages only its own A box and one half of B (rank 0
-//      Bre, rank 1 Bim), 32 KB per stage, 6 stages; rank 0 issues the MMAs for
-//      both SMs, each SM's tensor core reads its own A rows and both halves of
-//      B, and each CTA's TMEM holds its 128 rows. Per MMA an SM writes and
-//      reads 8 KB of shared memory instead of 12 KB, the rate that limits the
-//      one-CTA form. Both CTAs' TMA loads complete on rank 0's full barrier;
-//      the MMA commits arrive on both CTAs' empty and accumulator barriers;
-//      rank 1's drain warps release an accumulator on rank 0's barrier.
-// In variants 1 and 2 a cluster's second tile past the last row tile is
-// computed but not written.
-template <int V>
+//   clusters of two CTAs on vertically adjacent tiles of the same column tile,
+//      computed by 2-SM MMAs (tcgen05.mma.cta_group::2, M = 256): each CTA stages
+//      only its own A box and one half of B (rank 0 Bre, rank 1 Bim), 32 KB per
+//      stage, 6 stages; rank 0 issues the MMAs for both SMs, each SM's tensor core
+//      reads its own A rows and both halves of B, and each CTA's TMEM holds its 128
+//      rows. Per MMA an SM writes and reads 8 KB of shared memory instead of 12 KB,
+//      the rate that limits the one-CTA form. Both CTAs' TMA loads complete on rank
+//      0's full barrier; the MMA commits arrive on both CTAs' empty and accumulator
+//      barriers; rank 1's drain warps release an accumulator on rank 0's barrier. A
+//      cluster's second tile past the last row tile is computed but not written.
+template <bool PAIR>
 struct UmShape {
-  static constexpr uint32_t stage_bytes = V == 2 ? UM_A_BYTES + UM_BH_BYTES : UM_A_BYTES + 2 * UM_BH_BYTES;
-  static constexpr int stages = V == 2 ? 6 : 4;
+  static constexpr uint32_t stage_bytes = PAIR ? UM_A_BYTES + UM_BH_BYTES : UM_A_BYTES + 2 * UM_BH_BYTES;
+  static constexpr int stages = PAIR ? 6 : 4;
 };
-static_assert(UmShape<0>::stages * UmShape<0>::stage_bytes <= UM_RING_BYTES, "ring");
-static_assert(UmShape<2>::stages * UmShape<2>::stage_bytes <= UM_RING_BYTES, "ring");
+static_assert(UmShape<false>::stages * UmShape<false>::stage_bytes <= UM_RING_BYTES, "ring");
+static_assert(UmShape<true>::stages * UmShape<true>::stage_bytes <= UM_RING_BYTES, "ring");
 
-template <int V>
+template <bool PAIR>
 __global__ void __launch_bounds__(UM_THREADS, 1)
     k_oz_umma(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmBr,
               const __grid_constant__ CUtensorMap tmBi, UmArgs g) {
-  constexpr bool PAIR = V != 0;
-  constexpr int STAGES = UmShape<V>::stages;
-  constexpr uint32_t STAGE_BYTES = UmShape<V>::stage_bytes;
+  constexpr int STAGES = UmShape<PAIR>::stages;
+  constexpr uint32_t STAGE_BYTES = UmShape<PAIR>::stage_bytes;
   extern __shared__ __align__(1024) unsigned char um_smem_raw[];
   // 1024-byte aligned stage ring (128-byte swizzle atoms), barriers after it
   const uint32_t raw = su32(um_smem_raw);
@@ -122,11 +115,11 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(full0 + 8 * s, 1);
-      mbar_init(empty0 + 8 * s, V == 1 ? 2 : 1);
+      mbar_init(empty0 + 8 * s, 1);
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(accf0 + 8 * b, 1);
-      mbar_init(acce0 + 8 * b, V == 2 ? 16 : 8);
+      mbar_init(acce0 + 8 * b, PAIR ? 16 : 8);
     }
     mbar_init(done_bar, 1);
     s_abort = 0;
@@ -134,7 +127,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == 1) {
-    if (V == 2) {
+    if (PAIR) {
       // one warp of each CTA of the pair allocates collectively: the same
       // columns in both SMs' tensor memory
       asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(&s_tmem)),
@@ -151,7 +144,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (PAIR) cluster_sync();  // the peer's barriers are initialised before any multicast or remote arrival
+  if (PAIR) cluster_sync();  // the peer's barriers are initialised before any remote arrival
   const uint32_t tmem = s_tmem;
   volatile int* abort = &s_abort;
 
@@ -194,8 +187,8 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
     if (lane == 0) {
       int ks = 0;
       bool ok = true;
-      // variant 2: both CTAs' copies complete on rank 0's full barrier
-      const uint32_t full_lead = V == 2 ? mapa_shared(full0, 0) : full0;
+      // in a pair both CTAs' copies complete on rank 0's full barrier
+      const uint32_t full_lead = PAIR ? mapa_shared(full0, 0) : full0;
       for (int lev = 0; lev < g.nsl && ok; ++lev) {
         const int64_t total = (int64_t)(lev + 1) * Kp;
         for (int64_t kg = 0; kg < total && ok; kg += UM_BK) {
@@ -203,7 +196,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
           if (!mbar_wait(empty0 + 8 * stage, (round & 1) ^ 1, abort, g.wait)) { ok = false; break; }
           const uint32_t sA = ring + stage * STAGE_BYTES;
           const int t = (int)(kg / Kp), kk = (int)(kg % Kp), u = lev - t;
-          if (V == 2) {
+          if (PAIR) {
             if (rank == 0) mbar_expect_tx(full0 + 8 * stage, 2 * STAGE_BYTES);
             tma_2d_pair(sA, &tmA, kk, t * g.mp + i0, full_lead + 8 * stage);
             if (rank == 0) tma_2d_pair(sA + UM_A_BYTES, &tmBr, kk, u * g.np + j0, full_lead + 8 * stage);
@@ -211,13 +204,8 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
           } else {
             mbar_expect_tx(full0 + 8 * stage, STAGE_BYTES);
             tma_2d(sA, &tmA, kk, t * g.mp + i0, full0 + 8 * stage);
-            if (V == 1) {
-              if (rank == 0) tma_2d_mc(sA + UM_A_BYTES, &tmBr, kk, u * g.np + j0, full0 + 8 * stage, (uint16_t)3);
-              else tma_2d_mc(sA + UM_A_BYTES + UM_BH_BYTES, &tmBi, kk, u * g.np + j0, full0 + 8 * stage, (uint16_t)3);
-            } else {
-              tma_2d(sA + UM_A_BYTES, &tmBr, kk, u * g.np + j0, full0 + 8 * stage);
-              tma_2d(sA + UM_A_BYTES + UM_BH_BYTES, &tmBi, kk, u * g.np + j0, full0 + 8 * stage);
-            }
+            tma_2d(sA + UM_A_BYTES, &tmBr, kk, u * g.np + j0, full0 + 8 * stage);
+            tma_2d(sA + UM_A_BYTES + UM_BH_BYTES, &tmBi, kk, u * g.np + j0, full0 + 8 * stage);
           }
           ++ks;
         }
@@ -226,16 +214,16 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
       // copies in flight finish before the CTA may exit (after an abort in a
       // cluster a stage may lack the peer's part and never complete: its own
       // copies land within microseconds, so wait about a millisecond there).
-      // In variant 2 only rank 0 holds the full barriers; rank 1 is held at
+      // In a pair only rank 0 holds the full barriers; rank 1 is held at
       // the final cluster barrier until rank 0 has drained them. (What the peer
       // alone issued is covered by abort_hold.)
-      if (V != 2 || rank == 0)
+      if (!PAIR || rank == 0)
         for (int q = (issued > STAGES ? issued - STAGES : 0); q < issued; ++q)
           mbar_drain(full0 + 8 * (q % STAGES), (q / STAGES) & 1, PAIR ? 2000000LL : UM_WAIT_CYCLES);
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && (V != 2 || rank == 0)) {
+    if (lane == 0 && (!PAIR || rank == 0)) {
       int ks = 0, ci = 0;
       bool ok = true;
       for (int lev = 0; lev < g.nsl && ok; ++lev) {
@@ -256,23 +244,22 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
               const uint64_t ad = sw128_desc(sA), bd = sw128_desc(sA + UM_A_BYTES);
 #pragma unroll
               for (int k = 0; k < UM_BK / 16; ++k) {  // 16 bf16 = 32 bytes along the swizzled row
-                if (V == 2) umma_bf16_pair(d, ad + 2 * k, bd + 2 * k, (kg != cb || k > 0) ? 1u : 0u);
+                if (PAIR) umma_bf16_pair(d, ad + 2 * k, bd + 2 * k, (kg != cb || k > 0) ? 1u : 0u);
                 else umma_bf16(d, ad + 2 * k, bd + 2 * k, (kg != cb || k > 0) ? 1u : 0u);
               }
-              if (V == 2) umma_commit_pair_mc(empty0 + 8 * stage, (uint16_t)3);
-              else if (V == 1) umma_commit_mc(empty0 + 8 * stage, (uint16_t)3);
+              if (PAIR) umma_commit_pair_mc(empty0 + 8 * stage, (uint16_t)3);
               else umma_commit(empty0 + 8 * stage);
               ++ks;
             }
             if (!ok) break;
-            if (V == 2) umma_commit_pair_mc(accf0 + 8 * buf, (uint16_t)3);
+            if (PAIR) umma_commit_pair_mc(accf0 + 8 * buf, (uint16_t)3);
             else umma_commit(accf0 + 8 * buf);
             ++ci;
           }
         }
       }
       // every MMA issued has completed before TMEM is released
-      if (V == 2) umma_commit_pair_mc(done_bar, (uint16_t)1);
+      if (PAIR) umma_commit_pair_mc(done_bar, (uint16_t)1);
       else umma_commit(done_bar);
       mbar_drain(done_bar, 0);
     }
@@ -282,8 +269,8 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
     const int h = (warp - 2) >> 2;      // column half (0: j0..j0+63, 1: j0+64..j0+127)
     const int row = i0 + 32 * q + lane;
     const uint32_t lane_base = tmem + ((uint32_t)(32 * q) << 16);
-    // variant 2: an accumulator is free once both CTAs' drain warps released it
-    const uint32_t acce_lead = V == 2 ? mapa_shared(acce0, 0) : acce0;
+    // in a pair an accumulator is free once both CTAs' drain warps released it
+    const uint32_t acce_lead = PAIR ? mapa_shared(acce0, 0) : acce0;
     int ir[64], ii[64];
 #pragma unroll
     for (int c = 0; c < 64; ++c) { ir[c] = 0; ii[c] = 0; }
@@ -316,7 +303,7 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
           tc_fence_before();
           __syncwarp();
           if (lane == 0) {
-            if (V == 2 && rank != 0) mbar_arrive_remote(acce_lead + 8 * buf);
+            if (PAIR && rank != 0) mbar_arrive_remote(acce_lead + 8 * buf);
             else mbar_arrive(acce0 + 8 * buf);
           }
           ++ci;
@@ -364,10 +351,10 @@ __global__ void __launch_bounds__(UM_THREADS, 1)
   __syncthreads();
   tc_fence_after();
   if (PAIR && s_abort) abort_hold();
-  // variant 2: both CTAs' MMAs and drains are finished before the collective release
-  if (V == 2) cluster_sync();
+  // a pair: both CTAs' MMAs and drains are finished before the collective release
+  if (PAIR) cluster_sync();
   if (warp == 1) {
-    if (V == 2)
+    if (PAIR)
       asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(UM_TMEM_COLS) : "memory");
     else
       asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(UM_TMEM_COLS) : "memory");
@@ -422,8 +409,7 @@ long long pipeline_wait_cycles() { return g_wait_cycles.load(); }
 // err: device int, zeroed by the caller, raised by the kernel on a wait timeout.
 int oz_umma_gemm(const __nv_bfloat16* As, const __nv_bfloat16* Brs, const __nv_bfloat16* Bis, int mp, int np, int Kp,
                  int m, int n, int nsl, int lower, const int* ea, const int* eb, double2* C, int64_t ldc, int* err,
-                 cudaStream_t st, int variant) {
-  if (variant < 0 || variant > 2) { set_error_message("oz_umma_gemm: variant 0..2"); return ZQ_ERR_ARG; }
+                 cudaStream_t st, bool pairs_of_ctas) {
   if (mp % UM_BM || np % UM_BN || Kp % UM_BK || nsl < 1) { set_error_message("oz_umma_gemm: bad padding"); return ZQ_ERR_ARG; }
   CUtensorMap ta, tbr, tbi;
   if (int rc = make_map(&ta, As, Kp, (int64_t)nsl * mp)) return rc;
@@ -435,9 +421,8 @@ int oz_umma_gemm(const __nv_bfloat16* As, const __nv_bfloat16* Brs, const __nv_b
     ZQ_CUDA(cudaGetDevice(&dev));
     const unsigned long long bit = 1ull << (dev & 63);
     if (!(attr_set.load() & bit)) {
-      ZQ_CUDA(cudaFuncSetAttribute(k_oz_umma<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, UM_SMEM));
-      ZQ_CUDA(cudaFuncSetAttribute(k_oz_umma<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, UM_SMEM));
-      ZQ_CUDA(cudaFuncSetAttribute(k_oz_umma<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, UM_SMEM));
+      ZQ_CUDA(cudaFuncSetAttribute(k_oz_umma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, UM_SMEM));
+      ZQ_CUDA(cudaFuncSetAttribute(k_oz_umma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, UM_SMEM));
       attr_set.fetch_or(bit);
     }
   }
@@ -446,7 +431,7 @@ int oz_umma_gemm(const __nv_bfloat16* As, const __nv_bfloat16* Brs, const __nv_b
   a.ea = ea; a.eb = eb; a.C = C; a.ldc = ldc; a.err = err;
   a.wait = g_wait_cycles.load();
   const int tm = mp / UM_BM, tn = np / UM_BN;
-  if (variant != 0) {
+  if (pairs_of_ctas) {
     // clusters of two row-adjacent tiles (the last pair of a column may hold a tile past the matrix)
     int pairs = 0;
     if (lower) for (int col = 0; col < tm; ++col) pairs += (tm - col + 1) / 2;
@@ -463,11 +448,10 @@ int oz_umma_gemm(const __nv_bfloat16* As, const __nv_bfloat16* Brs, const __nv_b
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (variant == 1) ZQ_CUDA(cudaLaunchKernelEx(&cfg, k_oz_umma<1>, ta, tbr, tbi, a));
-    else ZQ_CUDA(cudaLaunchKernelEx(&cfg, k_oz_umma<2>, ta, tbr, tbi, a));
+    ZQ_CUDA(cudaLaunchKernelEx(&cfg, k_oz_umma<true>, ta, tbr, tbi, a));
   } else {
     const dim3 grid = lower ? dim3((unsigned)(tm * (tm + 1) / 2), 1) : dim3((unsigned)(tm * tn), 1);
-    k_oz_umma<0><<<grid, UM_THREADS, UM_SMEM, st>>>(ta, tbr, tbi, a);
+    k_oz_umma<false><<<grid, UM_THREADS, UM_SMEM, st>>>(ta, tbr, tbi, a);
   }
   ZQ_LAUNCH_CHECK();
   return ZQ_OK;

@@ -63,21 +63,6 @@ __device__ __forceinline__ void abort_hold() {
   }
 }
 
-// the same box written to this CTA and its cluster peer (same shared offsets);
-// complete_tx is signalled on the mbarrier at `bar` in each destination
-__device__ __forceinline__ void tma_2d_mc(uint32_t dst, const CUtensorMap* tm, int x, int y, uint32_t bar, uint16_t mask) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.multicast::cluster [%0], [%1, {%2, %3}], "
-      "[%4], %5;" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(tm)), "r"(x), "r"(y), "r"(bar), "h"(mask)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit_mc(uint32_t bar, uint16_t mask) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
-                   bar),
-               "h"(mask)
-               : "memory");
-}
 // address of the same shared variable in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
   uint32_t r;
