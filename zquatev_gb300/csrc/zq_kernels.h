@@ -205,6 +205,7 @@ struct RefineArgs {
   int slices0;                 // Ozaki slices of the first step's products
   int slices_res;              // Ozaki slices of the products with the residual R = HX - X Lambda
   int values_only;             // the eigenvalues alone: no last update of X, no vectors in place
+  int digits;                  // the products' workspace holds digit slices only
   int coop;                    // no other solve runs beside this one: the FP32 reduction may take every SM
   cudaStream_t st;
   cudaStream_t st2;            // second stream: Q formation overlaps the tridiagonal solve
@@ -225,12 +226,13 @@ struct OzOpts {
   int nofill;      // structured: leave the upper triangle to the caller (who fills it with structured_fill)
   int prev_slices; // reuse_a: the slices of the previous call
   int* err;        // device flag a pipeline timeout raises, cleared and read by the caller (null: here, with a wait)
+  int digits;      // 1: digit slices at any accuracy (workspaces too small for residues)
 };
 int zgemm_ozaki(int opa1, int opb1, int opa2, int opb2, const ZgemmArgs& g, void* ws, size_t ws_bytes, cudaStream_t st,
                 const OzOpts& opt);
 // workspace of one product (K = the complex inner dimension of all segments)
-size_t zgemm_ozaki_bytes(int m, int n, int64_t K, int slices);
-size_t ozaki_workspace_bytes(int n);
+size_t zgemm_ozaki_bytes(int m, int n, int64_t K, int slices, bool digits = false);
+size_t ozaki_workspace_bytes(int n, bool digits = false);
 // the current device's pool for the scratch of single calls: stream-ordered,
 // keeps up to SCRATCH_KEEP bytes mapped between calls (zq_release_workspace
 // returns them)

@@ -556,12 +556,15 @@ int oz_umma_gemm(const __nv_bfloat16* As, const __nv_bfloat16* Brs, const __nv_b
 // decides for small products (the two of a solve at n = 512 0.3 ms on digits, 0.15
 // on residues; n = 4096 the same 9 ms). Two: fewer digit products (12).
 static int crt_bits(int slices) { return OZ_BETA * slices - 1; }
-static int use_crt(int slices, int64_t K) {
-  return ozaki_kernel() == 3 && slices >= 3 ? crt_moduli(crt_bits(slices), 2.0 * (double)K) : 0;
+// K: the splitting kernel's grid has a row of blocks per 64 terms.
+constexpr int64_t CRT_K_MAX = (int64_t)64 * 65535;
+static int use_crt(int slices, int64_t K, bool digits) {
+  if (digits || ozaki_kernel() != 3 || slices < 3 || K > CRT_K_MAX) return 0;
+  return crt_moduli(crt_bits(slices), 2.0 * (double)K);
 }
 
-size_t zgemm_ozaki_bytes(int m, int n, int64_t K, int slices) {
-  if (const int L = use_crt(slices, K)) {
+size_t zgemm_ozaki_bytes(int m, int n, int64_t K, int slices, bool digits) {
+  if (const int L = use_crt(slices, K, digits)) {
     const CrtShape s = crt_shape(m, n, (int)K, L, true);
     return s.a_bytes + s.b_bytes + s.r_bytes + sizeof(int) * (size_t)(s.mp + s.np + 64) + 9 * 256;
   }
@@ -570,8 +573,9 @@ size_t zgemm_ozaki_bytes(int m, int n, int64_t K, int slices) {
 }
 
 // workspace of the refinement's products, (m, n, K) = (2 nq, nq, nq) and
-// (nq, nq, 2 nq), at any slice count and with any product kernel
-size_t ozaki_workspace_bytes(int nq) {
+// (nq, nq, 2 nq), at any slice count and with any product kernel, or with digit slices
+// only (a third of it)
+size_t ozaki_workspace_bytes(int nq, bool digits_only) {
   size_t most = 0;
   const int64_t shapes[2][3] = {{2 * (int64_t)nq, nq, nq}, {nq, nq, 2 * (int64_t)nq}};
   for (const auto& q : shapes) {
@@ -580,7 +584,7 @@ size_t ozaki_workspace_bytes(int nq) {
     const int L = crt_moduli(crt_bits(OZ_SMAX), 2.0 * (double)q[2]);
     const CrtShape s = crt_shape((int)q[0], (int)q[1], (int)q[2], L > 0 ? L : 1, true);
     const size_t residues = s.a_bytes + s.b_bytes + s.r_bytes + sizeof(int) * (size_t)(s.mp + s.np + 64);
-    most = std::max(most, std::max(digits, residues));
+    most = std::max(most, digits_only ? digits : std::max(digits, residues));
   }
   return most + 9 * 256;
 }
@@ -677,7 +681,8 @@ int zgemm_ozaki(int opa1, int opb1, int opa2, int opb2, const ZgemmArgs& g, void
   const int64_t Kp = rup(2 * ((int64_t)g.k1 + (two ? g.k2 : 0)), OZ_TK);
   const int64_t mp = rup(m, OZ_PAD), np = rup(n, OZ_PAD);
   const int64_t Kc = (int64_t)g.k1 + (two ? g.k2 : 0);
-  if (zgemm_ozaki_bytes(m, n, Kc, nsl) > ws_bytes) { set_error_message("zgemm_ozaki: workspace too small"); return ZQ_ERR_LIMIT; }
+  const bool digits = opt.digits != 0;
+  if (zgemm_ozaki_bytes(m, n, Kc, nsl, digits) > ws_bytes) { set_error_message("zgemm_ozaki: workspace too small"); return ZQ_ERR_LIMIT; }
   if (g.alpha.x != 1.0 || g.alpha.y != 0.0 || g.beta.x != 0.0 || g.beta.y != 0.0) {
     set_error_message("zgemm_ozaki: only C = op(A) op(B) (alpha 1, beta 0)");
     return ZQ_ERR_ARG;
@@ -719,8 +724,8 @@ int zgemm_ozaki(int opa1, int opb1, int opa2, int opb2, const ZgemmArgs& g, void
     }
     return ZQ_OK;
   };
-  const int L = use_crt(nsl, Kc);
-  const bool reuse_a = opt.reuse_a && (L > 0) == (use_crt(opt.prev_slices, Kc) > 0) && (L == 0 || opt.prev_slices == nsl);
+  const int L = use_crt(nsl, Kc, digits);
+  const bool reuse_a = opt.reuse_a && (L > 0) == (use_crt(opt.prev_slices, Kc, digits) > 0) && (L == 0 || opt.prev_slices == nsl);
   if (L > 0) {
     const CrtShape sh = crt_shape(m, n, (int)Kc, L, true);
     const int bits = crt_bits(nsl);
@@ -833,20 +838,26 @@ extern "C" int zq_zgemm_accurate(int opa, int opb, int m, int n, int k, const do
   using namespace zq;
   if (m < 0 || n < 0 || k < 0 || opa < 0 || opa > 3 || opb < 0 || opb > 3) return ZQ_ERR_ARG;
   if (m == 0 || n == 0) return ZQ_OK;
-  const size_t bytes = zgemm_ozaki_bytes(m, n, k, 8);
+  size_t bytes = zgemm_ozaki_bytes(m, n, k, 8);
   void* ws = nullptr;
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
   cudaMemPool_t pool = nullptr;
   if (int rc = scratch_pool(&pool)) return rc;
-  ZQ_CUDA(cudaMallocFromPoolAsync(&ws, bytes, pool, st));
+  OzOpts opt{};
+  opt.slices = 8;
+  if (cudaMallocFromPoolAsync(&ws, bytes, pool, st) != cudaSuccess) {
+    // residues take 2.5 times the scratch of digit slices: where they do not fit, these
+    (void)cudaGetLastError();
+    opt.digits = 1;
+    bytes = zgemm_ozaki_bytes(m, n, k, 8, true);
+    ZQ_CUDA(cudaMallocFromPoolAsync(&ws, bytes, pool, st));
+  }
   ZgemmArgs g{};
   g.m = m; g.n = n; g.k1 = k;
   g.A1 = reinterpret_cast<const double2*>(A); g.lda1 = lda;
   g.B1 = reinterpret_cast<const double2*>(B); g.ldb1 = ldb;
   g.alpha = make_double2(1.0, 0.0); g.beta = make_double2(0.0, 0.0);
   g.C = reinterpret_cast<double2*>(C); g.ldc = ldc;
-  OzOpts opt{};
-  opt.slices = 8;
   const int rc = zgemm_ozaki(opa, opb, OP_N, OP_N, g, ws, bytes, st, opt);
   cudaFreeAsync(ws, st);
   return rc;
