@@ -248,9 +248,9 @@ int ensure_ws(Context* c, size_t bytes) {
   if (c->ws_bytes >= bytes) return ZQ_OK;
   if (c->ws_external) { set_msg("bound workspace too small"); return ZQ_ERR_ARG; }
   if (c->ws) { cudaStreamSynchronize(c->st); cudaStreamSynchronize(c->st2); cudaFree(c->ws); c->ws = nullptr; c->ws_bytes = 0; }
+  c->dc_n = -1;  // the plan's pointers refer to the old buffer, also where there is no new one
   ZQ_CUDA(cudaMalloc(&c->ws, bytes));
   c->ws_bytes = bytes;
-  c->dc_n = -1;  // plan pointers refer to the old buffer
   return ZQ_OK;
 }
 

@@ -148,6 +148,7 @@ enum Status : int {
   do {                                                                       \
     cudaError_t _e = (call);                                                 \
     if (_e != cudaSuccess) {                                                 \
+      (void)cudaGetLastError(); /* reported here: not the next call's */     \
       zq::set_last_error(_e, #call, __FILE__, __LINE__);                     \
       return (_e == cudaErrorMemoryAllocation) ? zq::ZQ_ERR_NOMEM : zq::ZQ_ERR_CUDA; \
     }                                                                        \
