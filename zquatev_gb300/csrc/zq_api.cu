@@ -224,11 +224,11 @@ static size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 struct Layout {
   size_t tri, small, dc, fq, nodes, descs, total;
 };
-static Layout layout_for(int n, int nbmax, int nbq, size_t nnodes, size_t ndescs) {
+static Layout layout_for(int n, int nbmax, int nbq, size_t nnodes, size_t ndescs, bool lean) {
   Layout L{};
   L.tri = align256(tridiag_workspace_bytes<double>(n, nbmax));
   L.small = align256(sizeof(double) * (size_t)(n + 4 * (size_t)n + n + n + 4 * (size_t)n + n + 16));
-  L.dc = align256(sizeof(double) * DcPlan::workspace_doubles(n));
+  L.dc = align256(sizeof(double) * DcPlan::workspace_doubles(n, lean));
   L.fq = align256(form_q_workspace_bytes(n, nbq));
   L.nodes = align256(sizeof(DcNode) * (nnodes + 1));
   L.descs = align256(DcPlan::desc_bytes(ndescs));
@@ -236,12 +236,12 @@ static Layout layout_for(int n, int nbmax, int nbq, size_t nnodes, size_t ndescs
   return L;
 }
 
-void solve_workspace_bytes(int n, size_t* fp64_bytes, size_t* refine_bytes) {
+void solve_workspace_bytes(int n, size_t* fp64_bytes, size_t* refine_bytes, bool lean) {
   DcPlan probe;
   probe.build(n);
-  const Layout L = layout_for(n, NBMAX, g_nbq, probe.num_nodes(), probe.num_descs());
+  const Layout L = layout_for(n, NBMAX, g_nbq, probe.num_nodes(), probe.num_descs(), lean);
   if (fp64_bytes) *fp64_bytes = L.total;
-  if (refine_bytes) *refine_bytes = refine_workspace_bytes(n, g_nbq) + ozaki_workspace_bytes(n) + 4096 + 256;
+  if (refine_bytes) *refine_bytes = refine_workspace_bytes(n, g_nbq) + ozaki_workspace_bytes(n, lean) + 4096 + 256;
 }
 
 int ensure_ws(Context* c, size_t bytes) {
@@ -251,6 +251,31 @@ int ensure_ws(Context* c, size_t bytes) {
   c->dc_n = -1;  // the plan's pointers refer to the old buffer, also where there is no new one
   ZQ_CUDA(cudaMalloc(&c->ws, bytes));
   c->ws_bytes = bytes;
+  return ZQ_OK;
+}
+
+// The divide-and-conquer plan of order n in a workspace for it. Where the workspace does
+// not fit (an allocation that fails, a bound one that is too small), one without the
+// scratch of the residue merges is tried.
+int ensure_plan(Context* c, int n) {
+  if (c->dc_n == n) return ZQ_OK;
+  DcPlan probe;
+  probe.build(n);
+  Layout L{};
+  for (int lean = 0;; ++lean) {
+    L = layout_for(n, NBMAX, g_nbq, probe.num_nodes(), probe.num_descs(), lean != 0);
+    const int rc = ensure_ws(c, L.total);
+    c->lean = lean != 0;
+    if (rc == ZQ_OK) break;
+    if (lean || (rc != ZQ_ERR_NOMEM && !c->ws_external)) return rc;
+  }
+  c->dc_n = -1;
+  c->dc = probe;
+  char* p = reinterpret_cast<char*>(c->ws) + L.tri + L.small;
+  double* dcws = reinterpret_cast<double*>(p); p += L.dc + L.fq;
+  DcNode* nodes = reinterpret_cast<DcNode*>(p); p += L.nodes;
+  if (int rc = c->dc.upload(dcws, nodes, reinterpret_cast<DgemmDesc*>(p), c->st, nullptr, c->lean)) return rc;
+  c->dc_n = n;
   return ZQ_OK;
 }
 
@@ -292,21 +317,8 @@ int solve_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, bool
   const char* tenv = getenv("ZQ_TIMING");
   StageTimer tm(tenv && tenv[0] == '1');
   const int nbq = g_nbq;
-  if (c->dc_n != n) {
-    DcPlan probe;
-    probe.build(n);
-    Layout L = layout_for(n, NBMAX, nbq, probe.num_nodes(), probe.num_descs());
-    if (int rc = ensure_ws(c, L.total)) return rc;
-    c->dc = probe;
-    char* base = reinterpret_cast<char*>(c->ws);
-    char* p = base + L.tri + L.small;
-    double* dcws = reinterpret_cast<double*>(p); p += L.dc + L.fq;
-    DcNode* nodes = reinterpret_cast<DcNode*>(p); p += L.nodes;
-    DgemmDesc* descs = reinterpret_cast<DgemmDesc*>(p);
-    if (int rc = c->dc.upload(dcws, nodes, descs, c->st)) return rc;
-    c->dc_n = n;
-  }
-  Layout L = layout_for(n, NBMAX, nbq, c->dc.num_nodes(), c->dc.num_descs());
+  if (int rc = ensure_plan(c, n)) return rc;
+  Layout L = layout_for(n, NBMAX, nbq, c->dc.num_nodes(), c->dc.num_descs(), c->lean);
   char* base = reinterpret_cast<char*>(c->ws);
   void* tri_ws = base;
   double* sm = reinterpret_cast<double*>(base + L.tri);
@@ -500,28 +512,23 @@ static int zquatev_host(int n2, double2* D, int ld2, double* eig, bool vectors, 
 // refined (mixed-precision) path
 // ----------------------------------------------------------------------------
 
-int ensure_plan(Context* c, int n) {
-  if (c->dc_n == n) return ZQ_OK;
-  DcPlan probe;
-  probe.build(n);
-  Layout L = layout_for(n, NBMAX, g_nbq, probe.num_nodes(), probe.num_descs());
-  if (int rc = ensure_ws(c, L.total)) return rc;
-  c->dc = probe;
-  char* base = reinterpret_cast<char*>(c->ws);
-  char* p = base + L.tri + L.small;
-  double* dcws = reinterpret_cast<double*>(p); p += L.dc + L.fq;
-  DcNode* nodes = reinterpret_cast<DcNode*>(p); p += L.nodes;
-  if (int rc = c->dc.upload(dcws, nodes, reinterpret_cast<DgemmDesc*>(p), c->st)) return rc;
-  c->dc_n = n;
-  return ZQ_OK;
-}
-
-// `spare`: take the workspace only if that leaves as much free again (else ZQ_ERR_NOMEM)
+// The refinement's workspace; rb.digits: it holds the products' digit slices but not
+// their residues (the full one does not fit). `spare`: take it only if that leaves as
+// much free again (else ZQ_ERR_NOMEM)
 static int refined_reserve(Context* c, int n, int mode, bool spare) {
   if (int rc = ensure_plan(c, n)) return rc;
   RefineBuffers& rb = c->rb;
-  const size_t need = refine_workspace_bytes(n, g_nbq) + (mode == 1 ? ozaki_workspace_bytes(n) : 0) + 4096;
-  if (rb.bytes < need) {
+  const size_t base = refine_workspace_bytes(n, g_nbq) + 4096;
+  const size_t need = base + (mode == 1 ? ozaki_workspace_bytes(n) : 0);
+  const size_t least = base + (mode == 1 ? ozaki_workspace_bytes(n, true) : 0);
+  rb.digits = rb.bytes < need;
+  if (rb.digits && rb.bytes >= least && rb.external) return ZQ_OK;
+  if (rb.digits && rb.bytes >= least) {  // as an earlier call left it: worth another try?
+    size_t free_b = 0, total_b = 0;
+    ZQ_CUDA(cudaMemGetInfo(&free_b, &total_b));
+    if (free_b + rb.bytes < need) return ZQ_OK;
+  }
+  if (rb.digits) {
     if (rb.external) { set_msg("bound refinement workspace too small"); return ZQ_ERR_ARG; }
     if (spare) {
       size_t free_b = 0, total_b = 0;
@@ -529,8 +536,13 @@ static int refined_reserve(Context* c, int n, int mode, bool spare) {
       if (need > free_b / 2) return ZQ_ERR_NOMEM;
     }
     if (rb.dev) { cudaStreamSynchronize(c->st); cudaFree(rb.dev); rb.dev = nullptr; rb.bytes = 0; }
-    ZQ_CUDA(cudaMalloc(&rb.dev, need));
-    rb.bytes = need;
+    rb.digits = cudaMalloc(&rb.dev, need) != cudaSuccess;
+    if (rb.digits) {
+      (void)cudaGetLastError();
+      rb.dev = nullptr;
+      ZQ_CUDA(cudaMalloc(&rb.dev, least));
+    }
+    rb.bytes = rb.digits ? least : need;
   }
   return ZQ_OK;
 }
@@ -538,7 +550,7 @@ static int refined_reserve(Context* c, int n, int mode, bool spare) {
 int refined_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, cudaStream_t st, int mode, bool vectors) {
   if (int rc = refined_reserve(c, n, mode, false)) return rc;
   RefineBuffers& rb = c->rb;
-  Layout L = layout_for(n, NBMAX, g_nbq, c->dc.num_nodes(), c->dc.num_descs());
+  Layout L = layout_for(n, NBMAX, g_nbq, c->dc.num_nodes(), c->dc.num_descs(), c->lean);
   DgemmDesc* desc1 = reinterpret_cast<DgemmDesc*>(reinterpret_cast<char*>(c->ws) + L.tri + L.small + L.dc + L.fq + L.nodes) +
                      c->dc.num_descs();
   RefineArgs ra{};
@@ -546,7 +558,8 @@ int refined_device(Context* c, double2* dD, int64_t ldd, int n, double* deig, cu
   ra.ws = reinterpret_cast<char*>(rb.dev) + 4096;
   const size_t rws = refine_workspace_bytes(n, g_nbq);
   ra.ows = (mode == 1) ? reinterpret_cast<char*>(ra.ws) + ((rws + 255) & ~(size_t)255) : nullptr;
-  ra.ows_bytes = (mode == 1) ? ozaki_workspace_bytes(n) : 0;
+  ra.ows_bytes = (mode == 1) ? ozaki_workspace_bytes(n, rb.digits) : 0;
+  ra.digits = rb.digits ? 1 : 0;
   ra.dc = &c->dc;
   ra.coop = c->coop ? 1 : 0;
   ra.values_only = vectors ? 0 : 1;
@@ -801,19 +814,7 @@ int zq_stedc_device(int n, const double* d, const double* e, double* lam, double
   if (int rc = get_context(&c)) return rc;
   std::lock_guard<std::mutex> lk(c->mu);
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (c->dc_n != n) {
-    DcPlan probe;
-    probe.build(n);
-    Layout L = layout_for(n, NBMAX, g_nbq, probe.num_nodes(), probe.num_descs());
-    if (int rc = ensure_ws(c, L.total)) return rc;
-    c->dc = probe;
-    char* base = reinterpret_cast<char*>(c->ws);
-    char* p = base + L.tri + L.small;
-    double* dcws = reinterpret_cast<double*>(p); p += L.dc + L.fq;
-    DcNode* nodes = reinterpret_cast<DcNode*>(p); p += L.nodes;
-    if (int rc = c->dc.upload(dcws, nodes, reinterpret_cast<DgemmDesc*>(p), c->st)) return rc;
-    c->dc_n = n;
-  }
+  if (int rc = ensure_plan(c, n)) return rc;
   ZQ_CUDA(cudaEventRecord(c->ev_fork, st));
   ZQ_CUDA(cudaStreamWaitEvent(c->st, c->ev_fork, 0));
   double* Zi = nullptr;

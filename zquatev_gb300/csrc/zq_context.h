@@ -19,6 +19,7 @@ struct RefineBuffers {
   void* dev = nullptr;
   size_t bytes = 0;
   bool external = false;  // bound by the caller: never freed or grown here
+  bool digits = false;    // room for the products' digit slices only
   int last_iters = 0;
   double last_emax = 0.0;
   int last_fallback = 0;
@@ -38,6 +39,7 @@ struct Context {
   size_t ws_bytes = 0;
   bool ws_external = false;  // bound by the caller: never freed or grown here
   int dc_n = -1;
+  bool lean = false;         // the workspace of that plan is without the residue merges' scratch
   DcPlan dc;
   // Device flags of the FP64 path (two ints, made by the first solve), raised when a
   // device-side wait ran out: [0] in the last solve, whose eigenvalues are NaN then,
@@ -64,8 +66,8 @@ int context_create(int device, Context** out);
 void context_destroy(Context* c);
 // Device bytes one solve of quaternion size n needs: the FP64 path's workspace
 // and, for refined = true, the refinement buffers on top (with the Ozaki
-// product's slices).
-void solve_workspace_bytes(int n, size_t* fp64_bytes, size_t* refine_bytes);
+// products' residues). lean: the least it runs in, without residues.
+void solve_workspace_bytes(int n, size_t* fp64_bytes, size_t* refine_bytes, bool lean = false);
 // Use caller-owned workspace for the next solves (nullptr/0 unbinds).
 void context_bind(Context* c, void* ws, size_t ws_bytes, void* rws, size_t rws_bytes);
 

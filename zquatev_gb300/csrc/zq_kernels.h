@@ -133,7 +133,8 @@ struct DcPlan {
   int* err = nullptr;        // raised when one of their pipeline waits ran out: the eigenvalues become NaN
   int* tc_err = nullptr;  // run_single: merges of large nodes on the tensor cores (timeout flag) when set
 
-  static size_t workspace_doubles(int n);
+  // lean: without the scratch of the residue merges, which then run on the FP64 pipe
+  static size_t workspace_doubles(int n, bool lean = false);
   size_t forest_doubles() const;  // the same for a built plan of several matrices, without their table
   int build(int n);
   // several tridiagonals at once: orders ns, eigenvalues at eoffs of the
@@ -145,7 +146,7 @@ struct DcPlan {
     return (t + 1 < (int)gemm_off.size() ? gemm_off[t + 1] : (int)gemm_host.size()) - gemm_off[t];
   }
   // mats: the table's place where the workspace is not the plan's alone (null: in the workspace)
-  int upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t st, DcMat* mats = nullptr);
+  int upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t st, DcMat* mats = nullptr, bool lean = false);
   // d (n), e (n-1) on device; lam_out (n) on device; z_out points into the workspace
   // flags (two ints, null: the plan's own, cleared here): raised when a wait of a residue
   // product ran out; the eigenvalues become NaN when [0] is up, which then raises [1] too

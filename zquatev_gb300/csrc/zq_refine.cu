@@ -511,15 +511,17 @@ size_t refine_workspace_bytes(int n, int nbq) {
 // tiles computed, upper filled); +-2 the lower triangle only, the caller fills.
 // prev_slices > 0: the A operand is the previous call's, cut into that many slices.
 // err: device flag of the tensor-core pipelines' timeouts, read once per step.
-static int zgemm_acc(int mode, int opa1, int opb1, int opa2, int opb2, const ZgemmArgs& g, void* ows, size_t ows_bytes,
-                     cudaStream_t st, int slices, int structured, int prev_slices, int* err) {
+static int zgemm_acc(const RefineArgs& ra, int opa1, int opb1, int opa2, int opb2, const ZgemmArgs& g, int slices,
+                     int structured, int prev_slices, int* err) {
   const int sym = structured > 0 ? 1 : (structured < 0 ? -1 : 0);
   const bool fill = structured == 1 || structured == -1;
-  if (mode == 1) {
+  const cudaStream_t st = ra.st;
+  if (ra.mode == 1) {
     OzOpts o{};
     o.slices = slices; o.structured = sym; o.reuse_a = prev_slices > 0; o.prev_slices = prev_slices; o.nofill = fill ? 0 : 1;
     o.err = err;
-    return zgemm_ozaki(opa1, opb1, opa2, opb2, g, ows, ows_bytes, st, o);
+    o.digits = ra.digits;
+    return zgemm_ozaki(opa1, opb1, opa2, opb2, g, ra.ows, ra.ows_bytes, st, o);
   }
   if (int rc = zgemm<double>(opa1, opb1, opa2, opb2, g, 1, st)) return rc;
   if (fill) return structured_fill(g.C, g.ldc, g.m, sym, st);
@@ -760,9 +762,9 @@ int refined_solve(RefineArgs& ra) {
     g = ZgemmArgs{};
     g.m = n2; g.n = n; g.k1 = n; g.A1 = H0; g.lda1 = n2; g.B1 = U; g.ldb1 = ldd;
     g.alpha = one; g.beta = zero; g.C = P1; g.ldc = n2;
-    if (int rc = zgemm_acc(ra.mode, OP_N, OP_N, OP_N, OP_N, g, ra.ows, ra.ows_bytes, st, sl, 0, 0, oz_err)) return rc;
+    if (int rc = zgemm_acc(ra, OP_N, OP_N, OP_N, OP_N, g, sl, 0, 0, oz_err)) return rc;
     g.B1 = V; g.C = P2;
-    if (int rc = zgemm_acc(ra.mode, OP_N, OP_R, OP_N, OP_N, g, ra.ows, ra.ows_bytes, st, sl, 0, sl, oz_err)) return rc;
+    if (int rc = zgemm_acc(ra, OP_N, OP_R, OP_N, OP_N, g, sl, 0, sl, oz_err)) return rc;
     // R = HX - X diag(lamr), lamr the current eigenvalue estimates (the
     // divide-and-conquer values, then the previous step's Rayleigh quotients).
     // S = X^H H X = X^H R + G diag(lamr) for any diagonal lamr; with R small
@@ -775,17 +777,17 @@ int refined_solve(RefineArgs& ra) {
     g = ZgemmArgs{};
     g.m = n; g.n = n; g.k1 = n2; g.A1 = X; g.lda1 = ldd; g.B1 = X; g.ldb1 = ldd;
     g.alpha = one; g.beta = zero; g.C = G1; g.ldc = n;
-    if (int rc = zgemm_acc(ra.mode, OP_C, OP_N, OP_N, OP_N, g, ra.ows, ra.ows_bytes, st, sl, 1, 0, oz_err)) return rc;
+    if (int rc = zgemm_acc(ra, OP_C, OP_N, OP_N, OP_N, g, sl, 1, 0, oz_err)) return rc;
     g.B1 = HX; g.ldb1 = n2; g.C = S1;
-    if (int rc = zgemm_acc(ra.mode, OP_C, OP_N, OP_N, OP_N, g, ra.ows, ra.ows_bytes, st, ss_slices, 2, sl, oz_err)) return rc;
+    if (int rc = zgemm_acc(ra, OP_C, OP_N, OP_N, OP_N, g, ss_slices, 2, sl, oz_err)) return rc;
     // G2 = U^T V - V^T U ; S2 = U^T R_bot - V^T R_top + G2 Lambda
     g = ZgemmArgs{};
     g.m = n; g.n = n; g.k1 = n; g.k2 = n;
     g.A1 = U; g.lda1 = ldd; g.B1 = V; g.ldb1 = ldd; g.A2 = V; g.lda2 = ldd; g.B2 = U; g.ldb2 = ldd; g.s2 = -1.0;
     g.alpha = one; g.beta = zero; g.C = G2; g.ldc = n;
-    if (int rc = zgemm_acc(ra.mode, OP_T, OP_N, OP_T, OP_N, g, ra.ows, ra.ows_bytes, st, sl, -1, 0, oz_err)) return rc;
+    if (int rc = zgemm_acc(ra, OP_T, OP_N, OP_T, OP_N, g, sl, -1, 0, oz_err)) return rc;
     g.B1 = HX + n; g.ldb1 = n2; g.B2 = HX; g.ldb2 = n2; g.C = S2;
-    if (int rc = zgemm_acc(ra.mode, OP_T, OP_N, OP_T, OP_N, g, ra.ows, ra.ows_bytes, st, ss_slices, -2, sl, oz_err)) return rc;
+    if (int rc = zgemm_acc(ra, OP_T, OP_N, OP_T, OP_N, g, ss_slices, -2, sl, oz_err)) return rc;
     ZQ_CUDA(launch_pdl_smem(k_add_glam, dim3(grid_for((int64_t)nn)), dim3(256), 0, st, S1, G1, n, lamr));
     ZQ_LAUNCH_CHECK();
     ZQ_CUDA(launch_pdl_smem(k_add_glam, dim3(grid_for((int64_t)nn)), dim3(256), 0, st, S2, G2, n, lamr));
@@ -836,9 +838,9 @@ int refined_solve(RefineArgs& ra) {
     g.m = n; g.n = n; g.k1 = n; g.k2 = n;
     g.A1 = U; g.lda1 = ldd; g.B1 = Et; g.ldb1 = n; g.A2 = V; g.lda2 = ldd; g.B2 = Eb; g.ldb2 = n; g.s2 = -1.0;
     g.alpha = one; g.beta = zero; g.C = P1; g.ldc = n2;
-    if (int rc = zgemm_acc(ra.mode, OP_N, OP_N, OP_R, OP_N, g, ra.ows, ra.ows_bytes, st, sl_upd, 0, 0, oz_err)) return rc;
+    if (int rc = zgemm_acc(ra, OP_N, OP_N, OP_R, OP_N, g, sl_upd, 0, 0, oz_err)) return rc;
     g.A1 = V; g.A2 = U; g.s2 = 1.0; g.C = P1 + n;
-    if (int rc = zgemm_acc(ra.mode, OP_N, OP_N, OP_R, OP_N, g, ra.ows, ra.ows_bytes, st, sl_upd, 0, 0, oz_err)) return rc;
+    if (int rc = zgemm_acc(ra, OP_N, OP_N, OP_R, OP_N, g, sl_upd, 0, 0, oz_err)) return rc;
     ZQ_CUDA(launch_pdl_smem(k_add_c128, dim3(grid_for((int64_t)n2 * n)), dim3(256), 0, st, P1, n2, X, ldd, n2, n));
     ZQ_LAUNCH_CHECK();
     ra.iters = it + 1;

@@ -400,8 +400,11 @@ long long zq_server_submit(zq_server* s, int n2, double* D, int ld2, double* eig
   if (r->small) {
     r->footprint = (size_t)zq_solve_footprint(n2, 2);
   } else {
-    solve_workspace_bytes(r->n, &r->ws_fp64, &r->ws_ref);
-    r->footprint = r->mat_bytes + r->ws_fp64 + (path_for(r->n) == 1 ? r->ws_ref : 0);
+    // the workspace at its best, or the least where that alone exceeds the budget
+    for (int lean = 0; lean == 0 || (lean == 1 && r->footprint > s->budget); ++lean) {
+      solve_workspace_bytes(r->n, &r->ws_fp64, &r->ws_ref, lean != 0);
+      r->footprint = r->mat_bytes + r->ws_fp64 + (path_for(r->n) == 1 ? r->ws_ref : 0);
+    }
   }
   std::lock_guard<std::mutex> lk(s->mu);
   if (r->footprint > s->budget) {

@@ -612,10 +612,10 @@ static size_t dc_crt_doubles(int n) {
   return crt_dgemm_workspace(h, n, h) / sizeof(double) + 64;
 }
 
-size_t DcPlan::workspace_doubles(int n) {
+size_t DcPlan::workspace_doubles(int n, bool lean) {
   // Z x2, M, lam x2, dmod, es, scal + the per-position DcWork arrays, the matrix table
   const size_t nn = (size_t)n * n;
-  return 3 * nn + 2 * (size_t)n + 2 * (size_t)n + 8 + 16 * (size_t)n + 64 + dc_crt_doubles(n);
+  return 3 * nn + 2 * (size_t)n + 2 * (size_t)n + 8 + 16 * (size_t)n + 64 + (lean ? 0 : dc_crt_doubles(n));
 }
 
 size_t DcPlan::forest_doubles() const {
@@ -728,7 +728,7 @@ int DcPlan::build(const std::vector<int>& ns, const std::vector<long long>& eoff
 }
 
 // Binds device pointers into the descriptor copies and uploads everything.
-int DcPlan::upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t st, DcMat* mats) {
+int DcPlan::upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t st, DcMat* mats, bool lean) {
   base = ws;
   Z[0] = ws; Z[1] = ws + nn; Mb = ws + 2 * nn;
   double* p = ws + 3 * nn;
@@ -747,7 +747,7 @@ int DcPlan::upload(double* ws, DcNode* dnodes, DgemmDesc* ddescs, cudaStream_t s
   w.perm = ip; ip += n; w.nd_col = ip; ip += n; w.df_col = ip; ip += n; w.df_scol = ip; ip += n;
   w.rot_p = ip; ip += n; w.rot_j = ip; ip += n; w.r_orig = ip; ip += n;
   // a single matrix: after the position arrays, on a 256-byte boundary of the workspace
-  crt_ws = mats_host.size() == 1 && n >= DC_CRT_MIN ? ws + ((3 * nn + 20 * (size_t)n + 24 + 31) & ~(size_t)31) : nullptr;
+  crt_ws = !lean && mats_host.size() == 1 && n >= DC_CRT_MIN ? ws + ((3 * nn + 20 * (size_t)n + 24 + 31) & ~(size_t)31) : nullptr;
   nodes_dev = dnodes;
   descs_dev = ddescs;
   // bind pointers: at depth t, A (children) lives in Z[(t+1)&1], output in Z[t&1]
