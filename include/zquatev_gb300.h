@@ -199,9 +199,10 @@ int zq_profile_flops(int cls, double* flops);
  * entry points; every launch is counted on the host right after it is made). */
 long long zq_launch_count(void);
 
-/* Frees the cached device workspace of the current device, the device copy of D
- * that the host-memory entry points keep between calls (n2^2 complex), and the
- * scratch pool's idle memory. */
+/* Frees what the calls keep on the current device between them, after the work in
+ * flight there: the solves', the refinement's and the batches' workspaces, the device
+ * copy of D of the host-memory entry points (n2^2 complex), and the scratch pool's
+ * memory. */
 int zq_release_workspace(void);
 
 /* ---------------------------------------------------------------- serving

@@ -916,6 +916,7 @@ long long zq_launch_count(void) { return zq::g_launches.load(std::memory_order_r
 int zq_release_workspace(void) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return ZQ_ERR_CUDA;
+  cudaDeviceSynchronize();  // what is freed in stream order, after the work in flight, is free now
   scratch_pool_trim();
   std::lock_guard<std::mutex> lk(g_ctx_mu);
   Context* c = g_ctx[dev];
@@ -930,6 +931,12 @@ int zq_release_workspace(void) {
   if (c->hbuf) cudaFree(c->hbuf);
   c->hbuf = nullptr;
   c->hbuf_bytes = 0;
+  if (c->rb.dev) cudaFree(c->rb.dev);
+  c->rb.dev = nullptr;
+  c->rb.bytes = 0;
+  if (c->bb.dev) cudaFree(c->bb.dev);
+  c->bb.dev = nullptr;
+  c->bb.bytes = 0;
   c->forest.release();
   return ZQ_OK;
 }
