@@ -83,7 +83,8 @@ __device__ __forceinline__ Q4<double> q_of(const double2* a, const double2* b, i
 
 // Load [A; B] (lower triangles) and reduce it to tridiagonal form; the reflectors go
 // to the columns of the matrix in global memory. Returns the scale: the matrix is
-// brought to largest entry in [1, 2), so no sum of squares needs its own.
+// brought to largest entry in [1, 2) (subnormal numbers to 2^-52 and more), so no sum
+// of squares needs its own.
 __device__ double small_reduce(double2* A, double2* B, int64_t gld, int n, double* s, const SmallOffsets& o, int lane) {
   const int ld = n | 1;
   double2* ma = reinterpret_cast<double2*>(s);
@@ -112,7 +113,8 @@ __device__ double small_reduce(double2* A, double2* B, int64_t gld, int n, doubl
   }
   int ex = (int)(top >> 52);
   const bool finite = ex < 2047;
-  ex = ex < 1 ? 1023 : (ex > 2045 ? 2045 : ex);  // zero (or subnormal) matrices stay as they are
+  // a zero matrix stays as it is; one of subnormal numbers comes as near as 2^1022 takes it
+  ex = top == 0ull ? 1023 : (ex < 1 ? 1 : (ex > 2045 ? 2045 : ex));
   // (a matrix that holds an Inf or a NaN becomes NaN as a whole)
   const double scale = __hiloint2double(ex << 20, 0);
   const double inv = finite ? __hiloint2double((2046 - ex) << 20, 0) : __longlong_as_double(0x7ff8000000000000ll);
