@@ -28,6 +28,7 @@
 #include "zq_common.cuh"
 #include "zq_context.h"
 #include "zq_kernels.h"
+#include "zq_recip.cuh"
 #include "zq_resident.h"
 
 #include <algorithm>
@@ -166,8 +167,8 @@ __device__ __forceinline__ unsigned long long warp_max_bits(unsigned long long v
 // relative to max |lambda|.
 //
 // FP64 instructions bound it, so magnitudes are compared as integers (bit patterns
-// without the sign) and the gap's reciprocal is the approximate instruction with one
-// cubic step. max |lambda| is gathered by the whole block: one thread's chain over
+// without the sign) and the gap's reciprocal is that of zq_recip.cuh (matrices that FP32
+// can hold have gaps of at least 1e-61). max |lambda| is gathered by the whole block: one thread's chain over
 // the 1024 partials took longer than the rest up to n ~ 1000 (n = 750: 182 us a call).
 __global__ void k_oa_build_e(const double2* __restrict__ S1, const double2* __restrict__ S2,
                              const double2* __restrict__ G1, const double2* __restrict__ G2, int64_t ld, int n,
@@ -216,13 +217,7 @@ __global__ void k_oa_build_e(const double2* __restrict__ S1, const double2* __re
     double2 e1, e2;
     bool cl = false;
     // uncoupled equal eigenvalues (0 <= 0) need no correction: no reciprocal of zero
-    double igap = 0.0;
-    if (i != j && gap != 0.0) {
-      double y;
-      asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(gap));
-      const double h = fma(-gap, y, 1.0);
-      igap = fma(y, fma(h, h, h), y);
-    }
+    const double igap = i != j && gap != 0.0 ? recip(gap) : 0.0;
     if (i == j) {
       e1 = make_double2(0.5 * r1.x, 0.5 * r1.y);
     } else if (a1 <= bound) {

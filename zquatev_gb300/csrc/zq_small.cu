@@ -22,6 +22,7 @@
 #include "zq_common.cuh"
 #include "zq_kernels.h"
 #include "zq_quat.cuh"
+#include "zq_recip.cuh"
 
 namespace zq {
 namespace {
@@ -52,14 +53,7 @@ __host__ __device__ inline SmallOffsets small_offsets(int n) {
 
 __device__ __forceinline__ int exponent_of(double v) { return (__double2hiint(v) >> 20) & 0x7ff; }
 
-// 1 / sqrt(q) for q in [2^-900, 2^900]: the approximation instruction, then a step of
-// third order (relative error 2^-20 -> below 2^-58 before the last rounding)
-__device__ __forceinline__ double small_rsqrt(double q) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(q));
-  const double h = fma(-(q * y), y, 1.0);
-  return fma(y * h, fma(0.375, h, 0.5), y);
-}
+// the range of recip_sqrt
 __device__ __forceinline__ bool mid_range(double q) {
   const int e = exponent_of(q);
   return e > 123 && e < 1923;
@@ -281,7 +275,7 @@ __device__ int small_sweeps(int n, double* s, const SmallOffsets& o, QlState& q)
       const double ff = sn * ei, bb = c * ei, qq = fma(ff, ff, g * g);
       double r;
       if (mid_range(qq)) {
-        const double y = small_rsqrt(qq);
+        const double y = recip_sqrt(qq);
         r = qq * y; sn = ff * y; c = g * y;
       } else {
         r = hypot(ff, g);

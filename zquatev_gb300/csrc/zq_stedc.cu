@@ -25,6 +25,7 @@
 //       gemm     - Z_node = blockdiag(Z1, Z2) * M  (grouped DGEMM).
 #include "zq_common.cuh"
 #include "zq_kernels.h"
+#include "zq_recip.cuh"
 #include "zq_crt.h"
 #include "zq_tc32.h"
 
@@ -248,17 +249,11 @@ __global__ void __launch_bounds__(256) k_dc_prepare(DcNode* nodes, DcWork w, con
 // iteration's control flow stays warp-uniform)
 //
 // FP64 instructions bound it (K^2 poles and roots, ~7 iterations), so each pole
-// takes ten: the products rho z^2 are formed once (w.sz), the reciprocal is
-// 1/del from the approximate instruction and one cubically convergent Newton
-// step (relative error below 2^-52), and the two sides of the root share one
+// takes ten: the products rho z^2 are formed once (w.sz), the reciprocals of the
+// distances are those of zq_recip.cuh (kept poles of a scaled node lie 1e-15 and
+// more apart, their roots 1e-31 and more from them: in its range), and the two sides of the root share one
 // accumulation loop each. The root is first approached in FP32 (dc_approach),
 // whose instructions cost a sixteenth, so that two or three FP64 iterations remain.
-__device__ __forceinline__ double dc_recip(double d) {
-  double y;
-  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
-  const double e = fma(-d, y, 1.0);
-  return fma(y, fma(e, e, e), y);
-}
 // The step of the two-pole rational model around tau, for root i between the
 // poles at distances di, dj (i = K - 1: one pole): f the function's value, dpsi,
 // dphi the derivatives of its two sums. False: no step.
@@ -349,7 +344,7 @@ __global__ void __launch_bounds__(128) k_dc_secular(const DcNode* nodes, int cnt
     const double gap = D[i + 1] - D[i];
     const double mid = 0.5 * gap;
     double fs = 0.0;
-    for (int k = lane; k < K; k += 32) fs = fma(rz[k], dc_recip((D[k] - D[i]) - mid), fs);
+    for (int k = lane; k < K; k += 32) fs = fma(rz[k], recip((D[k] - D[i]) - mid), fs);
     const double f = 1.0 + warp_sum(fs);
     if (f >= 0.0) { o = i; lo = 0.0; hi = mid; }
     else { o = i + 1; lo = -mid; hi = 0.0; }
@@ -366,14 +361,14 @@ __global__ void __launch_bounds__(128) k_dc_secular(const DcNode* nodes, int cnt
     double psi = 0.0, phi = 0.0, dpsi = 0.0, dphi = 0.0;
 #pragma unroll 4
     for (int k = lane; k <= i; k += 32) {
-      const double inv = dc_recip((D[k] - Do) - tau);
+      const double inv = recip((D[k] - Do) - tau);
       const double t = rz[k] * inv;
       psi += t;
       dpsi = fma(t, inv, dpsi);
     }
 #pragma unroll 4
     for (int k = above; k < K; k += 32) {
-      const double inv = dc_recip((D[k] - Do) - tau);
+      const double inv = recip((D[k] - Do) - tau);
       const double t = rz[k] * inv;
       phi += t;
       dphi = fma(t, inv, dphi);
@@ -428,7 +423,7 @@ __global__ void __launch_bounds__(128) k_dc_zhat(const DcNode* nodes, int cnt, D
   for (int j = lane; j < K - 1; j += 32) {
     const double num = (D[O[j]] - Dk) + T[j];  // lambda_j - D_k
     const double den = (j < k) ? (D[j] - Dk) : (D[j + 1] - Dk);
-    prod *= num * dc_recip(den);
+    prod *= num * recip(den);
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) prod *= __shfl_xor_sync(0xffffffffu, prod, off);
@@ -476,7 +471,7 @@ __global__ void __launch_bounds__(128) k_dc_vectors(const DcNode* nodes, int cnt
     double ss = 0.0;
     for (int k = tid; k < K; k += blockDim.x) {
       const double del = (D[k] - Do) - t;
-      const double vk = w.zhat[a + k] * dc_recip(del);
+      const double vk = w.zhat[a + k] * recip(del);
       ss += vk * vk;
     }
     ss = warp_sum(ss);
@@ -486,7 +481,7 @@ __global__ void __launch_bounds__(128) k_dc_vectors(const DcNode* nodes, int cnt
     const double inv = 1.0 / nrm;
     for (int k = tid; k < K; k += blockDim.x) {
       const double del = (D[k] - Do) - t;
-      col[w.nd_col[a + k]] = (ZT)(w.zhat[a + k] * dc_recip(del) * inv);
+      col[w.nd_col[a + k]] = (ZT)(w.zhat[a + k] * recip(del) * inv);
     }
   } else {
     if (tid == 0) col[w.df_scol[a + (s - K)]] = (ZT)1;
