@@ -5,7 +5,8 @@
 // accumulation).
 //
 //   * Every row of A (column of B) is scaled by a power of two above its
-//     largest entry and rounded to integers of `bits` bits (55 for FP64).
+//     largest entry and rounded to integers of `bits` bits (55 for complex FP64
+//     products, 60 for real ones).
 //   * For each of L pairwise coprime moduli p <= 253 the integers are reduced to
 //     symmetric residues, |r| <= 127: exact in bf16, products below 2^14, so
 //     sums of 512 are exact in FP32; they are emptied into int32 and reduced
@@ -59,8 +60,8 @@ constexpr int CB_THREADS = 320;
 constexpr int CB_SMEM = 1024 + CB_STAGES * CB_STAGE + 256 + 16384;  // slack: see UM_SMEM (zq_ozaki_umma.cu)
 constexpr int CB_GROUP = 8;           // row tiles per group of the job order
 
-// per modulus: 2^14, 2^28, 2^42 mod p (symmetric), p, 1/p
-struct CrtMod { float c1, c2, c3, p, ip; };
+// per modulus: 2^14, 2^28, 2^42, 2^56 mod p (symmetric), p, 1/p
+struct CrtMod { float c1, c2, c3, c4, p, ip; };
 struct CrtMods { CrtMod v[CRT_MAX]; };
 
 constexpr int crt_sym(long long v, int p) {
@@ -75,6 +76,7 @@ constexpr CrtMods crt_mods() {
     m.v[l].c1 = (float)crt_sym(1ll << 14, p);
     m.v[l].c2 = (float)crt_sym(1ll << 28, p);
     m.v[l].c3 = (float)crt_sym(1ll << 42, p);
+    m.v[l].c4 = (float)crt_sym(1ll << 56, p);
     m.v[l].p = (float)p;
     m.v[l].ip = 1.0f / (float)p;
   }
@@ -85,8 +87,9 @@ __constant__ CrtMods g_crt_mods = crt_mods();
 // ------------------------------------------------------------------ residues
 __device__ __forceinline__ float crt_rint(float v) { return __fadd_rn(__fadd_rn(v, 12582912.f), -12582912.f); }
 
-// v 2^(bits - e) rounded to an integer, as four 14-bit limbs with its sign
-__device__ __forceinline__ void crt_limbs(double v, int e, int bits, float (&f)[4]) {
+// v 2^(bits - e) rounded to an integer, as four (56 bits) or five 14-bit limbs with its sign
+template <int NL>
+__device__ __forceinline__ void crt_limbs(double v, int e, int bits, float (&f)[NL]) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v);
   const unsigned neg = (unsigned)(b >> 32) & 0x80000000u;
   const int ex = (int)((b >> 52) & 0x7ff);
@@ -99,12 +102,15 @@ __device__ __forceinline__ void crt_limbs(double v, int e, int bits, float (&f)[
     else if (sh > -55) V = (mant + (1ull << (-sh - 1))) >> (-sh);
   }
 #pragma unroll
-  for (int q = 0; q < 4; ++q)  // 0x4B000000 | d is 2^23 + d
+  for (int q = 0; q < NL; ++q)  // 0x4B000000 | d is 2^23 + d
     f[q] = __uint_as_float(__float_as_uint(__uint_as_float(0x4B000000u | ((unsigned)(V >> (14 * q)) & 0x3fffu)) - 8388608.f) ^ neg);
 }
-// symmetric residue of the limbs' integer (all steps exact: the sum is below 2^23)
-__device__ __forceinline__ float crt_residue(const float (&f)[4], const CrtMod& m) {
-  const float x = fmaf(f[3], m.c3, fmaf(f[2], m.c2, fmaf(f[1], m.c1, f[0])));
+// symmetric residue of the limbs' integer (all steps exact: the sum is below 2^23, the
+// fifth limb of 60 bits below 2^4)
+template <int NL>
+__device__ __forceinline__ float crt_residue(const float (&f)[NL], const CrtMod& m) {
+  float x = fmaf(f[3], m.c3, fmaf(f[2], m.c2, fmaf(f[1], m.c1, f[0])));
+  if constexpr (NL > 4) x = fmaf(f[4], m.c4, x);
   return fmaf(-crt_rint(x * m.ip), m.p, x);
 }
 __device__ __forceinline__ unsigned crt_pack(float a, float b) {
@@ -164,7 +170,8 @@ __global__ void __launch_bounds__(256, 3) k_crt_split(CrtSide s, bool is_a, int 
   const int g = lane & 7, r = warp * 4 + (lane >> 3);
   const int idx = i0 + r;
   const int e = idx < count ? exps[idx] : -1100;
-  float fr[8][4], fi[CPLX ? 8 : 1][4];
+  constexpr int NL = CPLX ? 4 : 5;  // complex products of up to 55 bits, real ones of 60
+  float fr[8][NL], fi[CPLX ? 8 : 1][NL];
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
     const E v = tile[r][8 * g + (u ^ g)];
@@ -665,7 +672,11 @@ int crt_join(const CrtShape& sh, const void* r, int m, int n, int bits, const in
   return ZQ_OK;
 }
 
-constexpr int CRT_FP64_BITS = 55;
+// Bits of a real operand's largest entry. A double's 53 and seven more: entries below
+// the largest of their row or column lose only what lies 2^-60 under it (with 55 bits
+// localised eigenvectors came out up to 1.5 times less orthogonal than FP64 merges
+// leave them, with 60 as orthogonal; one modulus in 16 more)
+constexpr int CRT_FP64_BITS = 60;
 
 size_t crt_dgemm_workspace(int m, int n, int k) {
   const int L = crt_moduli(CRT_FP64_BITS, k);
