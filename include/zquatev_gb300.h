@@ -46,7 +46,7 @@ int zquatev_device(int n2, double* dD, int ld2, double* deig, void* stream);
 int zquatev_values_device(int n2, double* dD, int ld2, double* deig, void* stream);
 
 /* Real symmetric tridiagonal eigensolver (the stage that replaces zhbev at
- * zquatev.cc:74-84): d (n), e (n-1, the off-diagonal), lam (n, ascending) and
+ * zquatev.cc:74-84): d (n), e (n-1, the off-diagonal, of either sign), lam (n, ascending) and
  * Z (n x ldz, column-major eigenvectors) all in device memory. */
 int zq_stedc_device(int n, const double* d, const double* e, double* lam, double* Z, int ldz, void* stream);
 

@@ -817,10 +817,9 @@ int zq_stedc_device(int n, const double* d, const double* e, double* lam, double
   if (int rc = ensure_plan(c, n)) return rc;
   ZQ_CUDA(cudaEventRecord(c->ev_fork, st));
   ZQ_CUDA(cudaStreamWaitEvent(c->st, c->ev_fork, 0));
-  double* Zi = nullptr;
-  if (int rc = c->dc.run(d, e, lam, Zi, c->st)) return rc;
-  ZQ_CUDA(cudaMemcpy2DAsync(Z, sizeof(double) * (size_t)ldz, Zi, sizeof(double) * n, sizeof(double) * n, n,
-                            cudaMemcpyDeviceToDevice, c->st));
+  const Layout L = layout_for(n, NBMAX, g_nbq, c->dc.num_nodes(), c->dc.num_descs(), c->lean);
+  double* sm = reinterpret_cast<double*>(reinterpret_cast<char*>(c->ws) + L.tri);  // 12 n doubles, unused here
+  if (int rc = c->dc.run_signed(d, e, lam, Z, ldz, sm, sm + n, c->st)) return rc;
   ZQ_CUDA(cudaEventRecord(c->ev_join, c->st));
   ZQ_CUDA(cudaStreamWaitEvent(st, c->ev_join, 0));
   return ZQ_OK;

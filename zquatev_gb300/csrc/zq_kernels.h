@@ -157,6 +157,9 @@ struct DcPlan {
   int run_forest(const double* d, const double* e, double* eig, int* info, cudaStream_t st);
   // same tree with Z and the merge products in FP32 (eigenvalues and the
   // secular equation stay FP64): the refined path's decomposition
+  // the same for couplings e of either sign, Z stored at ldz: e_abs and signs are n doubles of scratch each
+  int run_signed(const double* d, const double* e, double* lam_out, double* Z_out, int64_t ldz, double* e_abs,
+                 double* signs, cudaStream_t st);
   int run_single(const double* d, const double* e, double* lam_out, float*& z_out, cudaStream_t st);
   // descriptor area bytes for upload(): double descriptors + 2 spare + float descriptors
   static size_t desc_bytes(size_t ndescs) {

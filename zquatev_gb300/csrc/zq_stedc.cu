@@ -588,6 +588,39 @@ __global__ void __launch_bounds__(256) k_dc_merge(const DcNode* nodes, int cnt, 
   }
 }
 
+// Couplings of either sign: with S the diagonal of the couplings' running signs, S T S
+// has their moduli (the tear needs rho > 0) and the same eigenvalues. One block.
+constexpr int DC_SIGN_T = 1024;
+__global__ void __launch_bounds__(DC_SIGN_T) k_dc_signs(const double* __restrict__ e, int n, double* __restrict__ e_abs,
+                                                        double* __restrict__ signs) {
+  pdl_wait();
+  __shared__ unsigned s_odd[DC_SIGN_T / 32];  // per warp: which threads' chunks hold an odd number of negative couplings
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int per = (n + DC_SIGN_T - 1) / DC_SIGN_T, i0 = min(tid * per, n), i1 = min(i0 + per, n);
+  bool odd = false;  // chunk: positions i0 .. i1, the coupling e[i - 1] leads to position i
+  for (int i = i0; i < i1; ++i) odd ^= i > 0 && e[i - 1] < 0.0;
+  const unsigned mask = __ballot_sync(0xffffffffu, odd);
+  if (lane == 0) s_odd[warp] = mask;
+  __syncthreads();
+  int before = __popc(mask & ((1u << lane) - 1u));
+  for (int w = 0; w < warp; ++w) before += __popc(s_odd[w]);
+  bool neg = before & 1;
+  for (int i = i0; i < i1; ++i) {
+    neg ^= i > 0 && e[i - 1] < 0.0;
+    signs[i] = neg ? -1.0 : 1.0;
+    if (i > 0) e_abs[i - 1] = fabs(e[i - 1]);
+  }
+}
+// Z_out = S Z
+__global__ void __launch_bounds__(256) k_dc_signed_copy(const double* __restrict__ Z, int n, const double* __restrict__ signs,
+                                                        double* __restrict__ Z_out, int64_t ldz) {
+  pdl_wait();
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= n) return;
+  const double s = signs[r];
+  for (int c = blockIdx.y; c < n; c += gridDim.y) Z_out[r + (int64_t)c * ldz] = s * Z[r + (int64_t)c * n];
+}
+
 __global__ void k_dc_setrho(DcNode* nodes, int cnt, const double* es) {
   pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -909,6 +942,19 @@ int DcPlan::run(const double* d, const double* e, double* lam_out, double*& z_ou
   if (n <= 0) return ZQ_OK;
   if (int rc = dc_run<double>(*this, d, e, lam_out, Z, Mb, descs_dev, st, nullptr, flags)) return rc;
   z_out = Z[0];
+  return ZQ_OK;
+}
+
+int DcPlan::run_signed(const double* d, const double* e, double* lam_out, double* Z_out, int64_t ldz, double* e_abs,
+                       double* signs, cudaStream_t st) {
+  if (n <= 0) return ZQ_OK;
+  ZQ_CUDA(launch_pdl_smem(k_dc_signs, dim3(1), dim3(DC_SIGN_T), 0, st, e, n, e_abs, signs));
+  ZQ_LAUNCH_CHECK();
+  double* Zi = nullptr;
+  if (int rc = run(d, e_abs, lam_out, Zi, st)) return rc;
+  ZQ_CUDA(launch_pdl_smem(k_dc_signed_copy, dim3((unsigned)ceil_div(n, 256), (unsigned)std::min(n, 8192)), dim3(256), 0, st, Zi, n, signs,
+                          Z_out, ldz));
+  ZQ_LAUNCH_CHECK();
   return ZQ_OK;
 }
 
