@@ -68,10 +68,31 @@ BatchForest::~BatchForest() { release(); }
 void BatchForest::release() {
   for (Chunk* c : chunks_) delete c;
   chunks_.clear();
-  if (dev_) cudaFree(dev_);
+  drop();
+  items_.clear();
+}
+
+void BatchForest::drop() {
+  if (dev_ && pooled_) cudaFreeAsync(dev_, st_);
+  else if (dev_) cudaFree(dev_);
   dev_ = nullptr;
   bytes_ = 0;
-  items_.clear();
+}
+
+int BatchForest::reserve(size_t bytes, cudaStream_t st) {
+  if (bytes_ >= bytes) return ZQ_OK;
+  drop();
+  st_ = st;
+  const cudaError_t e = pooled_ ? cudaMallocAsync(&dev_, bytes, st) : cudaMalloc(&dev_, bytes);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    dev_ = nullptr;
+    release();
+    set_error_message("batch: device allocation failed");
+    return ZQ_ERR_NOMEM;
+  }
+  bytes_ = bytes;
+  return ZQ_OK;
 }
 
 int BatchForest::build(const std::vector<ForestItem>& items, cudaStream_t st) {
@@ -151,19 +172,7 @@ int BatchForest::build(const std::vector<ForestItem>& items, cudaStream_t st) {
     scratch = std::max(scratch, up(sizeof(double) * 11 * N) + c->tri_ws_bytes + up(sizeof(double) * c->dc.forest_doubles()));
     i0 = i1;
   }
-  const size_t total = tables + scratch;
-  if (bytes_ < total) {
-    if (dev_) cudaFree(dev_);
-    dev_ = nullptr;
-    bytes_ = 0;
-    if (cudaMalloc(&dev_, total) != cudaSuccess) {
-      cudaGetLastError();
-      release();
-      set_error_message("batch: device allocation failed");
-      return ZQ_ERR_NOMEM;
-    }
-    bytes_ = total;
-  }
+  if (int rc = reserve(tables + scratch, st)) return rc;
   char* p = reinterpret_cast<char*>(dev_);
   auto take = [&](size_t b) { char* q = p; p += up(b); return q; };
   info_ = reinterpret_cast<int*>(take(sizeof(int) * items.size()));

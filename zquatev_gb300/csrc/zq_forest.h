@@ -36,7 +36,12 @@ struct ForestItem {
 // of the same object on another stream.
 class BatchForest {
  public:
+  // pooled: the device memory comes from the device's stream-ordered pool, in the order
+  // of the stream given to build(), instead of cudaMalloc
+  explicit BatchForest(bool pooled = false) : pooled_(pooled) {}
   ~BatchForest();
+  BatchForest(const BatchForest&) = delete;
+  BatchForest& operator=(const BatchForest&) = delete;
   int build(const std::vector<ForestItem>& items, cudaStream_t st);
   bool matches(const std::vector<ForestItem>& items) const { return items == items_; }
   // build()'s code where the batch cannot run jointly (no room for its scratch, no cluster
@@ -52,9 +57,13 @@ class BatchForest {
   void release();
 
  private:
+  int reserve(size_t bytes, cudaStream_t st);
+  void drop();
   struct Chunk;                    // a part of the batch; the parts run one after another on the same scratch
   std::vector<ForestItem> items_;
   std::vector<Chunk*> chunks_;
+  const bool pooled_;
+  cudaStream_t st_ = nullptr;  // pooled: the memory's stream
   void* dev_ = nullptr;
   size_t bytes_ = 0;
   int* info_ = nullptr;

@@ -217,14 +217,12 @@ void lane_loop(Server* s, Context* c) {
   }
 }
 
-constexpr size_t FOREST_KEEP = (size_t)64 << 20;  // scratch a batch worker keeps between batches
-
 void batch_loop(Server* s, Context* c) {
   cudaSetDevice(s->device);
   const size_t tb = batched_task_bytes();
   std::vector<char> htasks;
   std::vector<int> hinfo;
-  BatchForest forest;  // the orders above a warp's, all together (a CTA each: 10 ms at n = 48)
+  BatchForest forest(true);  // the orders above a warp's, all together (a CTA each: 10 ms at n = 48)
   for (;;) {
     std::vector<Req*> batch, all;
     {
@@ -255,7 +253,7 @@ void batch_loop(Server* s, Context* c) {
       items.push_back(ForestItem{r->n, r->n2, (long long)(r->dD - D0), (long long)(r->deig - E0)});
     }
     int rc = ZQ_OK;
-    if (!items.empty() && !forest.matches(items)) {
+    if (!items.empty()) {
       rc = forest.build(items, c->st);
       if (BatchForest::declined(rc)) {  // no room for it: a CTA each
         rc = ZQ_OK;
@@ -303,11 +301,10 @@ void batch_loop(Server* s, Context* c) {
       for (size_t q = 0; q < all.size() && rc == ZQ_OK; ++q) rc = copy_back(all[q], c->st);
       cudaFreeAsync(mem, c->st);
     }
+    forest.release();  // its tables and scratch are within the requests' footprints: not kept beyond them
     for (Req* r : all) cudaFreeAsync(r->dD, c->st);
     const cudaError_t e = cudaStreamSynchronize(c->st);
     if (rc == ZQ_OK && e != cudaSuccess) { set_last_error(e, "server batch", __FILE__, __LINE__); rc = ZQ_ERR_CUDA; }
-    // its tables and scratch are within the finished requests' footprints: not kept beyond them
-    if (forest.bytes() > FOREST_KEEP) forest.release();
     for (size_t q = 0; q < joint.size(); ++q) finish(s, joint[q], rc != ZQ_OK ? rc : jinfo[q], 2);
     for (int q = 0; q < k; ++q) finish(s, batch[q], rc != ZQ_OK ? rc : hinfo[q], 2);
   }
