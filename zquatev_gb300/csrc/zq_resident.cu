@@ -779,37 +779,28 @@ __device__ bool reduce_matrix(const TriTask<R>& tk, const TriGroup<R>& gr, int r
 template <typename R, int T, bool CL>
 __global__ void __launch_bounds__(RT_THREADS, 1) k_tri_resident(const TriArgs<R> a) {
   extern __shared__ __align__(16) unsigned char rt_smem[];
-  __shared__ int s_task;
-  __shared__ int s_ok;
+  constexpr int LPR = sizeof(R) == 8 ? 32 : 8;
   const int group = blockIdx.x / a.G, rank = blockIdx.x % a.G;
   const TriGroup<R> gr = tri_group<R>(a.ws + (size_t)group * a.ws_stride, a.G, a.m_max, T);
   unsigned target = 0;
-  bool ok = true;
-  if (!a.tasks) {
-    ok = reduce_matrix<R, T, sizeof(R) == 8 ? 32 : 8, CL>(a.one, gr, rank, a.G, rt_smem, target, a.err, a.limit);
-    if (!ok && rank == 0 && threadIdx.x == 0) a.one.d[a.one.k0] = __longlong_as_double(0x7ff8000000000000ll);
-    return;
-  }
-  // a queue of matrices: the group's first CTA takes one for all of them
-  for (int it = 0;; ++it) {
-    if (rank == 0 && threadIdx.x == 0) gr.slot[it & 1] = atomicAdd(a.queue, 1);
-    if constexpr (CL) cluster_barrier();
-    else if (!group_barrier(gr.counter, target, a.G, gr.abort, a.err, a.limit, &s_ok)) return;
-    if (threadIdx.x == 0) s_task = __ldcg(gr.slot + (it & 1));
-    __syncthreads();
-    const int t = s_task;
-    if (t >= a.ntasks) return;
-    TriTask<R> tk = a.tasks[t];
-    if (!tk.M) tk.M = a.base + tk.off;
-    if (tk.n > 0) {
-      ok = reduce_matrix<R, T, sizeof(R) == 8 ? 32 : 8, CL>(tk, gr, rank, a.G, rt_smem, target, a.err, a.limit);
-      if (!ok) {
-        if (rank == 0 && threadIdx.x == 0) tk.d[0] = __longlong_as_double(0x7ff8000000000000ll);
-        return;
-      }
+  if constexpr (CL) {
+    // a queue of matrices: each cluster's first CTA takes one for all of them
+    __shared__ int s_task;
+    for (int it = 0; a.tasks; ++it) {
+      if (rank == 0 && threadIdx.x == 0) gr.slot[it & 1] = atomicAdd(a.queue, 1);
+      cluster_barrier();
+      if (threadIdx.x == 0) s_task = __ldcg(gr.slot + (it & 1));
+      __syncthreads();
+      const int t = s_task;
+      if (t >= a.ntasks) return;
+      TriTask<R> tk = a.tasks[t];
+      if (!tk.M) tk.M = a.base + tk.off;
+      if (tk.n > 0) reduce_matrix<R, T, LPR, true>(tk, gr, rank, a.G, rt_smem, target, a.err, a.limit);
+      __syncthreads();
     }
-    __syncthreads();
   }
+  if (!reduce_matrix<R, T, LPR, CL>(a.one, gr, rank, a.G, rt_smem, target, a.err, a.limit) && rank == 0 && threadIdx.x == 0)
+    a.one.d[a.one.k0] = __longlong_as_double(0x7ff8000000000000ll);
 }
 
 template <typename R>

@@ -26,12 +26,12 @@ struct TriGroup {
   int* slot;          // the task taken from the queue (two, in turn)
   double *cpart, *npart;  // per CTA: partials of c and of |x|^2
   double* q2;             // |x_1|^2 of the column
-  Q4<R>*g1, *x, *y, *col, *part;
+  Q4<R>*x, *y, *col, *part;
 };
 
 inline __host__ __device__ size_t tri_group_bytes(int G, int m, int T, size_t real_bytes) {
   const size_t nt = (size_t)((m + T - 1) / T);
-  return 256 + sizeof(double) * 3 * (size_t)G + 4 * real_bytes * (8 + 3 * (size_t)m + nt * (size_t)m) + 256;
+  return 256 + sizeof(double) * 2 * (size_t)G + 4 * real_bytes * (3 * (size_t)m + nt * (size_t)m) + 256;
 }
 
 template <typename R>
@@ -43,8 +43,7 @@ __device__ __forceinline__ TriGroup<R> tri_group(unsigned char* base, int G, int
   g.cpart = reinterpret_cast<double*>(base + 256);
   g.npart = g.cpart + G;
   g.q2 = reinterpret_cast<double*>(base + 128);
-  g.g1 = reinterpret_cast<Q4<R>*>(base + ((256 + sizeof(double) * 3 * (size_t)G + 31) & ~(size_t)31));
-  g.x = g.g1 + 8;
+  g.x = reinterpret_cast<Q4<R>*>(base + ((256 + sizeof(double) * 2 * (size_t)G + 31) & ~(size_t)31));
   g.y = g.x + m;
   g.col = g.y + m;
   g.part = g.col + m;
