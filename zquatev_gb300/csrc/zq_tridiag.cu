@@ -107,7 +107,10 @@ __device__ bool head_math(const TridiagView<R>& v, int j, int nnp, double& f, do
   sq = warp_sum(sq);
   const double nu = sc * sqrt(sq);
   if (lane != 0) return false;
-  const double q1 = sqrt(qa0 * qa0 + qa1 * qa1 + qb0 * qb0 + qb1 * qb1);
+  // |x_1| in units of the largest entry: its squares stay in range at any scale of the matrix
+  const double inv = sc > 0.0 ? 1.0 / sc : 0.0;
+  const double a0 = qa0 * inv, a1 = qa1 * inv, b0 = qb0 * inv, b1 = qb1 * inv;
+  const double q1 = sc * sqrt(a0 * a0 + a1 * a1 + b0 * b0 + b1 * b1);
   f = 0.0;
   m[0] = m[1] = m[2] = m[3] = 0.0;
   ee[0] = qa0; ee[1] = qa1; ee[2] = qb0; ee[3] = qb1;   // L == 1: the entry itself is e_j
