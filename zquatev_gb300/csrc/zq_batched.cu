@@ -102,7 +102,10 @@ __device__ void batch_solve_group(const BatchTask& tk, const BatchArgs& a, doubl
     if (tid == 0) {
       const double nu = mx * sqrt(ssq);
       const double2 qa = A[j + 1 + (int64_t)j * ld], qb = B[j + 1 + (int64_t)j * ld];
-      const double q1 = sqrt(qa.x * qa.x + qa.y * qa.y + qb.x * qb.x + qb.y * qb.y);
+      // (in units of the largest entry, so that no square leaves the range of doubles)
+      const double inv = mx > 0.0 ? 1.0 / mx : 0.0;
+      const double u0 = qa.x * inv, u1 = qa.y * inv, u2 = qb.x * inv, u3 = qb.y * inv;
+      const double q1 = mx * sqrt(u0 * u0 + u1 * u1 + u2 * u2 + u3 * u3);
       double f = 0.0, m0 = 0, m1 = 0, m2 = 0, m3 = 0;
       double ee0 = qa.x, ee1 = qa.y, ee2 = qb.x, ee3 = qb.y;
       if (L >= 2) {
@@ -210,8 +213,10 @@ __device__ void batch_solve_group(const BatchTask& tk, const BatchArgs& a, doubl
     double a0 = 1.0, a1 = 0.0, b0 = 0.0, b1 = 0.0;
     phi[0] = a0; phi[1] = a1; phi[2] = b0; phi[3] = b1;
     for (int k = 0; k + 1 < n; ++k) {
-      const double ea0 = e4[4 * k], ea1 = e4[4 * k + 1], eb0 = e4[4 * k + 2], eb1 = e4[4 * k + 3];
-      const double nrm = sqrt(ea0 * ea0 + ea1 * ea1 + eb0 * eb0 + eb1 * eb1);
+      double ea0 = e4[4 * k], ea1 = e4[4 * k + 1], eb0 = e4[4 * k + 2], eb1 = e4[4 * k + 3];
+      const double em = fmax(fmax(fabs(ea0), fabs(ea1)), fmax(fabs(eb0), fabs(eb1)));
+      if (em > 0.0) { const double inv = 1.0 / em; ea0 *= inv; ea1 *= inv; eb0 *= inv; eb1 *= inv; }
+      const double nrm = em * sqrt(ea0 * ea0 + ea1 * ea1 + eb0 * eb0 + eb1 * eb1);
       offd[k] = nrm;
       if (nrm > 0.0) {
         const double na0 = (ea0 * a0 - ea1 * a1) - (eb0 * b0 + eb1 * b1);
@@ -244,7 +249,7 @@ __device__ void batch_solve_group(const BatchTask& tk, const BatchArgs& a, doubl
         int m = l;
         for (; m < n - 1; ++m) {
           const double dd = fabs(d[m]) + fabs(d[m + 1]);
-          if (fabs(offd[m]) <= eps * dd || fabs(offd[m]) < 1e-300) break;
+          if (fabs(offd[m]) <= eps * dd || fabs(offd[m]) < 2.2250738585072014e-308) break;
         }
         s_done = (m == l) || (iter >= 60);
         if (iter >= 60 && m != l) sflag[0] += 1;
