@@ -323,12 +323,13 @@ __device__ float dc_approach(const float2* D, const float* rz, int K, int i, int
   }
   return tau;
 }
-// Nodes with more poles than this start from the FP32 root (with it at every order
-// n = 3000 took 5.0 ms instead of 6.4, with this line 5.4). Smaller ones start in the middle of the gap: with an FP32 start there,
-// whose time no longer matters, the eigenvalues of Toeplitz matrices (equal halves, so
-// most poles coincide) had errors of 2.9e-16 of the norm (root mean square, n = 40 to
-// 4000) instead of 2.2e-16; other matrices' are no different.
-constexpr int DC_APPROACH_MIN = 64;
+// Nodes with more poles than this start from the FP32 root (n = 3000: 5.2 ms; from the
+// middle of the gap at every order 1.4 ms more). One or two poles start in the middle:
+// there the FP64 iteration hits the roots of equal leaves, as of a Toeplitz matrix,
+// exactly, and an error made there goes up the whole tree (root mean square of such
+// eigenvalues' errors over the norm, n = 40 to 4000: 2.9e-16 with an FP32 start, 2.1e-16
+// without; lines at 4, 8 and 64 poles 2.3e-16, 2.3e-16 and 2.2e-16 at up to 5% more time).
+constexpr int DC_APPROACH_MIN = 2;
 __global__ void __launch_bounds__(128) k_dc_secular(const DcNode* nodes, int cnt, DcWork w) {
   pdl_wait();
   const int pos = (int)((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5);
