@@ -533,7 +533,7 @@ def batched_case(count: int, fp64_peak: float, seed: int = 2024) -> dict:
     del master, work
     return {"workload": f"{count} matrices, n log-uniform in [8, 256] (n2 16..512), random as config 0, per-matrix seeds",
             "ms": ms, "solves_per_s": count / (ms * 1e-3), "gpu_launches": int(launches),
-            "launch": "one CUDA-graph replay of the persistent kernel (zq_batch_plan)",
+            "launch": "one CUDA-graph replay (zq_batch_plan): the joint solve's steps, then the small matrices' kernel",
             "tuned_shape": shape,
             "fp64_loop_solves_per_s": count / loop_s, "speedup_vs_fp64_loop": loop_s / (ms * 1e-3),
             "fp64_loop_sample": f"{len(sample)} matrices (every 16th), scaled x{count / len(sample):.0f}",

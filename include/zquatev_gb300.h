@@ -156,8 +156,8 @@ int zq_set_tuned_nb(int n2, int precision, int nb);
 
 /* Batch plan: one layout of small matrices (every n2 <= 512; arguments as
  * zquatev_batched_device) solved repeatedly. Tasks are ordered largest first
- * and uploaded once. ctas_per_sm 1..4 fixes the persistent kernel's launch
- * shape; 0 lets the first run choose it by timing each candidate on the
+ * and uploaded once. ctas_per_sm 1..4 fixes the launch shape of the small
+ * matrices' kernel; 0 lets the first run choose it by timing each candidate on the
  * caller's batch (the input is restored between candidates). The launch is
  * captured in a CUDA graph; each run replays it on `stream` without
  * synchronising (recaptured when dD or deig change). zq_batch_plan_info waits
@@ -214,10 +214,9 @@ int zq_release_workspace(void);
  * 80% of the free device memory at creation). An admitted request's matrix is
  * copied to the device at once and stays there until its result is copied
  * back into D and eig. Requests with n2 <= batch_max_n2 (at most 512) are
- * solved together in launches of the persistent batched kernel (every one that
- * is ready when a batch slot frees up, at most max_batch); larger ones run on
- * `lanes` concurrent lanes through the drop-in's default path (refined above
- * n2 = 512, FP64 below; FP64 fallback). D and eig must stay valid until zq_server_wait returns for the
+ * solved together (every one that is ready when a batch slot frees up, at most
+ * max_batch); larger ones run on `lanes` concurrent lanes (refined from n2 = 96,
+ * FP64 below; FP64 fallback). D and eig must stay valid until zq_server_wait returns for the
  * request. No counterpart in the reference. */
 typedef struct zq_server zq_server;
 typedef struct zq_server_stats {

@@ -309,7 +309,7 @@ int apply_q(const ApplyQTask* tasks, const int* task_of, const ApplyQTask& one, 
   if (cols <= 0 || nmax <= 0) return ZQ_OK;
   int rc;
   // rows in registers: the smallest count that holds the largest order. One
-  // warp per column up to 64 rows (no block barrier), four above
+  // warp per column up to 32 rows (no block barrier), four above
   if (nmax <= 16) rc = launch<1, 2>(tasks, task_of, one, first, cols, st);
   else if (nmax <= 32) rc = launch<1, 4>(tasks, task_of, one, first, cols, st);
   else if (nmax <= 64) rc = launch<4, 2>(tasks, task_of, one, first, cols, st);

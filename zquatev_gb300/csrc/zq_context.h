@@ -49,8 +49,8 @@ struct Context {
   RefineBuffers rb;
   BatchBuffers bb;
   BatchForest forest;  // layout and scratch of the last batch's mid-size matrices, rebuilt when the layout changes
-  // solves of this context may use cooperative launches (off for the
-  // server's lanes, whose solves run beside each other)
+  // no other solve runs beside this context's (false for the server's lanes): the
+  // resident reduction takes every SM, else a quarter of them where that is enough
   bool coop = true;
   // device copy of D for the host-memory entry points, kept between calls
   // (a 1 GB cudaMallocAsync + cudaFreeAsync per n2 = 8192 call cost ~44 ms in

@@ -25,7 +25,7 @@
 // GPU, where one CTA pair per tile ran all digit products in turn. Measured
 // before and after: 8192 x 4096 x 4096 complex 28.9 -> 13.0 ms (k_crt_mma 7.5 ms,
 // 1770 TFLOP/s executed; splitting 1.4, joining 1.2), 1500 x 1100 x 3000 1.61 ->
-// 0.79 ms, 300 x 300 x 300 products of a solve 0.26 -> 0.10 ms each.
+// 0.74 ms, 300 x 300 x 300 products of a solve 0.26 -> 0.10 ms each.
 //
 // k_crt_mma is persistent: each pair of CTAs (cta_group::2, 256 x 256 output
 // tiles) takes jobs (modulus and product, tile); the roles of k_oz_umma's pairs

@@ -41,8 +41,11 @@
 // Tiles are dealt in the order of their columns from the last one back, so
 // that the live tiles of every stage are spread evenly.
 //
-// The group is one cooperative launch; every wait is bounded (the abort flag
-// and the caller's error flag are raised, NaN is left in d, and all CTAs return).
+// A group of one CTA per SM is one cooperative launch and meets at a counter; that
+// wait is bounded (when it runs out, the abort flag and the caller's error flag are
+// raised, NaN is left in d, and all CTAs return). A cluster meets at its hardware
+// barrier, which has no limit and needs none: its CTAs are scheduled together and
+// all pass the same barriers.
 #include "zq_common.cuh"
 #include "zq_kernels.h"
 #include "zq_quat.cuh"
@@ -142,7 +145,10 @@ __device__ __forceinline__ double pow2_biased(int be) {
 
 // Sums of the vector phases. FP64 data: doubles. FP32 data: unevaluated pairs of
 // floats (hi + lo, ~48 bits; Dekker/Knuth two-sums and FMA products): the FP64 pipe
-// takes ~75 cycles per dependent instruction here, a pair's sum ~30.
+// takes ~75 cycles per dependent instruction here, a pair's sum ~30. What follows from
+// them is rounded to 24 bits (f, h, c / 2) or describes data that are (e); against sums
+// in double the first correction of the refinement is the same (its maximum, 33 random
+// matrices of n = 60 to 2500: geometric mean of the ratios 1.00).
 struct Pair { float hi, lo; };
 __device__ __forceinline__ Pair sum2(Pair a, Pair b) {
   const float s = a.hi + b.hi, t = s - a.hi;

@@ -43,7 +43,8 @@
 // with pdl_wait), so a kernel's launch overlaps the tail of the previous one.
 // All arithmetic is FP64 (template R = double) for the plain path; the same
 // kernels instantiate with R = float for the mixed-precision path, where norms
-// and reflector scalars are still formed in double.
+// and reflector scalars are formed in double here and in pairs of floats (48
+// bits) in the resident kernel.
 #include "zq_common.cuh"
 #include "zq_kernels.h"
 #include "zq_resident.h"

@@ -4,8 +4,8 @@ Each request is one ts::zquatev call (zquatev.h:54) on host arrays with the
 reference's argument meaning: D is a Fortran-ordered (ld2, n2) complex128 array
 whose left half holds [A; B] and is overwritten with the eigenvectors; eig[:n]
 receives the eigenvalues; wait() returns the solver's info. The server admits
-requests by HBM footprint, batches the small ones into persistent-kernel
-launches and runs the larger ones on concurrent lanes; all of it happens in the
+requests by HBM footprint, solves the small ones together as they
+arrive and runs the larger ones on concurrent lanes; all of it happens in the
 native library, this class only keeps the arrays alive until their request is
 waited for.
 """
